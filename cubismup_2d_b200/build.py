@@ -19,7 +19,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libcup2d.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
-SOURCES = ["context.cu", "fluid.cu", "obstacles.cu", "fish.cu", "poisson.cu", "noalloc.cu", "varrho.cu",
+SOURCES = ["context.cu", "fluid.cu", "obstacles.cu", "fish.cu", "poisson.cu", "poisson32.cu", "noalloc.cu", "varrho.cu",
            "adjoint.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
@@ -27,10 +27,10 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std
 
 
 def flags_for(src):
-    """poisson.cu contracts multiply-adds: its FFTs need not follow the
+    """poisson.cu and poisson32.cu contract multiply-adds: their FFTs need not follow the
     reference's (FFTW's) rounding, and the one value compared exactly, the
     faded RHS, is written with explicit round-to-nearest intrinsics."""
-    if src == "poisson.cu":
+    if src in ("poisson.cu", "poisson32.cu"):
         return [f if f != "-fmad=false" else "-fmad=true" for f in FLAGS]
     return FLAGS
 

@@ -424,8 +424,8 @@ k_adj_geo_dot(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* 
 
 // ---- the boundary-strip fade F (cub2rhs) ----------------------------------
 __device__ __forceinline__ double fade_w2(const GridDesc& g, int gx, int gy) {
-  const double fadeLenX = g.fadeLenX, invFadeX = 1 / fmax(fadeLenX, EPSd);
-  const double fadeLenY = g.fadeLenY, invFadeY = 1 / fmax(fadeLenY, EPSd);
+  const double fadeLenX = g.fadeLenX, invFadeX = g.invFadeX;
+  const double fadeLenY = g.fadeLenY, invFadeY = g.invFadeY;
   const double px = cell_x(g, gx >> 5, gx & 31), py = cell_y(g, gy >> 5, gy & 31);
   const double yt = invFadeY * fmax(0.0, fadeLenY - g.ext[1] + py);
   const double yb = invFadeY * fmax(0.0, fadeLenY - py);

@@ -465,6 +465,8 @@ int cup2d_create(const cup2d_config* cfg, cup2d_ctx** out) {
   g.nu = cfg->nu; g.CFL = cfg->CFL; g.dlm = cfg->dlm;
   g.fadeLenX = cfg->fadeLen * cfg->extent;                     // Simulation.cpp:97-98
   g.fadeLenY = cfg->fadeLen * cfg->extent;
+  g.invFadeX = 1 / std::max(g.fadeLenX, EPSd);                 // PoissonSolver.cpp:62-65
+  g.invFadeY = 1 / std::max(g.fadeLenY, EPSd);
   g.implicitPenal = cfg->implicit_penalization ? 1 : 0;
   const size_t n = c.ncells();
   int rc = CUP2D_OK;
@@ -1840,6 +1842,7 @@ void trace_bind_fluid(unsigned long long*);
 void trace_bind_obstacles(unsigned long long*);
 void trace_bind_fish(unsigned long long*);
 void trace_bind_poisson(unsigned long long*);
+void trace_bind_poisson32(unsigned long long*);
 }
 extern "C" int cup2d_trace(cup2d_ctx* ctx, unsigned long long* out, int reset) {
   using namespace cup2d;
@@ -1849,6 +1852,7 @@ extern "C" int cup2d_trace(cup2d_ctx* ctx, unsigned long long* out, int reset) {
   if (!buf) {
     if (cudaMalloc(&buf, sizeof(unsigned long long) * (2 * TR_N + 8 * TRACE_ITEMS)) != cudaSuccess) return CUP2D_ENOMEM;
     trace_bind_fluid(buf); trace_bind_obstacles(buf); trace_bind_fish(buf); trace_bind_poisson(buf);
+    trace_bind_poisson32(buf);
     reset = 1;
   }
   cudaDeviceSynchronize();

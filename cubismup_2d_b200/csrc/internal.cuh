@@ -35,6 +35,7 @@ struct GridDesc {
   double ext[2];                  // SimulationData::extents (SimulationData.cpp:34-35)
   double nu, CFL, dlm;
   double fadeLenX, fadeLenY;
+  double invFadeX, invFadeY;      // 1 / max(fadeLen, eps): formed once, not per cell
   int implicitPenal;              // cup2d_config.implicit_penalization
 };
 
@@ -464,8 +465,8 @@ __device__ __forceinline__ bool fade_touch(const GridDesc& g, int bx, int by) {
 // adds cell (ix, iy) of block (bx, by), of RHS b, to s (PoissonSolver.cpp:86-95)
 __device__ __forceinline__ void fade_accumulate(const GridDesc& g, int bx, int by, int ix, int iy,
                                                 double b, double (&s)[3]) {
-  const double fadeLenX = g.fadeLenX, invFadeX = 1 / fmax(fadeLenX, EPSd);
-  const double fadeLenY = g.fadeLenY, invFadeY = 1 / fmax(fadeLenY, EPSd);
+  const double fadeLenX = g.fadeLenX, invFadeX = g.invFadeX;
+  const double fadeLenY = g.fadeLenY, invFadeY = g.invFadeY;
   const double px = cell_x(g, bx, ix), py = cell_y(g, by, iy);
   const double yt = invFadeY * fmax(0.0, fadeLenY - g.ext[1] + py);
   const double yb = invFadeY * fmax(0.0, fadeLenY - py);

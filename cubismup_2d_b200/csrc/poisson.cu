@@ -16,10 +16,11 @@
 //    power-of-two lengths keep every FFT in shared memory.
 //  - periodic (Poisson/FFTW_periodic.h:77-166): the same passes without
 //    padding and with the spectral multiplier -1/|k|^2.
-// FFTs are compile-time-length Stockham radix-4 (one radix-2 stage when
-// log2 L is odd) in shared memory padded by one element per 16 against bank
-// conflicts, twiddles from one host-computed table; one CTA transforms a few
-// rows (or columns) with L/4 threads each.
+// FFTs are compile-time-length Stockham transforms in shared memory, padded
+// by one element per 16 against bank conflicts: radix-16 (or radix-8) passes
+// with 16 (8) values per thread in registers and one pass of the remaining
+// factor, twiddles from host-computed tables; one CTA transforms a few rows
+// (or columns).
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -27,7 +28,7 @@
 #include <mutex>
 #include <tuple>
 #include <vector>
-#include "context.hpp"
+#include "poisson.cuh"
 
 namespace cup2d {
 
@@ -39,292 +40,178 @@ struct Poisson {
   int Lrow = 0;          // complex FFT length of the row passes (M/2)
   int Lcol = 0;          // complex FFT length of the column pass
   int nkx = 0;           // spectrum columns (Lrow + 1)
-  double2* spec = nullptr;   // [Lcol rows][nkx] row-major spectrum
-  double* ghat = nullptr;    // [Lcol/2 + 1][nkx] free-space kernel
+  double2* spec = nullptr;   // the half spectrum: FP64 in column pairs (spec_at), FP32 [Lcol rows][nkx]
+  // FP64: the column pass's multiplier [nkx][Lcol/2 + 1], the free-space
+  // kernel or the periodic -1/|k|^2, halved (r2c_split writes twice the
+  // spectrum); a column's values are consecutive
+  double* ghat = nullptr;
   double2* tw = nullptr;     // exp(-2 pi i k / twLen)
   int twLen = 0;
+  double2* tRow[2] = {nullptr, nullptr};   // pass tables of the row transforms, 8 and 16 values per thread
+  double2* tCol = nullptr;                 // and of the column transforms
   bool fp32 = false;         // CUP2D_PREC_FP32: float2 spectrum in spec, FP32 passes
   float2* tw32 = nullptr;    // tw rounded to FP32
-  float* ghat32 = nullptr;   // ghat rounded to FP32
+  float* ghat32 = nullptr;   // the free-space kernel rounded to FP32, [Lcol/2 + 1][nkx]
   int rb = 1, cb = 1;        // rows / columns per CTA
   int MX = 0, MY = 0;        // free space: the padded grid (powers of two >= 2Nx, 2Ny)
   // elements per thread of the forward and inverse row passes (FP64 free
   // space and periodic), and the times the autotuner measured (us; r2c with
   // 8 and 16, c2r with 8 and 16; zero when not tuned)
-  int eR2C = 8, eC2R = 16;
+  int eR2C = 16, eC2R = 16;
   bool tuned = false;
   double tuneUs[4] = {0, 0, 0, 0};
 };
 
 namespace {
 
-// The transforms are written once for a complex type C: double2 (the FP64
-// solve) or float2 (the FP32 solve of CUP2D_PREC_FP32).
-template <class C> struct CT;
-template <> struct CT<double2> { using R = double; };
-template <> struct CT<float2> { using R = float; };
-template <class C> __device__ __forceinline__ C mk(typename CT<C>::R a, typename CT<C>::R b);
-template <> __device__ __forceinline__ double2 mk<double2>(double a, double b) { return make_double2(a, b); }
-template <> __device__ __forceinline__ float2 mk<float2>(float a, float b) { return make_float2(a, b); }
-template <class C> __device__ __forceinline__ C cmul(C a, C b) {
-  return mk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-template <class C> __device__ __forceinline__ C cadd(C a, C b) { return mk<C>(a.x + b.x, a.y + b.y); }
-template <class C> __device__ __forceinline__ C csub(C a, C b) { return mk<C>(a.x - b.x, a.y - b.y); }
-template <class C> __device__ __forceinline__ C conjg(C a) { return mk<C>(a.x, -a.y); }
-
-__device__ __forceinline__ int pad(int i) { return i + (i >> 4); }
-
 // Per transform length L: padded stride SL of one sequence (one spare
 // element per 16, plus 4 so that consecutive sequences start in different
 // halves of the shared-memory banks), the staged quarter twiddle table
 // (w^j, j < L/4), the sequences per CTA B and the threads per CTA NT
 // (L/E per sequence: every thread owns E = 16 or 8 elements of a pass).
-// ---- per-pass twiddle tables ---------------------------------------------
-// The passes of fft_inplace<L, ..., E> (fft_passes): sub-transform sizes
-// NS = 1, E, E^2, ... with radix E while NS E <= L, then one pass of radix
-// L/NS.  The pass over sub-transforms of size NS scales input m of the
-// butterfly with k = j mod NS by W^(m k), W = exp(-2 pi i/(R NS)).  For each
-// pass with NS > 1 the tables hold W^(p k), k < NS, for the powers p = 1, 2,
-// 4, 8 below R (one table of NS entries each): the butterflies of a warp
-// read consecutive entries (no shared-memory bank conflicts, where indexing
-// one table by m k made every lane of a warp hit the same banks), and the
-// other powers are products of at most three table values.
-constexpr int tw_npow(int R) { return R >= 16 ? 4 : (R >= 8 ? 3 : (R >= 4 ? 2 : (R >= 2 ? 1 : 0))); }
-// offset of the tables of the pass over sub-transforms of size NS
-template <int L, int E> constexpr int tw_off(int NS) {
-  int off = 0, ns = 1;
-  while (ns < L && ns < NS) {
-    const int r = ns * E <= L ? E : L / ns;
-    if (ns > 1) off += tw_npow(r) * ns;
-    ns *= r;
-  }
-  return off;
-}
-template <int L, int E> constexpr int tw_size() { return tw_off<L, E>(L); }
-// entries staged per CTA: enough for the element counts E = 8 and 16
-template <int L> constexpr int tw_max() {
-  const int a = tw_size<L, 8>(), b = tw_size<L, 16>();
-  return a > b ? (a > 0 ? a : 1) : (b > 0 ? b : 1);
-}
-
 template <int L, int E = 16> struct Len {
   static constexpr int SL = L + L / 16 + 4;
-  static constexpr int TW = tw_max<L>();
   static constexpr int B = 2048 / L < 1 ? 1 : (2048 / L > 8 ? 8 : 2048 / L);
   static constexpr int NT0 = B * L / E;
   static constexpr int NT = NT0 < 64 ? 64 : (NT0 > 512 ? 512 : NT0);
   static constexpr int REGS = E == 16 ? 128 : 64;   // register budget per thread
   static constexpr int MINB = 65536 / (NT * REGS) < 1 ? 1 : 65536 / (NT * REGS);
 };
-// elements per thread: the row passes have two instantiations each (8 and
-// 16: a forward row of 4096 points runs faster with 16, shorter rows with
-// 8, measured on B200), chosen per grid at set-up (table below, or timed
-// by poisson_autotune); the column pass uses 16 (faster at every length
-// measured)
-constexpr int E_ROWS = 8;
-constexpr int E_C2R = 16;
-constexpr int E_COLS = 16;
-// the same for the FP32 transforms (half the registers per value)
-constexpr int E_ROWS32 = 8;
-constexpr int E_C2R32 = 8;
-constexpr int E_COLS32 = 16;
+// ---- FP64: twiddles and DFT in one, on fused multiply-adds -----------------
+// A pass of radix R over sub-transforms of size NS, y_q = sum_m x_m W^(m k)
+// W_R^(m q) with W = exp(-2 pi i / (R NS)), as log2 R levels of two-point
+// butterflies a +- w b whose twiddles include W^(m k): the level that joins
+// transforms of h values into 2h uses w_q = exp(-2 pi i (k + q NS)/(2 h NS)),
+// q < h, and w_q for q >= h/2 is a quarter turn of w_(q - h/2).  With the
+// table holding (c, t) = (cos, tan) of an angle, w b = c (b.x - t b.y, b.y +
+// t b.x) and a butterfly is six multiply-adds (the "ratio" butterfly of
+// Linzer and Feig, 1993); c t is the sine to rounding at every angle, so no
+// branch on it is needed (c is never zero: cos(pi/2) rounds to 6e-17).  A
+// radix-16 pass takes 192 FP64 instructions a thread instead of about 280
+// (15 scalings, 11 products for the powers of W that the table did not hold,
+// 9 internal twiddles and 144 additions).
+// Table of a pass: level h's entries j = k + q NS < NS max(1, h/2), level
+// after level, R NS / 2 in all.
+template <int L, int E> constexpr int pass_radix(int ns) { return ns * E <= L ? E : L / ns; }
+template <int L, int E> constexpr int tab_off(int NS) {
+  int off = 0;
+  for (int ns = 1; ns < L && ns < NS; ns *= pass_radix<L, E>(ns))
+    if (ns > 1) off += pass_radix<L, E>(ns) * ns / 2;
+  return off;
+}
+template <int L, int E> constexpr int tab_size() { return tab_off<L, E>(L); }
+// A pass's table is staged in shared memory if it has at most this many
+// entries (16 KB); the last pass of 4096 points (2048 entries, each read once
+// a transform) reads it through the L1 instead, which leaves room for two
+// CTAs an SM.
+constexpr int TAB_STAGED = 1024;
+template <int L, int E> constexpr int tab_staged() {
+  int n = 0;
+  for (int ns = 1; ns < L; ns *= pass_radix<L, E>(ns))
+    if (ns > 1 && pass_radix<L, E>(ns) * ns / 2 <= TAB_STAGED) n += pass_radix<L, E>(ns) * ns / 2;
+  return n;
+}
+struct Tab { const double2 *s, *g; };            // the staged part, the whole table in global memory
 
-constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
-
-// Stages the per-pass tables of fft_inplace<L, ..., E> from the global
-// table tw[j] = exp(-2 pi i j / twLen) (twLen a power of two, a multiple of
-// 4 L): the tables of the pass over sub-transforms of size NS and of every
-// later pass.  Entry t = p NS + k of a pass of radix R holds
-// W^(k 2^p) = tw[(k 2^p) twLen / (R NS)]; the passes' sizes are
-// compile-time powers of two, so every index is a shift.
-template <int L, int E, int NS, class C>
-__device__ __forceinline__ void load_twiddles_from(C* tws, const C* __restrict__ tw, int twShift) {
-  if constexpr (NS < L) {
-    constexpr int R = NS * E <= L ? E : L / NS;
-    if constexpr (NS > 1) {
-      constexpr int n = tw_npow(R) * NS, off = tw_off<L, E>(NS), sh = ilog2(R * NS);
-      for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int p = t / NS, k = t - p * NS;
-        tws[off + t] = tw[(size_t)(k << p) << (twShift - sh)];
-      }
-    }
-    load_twiddles_from<L, E, NS * R>(tws, tw, twShift);
-  }
-}
-template <int L, int E, class C>
-__device__ __forceinline__ void load_twiddles(C* tws, const C* __restrict__ tw, int twLen) {
-  load_twiddles_from<L, E, 1>(tws, tw, __ffs(twLen) - 1);
-}
-
-// Scales xb[m], 0 < m < R, of the butterfly k of the pass over
-// sub-transforms of size NS by W^(m k) (conjugated for the inverse).
-template <int L, int E, int R, int NS, bool INV, class C>
-__device__ __forceinline__ void apply_twiddles(C* xb, const C* tws, int k) {
-  const C* t = tws + tw_off<L, E>(NS) + k;
-  auto ld = [&](int pi) { C w = t[pi * NS]; if (INV) w.y = -w.y; return w; };
-  const C w1 = ld(0);
-  xb[1] = cmul(xb[1], w1);
-  if constexpr (R > 2) {
-    const C w2 = ld(1), w3 = cmul(w1, w2);
-    xb[2] = cmul(xb[2], w2);
-    xb[3] = cmul(xb[3], w3);
-    if constexpr (R > 4) {
-      const C w4 = ld(2);
-      xb[4] = cmul(xb[4], w4);
-      xb[5] = cmul(xb[5], cmul(w1, w4));
-      xb[6] = cmul(xb[6], cmul(w2, w4));
-      xb[7] = cmul(xb[7], cmul(w3, w4));
-      if constexpr (R > 8) {
-        const C w8 = ld(3), w12 = cmul(w4, w8);
-        xb[8] = cmul(xb[8], w8);
-        xb[9] = cmul(xb[9], cmul(w1, w8));
-        xb[10] = cmul(xb[10], cmul(w2, w8));
-        xb[11] = cmul(xb[11], cmul(w3, w8));
-        xb[12] = cmul(xb[12], w12);
-        xb[13] = cmul(xb[13], cmul(w1, w12));
-        xb[14] = cmul(xb[14], cmul(w2, w12));
-        xb[15] = cmul(xb[15], cmul(w3, w12));
-      }
-    }
-  }
-}
-
-// asynchronous global -> shared copies (sm_80+ cp.async), so that every
-// load of a CTA's rows or columns is in flight at once
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n"
-               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n"
-               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n"
-               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" :: "n"(N) : "memory");
-}
-
-// ---- small DFTs in registers (forward exp(-2 pi i mq/R), inverse exp(+)) --
-// multiply by -i (forward) or +i (inverse)
-template <bool INV, class C> __device__ __forceinline__ C mul_mi(C a) {
-  return INV ? mk<C>(-a.y, a.x) : mk<C>(a.y, -a.x);
-}
-template <bool INV, class C>
-__device__ __forceinline__ void dft4(C& x0, C& x1, C& x2, C& x3) {
-  const C t0 = cadd(x0, x2), t1 = csub(x0, x2), t2 = cadd(x1, x3), t3 = mul_mi<INV>(csub(x1, x3));
-  x0 = cadd(t0, t2); x2 = csub(t0, t2);
-  x1 = cadd(t1, t3); x3 = csub(t1, t3);
-}
-constexpr double C8 = 0.92387953251128675613;   // cos(pi/8)
-constexpr double S8 = 0.38268343236508977173;   // sin(pi/8)
-constexpr double R2 = 0.70710678118654752440;   // sqrt(2)/2
-// W16^e for e in [0, 16): the first quadrant from (1, C8, R2, S8), the rest
-// by exact quarter turns
-template <bool INV, class C>
-__device__ __forceinline__ C w16(int e) {
-  using R = typename CT<C>::R;
-  const int q = e >> 2, r = e & 3;
-  const R cr = (R)(r == 0 ? 1.0 : (r == 1 ? C8 : (r == 2 ? R2 : S8)));
-  const R sr = (R)(r == 0 ? 0.0 : (r == 1 ? S8 : (r == 2 ? R2 : C8)));
-  C v = mk<C>(cr, -sr);
-  for (int k = 0; k < q; k++) v = mk<C>(v.y, -v.x);
-  if (INV) v.y = -v.y;
-  return v;
-}
-// DFT of R values in x[0..R); the result for output q is in x[out_reg<R>(q)]
+// register of output q of a butterfly of radix R
 template <int R> __device__ __forceinline__ constexpr int out_reg(int q) {
-  return R == 16 ? 4 * (q & 3) + (q >> 2) : q;
+  int p = 0;
+  for (int b = 0; (1 << b) < R; b++) p |= ((q >> b) & 1) * (R >> (b + 1));
+  return p;
 }
-template <bool INV, class C> __device__ __forceinline__ void dft8(C* x) {
-  // m = m1 + 2 m2: DFT4 over m2, twiddle W8^(m1 q2), DFT2 over m1
-  dft4<INV>(x[0], x[2], x[4], x[6]);
-  dft4<INV>(x[1], x[3], x[5], x[7]);
-  C y[8];
+
+// a +- w b, w = c (1 + i t) (conjugated for the inverse), or w a quarter
+// turn further on (TURN: times -i, for the inverse +i)
+template <bool INV, bool TURN>
+__device__ __forceinline__ void ratio_butterfly(double2& a, double2& b, double c, double t) {
+  const double ti = INV ? -t : t;
+  const double p = fma(-ti, b.y, b.x), q = fma(ti, b.x, b.y);
+  const double re = TURN ? (INV ? -q : q) : p, im = TURN ? (INV ? p : -p) : q;
+  b = make_double2(fma(-c, re, a.x), fma(-c, im, a.y));
+  a = make_double2(fma(c, re, a.x), fma(c, im, a.y));
+}
+// the same for w = 1 or a quarter turn
+template <bool INV, bool TURN>
+__device__ __forceinline__ void unit_butterfly(double2& a, double2& b) {
+  const double2 d = TURN ? mul_mi<INV>(b) : b, s = a;
+  a = cadd(s, d);
+  b = csub(s, d);
+}
+// level h of a radix-R butterfly in x (in place: output q of the group at r
+// sits where its bits, lowest first, select R/2, R/4, ...)
+template <int R, int H, int NS, bool INV, bool ZIN>
+__device__ __forceinline__ void radix_level(double2* x, const double2* tb, int k) {
+  constexpr int S = R / (2 * H), HT = H / 2 > 0 ? H / 2 : 1;
+  constexpr int TOFF = H == 1 ? 0 : NS * H / 2;
+  constexpr double CC[4] = {1.0, 0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173};
+  constexpr double TT[4] = {0.0, -0.41421356237309504880, -1.0, -2.41421356237309504880};
 #pragma unroll
-  for (int q2 = 0; q2 < 4; q2++) {
-    const C z0 = x[2 * q2], z1 = cmul(x[2 * q2 + 1], w16<INV, C>(2 * q2));
-    y[q2] = cadd(z0, z1); y[q2 + 4] = csub(z0, z1);
+  for (int q = 0; q < HT; q++) {
+    double2 w = make_double2(0, 0);
+    if (NS > 1) w = NS * R / 2 > TAB_STAGED ? __ldg(tb + TOFF + q * NS + k) : tb[TOFF + q * NS + k];
+#pragma unroll
+    for (int turn = 0; turn < (H > 1 ? 2 : 1); turn++) {
+      const int p = out_reg<R>(q + turn * HT);
+#pragma unroll
+      for (int r = 0; r < S; r++) {
+        double2 &a = x[r + p], &b = x[r + S + p];
+        if (ZIN && H == 1) b = a;                 // the upper inputs are zero
+        else if (NS == 1 && q == 0) { if (turn) unit_butterfly<INV, true>(a, b); else unit_butterfly<INV, false>(a, b); }
+        else {
+          const double c = NS > 1 ? w.x : CC[q * (8 / H) & 3], t = NS > 1 ? w.y : TT[q * (8 / H) & 3];
+          if (turn) ratio_butterfly<INV, true>(a, b, c, t); else ratio_butterfly<INV, false>(a, b, c, t);
+        }
+      }
+    }
   }
-#pragma unroll
-  for (int q = 0; q < 8; q++) x[q] = y[q];
 }
-template <bool INV, class C> __device__ __forceinline__ void dft16(C* x) {
-  // m = m1 + 4 m2: DFT4 over m2 (result z[m1][q2] in x[m1 + 4 q2]),
-  // twiddle W16^(m1 q2), DFT4 over m1 (output q2 + 4 q1 in x[4 q2 + q1])
-#pragma unroll
-  for (int m1 = 0; m1 < 4; m1++) dft4<INV>(x[m1], x[m1 + 4], x[m1 + 8], x[m1 + 12]);
-#pragma unroll
-  for (int m1 = 1; m1 < 4; m1++)
-#pragma unroll
-    for (int q2 = 1; q2 < 4; q2++) x[m1 + 4 * q2] = cmul(x[m1 + 4 * q2], w16<INV, C>(m1 * q2));
-#pragma unroll
-  for (int q2 = 0; q2 < 4; q2++) dft4<INV>(x[4 * q2], x[4 * q2 + 1], x[4 * q2 + 2], x[4 * q2 + 3]);
+// butterfly k of the pass over sub-transforms of size NS
+template <int L, int E, int R, int NS, bool INV, bool ZIN>
+__device__ __forceinline__ void radix_step(double2* x, Tab tab, int k) {
+  const double2* tb = (NS * R / 2 > TAB_STAGED ? tab.g : tab.s) + tab_off<L, E>(NS);
+  radix_level<R, 1, NS, INV, ZIN>(x, tb, k);
+  if constexpr (R > 2) radix_level<R, 2, NS, INV, ZIN>(x, tb, k);
+  if constexpr (R > 4) radix_level<R, 4, NS, INV, ZIN>(x, tb, k);
+  if constexpr (R > 8) radix_level<R, 8, NS, INV, ZIN>(x, tb, k);
 }
-template <int R, bool INV, class C> __device__ __forceinline__ void dft(C* x) {
-  if constexpr (R == 2) { const C t = x[0]; x[0] = cadd(t, x[1]); x[1] = csub(t, x[1]); }
-  else if constexpr (R == 4) dft4<INV>(x[0], x[1], x[2], x[3]);
-  else if constexpr (R == 8) dft8<INV>(x);
-  else dft16<INV>(x);
+// the staged tables of a transform, n threads from thread `first`
+template <int L, int E>
+__device__ __forceinline__ Tab stage_tables(double2* s, const double2* __restrict__ g) {
+  for (int t = threadIdx.x; t < tab_staged<L, E>(); t += blockDim.x) cp_async16(s + t, g + t);
+  return {s, g};
 }
 
-// pad(j + u T + m Q) given pj = pad(j): a multiple C of 16 added to an index
-// adds C + C/16 to its padded position, an immediate offset
-template <int T, int Q>
-__device__ __forceinline__ int pad_at(int pj, int j, int u, int m) {
-  if constexpr (T % 16 == 0 && Q % 16 == 0) return pj + u * (T + T / 16) + m * (Q + Q / 16);
-  else return pad(j + u * T + m * Q);
-}
-// pad(o + q NS) given po = pad(o), for an output o of a pass over sub-transforms
-// of size NS: with NS = 1, o is a multiple of R (a divisor of 16) and q < R
-// stays inside o's group of 16
-template <int NS>
-__device__ __forceinline__ int pad_out(int po, int o, int q) {
-  if constexpr (NS % 16 == 0) return po + q * (NS + NS / 16);
-  else if constexpr (NS == 1) return po + q;
-  else return pad(o + q * NS);
-}
-
-// One in-place Stockham pass of radix R over sub-transforms of size NS on
-// nseq sequences A + q*SL: butterfly j (k = j mod NS) reads x_m =
-// a[j + m L/R], scales by w^(m k L/(R NS)), takes the DFT_R and writes
-// output q at (j - k) R + k + q NS.  Thread t of a sequence owns the 16/R
-// butterflies t + u L/16.  Loads go to registers before the barrier,
-// stores after it, so one buffer suffices.
-template <int L, int R, int NS, bool INV, bool HIN, bool HOUT, int E, class C>
-__device__ __forceinline__ void fft_pass(C* A, int nseq, const C* tws)
+// One in-place Stockham pass of radix R over sub-transforms of size NS of the
+// sequence a (padded indexing), by L/E threads, this one thread j of them
+// (if act): butterfly jb (k = jb mod NS) reads x_m = a[jb + m L/R], scales
+// by W^(m k), takes the DFT_R and writes output q at (jb - k) R + k + q NS.
+// Thread j owns the E/R butterflies j + u L/E.  Loads go to registers before
+// the barrier, stores after it, so one buffer suffices.
+template <int L, int R, int NS, bool INV, bool HIN, bool HOUT, int E>
+__device__ __forceinline__ void fft_pass(double2* a, bool act, int j, Tab tab)
 {
-  constexpr int SL = Len<L>::SL, T = L / E, NB = E / R, Q = L / R;
+  constexpr int T = L / E, NB = E / R, Q = L / R;
   // first pass of an input whose upper half is zero: inputs m >= R/2 sit at
   // indices >= L/2 (then NB == 1); last pass of which only the lower half of
   // the output is kept: outputs q >= R/2 land at indices >= L/2
   constexpr bool ZIN = HIN && NS == 1, HALFO = HOUT && NS * R == L;
-  const int tid = threadIdx.x;
-  const bool act = tid < nseq * T;
-  const int sq = act ? tid / T : 0, j = tid - sq * T;
-  C* a = A + sq * SL;
-  C x[E];
+  double2 x[E];
   if (act) {
     const int pj = pad(j);
 #pragma unroll
     for (int u = 0; u < NB; u++)
 #pragma unroll
       for (int m = 0; m < R; m++)
-        x[u * R + m] = (ZIN && m >= R / 2) ? mk<C>(0, 0)
+        x[u * R + m] = (ZIN && m >= R / 2) ? make_double2(0, 0)
                                            : a[pad_at<T, Q>(pj, j, u, m)];
   }
   __syncthreads();
   if (act) {
 #pragma unroll
     for (int u = 0; u < NB; u++) {
-      C* xb = x + u * R;
+      double2* xb = x + u * R;
       const int jb = j + u * T, k = jb & (NS - 1);
-      if (NS > 1 && k) apply_twiddles<L, E, R, NS, INV>(xb, tws, k);
-      dft<R, INV>(xb);
+      radix_step<L, E, R, NS, INV, ZIN>(xb, tab, k);
       const int o = (jb - k) * R + k, po = pad(o);
 #pragma unroll
       for (int q = 0; q < (HALFO ? R / 2 : R); q++) a[pad_out<NS>(po, o, q)] = xb[out_reg<R>(q)];
@@ -333,26 +220,24 @@ __device__ __forceinline__ void fft_pass(C* A, int nseq, const C* tws)
   __syncthreads();
 }
 
-template <int L, int NS, bool INV, bool HIN, bool HOUT, int E, class C>
-__device__ __forceinline__ void fft_passes(C* A, int nseq, const C* tws) {
-  if constexpr (NS * E <= L) {
-    fft_pass<L, E, NS, INV, HIN, HOUT, E>(A, nseq, tws);
-    fft_passes<L, NS * E, INV, HIN, HOUT, E>(A, nseq, tws);
-  } else if constexpr (NS < L) {
-    fft_pass<L, L / NS, NS, INV, HIN, HOUT, E>(A, nseq, tws);
+template <int L, int NS, bool INV, bool HIN, bool HOUT, int E>
+__device__ __forceinline__ void fft_passes(double2* a, bool act, int j, Tab tab) {
+  if constexpr (NS < L) {
+    constexpr int R = pass_radix<L, E>(NS);
+    fft_pass<L, R, NS, INV, HIN, HOUT, E>(a, act, j, tab);
+    fft_passes<L, NS * R, INV, HIN, HOUT, E>(a, act, j, tab);
   }
 }
 
-// In-place Stockham autosort FFT of nseq sequences of length L (A + q*SL,
-// padded indexing; a power of two >= 16): radix-16 passes and one radix
-// 2/4/8 pass for the remaining factor.  Forward exp(-2 pi i jk/L), inverse
-// exp(+...), unnormalised.  Needs blockDim.x >= nseq * L/E.  HIN: the
-// upper half of the input is zero and never read; HOUT: only the lower half
-// of the output is written.
-template <int L, bool INV, bool HIN = false, bool HOUT = false, int E = 16, class C>
-__device__ void fft_inplace(C* A, int nseq, const C* tws)
+// In-place Stockham autosort FFT of length L (a power of two >= 16; padded
+// indexing): radix-E passes and one of the remaining factor.  Forward
+// exp(-2 pi i jk/L), inverse exp(+...), unnormalised.  HIN: the upper half
+// of the input is zero and never read; HOUT: only the lower half of the
+// output is written.
+template <int L, bool INV, bool HIN = false, bool HOUT = false, int E = 16>
+__device__ void fft_inplace(double2* a, bool act, int j, Tab tab)
 {
-  fft_passes<L, 1, INV, HIN, HOUT, E>(A, nseq, tws);
+  fft_passes<L, 1, INV, HIN, HOUT, E>(a, act, j, tab);
 }
 
 // sub-transform size NS of the last pass of fft_inplace<L, ..., E>
@@ -362,43 +247,25 @@ template <int L, int E> constexpr int last_ns() {
   return ns == L ? ns / E : ns;
 }
 // the passes of fft_passes<L, NS, ...> whose sub-transform size is below NSEND
-template <int L, int NS, int NSEND, bool INV, bool HIN, int E, class C>
-__device__ __forceinline__ void fft_passes_below(C* A, int nseq, const C* tws) {
+template <int L, int NS, int NSEND, bool INV, bool HIN, int E>
+__device__ __forceinline__ void fft_passes_below(double2* a, bool act, int j, Tab tab) {
   if constexpr (NS < NSEND) {
-    constexpr int R = NS * E <= L ? E : L / NS;
-    fft_pass<L, R, NS, INV, HIN, false, E>(A, nseq, tws);
-    fft_passes_below<L, NS * R, NSEND, INV, HIN, E>(A, nseq, tws);
+    constexpr int R = pass_radix<L, E>(NS);
+    fft_pass<L, R, NS, INV, HIN, false, E>(a, act, j, tab);
+    fft_passes_below<L, NS * R, NSEND, INV, HIN, E>(a, act, j, tab);
   }
 }
 
-// Spectral convolution of nseq sequences in place: fft_inplace<L, false,
-// HIN>, X[r] = mul(sequence, r, X[r]), fft_inplace<L, true, false, HOUT>.  The
-// last forward pass, the multiplier and the first inverse pass run in
-// registers: butterfly jb = j + u L/E of the last forward pass (radix R,
-// NS = L/R, no stride: k = jb) produces X[jb + q NS] = X[j + (u + (E/R) q)
-// L/E], which is input m = u + (E/R) q of thread j's radix-E first inverse
-// butterfly (NS = 1).  With L <= E (one pass each way) the three steps run
-// one after the other.
-template <int L, bool HIN, bool HOUT, int E, class C, class Mul>
-__device__ __forceinline__ void fft_convolve(C* A, int nseq, const C* tws, Mul mul)
+// Middle of a spectral convolution in place: the last forward pass, X[r] =
+// mul(r, X[r]) and the first inverse pass in registers: butterfly jb = j +
+// u L/E of the last forward pass (radix R, NS = L/R, no stride: k = jb)
+// produces X[jb + q NS] = X[j + (u + (E/R) q) L/E], which is input m = u +
+// (E/R) q of thread j's radix-E first inverse butterfly (NS = 1).
+template <int L, int E, class Mul>
+__device__ __forceinline__ void fft_turn(double2* a, bool act, int j, Tab tab, Mul mul)
 {
-  constexpr int SL = Len<L>::SL, T = L / E, NS = last_ns<L, E>(), R = L / NS, NB = E / R;
-  if constexpr (L <= E) {
-    fft_inplace<L, false, HIN, false, E>(A, nseq, tws);
-    for (int idx = threadIdx.x; idx < nseq * L; idx += blockDim.x) {
-      const int sq = idx / L, r = idx - sq * L;
-      A[sq * SL + pad(r)] = mul(sq, r, A[sq * SL + pad(r)]);
-    }
-    __syncthreads();
-    fft_inplace<L, true, false, HOUT, E>(A, nseq, tws);
-    return;
-  }
-  fft_passes_below<L, 1, NS, false, HIN, E>(A, nseq, tws);
-  const int tid = threadIdx.x;
-  const bool act = tid < nseq * T;
-  const int sq = act ? tid / T : 0, j = tid - sq * T;
-  C* a = A + sq * SL;
-  C x[E];
+  constexpr int T = L / E, NS = last_ns<L, E>(), R = L / NS, NB = E / R;
+  double2 x[E];
   if (act) {
     const int pj = pad(j);
 #pragma unroll
@@ -408,66 +275,75 @@ __device__ __forceinline__ void fft_convolve(C* A, int nseq, const C* tws, Mul m
   }
   __syncthreads();
   if (act) {
-    C y[E];
+    double2 y[E];
 #pragma unroll
     for (int u = 0; u < NB; u++) {
-      C* xb = x + u * R;
+      double2* xb = x + u * R;
       const int jb = j + u * T;
-      if (jb) apply_twiddles<L, E, R, NS, false>(xb, tws, jb);
-      dft<R, false>(xb);
+      radix_step<L, E, R, NS, false, false>(xb, tab, jb);
 #pragma unroll
-      for (int q = 0; q < R; q++) y[u + NB * q] = mul(sq, jb + q * NS, xb[out_reg<R>(q)]);
+      for (int q = 0; q < R; q++) y[u + NB * q] = mul(jb + q * NS, xb[out_reg<R>(q)]);
     }
-    dft<E, true>(y);
+    radix_step<L, E, E, 1, true, false>(y, tab, 0);
 #pragma unroll
     for (int q = 0; q < E; q++) a[pad_out<1>(pad(j * E), j * E, q)] = y[out_reg<E>(q)];
   }
   __syncthreads();
-  fft_passes<L, E, true, false, HOUT, E>(A, nseq, tws);
 }
 
-// The first pass of a forward FFT (NS = 1, radix R) with its inputs read
-// straight from global memory (ld(sequence, index)) into registers: the
-// sequence is never staged in shared memory before the pass.  With ZIN the
-// upper half of the input is zero and not read.  The outputs go to
-// shared memory; the caller's barrier makes them visible.
-template <int L, int R, bool ZIN, int E, class C, class Ld>
-__device__ __forceinline__ void fft_first_pass_global(C* A, int nseq, Ld ld)
+// Spectral convolution in place: fft_inplace<L, false, HIN>, X[r] = mul(r,
+// X[r]), fft_inplace<L, true, false, HOUT>, with the turn in registers.  With
+// L <= E (one pass each way) the three steps run one after the other.
+template <int L, bool HIN, bool HOUT, int E, class Mul>
+__device__ __forceinline__ void fft_convolve(double2* a, bool act, int j, Tab tab, Mul mul)
 {
-  constexpr int SL = Len<L>::SL, T = L / E, NB = E / R, Q = L / R;
-  const int tid = threadIdx.x;
-  if (tid >= nseq * T) return;
-  const int sq = tid / T, j = tid - sq * T;
-  C* a = A + sq * SL;
-  C x[E];
-#pragma unroll
-  for (int u = 0; u < NB; u++)
-#pragma unroll
-    for (int m = 0; m < R; m++)
-      x[u * R + m] = (ZIN && m >= R / 2) ? mk<C>(0, 0) : ld(sq, j + u * T + m * Q);
-#pragma unroll
-  for (int u = 0; u < NB; u++) {
-    C* xb = x + u * R;
-    dft<R, false>(xb);
-    const int o = (j + u * T) * R, po = pad(o);
-#pragma unroll
-    for (int q = 0; q < R; q++) a[pad_out<1>(po, o, q)] = xb[out_reg<R>(q)];
+  if constexpr (L <= E) {
+    fft_inplace<L, false, HIN, false, E>(a, act, j, tab);
+    if (act)
+      for (int r = j; r < L; r += L / E) a[pad(r)] = mul(r, a[pad(r)]);
+    __syncthreads();
+    fft_inplace<L, true, false, HOUT, E>(a, act, j, tab);
+  } else {
+    fft_passes_below<L, 1, last_ns<L, E>(), false, HIN, E>(a, act, j, tab);
+    fft_turn<L, E>(a, act, j, tab, mul);
+    fft_passes<L, E, true, false, HOUT, E>(a, act, j, tab);
   }
 }
 
+// The first pass of a forward FFT (NS = 1, radix E) with its inputs read
+// straight from global memory (ld(index)) into registers: the sequence is
+// never staged in shared memory before the pass.  With the loads in flight
+// every thread calls mid() (the CTA's set-up; it may hold a barrier), then
+// the values pass through fix(index, value).  With ZIN the upper half of the
+// input is zero and not read.  The outputs go to shared memory; the caller's
+// barrier makes them visible.
+template <int L, bool ZIN, int E, class Ld, class Mid, class Fix>
+__device__ __forceinline__ void fft_first_pass_global(double2* a, bool act, int j, Tab tab, Ld ld, Mid mid, Fix fix)
+{
+  constexpr int Q = L / E, N = ZIN ? E / 2 : E;
+  double2 x[E];
+#pragma unroll
+  for (int m = 0; m < E; m++) x[m] = m < N && act ? ld(j + m * Q) : make_double2(0, 0);
+  mid();
+  if (!act) return;
+#pragma unroll
+  for (int m = 0; m < N; m++) x[m] = fix(j + m * Q, x[m]);
+  radix_step<L, E, E, 1, false, ZIN>(x, tab, 0);
+  const int o = j * E, po = pad(o);
+#pragma unroll
+  for (int q = 0; q < E; q++) a[pad_out<1>(po, o, q)] = x[out_reg<E>(q)];
+}
+
 // The last pass of an inverse FFT (NS * R = L) with its outputs written
-// straight to global memory (st(sequence, index, value)) from registers;
-// with HOUT only the lower half of the output is formed.
-template <int L, int R, int NS, bool HOUT, int E, class C, class St>
-__device__ __forceinline__ void fft_last_pass_global(C* A, int nseq, const C* tws, St st)
+// straight to global memory (st(index, value)) from registers; with HOUT
+// only the lower half of the output is formed.
+template <int L, int R, int NS, bool HOUT, int E, class St>
+__device__ __forceinline__ void fft_last_pass_global(const double2* a, bool act, int j, Tab tab, St st)
 {
   static_assert(NS * R == L, "the last pass");
-  constexpr int SL = Len<L>::SL, T = L / E, NB = E / R, Q = L / R;
-  const int tid = threadIdx.x;
-  if (tid >= nseq * T) return;
-  const int sq = tid / T, j = tid - sq * T;
-  const C* a = A + sq * SL;
-  C x[E];
+  constexpr int T = L / E, NB = E / R, Q = L / R;
+  if (!act) return;
+  double2 x[E];
   const int pj = pad(j);
 #pragma unroll
   for (int u = 0; u < NB; u++)
@@ -475,150 +351,129 @@ __device__ __forceinline__ void fft_last_pass_global(C* A, int nseq, const C* tw
     for (int m = 0; m < R; m++) x[u * R + m] = a[pad_at<T, Q>(pj, j, u, m)];
 #pragma unroll
   for (int u = 0; u < NB; u++) {
-    C* xb = x + u * R;
+    double2* xb = x + u * R;
     const int jb = j + u * T, k = jb & (NS - 1);
-    if (NS > 1 && k) apply_twiddles<L, E, R, NS, true>(xb, tws, k);
-    dft<R, true>(xb);
+    radix_step<L, E, R, NS, true, false>(xb, tab, k);
     const int o = (jb - k) * R + k;
 #pragma unroll
-    for (int q = 0; q < (HOUT ? R / 2 : R); q++) st(sq, o + q * NS, xb[out_reg<R>(q)]);
+    for (int q = 0; q < (HOUT ? R / 2 : R); q++) st(o + q * NS, xb[out_reg<R>(q)]);
   }
 }
 
-struct FadeArgs {
-  int enabled;
-  Scalars* sc;           // receives fadeCorr (from the first CTA)
-  GridDesc g;
-  double* writeback;     // rhs buffer receives the faded values (cub2rhs writes tmp)
-  const double* partials;   // fade sums of the strip blocks, three each
-  int nstrip;
-  int bandX, bandY;         // cells of the fade band from each edge, (int)(fadeLen / h) + 2 (host-formed)
+// fadeCorr ahead of the first row pass, by one warp
+__global__ void k_fade_corr(FadeArgs fa) {
+  pdl_begin();
+  const double corr = fade_corr(fa.partials, fa.nstrip);
+  if (threadIdx.x == 0) fa.sc->fadeCorr = corr;
+}
+// Strips of more blocks than this have fadeCorr formed once by k_fade_corr;
+// up to here (one round trip of fade_corr's loads) every CTA of the row pass
+// forms it while its rows land, which costs less than one more dependent
+// kernel.  At 380 blocks (4096 x 2048) the three round trips of every CTA had
+// made the other warps wait at the barrier.
+constexpr int FADE_IN_PLACE = 128;
+
+// ---- FP64 row and column passes ---------------------------------------------
+// The half spectrum between the passes lies in groups of SPEC_K columns:
+// entry (r, k) at ((k / SPEC_K) rows + r) SPEC_K + k mod SPEC_K.  A row pass
+// then writes (reads) 64-byte runs, and 32 rows of a column lie in 16
+// 128-byte lines; row-major, every 16-byte access of the column pass touched
+// its own line, and those took as many L1 cycles as its whole shared-memory
+// traffic.  Forward rows, columns, inverse rows at 4096 x 2048, in us: groups
+// of one column (transposed) 127, 141, 94; two 87, 157, 76; four 79, 172, 67;
+// eight 77, 215, 61; at 1024 x 512 two 15.0, 15.6, 11.5 and four 14.1, 16.6,
+// 10.6.
+constexpr int SPEC_LOG = 2, SPEC_K = 1 << SPEC_LOG;
+__host__ __device__ __forceinline__ size_t spec_at(int rows, int r, int k) {
+  return (((size_t)(k >> SPEC_LOG) * rows + r) << SPEC_LOG) | (k & (SPEC_K - 1));
+}
+
+// rows per CTA B, threads NT (L/E per row), padded stride SL of a row
+template <int L, int E> struct Row64 {
+  static constexpr int B = Len<L, E>::B, NT = Len<L, E>::NT, MINB = Len<L, E>::MINB, SL = Len<L, E>::SL;
 };
-
-// fadeCorr for this CTA, formed by warp 0 (blockDim.x >= 32) into *s;
-// visible to the CTA after its next barrier
-__device__ __forceinline__ void fade_corr_cta(const FadeArgs& fa, double* s) {
-  if (threadIdx.x < 32) {
-    const double corr = fade_corr(fa.partials, fa.nstrip);
-    if (threadIdx.x == 0) {
-      *s = corr;
-      if (blockIdx.x == 0) fa.sc->fadeCorr = corr;
-    }
-  }
+// columns per CTA: consecutive lanes take the columns of one pair (CB > 1),
+// and the stride SL puts the columns of eight lanes in different banks
+template <int L> struct Col64 {
+  static constexpr int CB = L <= 256 ? 8 : (L == 512 ? 4 : (L <= 2048 ? 2 : 1));
+  static constexpr int NT = CB * L / 16 < 64 ? 64 : CB * L / 16;
+  static constexpr int MINB = 65536 / (NT * 128) < 1 ? 1 : 65536 / (NT * 128);
+  static constexpr int SL0 = L + L / 16 + 1, WANT = CB == 1 ? 4 : 8 / CB;
+  static constexpr int SL = SL0 + ((WANT - SL0) % 8 + 8) % 8;
+  static constexpr int GR = L / 2 + 2;                  // multiplier values staged per column
+  static constexpr size_t SMEM = sizeof(double2) * ((size_t)CB * SL + tab_staged<L, 16>()) + sizeof(double) * CB * GR;
+};
+template <int L, int E> constexpr size_t smem_row64() {
+  return sizeof(double2) * ((size_t)Row64<L, E>::B * Row64<L, E>::SL + tab_staged<L, E>());
 }
 
-// PoissonSolver::cub2rhs (PoissonSolver.cpp:101-125) for one cell
-__device__ __forceinline__ double fade_cell(const GridDesc& g, int gx, int gy, double b, double corr) {
-  const double fadeLenX = g.fadeLenX, invFadeX = 1 / fmax(fadeLenX, EPSd);
-  const double fadeLenY = g.fadeLenY, invFadeY = 1 / fmax(fadeLenY, EPSd);
-  const double px = gx_pos(g, gx), py = gy_pos(g, gy);
-  const double yt = invFadeY * fmax(0.0, fadeLenY - g.ext[1] + py);
-  const double yb = invFadeY * fmax(0.0, fadeLenY - py);
-  const double xt = invFadeX * fmax(0.0, fadeLenX - g.ext[0] + px);
-  const double xb = invFadeX * fmax(0.0, fadeLenX - px);
-  const double fadeArg = fmin(fmax(fmax(yt, yb), fmax(xt, xb)), 1.0);
-  const double f2 = fadeArg * fadeArg;
-  const double fadeRHS = b * f2;
-  const double fadeCorrection = corr * (corr > 0 ? fmax(fadeRHS, 0.0) : -fmin(fadeRHS, 0.0));
-  return __dadd_rn(__dmul_rn(b, 1 - f2), fadeCorrection);   // never contracted into an FMA
-}
-
-// Real FFT of length 2L from the complex FFT Z of length L of its value
-// pairs, even/odd split: X[k] = Fe[k] + W^k Fo[k], W = exp(-i pi / L),
-// k in [0, L]; written to row row0 + r of out.  Thread t takes k = t + q NT
-// of every row; its twiddles are read first, all in flight at once (read
-// inside the loop, every iteration waited for its own).
-template <int L, int ER, class C>
-__device__ __forceinline__ void r2c_split(const C* A, int nb, int row0, C* __restrict__ out,
-                                          int outStride, const C* __restrict__ tw, int twLen)
+// Twice the real FFT of length 2L from the complex FFT Z of length L of its
+// value pairs: 2 X[k] = Fe + W^k Fo and 2 X[L - k] = conj(Fe - W^k Fo) with
+// Fe = Z_k + conj(Z_(L-k)), Fo = -i (Z_k - conj(Z_(L-k))), W = exp(-i pi/L), k in
+// [0, L/2); 2 X[L/2] = 2 conj(Z_(L/2)).  (The column pass's multiplier carries
+// the 1/2.)  A thread's twiddles are read first, all in flight at once.
+template <int L, int E>
+__device__ __forceinline__ void r2c_split(const double2* A, int nb, int row0, double2* __restrict__ out, int rows,
+                                          const double2* __restrict__ tw, int twLen)
 {
-  using R = typename CT<C>::R;
-  constexpr int SL = Len<L, ER>::SL, NT = Len<L, ER>::NT, KPT = (L + 1 + NT - 1) / NT;
-  constexpr int KB = KPT < 8 ? KPT : 8;                 // twiddles in flight per batch
+  constexpr int SL = Row64<L, E>::SL, NT = Row64<L, E>::NT, H = L / 2, KPT = (H + NT - 1) / NT;
   const int twStep = twLen / (2 * L);
+  double2 w[KPT];
 #pragma unroll
-  for (int q0 = 0; q0 < KPT; q0 += KB) {
-    C w[KB];
+  for (int q = 0; q < KPT; q++) {
+    const int k = threadIdx.x + q * NT;
+    w[q] = k < H ? tw[k * twStep] : make_double2(0, 0);
+  }
+  if (threadIdx.x < nb) {
+    const double2 z = A[threadIdx.x * SL + pad(H)];
+    out[spec_at(rows, row0 + threadIdx.x, H)] = make_double2(2 * z.x, -2 * z.y);
+  }
 #pragma unroll
-    for (int q = 0; q < KB; q++) {
-      const int k = threadIdx.x + (q0 + q) * NT;
-      w[q] = q0 + q < KPT && k <= L ? tw[k * twStep] : mk<C>(0, 0);
-    }
-#pragma unroll
-    for (int q = 0; q < KB; q++) {
-      const int k = threadIdx.x + (q0 + q) * NT;
-      if (q0 + q >= KPT || k > L) break;                // k grows with q
-      for (int r = 0; r < nb; r++) {
-        const C Zk = A[r * SL + pad(k == L ? 0 : k)];
-        const C Zc = conjg(A[r * SL + pad(k == 0 ? 0 : L - k)]);
-        const C Fe = mk<C>(R(0.5) * (Zk.x + Zc.x), R(0.5) * (Zk.y + Zc.y));
-        const C d = csub(Zk, Zc);
-        const C Fo = mk<C>(R(0.5) * d.y, R(-0.5) * d.x);  // (Zk - Zc) / (2i)
-        out[(size_t)(row0 + r) * outStride + k] = cadd(Fe, cmul(w[q], Fo));
-      }
+  for (int q = 0; q < KPT; q++) {
+    const int k = threadIdx.x + q * NT;
+    if (k >= H) break;                                  // k grows with q
+    for (int r = 0; r < nb; r++) {
+      const double2 Za = A[r * SL + pad(k)], Zb = conjg(A[r * SL + pad(k == 0 ? 0 : L - k)]);
+      const double2 Fe = cadd(Za, Zb), d = csub(Za, Zb), t = cmul(w[q], make_double2(d.y, -d.x));
+      out[spec_at(rows, row0 + r, k)] = cadd(Fe, t);
+      out[spec_at(rows, row0 + r, L - k)] = conjg(csub(Fe, t));
     }
   }
 }
 
-// inMode 0: rows of `in`; 1: the free-space Green's function on the MY x MX
-// padded grid (FFTW_freespace.cpp:108-119) computed on the fly.  Each row of 2L
-// reals is the complex sequence (x[2n], x[2n+1]) of length L.
-template <int L, bool HIN, int ER>
-__global__ void __launch_bounds__(Len<L, ER>::NT, Len<L, ER>::MINB)
-k_rows_r2c(const double* in, int inStride, int nrows, int ncolsIn, int inMode,
-           double2* __restrict__ out, int outStride,
-           const double2* __restrict__ tw, int twLen, FadeArgs fa, double h, int MX, int MY)
+// Forward row pass: each row of 2L reals is the complex sequence (x[2n],
+// x[2n+1]) of length L.  GREEN: the rows are the free-space Green's function
+// on the MY x MX padded grid (FFTW_freespace.cpp:108-119), formed on the fly;
+// else rows of `in`, faded as they are read (cub2rhs, PoissonSolver.cpp:
+// 61-141) and the band cells written back.
+template <int L, bool HIN, int E, bool GREEN>
+__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+k_rows_r2c(const double* in, int inStride, int nrows, int ncolsIn, double2* __restrict__ out, int outRows,
+           const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen, FadeArgs fa, double h,
+           int MX, int MY)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_R2C);
-  constexpr int SL = Len<L, ER>::SL, RB = Len<L, ER>::B, NT = Len<L, ER>::NT;
+  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B;
   extern __shared__ double2 sm[];
   double2* A = sm;
-  double2* tws = sm + RB * SL;
   const int row0 = blockIdx.x * RB;
   const int nb = min(RB, nrows - row0);
-  if (inMode == 0) {
-    // the first pass reads the rows itself, fading the band cells as it
-    // goes (cub2rhs, PoissonSolver.cpp:61-141) and writing them back
-    __shared__ double sCorr0;
-    if (fa.enabled) fade_corr_cta(fa, &sCorr0);
-    load_twiddles<L, ER>(tws, tw, twLen);
+  __shared__ double sCorr0;
+  const int sq = threadIdx.x / (L / E), j = threadIdx.x % (L / E);
+  const bool act = sq < nb;
+  double2* a = A + sq * SL;
+  const int row = row0 + sq;
+  Tab tb{sm + RB * SL, tab};
+  auto mid = [&]() {                                    // while the rows' values are on their way
+    if (!GREEN && fa.enabled) fade_corr_cta(fa, &sCorr0);
+    stage_tables<L, E>(sm + RB * SL, tab);
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
-    const double corr = fa.enabled ? sCorr0 : 0.0;
-    const int bandX = fa.enabled ? fa.bandX : 0;
-    const int bandY = fa.enabled ? fa.bandY : 0;
-    auto ld = [&](int r, int n) {
-      const int row = row0 + r;
-      const double* src = in + (size_t)row * inStride + 2 * n;
-      double2 v = make_double2(0, 0);
-      if (2 * n + 1 < ncolsIn) v = *reinterpret_cast<const double2*>(src);
-      else if (2 * n < ncolsIn) v.x = src[0];
-      if (fa.enabled && 2 * n + 1 < ncolsIn) {
-        const bool rowBand = row < bandY || row >= fa.g.ny - bandY;
-        if (rowBand || 2 * n < bandX || 2 * n + 1 >= fa.g.nx - bandX) {
-          double* x = &v.x;
-          for (int q = 0; q < 2; q++) {
-            const int col = 2 * n + q;
-            if (rowBand || col < bandX || col >= fa.g.nx - bandX) {
-              x[q] = fade_cell(fa.g, col, row, x[q], corr);
-              fa.writeback[(size_t)row * inStride + col] = x[q];
-            }
-          }
-        }
-      }
-      return v;
-    };
-    fft_first_pass_global<L, ER, HIN, ER>(A, nb, ld);
-    __syncthreads();
-    fft_passes<L, ER, false, false, false, ER>(A, nb, tws);
-    r2c_split<L, ER>(A, nb, row0, out, outStride, tw, twLen);
-    return;
-  }
-  {
-    // inMode 1: the Green's function, formed in place
-    for (int idx = threadIdx.x; idx < RB * L; idx += NT) {
-      const int r = idx / L, n = idx & (L - 1), row = row0 + r;
-      if (r >= nb) continue;
+  };
+  if (GREEN) {
+    auto ld = [&](int n) {
       double x[2];
       for (int q = 0; q < 2; q++) {
         const int col = 2 * n + q;
@@ -638,358 +493,184 @@ k_rows_r2c(const double* in, int inStride, int nrows, int ncolsIn, int inMode,
         }
         x[q] = val;
       }
-      A[r * SL + pad(n)] = make_double2(x[0], x[1]);
-    }
+      return make_double2(x[0], x[1]);
+    };
+    fft_first_pass_global<L, HIN, E>(a, act, j, tb, ld, mid, [](int, double2 v) { return v; });
+  } else {
+    // Nx is even: a value pair lies inside the row or beyond it
+    auto ld = [&](int n) {
+      return 2 * n < ncolsIn ? *reinterpret_cast<const double2*>(in + (size_t)row * inStride + 2 * n)
+                             : make_double2(0, 0);
+    };
+    const bool rowBand = fa.enabled && (row < fa.bandY || row >= fa.g.ny - fa.bandY);
+    // (no band, and no cell looked at, with the fade off)
+    const int bandLo = !fa.enabled ? 0 : rowBand ? fa.g.nx : fa.bandX;
+    const int bandHi = fa.enabled ? fa.g.nx - fa.bandX : ncolsIn;
+    const double rowFade = fade_row(fa.g, row);
+    auto fix = [&](int n, double2 v) {
+      if ((2 * n < bandLo || 2 * n + 1 >= bandHi) && 2 * n < ncolsIn) {
+        double* x = &v.x;
+        for (int q = 0; q < 2; q++) {
+          const int col = 2 * n + q;
+          if (col < bandLo || col >= bandHi) {
+            x[q] = fade_cell(rowFade, fade_col(fa.g, col), x[q], sCorr0);
+            fa.writeback[(size_t)row * inStride + col] = x[q];
+          }
+        }
+      }
+      return v;
+    };
+    fft_first_pass_global<L, HIN, E>(a, act, j, tb, ld, mid, fix);
   }
-  load_twiddles<L, ER>(tws, tw, twLen);
   __syncthreads();
-  fft_inplace<L, false, HIN, false, ER>(A, nb, tws);
-  r2c_split<L, ER>(A, nb, row0, out, outStride, tw, twLen);
+  fft_passes<L, E, false, false, false, E>(a, act, j, tb);
+  r2c_split<L, E>(A, nb, row0, out, outRows, tw, twLen);
 }
 
-// mode 0: forward, x G^ (real, symmetric in ky), inverse, keep nrowsOut rows
-// mode 1: forward; write Re * norm for ky <= L/2 into ghat (kernel set-up)
-// mode 2: forward, periodic multiplier -1/|k|^2 / (MX MY), inverse
-// Rows r >= nrowsIn of the input are zero and never read.
-template <int L, bool FS>
-__global__ void __launch_bounds__(Len<L, E_COLS>::NT, Len<L, E_COLS>::MINB)
-k_cols(double2* __restrict__ data, int stride, int ncols, int nrowsIn, int nrowsOut,
-       const double* __restrict__ ghatIn, double* __restrict__ ghatOut, int mode,
-       const double2* __restrict__ tw, int twLen, double norm, int MXp, int MYp)
+// Column pass (at 4096 points: 172 us for 4097 columns, 280 before the
+// multiply-add butterflies, the grouped spectrum, the multiplier stored by
+// columns, and the first and last passes straight from and to global memory).
+// Bound by the L1: 23 M shared-memory wavefronts (four exchanges of 64 KB a
+// column) and 10 M of global accesses, 73% of its cycles; FP64 pipe 36%,
+// DRAM 30%.  CONV: forward, times the real multiplier g (symmetric in ky),
+// inverse, keep nrowsOut rows; else (set-up of the free-space kernel) forward
+// alone, Re * norm of the first L/2 + 1 values to gOut.  Rows r >= nrowsIn of
+// the input are zero and never read; FS: they are at least the upper half,
+// and at most the lower half of the output is kept.
+template <int L, bool FS, bool CONV>
+__global__ void __launch_bounds__(Col64<L>::NT, Col64<L>::MINB)
+k_cols(double2* __restrict__ data, int rows, int ncols, int nrowsIn, int nrowsOut, const double* __restrict__ g,
+       double* __restrict__ gOut, const double2* __restrict__ tab, double norm)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_COLS);
-  constexpr int SL = Len<L, E_COLS>::SL, CB = Len<L, E_COLS>::B, NT = Len<L, E_COLS>::NT, GR = L / 2 + 1;
+  using P = Col64<L>;
+  constexpr int CB = P::CB, GN = L / 2 + 1;
   extern __shared__ double2 sm[];
-  double2* A = sm;
-  double2* tws = sm + CB * SL;
-  double* Gs = reinterpret_cast<double*>(tws + Len<L>::TW);   // [GR][CB] kernel rows
+  double* Gs = reinterpret_cast<double*>(sm + CB * P::SL + tab_staged<L, 16>());
   const int c0 = blockIdx.x * CB;
   const int nb = min(CB, ncols - c0);
-  // consecutive threads take consecutive columns of one row
-  for (int idx = threadIdx.x; idx < CB * nrowsIn; idx += NT) {
-    const int r = idx / CB, j = idx & (CB - 1);
-    if (j < nb) cp_async16(A + j * SL + pad(r), data + (size_t)r * stride + c0 + j);
-  }
-  cp_async_commit();
-  if (mode == 0) {
-    for (int idx = threadIdx.x; idx < CB * GR; idx += NT) {
-      const int r = idx / CB, j = idx & (CB - 1);
-      if (j < nb) cp_async8(Gs + r * CB + j, ghatIn + (size_t)r * stride + c0 + j);
+  const Tab tb = stage_tables<L, 16>(sm + CB * P::SL, tab);
+  if (CONV)
+    for (int idx = threadIdx.x; idx < nb * GN; idx += P::NT) {
+      const int q = idx / GN, r = idx - q * GN;
+      cp_async8(Gs + q * P::GR + r, g + (size_t)(c0 + q) * GN + r);
     }
-  }
   cp_async_commit();
-  // rows beyond the input are zero; the free-space solve never reads its
-  // upper half
-  for (int idx = threadIdx.x; idx < CB * ((FS ? L / 2 : L) - nrowsIn); idx += NT) {
-    const int r = nrowsIn + idx / CB, j = idx & (CB - 1);
-    A[j * SL + pad(r)] = make_double2(0, 0);
-  }
-  load_twiddles<L, E_COLS>(tws, tw, twLen);
-  if (mode == 1) {
-    cp_async_wait<0>();
-    __syncthreads();
-    fft_inplace<L, false, FS, false, E_COLS>(A, nb, tws);
-    for (int idx = threadIdx.x; idx < CB * nrowsOut; idx += NT) {
-      const int r = idx / CB, j = idx & (CB - 1);
-      if (j < nb) ghatOut[(size_t)r * stride + c0 + j] = A[j * SL + pad(r)].x * norm;
-    }
+  const int sq = threadIdx.x % CB, j = threadIdx.x / CB;
+  const bool act = sq < nb && j < L / 16;
+  double2* a = sm + sq * P::SL;
+  const int c = c0 + sq;
+  fft_first_pass_global<L, FS, 16>(a, act, j, tb,
+      [&](int r) { return r < nrowsIn ? __ldcg(data + spec_at(rows, r, c)) : make_double2(0, 0); },
+      [&]() { cp_async_wait<0>(); }, [](int, double2 v) { return v; });
+  __syncthreads();
+  if (!CONV) {
+    fft_passes<L, 16, false, false, false, 16>(a, act, j, tb);
+    if (act)
+      for (int r = j; r < GN; r += L / 16) gOut[(size_t)c * GN + r] = a[pad(r)].x * norm;
     return;
   }
-  cp_async_wait<0>();          // the columns and the kernel rows
-  __syncthreads();
-  if (mode == 0) {
-    fft_convolve<L, FS, FS, E_COLS>(A, nb, tws, [&](int j, int r, double2 z) {
-      const int ky = r <= L / 2 ? r : L - r;
-      const double f = Gs[ky * CB + j];
-      return make_double2(z.x * f, z.y * f);
-    });
+  auto mul = [&](int r, double2 z) {
+    const double f = Gs[sq * P::GR + (r <= L / 2 ? r : L - r)];
+    return make_double2(z.x * f, z.y * f);
+  };
+  auto st = [&](int r, double2 v) {
+    if (r < nrowsOut) data[spec_at(rows, r, c)] = v;
+  };
+  if constexpr (L <= 16) {
+    if (act)
+      for (int r = j; r < L; r += L / 16) a[pad(r)] = mul(r, a[pad(r)]);
+    __syncthreads();
+    fft_last_pass_global<L, 16, 1, FS, 16>(a, act, j, tb, st);
   } else {
-    fft_convolve<L, FS, FS, E_COLS>(A, nb, tws, [&](int j, int r, double2 z) {
-      // FFTW_periodic::_solve_spectral (FFTW_periodic.h:77-92)
-      const int i = c0 + j;
-      if (i == 0 && r == 0) return make_double2(0, 0);
-      const int kx = i <= MXp / 2 ? i : MXp - i, ky = r <= MYp / 2 ? r : MYp - r;
-      const double waveFactX = 2 * M_PI / MXp, waveFactY = 2 * M_PI / MYp;
-      const double rkx = kx * waveFactX, rky = ky * waveFactY;
-      const double f = -1 / (rkx * rkx + rky * rky) * norm;
-      return make_double2(z.x * f, z.y * f);
-    });
-  }
-  for (int idx = threadIdx.x; idx < CB * nrowsOut; idx += NT) {
-    const int r = idx / CB, j = idx & (CB - 1);
-    if (j < nb) data[(size_t)r * stride + c0 + j] = A[j * SL + pad(r)];
+    constexpr int NSL = last_ns<L, 16>();
+    fft_passes_below<L, 16, NSL, false, false, 16>(a, act, j, tb);
+    fft_turn<L, 16>(a, act, j, tb, mul);
+    fft_passes_below<L, 16, NSL, true, false, 16>(a, act, j, tb);
+    fft_last_pass_global<L, L / NSL, NSL, FS, 16>(a, act, j, tb, st);
   }
 }
 
-// inverse real FFT of length 2L from X[0..L]; writes the first ncolsOut values
-template <int L, bool HOUT, int EC>
-__global__ void __launch_bounds__(Len<L, EC>::NT, Len<L, EC>::MINB)
-k_rows_c2r(const double2* __restrict__ in, int inStride, int nrows, double* __restrict__ out,
-           int outStride, int ncolsOut, const double2* __restrict__ tw, int twLen)
+// the periodic multiplier of FFTW_periodic::_solve_spectral
+// (FFTW_periodic.h:77-92), half of -1/|k|^2 / (MX MY), as the column pass reads it
+__global__ void k_periodic_multiplier(double* __restrict__ g, int nkx, int MX, int MY, double norm) {
+  const int n = MY / 2 + 1;
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nkx * n; idx += gridDim.x * blockDim.x) {
+    const int i = idx / n, r = idx - i * n;
+    const int kx = i <= MX / 2 ? i : MX - i;
+    const double waveFactX = 2 * M_PI / MX, waveFactY = 2 * M_PI / MY;
+    const double rkx = kx * waveFactX, rky = r * waveFactY;
+    g[idx] = i == 0 && r == 0 ? 0.0 : 0.5 * (-1 / (rkx * rkx + rky * rky) * norm);
+  }
+}
+
+// Inverse real FFT of length 2L from X[0..L]; writes the first ncolsOut
+// values.  The pairs X[k], X[L - k] are read straight into registers and
+// merged: z[k] = s + i t, z[L - k] = conj(s) + i conj(t) with s = X_k +
+// conj(X_(L-k)), t = W^-k (X_k - conj(X_(L-k))), k < L/2; z[L/2] = 2 conj(X_(L/2)).
+template <int L, bool HOUT, int E>
+__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+k_rows_c2r(const double2* __restrict__ in, int inRows, int nrows, double* __restrict__ out,
+           int outStride, int ncolsOut, const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_C2R);
-  constexpr int SL = Len<L, EC>::SL, RB = Len<L, EC>::B, NT = Len<L, EC>::NT, H = L / 2;
+  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B, NT = Row64<L, E>::NT, H = L / 2;
+  constexpr int KPT = (H + NT - 1) / NT;
   extern __shared__ double2 sm[];
   double2* A = sm;
-  double2* tws = sm + RB * SL;
   const int row0 = blockIdx.x * RB;
   const int nb = min(RB, nrows - row0);
   const int twStep = twLen / (2 * L);
-  // X[0..L] of each row; X[L] lands in the spare slot pad(L) < SL
-  for (int idx = threadIdx.x; idx < RB * (L + 1); idx += NT) {
-    const int r = idx / (L + 1), k = idx - r * (L + 1);
-    if (r < nb) cp_async16(A + r * SL + pad(k), in + (size_t)(row0 + r) * inStride + k);
-  }
+  const Tab tb = stage_tables<L, E>(sm + RB * SL, tab);
   cp_async_commit();
-  load_twiddles<L, EC>(tws, tw, twLen);
-  // the split's W^-k of the pairs (k, L - k) this thread forms, read while
-  // the rows land
-  constexpr int KPT = (H + NT - 1) / NT;
-  double2 wk[KPT][2];
+  double2 wk[KPT], xh = make_double2(0, 0);
+  if (threadIdx.x < nb) xh = in[spec_at(inRows, row0 + threadIdx.x, H)];
 #pragma unroll
   for (int q = 0; q < KPT; q++) {
     const int k = threadIdx.x + q * NT;
-    if (k < H) {
-      wk[q][0] = conjg(tw[k * twStep]);
-      wk[q][1] = conjg(tw[(k == 0 ? H : L - k) * twStep]);
+    wk[q] = k < H ? tw[k * twStep] : make_double2(0, 0);
+  }
+#pragma unroll
+  for (int r = 0; r < RB; r++) {
+    if (r >= nb) break;
+    double2 xa[KPT], xb[KPT];
+#pragma unroll
+    for (int q = 0; q < KPT; q++) {
+      const int k = threadIdx.x + q * NT;
+      xa[q] = xb[q] = make_double2(0, 0);
+      if (k < H) {
+        xa[q] = in[spec_at(inRows, row0 + r, k)];
+        xb[q] = in[spec_at(inRows, row0 + r, L - k)];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < KPT; q++) {
+      const int k = threadIdx.x + q * NT;
+      if (k >= H) break;
+      double2 Xk = xa[q], Xc = conjg(xb[q]);
+      if (k == 0) { Xk.y = 0; Xc.y = 0; }             // c2r ignores Im X[0], Im X[L]
+      const double2 s = cadd(Xk, Xc), t = cmul(conjg(wk[q]), csub(Xk, Xc));
+      double2* a = A + r * SL;
+      a[pad(k)] = make_double2(s.x - t.y, s.y + t.x);
+      if (k > 0) a[pad(L - k)] = make_double2(s.x + t.y, t.x - s.y);
     }
   }
+  if (threadIdx.x < nb) A[threadIdx.x * SL + pad(H)] = make_double2(2 * xh.x, -2 * xh.y);
   cp_async_wait<0>();
   __syncthreads();
-  // z[k] = s + i t, s = X_k + conj(X_{L-k}), t = W^-k (X_k - conj(X_{L-k})):
-  // thread (k, r), k < L/2, forms the pair k, L-k of every row in place;
-  // k = 0 also L/2
-#pragma unroll
-  for (int q = 0; q < KPT; q++) {
-    const int k = threadIdx.x + q * NT;
-    if (k >= H) continue;
-    const int kk[2] = {k, k == 0 ? H : L - k};
-    for (int r = 0; r < nb; r++) {
-      double2* a = A + r * SL;
-      double2 Xa = a[pad(k)], Xb = a[pad(k == 0 ? L : L - k)];
-      if (k == 0) { Xa.y = 0; Xb.y = 0; }         // c2r ignores Im X[0], Im X[L]
-      double2 res[2];
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        double2 Xk, XL;
-        if (e == 0) { Xk = Xa; XL = Xb; }
-        else if (k == 0) { Xk = a[pad(H)]; XL = Xk; }
-        else { Xk = Xb; XL = Xa; }
-        const double2 Xc = conjg(XL);
-        const double2 sv = cadd(Xk, Xc), d = csub(Xk, Xc);
-        const double2 t = cmul(wk[q][e], d);
-        res[e] = make_double2(sv.x - t.y, sv.y + t.x);
-      }
-      a[pad(kk[0])] = res[0];
-      a[pad(kk[1])] = res[1];
-    }
-  }
-  __syncthreads();
   // the inverse FFT; its last pass writes the value pairs of the row
-  constexpr int NSL = last_ns<L, EC>();
-  fft_passes_below<L, 1, NSL, true, false, EC>(A, nb, tws);
-  fft_last_pass_global<L, L / NSL, NSL, HOUT, EC>(A, nb, tws, [&](int r, int n, double2 v) {
-    double* o = out + (size_t)(row0 + r) * outStride;
+  const int sq = threadIdx.x / (L / E), j = threadIdx.x % (L / E);
+  const bool act = sq < nb;
+  double2* a = A + sq * SL;
+  constexpr int NSL = last_ns<L, E>();
+  fft_passes_below<L, 1, NSL, true, false, E>(a, act, j, tb);
+  double* o = out + (size_t)(row0 + sq) * outStride;
+  fft_last_pass_global<L, L / NSL, NSL, HOUT, E>(a, act, j, tb, [&](int n, double2 v) {
     if (2 * n + 1 < ncolsOut) *reinterpret_cast<double2*>(o + 2 * n) = v;
     else if (2 * n < ncolsOut) o[2 * n] = v.x;
   });
-}
-
-// ---- FP32 transforms (CUP2D_PREC_FP32) ------------------------------------
-// The free-space and periodic solves with float2 spectra and FP32 passes:
-// the same kernels' structure, the fade and its write-back in FP64 (so the
-// RHS written back is the one of the FP64 path), rows converted to FP32 as
-// they enter shared memory, the pressure written back in FP64.
-template <int L, bool HIN>
-__global__ void __launch_bounds__(Len<L, E_ROWS32>::NT, Len<L, E_ROWS32>::MINB)
-k_rows_r2c32(const double* __restrict__ in, int inStride, int nrows, int ncolsIn,
-             float2* __restrict__ out, int outStride, const float2* __restrict__ tw, int twLen, FadeArgs fa)
-{
-  pdl_begin();
-  CUP2D_TRACE_SCOPE(TR_R2C);
-  constexpr int SL = Len<L, E_ROWS32>::SL, RB = Len<L, E_ROWS32>::B, NT = Len<L, E_ROWS32>::NT;
-  constexpr int PER = (RB * L + NT - 1) / NT;          // value pairs per thread
-  extern __shared__ float2 sm32[];
-  float2* A = sm32;
-  float2* tws = sm32 + RB * SL;
-  const int row0 = blockIdx.x * RB;
-  const int nb = min(RB, nrows - row0);
-  double2 v[PER];                                      // this thread's pairs, all loads in flight
-#pragma unroll
-  for (int u = 0; u < PER; u++) {
-    const int idx = threadIdx.x + u * NT;
-    const int r = idx / L, n = idx & (L - 1), row = row0 + r;
-    v[u] = make_double2(0, 0);
-    if (idx < RB * L && r < nb) {
-      if (2 * n + 1 < ncolsIn) v[u] = *reinterpret_cast<const double2*>(in + (size_t)row * inStride + 2 * n);
-      else if (2 * n < ncolsIn) v[u].x = in[(size_t)row * inStride + 2 * n];
-    }
-  }
-  __shared__ double sCorr;
-  if (fa.enabled) fade_corr_cta(fa, &sCorr);
-  load_twiddles<L, E_ROWS32>(tws, tw, twLen);
-  __syncthreads();
-  const double corr = fa.enabled ? sCorr : 0.0;
-  const int bandX = fa.enabled ? fa.bandX : 0;
-  const int bandY = fa.enabled ? fa.bandY : 0;
-#pragma unroll
-  for (int u = 0; u < PER; u++) {
-    const int idx = threadIdx.x + u * NT;
-    const int r = idx / L, n = idx & (L - 1), row = row0 + r;
-    if (idx >= RB * L || r >= nb) continue;
-    if (HIN && n >= L / 2) continue;                   // the zero upper half is never read
-    if (fa.enabled && 2 * n + 1 < ncolsIn) {
-      // fade band as in k_rows_r2c (cub2rhs, PoissonSolver.cpp:61-141)
-      const bool rowBand = row < bandY || row >= fa.g.ny - bandY;
-      double* x = &v[u].x;
-      for (int q = 0; q < 2; q++) {
-        const int col = 2 * n + q;
-        if (rowBand || col < bandX || col >= fa.g.nx - bandX) {
-          x[q] = fade_cell(fa.g, col, row, x[q], corr);
-          fa.writeback[(size_t)row * inStride + col] = x[q];
-        }
-      }
-    }
-    A[r * SL + pad(n)] = make_float2((float)v[u].x, (float)v[u].y);
-  }
-  __syncthreads();
-  fft_inplace<L, false, HIN, false, E_ROWS32>(A, nb, tws);
-  r2c_split<L, E_ROWS32>(A, nb, row0, out, outStride, tw, twLen);
-}
-
-// mode 0: forward, x G^, inverse, keep nrowsOut rows; mode 2: the periodic
-// multiplier -1/|k|^2 / (MX MY) (formed in FP64, applied in FP32)
-template <int L, bool FS>
-__global__ void __launch_bounds__(Len<L, E_COLS32>::NT, Len<L, E_COLS32>::MINB)
-k_cols32(float2* __restrict__ data, int stride, int ncols, int nrowsIn, int nrowsOut,
-         const float* __restrict__ ghat, int mode, const float2* __restrict__ tw, int twLen,
-         double norm, int MXp, int MYp)
-{
-  pdl_begin();
-  CUP2D_TRACE_SCOPE(TR_COLS);
-  constexpr int SL = Len<L, E_COLS32>::SL, CB = Len<L, E_COLS32>::B, NT = Len<L, E_COLS32>::NT, GR = L / 2 + 1;
-  extern __shared__ float2 sm32[];
-  float2* A = sm32;
-  float2* tws = sm32 + CB * SL;
-  float* Gs = reinterpret_cast<float*>(tws + Len<L>::TW);   // [GR][CB] kernel rows
-  const int c0 = blockIdx.x * CB;
-  const int nb = min(CB, ncols - c0);
-  for (int idx = threadIdx.x; idx < CB * nrowsIn; idx += NT) {
-    const int r = idx / CB, j = idx & (CB - 1);
-    if (j < nb) cp_async8(A + j * SL + pad(r), data + (size_t)r * stride + c0 + j);
-  }
-  if (mode == 0)
-    for (int idx = threadIdx.x; idx < CB * GR; idx += NT) {
-      const int r = idx / CB, j = idx & (CB - 1);
-      if (j < nb) cp_async4(Gs + r * CB + j, ghat + (size_t)r * stride + c0 + j);
-    }
-  cp_async_commit();
-  // rows beyond the input are zero; the free-space solve never reads its
-  // upper half
-  for (int idx = threadIdx.x; idx < CB * ((FS ? L / 2 : L) - nrowsIn); idx += NT) {
-    const int r = nrowsIn + idx / CB, j = idx & (CB - 1);
-    A[j * SL + pad(r)] = make_float2(0, 0);
-  }
-  load_twiddles<L, E_COLS32>(tws, tw, twLen);
-  cp_async_wait<0>();
-  __syncthreads();
-  if (mode == 0) {
-    fft_convolve<L, FS, FS, E_COLS32>(A, nb, tws, [&](int j, int r, float2 z) {
-      const int ky = r <= L / 2 ? r : L - r;
-      const float f = Gs[ky * CB + j];
-      return make_float2(z.x * f, z.y * f);
-    });
-  } else {
-    fft_convolve<L, FS, FS, E_COLS32>(A, nb, tws, [&](int j, int r, float2 z) {
-      // FFTW_periodic::_solve_spectral (FFTW_periodic.h:77-92)
-      const int i = c0 + j;
-      if (i == 0 && r == 0) return make_float2(0, 0);
-      const int kx = i <= MXp / 2 ? i : MXp - i, ky = r <= MYp / 2 ? r : MYp - r;
-      const double waveFactX = 2 * M_PI / MXp, waveFactY = 2 * M_PI / MYp;
-      const double rkx = kx * waveFactX, rky = ky * waveFactY;
-      const float f = (float)(-1 / (rkx * rkx + rky * rky) * norm);
-      return make_float2(z.x * f, z.y * f);
-    });
-  }
-  for (int idx = threadIdx.x; idx < CB * nrowsOut; idx += NT) {
-    const int r = idx / CB, j = idx & (CB - 1);
-    if (j < nb) data[(size_t)r * stride + c0 + j] = A[j * SL + pad(r)];
-  }
-}
-
-// inverse real FFT of length 2L from X[0..L] (float2); writes the first
-// ncolsOut values in FP64
-template <int L, bool HOUT>
-__global__ void __launch_bounds__(Len<L, E_C2R32>::NT, Len<L, E_C2R32>::MINB)
-k_rows_c2r32(const float2* __restrict__ in, int inStride, int nrows, double* __restrict__ out, int outStride,
-             int ncolsOut, const float2* __restrict__ tw, int twLen)
-{
-  pdl_begin();
-  CUP2D_TRACE_SCOPE(TR_C2R);
-  constexpr int SL = Len<L, E_C2R32>::SL, RB = Len<L, E_C2R32>::B, NT = Len<L, E_C2R32>::NT, H = L / 2;
-  extern __shared__ float2 sm32[];
-  float2* A = sm32;
-  float2* tws = sm32 + RB * SL;
-  const int row0 = blockIdx.x * RB;
-  const int nb = min(RB, nrows - row0);
-  const int twStep = twLen / (2 * L);
-  for (int idx = threadIdx.x; idx < RB * (L + 1); idx += NT) {
-    const int r = idx / (L + 1), k = idx - r * (L + 1);
-    if (r < nb) cp_async8(A + r * SL + pad(k), in + (size_t)(row0 + r) * inStride + k);
-  }
-  cp_async_commit();
-  load_twiddles<L, E_C2R32>(tws, tw, twLen);
-  // the split's W^-k of the pairs (k, L - k) this thread forms, read while
-  // the rows land (as in k_rows_c2r)
-  constexpr int KPT = (H + NT - 1) / NT;
-  float2 wk[KPT][2];
-#pragma unroll
-  for (int q = 0; q < KPT; q++) {
-    const int k = threadIdx.x + q * NT;
-    if (k < H) {
-      wk[q][0] = conjg(tw[k * twStep]);
-      wk[q][1] = conjg(tw[(k == 0 ? H : L - k) * twStep]);
-    }
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < KPT; q++) {
-    const int k = threadIdx.x + q * NT;
-    if (k >= H) continue;
-    const int kk[2] = {k, k == 0 ? H : L - k};
-    for (int r = 0; r < nb; r++) {
-      float2* a = A + r * SL;
-      float2 Xa = a[pad(k)], Xb = a[pad(k == 0 ? L : L - k)];
-      if (k == 0) { Xa.y = 0; Xb.y = 0; }
-      float2 res[2];
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        float2 Xk, XL;
-        if (e == 0) { Xk = Xa; XL = Xb; }
-        else if (k == 0) { Xk = a[pad(H)]; XL = Xk; }
-        else { Xk = Xb; XL = Xa; }
-        const float2 Xc = conjg(XL);
-        const float2 sv = cadd(Xk, Xc), d = csub(Xk, Xc);
-        const float2 t = cmul(wk[q][e], d);
-        res[e] = make_float2(sv.x - t.y, sv.y + t.x);
-      }
-      a[pad(kk[0])] = res[0];
-      a[pad(kk[1])] = res[1];
-    }
-  }
-  __syncthreads();
-  fft_inplace<L, true, false, HOUT, E_C2R32>(A, nb, tws);
-  const int half = (ncolsOut + 1) / 2;
-  for (int idx = threadIdx.x; idx < nb * half; idx += NT) {
-    const int r = idx / half, n = idx - r * half;
-    const float2 v = A[r * SL + pad(n)];
-    double* o = out + (size_t)(row0 + r) * outStride;
-    if (2 * n + 1 < ncolsOut) *reinterpret_cast<double2*>(o + 2 * n) = make_double2(v.x, v.y);
-    else o[2 * n] = v.x;
-  }
 }
 
 // ---- cosine-transform solver (FFTW_dirichlet.h:30-130) --------------------
@@ -1003,18 +684,18 @@ k_rows_c2r32(const float2* __restrict__ in, int inStride, int nrows, double* __r
 template <int L>
 __global__ void __launch_bounds__(Len<L>::NT, Len<L>::MINB)
 k_dct_rows_fwd(const double* in, int Nx, int nrows, double* __restrict__ D, int rb,
-               const double2* __restrict__ tw, int twLen, FadeArgs fa)
+               const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen, FadeArgs fa)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_FWD);
   constexpr int SL = Len<L>::SL;
   extern __shared__ double2 sm[];
   double2* A = sm;
-  double2* tws = sm + rb * SL;
-  double* Bx = reinterpret_cast<double*>(tws + Len<L>::TW);     // staged real row values
+  double* Bx = reinterpret_cast<double*>(sm + rb * SL + tab_staged<L, 16>());     // staged real row values
   __shared__ double sCorr;
   if (fa.enabled) fade_corr_cta(fa, &sCorr);
-  load_twiddles<L, 16>(tws, tw, twLen);
+  const Tab tb = stage_tables<L, 16>(sm + rb * SL, tab);
+  cp_async_commit();
   const int row0 = blockIdx.x * rb;
   const int nb = min(rb, nrows - row0);
   __syncthreads();
@@ -1026,7 +707,7 @@ k_dct_rows_fwd(const double* in, int Nx, int nrows, double* __restrict__ D, int 
     const int r = idx / L, col = idx - r * L, row = row0 + r;
     double v = in[(size_t)row * Nx + col];
     if (fa.enabled && (row < bandY || row >= fa.g.ny - bandY || col < bandX || col >= fa.g.nx - bandX)) {
-      v = fade_cell(fa.g, col, row, v, corr);
+      v = fade_cell(fade_row(fa.g, row), fade_col(fa.g, col), v, corr);
       fa.writeback[(size_t)row * Nx + col] = v;
     }
     Bx[r * L + col] = v;
@@ -1039,8 +720,10 @@ k_dct_rows_fwd(const double* in, int Nx, int nrows, double* __restrict__ D, int 
     const double y1 = Bx[r * L + (j1 < L ? j1 : 2 * L - 1 - j1)];
     A[r * SL + pad(n)] = make_double2(y0, y1);
   }
+  cp_async_wait<0>();
   __syncthreads();
-  fft_inplace<L, false>(A, nb, tws);
+  const int sq = threadIdx.x / (L / 16), js = threadIdx.x % (L / 16);
+  fft_inplace<L, false>(A + sq * SL, sq < nb, js, tb);
   double2* Z = A;
   const int st2 = twLen / (2 * L), st4 = twLen / (4 * L);
   // four iterations' global loads in flight before the first store
@@ -1063,15 +746,15 @@ k_dct_rows_fwd(const double* in, int Nx, int nrows, double* __restrict__ D, int 
 template <int L>
 __global__ void __launch_bounds__(Len<L>::NT, Len<L>::MINB)
 k_dct_cols(double* D, int Nx, int Ny, int cb, const float* __restrict__ cosX, const float* __restrict__ cosY,
-           double tol, const double2* __restrict__ tw, int twLen)
+           double tol, const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_COLS);
   constexpr int SL = Len<L>::SL;
   extern __shared__ double2 sm[];
   double2* A = sm;
-  double2* tws = sm + cb * SL;
-  load_twiddles<L, 16>(tws, tw, twLen);
+  const Tab tb = stage_tables<L, 16>(sm + cb * SL, tab);
+  cp_async_commit();
   const int n = Ny;                                   // L = 2n
   const int c0 = blockIdx.x * cb * 2;                 // first column of this CTA
   const int np = min(cb, (Nx - c0) / 2);              // column pairs
@@ -1081,8 +764,10 @@ k_dct_cols(double* D, int Nx, int Ny, int cb, const float* __restrict__ cosX, co
     const double2 ab = *reinterpret_cast<const double2*>(D + (size_t)row * Nx + c0 + 2 * q);
     A[q * SL + pad(j)] = ab;                          // a + i b
   }
+  cp_async_wait<0>();
   __syncthreads();
-  fft_inplace<L, false>(A, np, tws);
+  const int sq = threadIdx.x / (L / 16), js = threadIdx.x % (L / 16);
+  fft_inplace<L, false>(A + sq * SL, sq < np, js, tb);
   double2* Z = A;
   // each thread reads the pair (k, L-k) before writing the same pair, and
   // slot n is read by none, so the inverse input overwrites Z in place
@@ -1123,7 +808,7 @@ k_dct_cols(double* D, int Nx, int Ny, int cb, const float* __restrict__ cosX, co
   }
   for (int q = threadIdx.x; q < np; q += blockDim.x) W[q * SL + pad(n)] = make_double2(0, 0);
   __syncthreads();
-  fft_inplace<L, true, false, true>(W, np, tws);          // outputs m < n = L/2
+  fft_inplace<L, true, false, true>(W + sq * SL, sq < np, js, tb);          // outputs m < n = L/2
   double2* Y = W;
 #pragma unroll 4
   for (int idx = threadIdx.x; idx < np * n; idx += blockDim.x) {
@@ -1136,15 +821,15 @@ k_dct_cols(double* D, int Nx, int Ny, int cb, const float* __restrict__ cosX, co
 template <int L>
 __global__ void __launch_bounds__(Len<L>::NT, Len<L>::MINB)
 k_dct_rows_inv(const double* __restrict__ D, int Nx, int nrows, double* __restrict__ out, int rb,
-               const double2* __restrict__ tw, int twLen)
+               const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_INV);
   constexpr int SL = Len<L>::SL;
   extern __shared__ double2 sm[];
   double2* A = sm;
-  double2* tws = sm + rb * SL;
-  load_twiddles<L, 16>(tws, tw, twLen);
+  const Tab tb = stage_tables<L, 16>(sm + rb * SL, tab);
+  cp_async_commit();
   const int row0 = blockIdx.x * rb;
   const int nb = min(rb, nrows - row0);
   const int st2 = twLen / (2 * L), st4 = twLen / (4 * L);
@@ -1164,8 +849,10 @@ k_dct_rows_inv(const double* __restrict__ D, int Nx, int nrows, double* __restri
     const double2 t = cmul(conjg(tw[k * st2]), d);
     A[r * SL + pad(k)] = make_double2(s.x - t.y, s.y + t.x);
   }
+  cp_async_wait<0>();
   __syncthreads();
-  fft_inplace<L, true, false, true>(A, nb, tws);          // outputs m < L/2
+  const int sq = threadIdx.x / (L / 16), js = threadIdx.x % (L / 16);
+  fft_inplace<L, true, false, true>(A + sq * SL, sq < nb, js, tb);          // outputs m < L/2
   double2* z = A;
   for (int idx = threadIdx.x; idx < nb * (L / 2); idx += blockDim.x) {
     const int r = idx / (L / 2), m = idx - r * (L / 2);
@@ -1180,51 +867,38 @@ void set_smem(const void* f) { if (allow_max_dynamic_smem(f) != cudaSuccess) g_s
 
 // B padded sequences, the staged twiddles, and extraReals doubles
 template <int L> inline size_t smem_for(size_t extraReals = 0) {
-  return sizeof(double2) * ((size_t)Len<L>::B * Len<L>::SL + Len<L>::TW) + sizeof(double) * extraReals;
+  return sizeof(double2) * ((size_t)Len<L>::B * Len<L>::SL + tab_staged<L, 16>()) + sizeof(double) * extraReals;
 }
-
-template <int L> inline size_t smem_for32(size_t extraReals = 0) {
-  return sizeof(float2) * ((size_t)Len<L>::B * Len<L>::SL + Len<L>::TW) + sizeof(float) * extraReals;
-}
-
-#define CUP2D_FFT_LENGTHS(X) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
 
 void set_all_smem() {
-#define X(L) set_smem((const void*)k_rows_r2c<L, false, 8>); set_smem((const void*)k_rows_r2c<L, true, 8>); \
-             set_smem((const void*)k_rows_r2c<L, false, 16>); set_smem((const void*)k_rows_r2c<L, true, 16>); \
+#define X(L) set_smem((const void*)k_rows_r2c<L, false, 8, false>); set_smem((const void*)k_rows_r2c<L, true, 8, false>); \
+             set_smem((const void*)k_rows_r2c<L, false, 16, false>); set_smem((const void*)k_rows_r2c<L, true, 16, false>); \
+             set_smem((const void*)k_rows_r2c<L, false, 8, true>); \
              set_smem((const void*)k_rows_c2r<L, false, 8>); set_smem((const void*)k_rows_c2r<L, true, 8>); \
              set_smem((const void*)k_rows_c2r<L, false, 16>); set_smem((const void*)k_rows_c2r<L, true, 16>); \
-             set_smem((const void*)k_cols<L, false>); set_smem((const void*)k_cols<L, true>); \
-             set_smem((const void*)k_dct_rows_fwd<L>); \
-             set_smem((const void*)k_dct_cols<L>); set_smem((const void*)k_dct_rows_inv<L>); \
-             set_smem((const void*)k_rows_r2c32<L, false>); set_smem((const void*)k_rows_r2c32<L, true>); \
-             set_smem((const void*)k_rows_c2r32<L, false>); set_smem((const void*)k_rows_c2r32<L, true>); \
-             set_smem((const void*)k_cols32<L, false>); set_smem((const void*)k_cols32<L, true>);
+             set_smem((const void*)k_cols<L, false, true>); set_smem((const void*)k_cols<L, true, true>); \
+             set_smem((const void*)k_cols<L, false, false>); set_smem((const void*)k_dct_rows_fwd<L>); \
+             set_smem((const void*)k_dct_cols<L>); set_smem((const void*)k_dct_rows_inv<L>);
   CUP2D_FFT_LENGTHS(X)
 #undef X
+  if (!poisson32_setup()) g_smemOk = false;
 }
 
 template <int LL, int ER>
-void rows_r2c_e(cudaStream_t st, const double* in, int inStride, int nrows, int ncolsIn, int inMode,
-                double2* out, int outStride, const double2* tw, int twLen, FadeArgs fa, double h, int MX, int MY,
-                bool halfIn) {
-  const int grid = (nrows + Len<LL>::B - 1) / Len<LL>::B;
-  if (halfIn) launch_k(k_rows_r2c<LL, true, ER>, grid, Len<LL, ER>::NT, smem_for<LL>(), st,
-                       in, inStride, nrows, ncolsIn, inMode, out, outStride, tw, twLen, fa, h, MX, MY);
-  else launch_k(k_rows_r2c<LL, false, ER>, grid, Len<LL, ER>::NT, smem_for<LL>(), st,
-                in, inStride, nrows, ncolsIn, inMode, out, outStride, tw, twLen, fa, h, MX, MY);
+void rows_r2c_e(const Poisson& P, cudaStream_t st, const double* in, int nx, int ny, const FadeArgs& fa, bool halfIn) {
+  const int grid = (ny + Row64<LL, ER>::B - 1) / Row64<LL, ER>::B;
+  const auto k = halfIn ? k_rows_r2c<LL, true, ER, false> : k_rows_r2c<LL, false, ER, false>;
+  launch_k(k, grid, Row64<LL, ER>::NT, smem_row64<LL, ER>(), st, in, nx, ny, nx, P.spec, ny, P.tRow[ER == 16], P.tw,
+           P.twLen, fa, 0.0, 0, 0);
 }
 
 // e: elements per thread (8 or 16)
-bool rows_r2c(int L, cudaStream_t st, const double* in, int inStride, int nrows, int ncolsIn, int inMode,
-              double2* out, int outStride, const double2* tw, int twLen, FadeArgs fa, double h, int MX, int MY,
-              bool halfIn, int e) {
-  switch (L) {
+bool rows_r2c(const Poisson& P, cudaStream_t st, const double* in, int nx, int ny, const FadeArgs& fa, bool halfIn,
+              int e) {
+  switch (P.Lrow) {
 #define X(LL) case LL: \
-    if (e == 16) rows_r2c_e<LL, 16>(st, in, inStride, nrows, ncolsIn, inMode, out, outStride, tw, twLen, fa, h, \
-                                    MX, MY, halfIn); \
-    else rows_r2c_e<LL, 8>(st, in, inStride, nrows, ncolsIn, inMode, out, outStride, tw, twLen, fa, h, MX, MY, \
-                           halfIn); \
+    if (e == 16) rows_r2c_e<LL, 16>(P, st, in, nx, ny, fa, halfIn); \
+    else rows_r2c_e<LL, 8>(P, st, in, nx, ny, fa, halfIn); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -1232,16 +906,37 @@ bool rows_r2c(int L, cudaStream_t st, const double* in, int inStride, int nrows,
   return false;
 }
 
-bool cols(int L, cudaStream_t st, double2* data, int stride, int ncols, int nrowsIn, int nrowsOut,
-          double* ghat, int mode, const double2* tw, int twLen, double norm, int MXp, int MYp) {
-  switch (L) {
+// the Green's function's rows (all MY of them) into spec
+bool rows_green(const Poisson& P, cudaStream_t st, double h) {
+  FadeArgs fa{};
+  switch (P.Lrow) {
+#define X(LL) case LL: launch_k(k_rows_r2c<LL, false, 8, true>, (P.MY + Row64<LL, 8>::B - 1) / Row64<LL, 8>::B, \
+        Row64<LL, 8>::NT, smem_row64<LL, 8>(), st, nullptr, 0, P.MY, P.MX, P.spec, P.MY, P.tRow[0], P.tw, P.twLen, \
+        fa, h, P.MX, P.MY); return true;
+    CUP2D_FFT_LENGTHS(X)
+#undef X
+  }
+  return false;
+}
+
+bool cols(const Poisson& P, cudaStream_t st, int ny, bool fs) {
+  switch (P.Lcol) {
 #define X(LL) case LL: \
-    if (mode == 0) launch_k(k_cols<LL, true>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS>::NT, \
-        smem_for<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, stride, ncols, nrowsIn, \
-        nrowsOut, ghat, ghat, mode, tw, twLen, norm, MXp, MYp); \
-    else launch_k(k_cols<LL, false>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS>::NT, \
-        smem_for<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, stride, ncols, nrowsIn, \
-        nrowsOut, ghat, ghat, mode, tw, twLen, norm, MXp, MYp); \
+    launch_k(fs ? k_cols<LL, true, true> : k_cols<LL, false, true>, (P.nkx + Col64<LL>::CB - 1) / Col64<LL>::CB, \
+             Col64<LL>::NT, Col64<LL>::SMEM, st, P.spec, ny, P.nkx, ny, ny, P.ghat, nullptr, P.tCol, 0.0); \
+    return true;
+    CUP2D_FFT_LENGTHS(X)
+#undef X
+  }
+  return false;
+}
+
+// the columns of the Green's function to the multiplier
+bool cols_green(const Poisson& P, cudaStream_t st, double norm) {
+  switch (P.Lcol) {
+#define X(LL) case LL: \
+    launch_k(k_cols<LL, false, false>, (P.nkx + Col64<LL>::CB - 1) / Col64<LL>::CB, Col64<LL>::NT, \
+             Col64<LL>::SMEM, st, P.spec, P.MY, P.nkx, P.MY, 0, nullptr, P.ghat, P.tCol, norm); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -1250,22 +945,19 @@ bool cols(int L, cudaStream_t st, double2* data, int stride, int ncols, int nrow
 }
 
 template <int LL, int EC>
-void rows_c2r_e(cudaStream_t st, const double2* in, int inStride, int nrows, double* out, int outStride,
-                int ncolsOut, const double2* tw, int twLen, bool halfOut) {
-  const int grid = (nrows + Len<LL>::B - 1) / Len<LL>::B;
-  if (halfOut) launch_k(k_rows_c2r<LL, true, EC>, grid, Len<LL, EC>::NT, smem_for<LL>(), st,
-                        in, inStride, nrows, out, outStride, ncolsOut, tw, twLen);
-  else launch_k(k_rows_c2r<LL, false, EC>, grid, Len<LL, EC>::NT, smem_for<LL>(), st,
-                in, inStride, nrows, out, outStride, ncolsOut, tw, twLen);
+void rows_c2r_e(const Poisson& P, cudaStream_t st, double* out, int nx, int ny, bool halfOut) {
+  const int grid = (ny + Row64<LL, EC>::B - 1) / Row64<LL, EC>::B;
+  const auto k = halfOut ? k_rows_c2r<LL, true, EC> : k_rows_c2r<LL, false, EC>;
+  launch_k(k, grid, Row64<LL, EC>::NT, smem_row64<LL, EC>(), st, P.spec, ny, ny, out, nx, nx, P.tRow[EC == 16], P.tw,
+           P.twLen);
 }
 
 // e: elements per thread (8 or 16)
-bool rows_c2r(int L, cudaStream_t st, const double2* in, int inStride, int nrows, double* out, int outStride,
-              int ncolsOut, const double2* tw, int twLen, bool halfOut, int e) {
-  switch (L) {
+bool rows_c2r(const Poisson& P, cudaStream_t st, double* out, int nx, int ny, bool halfOut, int e) {
+  switch (P.Lrow) {
 #define X(LL) case LL: \
-    if (e == 8) rows_c2r_e<LL, 8>(st, in, inStride, nrows, out, outStride, ncolsOut, tw, twLen, halfOut); \
-    else rows_c2r_e<LL, 16>(st, in, inStride, nrows, out, outStride, ncolsOut, tw, twLen, halfOut); \
+    if (e == 8) rows_c2r_e<LL, 8>(P, st, out, nx, ny, halfOut); \
+    else rows_c2r_e<LL, 16>(P, st, out, nx, ny, halfOut); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -1273,58 +965,35 @@ bool rows_c2r(int L, cudaStream_t st, const double2* in, int inStride, int nrows
   return false;
 }
 
-bool rows_r2c32(int L, cudaStream_t st, const double* in, int inStride, int nrows, int ncolsIn,
-                float2* out, int outStride, const float2* tw, int twLen, FadeArgs fa, bool halfIn) {
-  switch (L) {
-#define X(LL) case LL: \
-    if (halfIn) launch_k(k_rows_r2c32<LL, true>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_ROWS32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outStride, tw, twLen, fa); \
-    else launch_k(k_rows_r2c32<LL, false>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_ROWS32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outStride, tw, twLen, fa); \
-    return true;
-    CUP2D_FFT_LENGTHS(X)
-#undef X
+// The pass tables of a transform (see radix_level) in device memory; E = 8
+// or 16 values per thread.
+// (c and s: cos and sin of -2 pi k / n.)
+double2* make_tables(int L, int E, const std::vector<long double>& c, const std::vector<long double>& s,
+                     cudaStream_t st) {
+  const int n = (int)c.size();
+  std::vector<double2> t;
+  for (int ns = 1; ns < L;) {
+    const int R = ns * E <= L ? E : L / ns;
+    if (ns > 1)
+      for (int h = 1; h < R; h *= 2)
+        for (int j = 0; j < ns * std::max(1, h / 2); j++) {
+          const int k = j * (n / (2 * h * ns));
+          const double ck = (double)c[k];
+          t.push_back(make_double2(ck, (double)(s[k] / ck)));
+        }
+    ns *= R;
   }
-  return false;
-}
-
-bool cols32(int L, cudaStream_t st, float2* data, int stride, int ncols, int nrowsIn, int nrowsOut,
-            const float* ghat, int mode, const float2* tw, int twLen, double norm, int MXp, int MYp) {
-  switch (L) {
-#define X(LL) case LL: \
-    if (mode == 0) launch_k(k_cols32<LL, true>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS32>::NT, \
-        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, stride, ncols, nrowsIn, nrowsOut, \
-        ghat, mode, tw, twLen, norm, MXp, MYp); \
-    else launch_k(k_cols32<LL, false>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS32>::NT, \
-        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, stride, ncols, nrowsIn, nrowsOut, \
-        ghat, mode, tw, twLen, norm, MXp, MYp); \
-    return true;
-    CUP2D_FFT_LENGTHS(X)
-#undef X
-  }
-  return false;
-}
-
-bool rows_c2r32(int L, cudaStream_t st, const float2* in, int inStride, int nrows, double* out, int outStride,
-                int ncolsOut, const float2* tw, int twLen, bool halfOut) {
-  switch (L) {
-#define X(LL) case LL: \
-    if (halfOut) launch_k(k_rows_c2r32<LL, true>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_C2R32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, out, outStride, ncolsOut, tw, twLen); \
-    else launch_k(k_rows_c2r32<LL, false>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_C2R32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, out, outStride, ncolsOut, tw, twLen); \
-    return true;
-    CUP2D_FFT_LENGTHS(X)
-#undef X
-  }
-  return false;
+  double2* d = nullptr;
+  if (cudaMalloc(&d, sizeof(double2) * std::max<size_t>(1, t.size())) != cudaSuccess) return nullptr;
+  if (!t.empty()) h2d_sync(d, t.data(), sizeof(double2) * t.size(), st);
+  return d;
 }
 
 bool dct_rows_fwd(int L, cudaStream_t st, const double* in, int Nx, int nrows, double* D,
-                  const double2* tw, int twLen, FadeArgs fa) {
+                  const double2* tab, const double2* tw, int twLen, FadeArgs fa) {
   switch (L) {
 #define X(LL) case LL: launch_k(k_dct_rows_fwd<LL>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL>::NT, \
-                  smem_for<LL>((size_t)Len<LL>::B * LL), st, in, Nx, nrows, D, Len<LL>::B, tw, twLen, fa); return true;
+                  smem_for<LL>((size_t)Len<LL>::B * LL), st, in, Nx, nrows, D, Len<LL>::B, tab, tw, twLen, fa); return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }
@@ -1332,11 +1001,11 @@ bool dct_rows_fwd(int L, cudaStream_t st, const double* in, int Nx, int nrows, d
 }
 
 bool dct_cols(int L, cudaStream_t st, double* D, int Nx, int Ny, const float* cx, const float* cy, double tol,
-              const double2* tw, int twLen) {
+              const double2* tab, const double2* tw, int twLen) {
   const int pairs = Nx / 2;
   switch (L) {
 #define X(LL) case LL: launch_k(k_dct_cols<LL>, (pairs + Len<LL>::B - 1) / Len<LL>::B, Len<LL>::NT, smem_for<LL>(), st,  \
-                  D, Nx, Ny, Len<LL>::B, cx, cy, tol, tw, twLen); return true;
+                  D, Nx, Ny, Len<LL>::B, cx, cy, tol, tab, tw, twLen); return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }
@@ -1344,10 +1013,10 @@ bool dct_cols(int L, cudaStream_t st, double* D, int Nx, int Ny, const float* cx
 }
 
 bool dct_rows_inv(int L, cudaStream_t st, const double* D, int Nx, int nrows, double* out,
-                  const double2* tw, int twLen) {
+                  const double2* tab, const double2* tw, int twLen) {
   switch (L) {
 #define X(LL) case LL: launch_k(k_dct_rows_inv<LL>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL>::NT, smem_for<LL>(), st,  \
-                  D, Nx, nrows, out, Len<LL>::B, tw, twLen); return true;
+                  D, Nx, nrows, out, Len<LL>::B, tab, tw, twLen); return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }
@@ -1403,24 +1072,33 @@ Poisson* poisson_create(Ctx& c) {
     P->Lrow = Nx;          // DCT of length Nx via a real FFT of length 2Nx
     P->Lcol = 2 * Ny;      // DCT of length Ny via a complex FFT of length 2Ny
   }
-  // the built-in choice, measured on B200 (forward rows of 4096 points: 115
-  // us with 16 elements per thread against 127 with 8; 1024 points: 17 us
-  // with 8 against 21; the inverse pass: 16 at both)
-  P->eR2C = P->Lrow >= 4096 ? 16 : 8;
+  // the built-in choice, measured on B200 (with the fade, as a step runs
+  // them): forward rows with 8 and with 16 values per thread take 10.9 and 12.3
+  // us at 512 points (512 x 256), 14.2 and 14.2 at 1024 (1024 x 512), 20.5 and
+  // 18.4 (1024 x 1024), 52.8 and 50.9 at 2048 (2048 x 2048), 87 and 77 at 4096;
+  // inverse rows 10.2 and 10.3, 12.2 and 10.8, 16.4 and 15.1, 54 and 55, 76
+  // and 66
+  P->eR2C = P->Lrow >= 1024 ? 16 : 8;
   P->eC2R = 16;
   if (!is_pow2(P->Lrow) || !is_pow2(P->Lcol) || P->Lrow < 16 || P->Lcol < 16 ||
       P->Lrow > 4096 || P->Lcol > 4096) { delete P; return nullptr; }   // shared-memory limit
   P->nkx = P->Lrow + 1;
   P->twLen = 4 * (P->Lrow > P->Lcol ? P->Lrow : P->Lcol);
   std::vector<double2> tw(P->twLen);
+  std::vector<long double> twc(P->twLen), tws(P->twLen);
   for (int k = 0; k < P->twLen; k++) {
     const long double a = -2.0L * 3.14159265358979323846264338327950288L * k / P->twLen;
-    tw[k] = make_double2((double)cosl(a), (double)sinl(a));
+    twc[k] = cosl(a);
+    tws[k] = sinl(a);
+    tw[k] = make_double2((double)twc[k], (double)tws[k]);
   }
   if (cudaMalloc(&P->tw, sizeof(double2) * P->twLen) != cudaSuccess) { delete P; return nullptr; }
   h2d_sync(P->tw, tw.data(), sizeof(double2) * P->twLen, c.stream);
+  if (!(P->tRow[0] = make_tables(P->Lrow, 8, twc, tws, c.stream)) ||
+      !(P->tRow[1] = make_tables(P->Lrow, 16, twc, tws, c.stream)) ||
+      !(P->tCol = make_tables(P->Lcol, 16, twc, tws, c.stream))) { poisson_destroy(P); return nullptr; }
   const size_t specRows = (size_t)P->Lcol;
-  if (cudaMalloc(&P->spec, sizeof(double2) * specRows * P->nkx) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+  if (cudaMalloc(&P->spec, sizeof(double2) * specRows * ((P->nkx + SPEC_K - 1) & ~(SPEC_K - 1))) != cudaSuccess) { poisson_destroy(P); return nullptr; }
   set_all_smem();
   if (!g_smemOk) { poisson_destroy(P); return nullptr; }
   if (P->type == CUP2D_POISSON_COSINE) {
@@ -1433,16 +1111,18 @@ Poisson* poisson_create(Ctx& c) {
     h2d_sync(P->cosX, cx.data(), sizeof(float) * Nx, c.stream);
     h2d_sync(P->cosY, cy.data(), sizeof(float) * Ny, c.stream);
   }
+  if (P->type != CUP2D_POISSON_COSINE &&
+      cudaMalloc(&P->ghat, sizeof(double) * (P->Lcol / 2 + 1) * P->nkx) != cudaSuccess) { poisson_destroy(P); return nullptr; }
   if (P->type == CUP2D_POISSON_FREESPACE) {
-    // G^ = Re FFT[G] / (MX MY) on the MY x MX padded grid, kept for ky <= MY/2
-    if (cudaMalloc(&P->ghat, sizeof(double) * (P->Lcol / 2 + 1) * P->nkx) != cudaSuccess) { poisson_destroy(P); return nullptr; }
-    FadeArgs fa{}; fa.enabled = 0;
+    // G^ = Re FFT[G] / (MX MY) on the MY x MX padded grid, kept for ky <= MY/2;
+    // a quarter of norm: twice the spectrum comes in here and in the solve
     // (always with 8 elements per thread: G^ does not depend on the tuning)
-    rows_r2c(P->Lrow, c.stream, nullptr, 0, P->MY, P->MX, 1, P->spec, P->nkx, P->tw, P->twLen, fa, c.g.h,
-             P->MX, P->MY, false, 8);
+    rows_green(*P, c.stream, c.g.h);
     CUP2D_LAUNCHED(c);
-    const double norm = 1.0 / ((double)P->MX * (double)P->MY);
-    cols(P->Lcol, c.stream, P->spec, P->nkx, P->nkx, P->MY, P->Lcol / 2 + 1, P->ghat, 1, P->tw, P->twLen, norm, 0, 0);
+    cols_green(*P, c.stream, 0.25 / ((double)P->MX * (double)P->MY));
+    CUP2D_LAUNCHED(c);
+  } else if (P->type == CUP2D_POISSON_PERIODIC) {
+    k_periodic_multiplier<<<4 * c.sms, 256, 0, c.stream>>>(P->ghat, P->nkx, Nx, Ny, 1.0 / ((double)Nx * (double)Ny));
     CUP2D_LAUNCHED(c);
   }
   if (c.cfg.precision == CUP2D_PREC_FP32) {
@@ -1459,7 +1139,9 @@ Poisson* poisson_create(Ctx& c) {
       if (cudaStreamSynchronize(c.stream) != cudaSuccess ||
           cudaMemcpy(g64.data(), P->ghat, sizeof(double) * ng, cudaMemcpyDeviceToHost) != cudaSuccess ||
           cudaMalloc(&P->ghat32, sizeof(float) * ng) != cudaSuccess) { poisson_destroy(P); return nullptr; }
-      for (size_t i = 0; i < ng; i++) g32[i] = (float)g64[i];
+      const size_t gn = (size_t)P->Lcol / 2 + 1;
+      for (size_t k = 0; k < (size_t)P->nkx; k++)
+        for (size_t r = 0; r < gn; r++) g32[r * P->nkx + k] = (float)(2 * g64[k * gn + r]);
       h2d_sync(P->ghat32, g32.data(), sizeof(float) * ng, c.stream);
     }
   }
@@ -1470,6 +1152,7 @@ void poisson_destroy(Poisson* P) {
   if (!P) return;
   cudaFree(P->spec); cudaFree(P->ghat); cudaFree(P->tw); cudaFree(P->cosX); cudaFree(P->cosY);
   cudaFree(P->tw32); cudaFree(P->ghat32);
+  cudaFree(P->tRow[0]); cudaFree(P->tRow[1]); cudaFree(P->tCol);
   delete P;
 }
 
@@ -1480,9 +1163,14 @@ void poisson_rows_fwd(Ctx& c) {
   Poisson* P = c.poisson;
   const int Nx = c.g.nx, Ny = c.g.ny;
   FadeArgs fa{c.solveNoFade ? 0 : 1, c.dsc, c.g, c.rhs, fade_partials(c), c.nfade,
-              (int)(c.g.fadeLenX / c.g.h) + 2, (int)(c.g.fadeLenY / c.g.h) + 2};
+              (int)(c.g.fadeLenX / c.g.h) + 2, (int)(c.g.fadeLenY / c.g.h) + 2, 0};
+  if (fa.enabled && c.nfade > FADE_IN_PLACE) {
+    fa.ready = 1;
+    launch_k(k_fade_corr, 1, 32, 0, c.stream, fa);
+    CUP2D_LAUNCHED(c);
+  }
   if (P->type == CUP2D_POISSON_COSINE) {
-    dct_rows_fwd(P->Lrow, c.stream, c.rhs, Nx, Ny, reinterpret_cast<double*>(P->spec), P->tw, P->twLen, fa);
+    dct_rows_fwd(P->Lrow, c.stream, c.rhs, Nx, Ny, reinterpret_cast<double*>(P->spec), P->tRow[1], P->tw, P->twLen, fa);
     CUP2D_LAUNCHED(c);
     return;
   }
@@ -1491,8 +1179,7 @@ void poisson_rows_fwd(Ctx& c) {
     rows_r2c32(P->Lrow, c.stream, c.rhs, Nx, Ny, Nx, reinterpret_cast<float2*>(P->spec), P->nkx, P->tw32,
                P->twLen, fa, P->type == CUP2D_POISSON_FREESPACE);
   else
-    rows_r2c(P->Lrow, c.stream, c.rhs, Nx, Ny, Nx, 0, P->spec, P->nkx, P->tw, P->twLen, fa, c.g.h, P->MX, P->MY,
-             P->type == CUP2D_POISSON_FREESPACE, P->eR2C);
+    rows_r2c(*P, c.stream, c.rhs, Nx, Ny, fa, P->type == CUP2D_POISSON_FREESPACE, P->eR2C);
   CUP2D_LAUNCHED(c);
 }
 
@@ -1500,20 +1187,20 @@ void poisson_cols(Ctx& c) {
   Poisson* P = c.poisson;
   const int Nx = c.g.nx, Ny = c.g.ny;
   if (P->type == CUP2D_POISSON_COSINE) {
-    dct_cols(P->Lcol, c.stream, reinterpret_cast<double*>(P->spec), Nx, Ny, P->cosX, P->cosY, P->tol, P->tw, P->twLen);
+    dct_cols(P->Lcol, c.stream, reinterpret_cast<double*>(P->spec), Nx, Ny, P->cosX, P->cosY, P->tol, P->tCol, P->tw, P->twLen);
   } else if (P->type == CUP2D_POISSON_FREESPACE) {
     if (P->fp32)
       cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), P->nkx, P->nkx, Ny, Ny, P->ghat32, 0,
              P->tw32, P->twLen, 0.0, 0, 0);
     else
-      cols(P->Lcol, c.stream, P->spec, P->nkx, P->nkx, Ny, Ny, P->ghat, 0, P->tw, P->twLen, 0.0, 0, 0);
+      cols(*P, c.stream, Ny, true);
   } else {
     const double norm = 1.0 / ((double)Nx * (double)Ny);
     if (P->fp32)
       cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), P->nkx, P->nkx, Ny, Ny, nullptr, 2,
              P->tw32, P->twLen, norm, Nx, Ny);
     else
-      cols(P->Lcol, c.stream, P->spec, P->nkx, P->nkx, Ny, Ny, nullptr, 2, P->tw, P->twLen, norm, Nx, Ny);
+      cols(*P, c.stream, Ny, false);
   }
   CUP2D_LAUNCHED(c);
 }
@@ -1522,7 +1209,7 @@ void poisson_rows_inv(Ctx& c) {
   Poisson* P = c.poisson;
   const int Nx = c.g.nx, Ny = c.g.ny;
   if (P->type == CUP2D_POISSON_COSINE) {
-    dct_rows_inv(P->Lrow, c.stream, reinterpret_cast<const double*>(P->spec), Nx, Ny, c.pres, P->tw, P->twLen);
+    dct_rows_inv(P->Lrow, c.stream, reinterpret_cast<const double*>(P->spec), Nx, Ny, c.pres, P->tRow[1], P->tw, P->twLen);
     CUP2D_LAUNCHED(c);
     return;
   }
@@ -1530,8 +1217,7 @@ void poisson_rows_inv(Ctx& c) {
     rows_c2r32(P->Lrow, c.stream, reinterpret_cast<const float2*>(P->spec), P->nkx, Ny, c.pres, Nx, Nx,
                P->tw32, P->twLen, P->type == CUP2D_POISSON_FREESPACE);
   else
-    rows_c2r(P->Lrow, c.stream, P->spec, P->nkx, Ny, c.pres, Nx, Nx, P->tw, P->twLen,
-             P->type == CUP2D_POISSON_FREESPACE, P->eC2R);        // free space keeps the first half
+    rows_c2r(*P, c.stream, c.pres, Nx, Ny, P->type == CUP2D_POISSON_FREESPACE, P->eC2R);        // free space keeps the first half
   CUP2D_LAUNCHED(c);
 }
 
@@ -1584,11 +1270,10 @@ cudaError_t poisson_autotune(Ctx& c) {
   for (int q = 0; q < 2; q++) {
     const int e = q ? 16 : 8;
     P->tuneUs[q] = median_us(c.stream, [&] {
-      rows_r2c(P->Lrow, c.stream, c.rhs, Nx, Ny, Nx, 0, P->spec, P->nkx, P->tw, P->twLen, fa, c.g.h, P->MX,
-               P->MY, fs, e);
+      rows_r2c(*P, c.stream, c.rhs, Nx, Ny, fa, fs, e);
     });
     P->tuneUs[2 + q] = median_us(c.stream, [&] {
-      rows_c2r(P->Lrow, c.stream, P->spec, P->nkx, Ny, c.pres, Nx, Nx, P->tw, P->twLen, fs, e);
+      rows_c2r(*P, c.stream, c.pres, Nx, Ny, fs, e);
     });
   }
   const cudaError_t err = cudaGetLastError();
