@@ -43,7 +43,7 @@ struct Poisson {
   double2* spec = nullptr;   // the half spectrum: FP64 in column pairs (spec_at), FP32 [Lcol rows][nkx]
   // FP64: the column pass's multiplier [nkx][Lcol/2 + 1], the free-space
   // kernel or the periodic -1/|k|^2, halved (r2c_split writes twice the
-  // spectrum); a column's values are consecutive
+  // spectrum); cosine: its multiplier [Nx][Ny]; a column's values are consecutive
   double* ghat = nullptr;
   double2* tw = nullptr;     // exp(-2 pi i k / twLen)
   int twLen = 0;
@@ -674,189 +674,231 @@ k_rows_c2r(const double2* __restrict__ in, int inRows, int nrows, double* __rest
 }
 
 // ---- cosine-transform solver (FFTW_dirichlet.h:30-130) --------------------
-// DCT-II (FFTW REDFT10, Y_k = 2 sum x_j cos(pi (j+1/2) k / n)) is the real
-// FFT of the even extension y = [x, reversed x] of length 2n:
-// Y_k = exp(-i pi k / 2n) FFT_2n(y)_k.  DCT-III (REDFT01,
-// x'_m = Y_0 + 2 sum_{k>=1} Y_k cos(pi k (m+1/2) / n)) is the inverse real FFT
-// of length 2n of Z_k = exp(+i pi k / 2n) Y_k (Z_n = 0), first n outputs.
+// DCT-II (FFTW REDFT10, C_k = 2 sum x_j cos(pi (j+1/2) k / n)) by an FFT of
+// length n (Makhoul 1980): v = (x_0, x_2, ..., x_5, x_3, x_1), V = FFT_n(v), and
+// with w = exp(-i pi / 2n), 2 w^k V_k = C_k - i C_(n-k).  DCT-III (REDFT01,
+// x_m = Y_0 + 2 sum_{k>=1} Y_k cos(pi k (m+1/2) / n)) is its inverse times 2n:
+// v = unnormalised inverse FFT of conj(w^k) (Y_k - i Y_(n-k)), Y_n = 0.  The
+// FFT of the even extension, twice as long, had twice the work and smem.
+// A real row of n = 2L values is a complex FFT of length L as in k_rows_r2c;
+// two real columns are one complex FFT of length Ny.  The spectrum lies as
+// the other solvers' (spec_at, entry (r, p) = columns 2p and 2p + 1).
+// B200, forward rows, columns, inverse rows (events around a launch, about 7 us of
+// them launch): 512 x 256 14.1, 12.3, 12.4 us (21.5, 17.9, 12.3 before);
+// 4096 x 2048 69, 87, 80 us (211, 188, 88 before).
 
-// rows: fade on load, DCT-II along x into D (real, Ny x Nx); L = Nx
-template <int L>
-__global__ void __launch_bounds__(Len<L>::NT, Len<L>::MINB)
-k_dct_rows_fwd(const double* in, int Nx, int nrows, double* __restrict__ D, int rb,
-               const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen, FadeArgs fa)
+// one real value of the spectrum
+__device__ __forceinline__ size_t dct_at(int rows, int r, int c) { return 2 * spec_at(rows, r, c >> 1) + (c & 1); }
+
+// values per thread of the cosine solver's row passes
+template <int L> constexpr int dct_e() { return L >= 1024 ? 16 : 8; }
+
+// rows: fade on load, DCT-II along x of n = 2L values into D
+template <int L, int E>
+__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+k_dct_rows_fwd(const double* in, int nrows, double* __restrict__ D, const double2* __restrict__ tab,
+               const double2* __restrict__ tw, int twLen, FadeArgs fa)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_FWD);
-  constexpr int SL = Len<L>::SL;
+  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B, NT = Row64<L, E>::NT, n = 2 * L, H = L / 2;
+  constexpr int PER = (RB * H + NT - 1) / NT;
   extern __shared__ double2 sm[];
   double2* A = sm;
-  double* Bx = reinterpret_cast<double*>(sm + rb * SL + tab_staged<L, 16>());     // staged real row values
   __shared__ double sCorr;
-  if (fa.enabled) fade_corr_cta(fa, &sCorr);
-  const Tab tb = stage_tables<L, 16>(sm + rb * SL, tab);
-  cp_async_commit();
-  const int row0 = blockIdx.x * rb;
-  const int nb = min(rb, nrows - row0);
-  __syncthreads();
-  const double corr = fa.enabled ? sCorr : 0.0;
-  const int bandX = fa.enabled ? fa.bandX : 0;
-  const int bandY = fa.enabled ? fa.bandY : 0;
-  // faded row values, then the even extension y[j] = x[j] (j < n), x[2n-1-j]
-  for (int idx = threadIdx.x; idx < nb * L; idx += blockDim.x) {
-    const int r = idx / L, col = idx - r * L, row = row0 + r;
-    double v = in[(size_t)row * Nx + col];
-    if (fa.enabled && (row < bandY || row >= fa.g.ny - bandY || col < bandX || col >= fa.g.nx - bandX)) {
-      v = fade_cell(fade_row(fa.g, row), fade_col(fa.g, col), v, corr);
-      fa.writeback[(size_t)row * Nx + col] = v;
+  const int row0 = blockIdx.x * RB;
+  const int nb = min(RB, nrows - row0);
+  // x[4m .. 4m+3] are v's pairs m and L - 1 - m
+  double2 x0[PER], x1[PER];
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const int idx = threadIdx.x + u * NT, r = idx / H, m = idx % H;
+    x0[u] = x1[u] = make_double2(0, 0);
+    if (r < nb) {
+      const double2* src = reinterpret_cast<const double2*>(in + (size_t)(row0 + r) * n + 4 * m);
+      x0[u] = src[0];
+      x1[u] = src[1];
     }
-    Bx[r * L + col] = v;
   }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < nb * L; idx += blockDim.x) {
-    const int r = idx / L, n = idx - r * L;
-    const int j0 = 2 * n, j1 = 2 * n + 1;
-    const double y0 = Bx[r * L + (j0 < L ? j0 : 2 * L - 1 - j0)];
-    const double y1 = Bx[r * L + (j1 < L ? j1 : 2 * L - 1 - j1)];
-    A[r * SL + pad(n)] = make_double2(y0, y1);
-  }
+  if (fa.enabled) fade_corr_cta(fa, &sCorr);
+  const Tab tb = stage_tables<L, E>(sm + RB * SL, tab);
+  cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
-  const int sq = threadIdx.x / (L / 16), js = threadIdx.x % (L / 16);
-  fft_inplace<L, false>(A + sq * SL, sq < nb, js, tb);
-  double2* Z = A;
-  const int st2 = twLen / (2 * L), st4 = twLen / (4 * L);
-  // four iterations' global loads in flight before the first store
-#pragma unroll 4
-  for (int idx = threadIdx.x; idx < nb * L; idx += blockDim.x) {
-    const int r = idx / L, k = idx - r * L;
-    const double2 Zk = Z[r * SL + pad(k)];
-    const double2 Zc = conjg(Z[r * SL + pad(k == 0 ? 0 : L - k)]);
-    const double2 Fe = make_double2(0.5 * (Zk.x + Zc.x), 0.5 * (Zk.y + Zc.y));
-    const double2 d = csub(Zk, Zc);
-    const double2 Fo = make_double2(0.5 * d.y, -0.5 * d.x);
-    const double2 X = cadd(Fe, cmul(tw[k * st2], Fo));          // FFT_2n(y)_k
-    const double2 Y = cmul(tw[k * st4], X);                     // exp(-i pi k/2n) X_k
-    D[(size_t)(row0 + r) * Nx + k] = Y.x;
+  const int bandX = fa.enabled ? fa.bandX : 0, bandY = fa.enabled ? fa.bandY : 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const int idx = threadIdx.x + u * NT, r = idx / H, m = idx % H, row = row0 + r;
+    if (r >= nb) continue;
+    if (fa.enabled) {
+      const bool rowBand = row < bandY || row >= fa.g.ny - bandY;
+      if (rowBand || 4 * m < bandX || 4 * m + 3 >= n - bandX) {
+        const double rowFade = fade_row(fa.g, row);
+        double v[4] = {x0[u].x, x0[u].y, x1[u].x, x1[u].y};
+        for (int q = 0; q < 4; q++) {
+          const int col = 4 * m + q;
+          if (!(rowBand || col < bandX || col >= n - bandX)) continue;
+          v[q] = fade_cell(rowFade, fade_col(fa.g, col), v[q], sCorr);
+          fa.writeback[(size_t)row * n + col] = v[q];
+        }
+        x0[u] = make_double2(v[0], v[1]);
+        x1[u] = make_double2(v[2], v[3]);
+      }
+    }
+    A[r * SL + pad(m)] = make_double2(x0[u].x, x1[u].x);
+    A[r * SL + pad(L - 1 - m)] = make_double2(x1[u].y, x0[u].y);
+  }
+  __syncthreads();
+  const int sq = threadIdx.x / (L / E), j = threadIdx.x % (L / E);
+  fft_inplace<L, false, false, false, E>(A + sq * SL, sq < nb, j, tb);
+  // the real-FFT split (r2c_split), then C_k and C_(n-k) of k and of L - k
+  constexpr int KPT = (H + NT - 1) / NT;
+  const int st2 = twLen / (2 * L), st8 = twLen / (8 * L);
+  auto put = [&](int r, int k, double2 z) {            // z = 2 w^k V_k
+    D[dct_at(nrows, row0 + r, k)] = z.x;
+    if (k != 0 && k != L) D[dct_at(nrows, row0 + r, n - k)] = -z.y;
+  };
+  if (threadIdx.x < nb) {
+    const double2 z = A[threadIdx.x * SL + pad(H)];
+    put(threadIdx.x, H, cmul(tw[H * st8], make_double2(2 * z.x, -2 * z.y)));
+  }
+#pragma unroll
+  for (int q = 0; q < KPT; q++) {
+    const int k = threadIdx.x + q * NT;
+    if (k >= H) break;                                  // k grows with q
+    const double2 w = tw[k * st2], wk = tw[k * st8], wl = tw[(L - k) * st8];
+    for (int r = 0; r < nb; r++) {
+      const double2 Za = A[r * SL + pad(k)], Zb = conjg(A[r * SL + pad(k == 0 ? 0 : L - k)]);
+      const double2 Fe = cadd(Za, Zb), d = csub(Za, Zb), t = cmul(w, make_double2(d.y, -d.x));
+      put(r, k, cmul(wk, cadd(Fe, t)));
+      put(r, L - k, cmul(wl, conjg(csub(Fe, t))));
+    }
   }
 }
 
-// columns, two per complex FFT of length L = 2 Ny: DCT-II along y, the
-// multiplier of FFTW_dirichlet::_solve (FFTW_dirichlet.h:49-61), DCT-III.
+// columns, two per complex FFT of length L = Ny: DCT-II along y, the
+// multiplier M[column][k] of FFTW_dirichlet::_solve, DCT-III
 template <int L>
-__global__ void __launch_bounds__(Len<L>::NT, Len<L>::MINB)
-k_dct_cols(double* D, int Nx, int Ny, int cb, const float* __restrict__ cosX, const float* __restrict__ cosY,
-           double tol, const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen)
+__global__ void __launch_bounds__(Col64<L>::NT, Col64<L>::MINB)
+k_dct_cols(double2* D, int npairs, const double* __restrict__ M, const double2* __restrict__ tab,
+           const double2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_COLS);
-  constexpr int SL = Len<L>::SL;
+  using P = Col64<L>;
+  constexpr int CB = P::CB, T = L / 16, H = L / 2;
   extern __shared__ double2 sm[];
-  double2* A = sm;
-  const Tab tb = stage_tables<L, 16>(sm + cb * SL, tab);
+  const int p0 = blockIdx.x * CB;
+  const int nb = min(CB, npairs - p0);
+  const Tab tb = stage_tables<L, 16>(sm + CB * P::SL, tab);
   cp_async_commit();
-  const int n = Ny;                                   // L = 2n
-  const int c0 = blockIdx.x * cb * 2;                 // first column of this CTA
-  const int np = min(cb, (Nx - c0) / 2);              // column pairs
-  for (int idx = threadIdx.x; idx < np * L; idx += blockDim.x) {
-    const int j = idx / np, q = idx - j * np;         // j: extended row index
-    const int row = j < n ? j : 2 * n - 1 - j;
-    const double2 ab = *reinterpret_cast<const double2*>(D + (size_t)row * Nx + c0 + 2 * q);
-    A[q * SL + pad(j)] = ab;                          // a + i b
-  }
-  cp_async_wait<0>();
+  const int sq = threadIdx.x % CB, j = threadIdx.x / CB;
+  const bool act = sq < nb && j < T;
+  double2* a = sm + sq * P::SL;
+  const int p = p0 + sq;
+  auto rowOf = [](int i) { return i < H ? 2 * i : 2 * L - 2 * i - 1; };     // of v's entry i
+  fft_first_pass_global<L, false, 16>(a, act, j, tb, [&](int i) { return D[spec_at(L, rowOf(i), p)]; },
+                                      [&]() { cp_async_wait<0>(); }, [](int, double2 v) { return v; });
   __syncthreads();
-  const int sq = threadIdx.x / (L / 16), js = threadIdx.x % (L / 16);
-  fft_inplace<L, false>(A + sq * SL, sq < np, js, tb);
-  double2* Z = A;
-  // each thread reads the pair (k, L-k) before writing the same pair, and
-  // slot n is read by none, so the inverse input overwrites Z in place
-  double2* W = Z;
-  const int st4 = twLen / (2 * L);                    // exp(-i pi k/2n) = tw[k twLen/(4n)]
-  const double MX = Nx, MY = Ny;
-  const double waveFactX = M_PI / MX, waveFactY = M_PI / MY;
-  const double norm_factor = 0.25 / (MX * MY);
-  // separate the two real columns, DCT-II values, multiplier, then the
-  // Hermitian spectra of both DCT-III inputs packed as Za + i Zb
-#pragma unroll 4
-  for (int idx = threadIdx.x; idx < np * n; idx += blockDim.x) {
-    const int q = idx / n, k = idx - q * n;
-    const double2 Zk = Z[q * SL + pad(k)];
-    const double2 Zc = conjg(Z[q * SL + pad(k == 0 ? 0 : L - k)]);
-    const double2 Ak = make_double2(0.5 * (Zk.x + Zc.x), 0.5 * (Zk.y + Zc.y));     // FFT of a
-    const double2 dd = csub(Zk, Zc);
-    const double2 Bk = make_double2(0.5 * dd.y, -0.5 * dd.x);                      // FFT of b
-    const double2 w = tw[k * st4];
-    double ya = cmul(w, Ak).x, yb = cmul(w, Bk).x;                                 // DCT-II
-    for (int e = 0; e < 2; e++) {
-      const int i = c0 + 2 * q + e, jj = k;
-      const double rkx = (i + 0.5) * waveFactX, rky = (jj + 0.5) * waveFactY;
-      const float denomF = 1 - cosX[i] / 2 - cosY[jj] / 2;                         // float, as written
-      const double denomFD = denomF;
-      const double denomSP = rkx * rkx + rky * rky;
-      double& y = e == 0 ? ya : yb;
-      y *= -norm_factor / ((1 - tol) * denomFD + tol * denomSP);
-      if (i == 0 && jj == 0) y = 0;                                                // in_out[0] = 0
-    }
-    // Z_k = exp(+i pi k/2n) Y_k for both columns, packed
+  fft_passes<L, 16, false, false, false, 16>(a, act, j, tb);
+  // per pair (k, L - k): the columns' transforms apart, DCT-II values,
+  // multiplier, and the packed input of the inverse in the same two slots
+  const int st4 = twLen / (4 * L);
+  auto turn = [&](int k, double2 w, double2 mk, double2 ml) {
+    const double2 Zk = a[pad(k)], Zl = conjg(a[pad(k == 0 ? 0 : L - k)]);
+    const double2 d = csub(Zk, Zl);
+    const double2 za = cmul(w, cadd(Zk, Zl)), zb = cmul(w, make_double2(d.y, -d.x));
     const double2 wc = conjg(w);
-    const double2 za = make_double2(wc.x * ya, wc.y * ya), zb = make_double2(wc.x * yb, wc.y * yb);
-    W[q * SL + pad(k)] = make_double2(za.x - zb.y, za.y + zb.x);                     // za + i zb
-    if (k > 0) {   // k' = 2n - k: conj(za) + i conj(zb)
-      W[q * SL + pad(L - k)] = make_double2(za.x + zb.y, -za.y + zb.x);
+    const double2 va = cmul(wc, make_double2(za.x * mk.x, k == 0 ? 0.0 : za.y * ml.x));
+    const double2 vb = cmul(wc, make_double2(zb.x * mk.y, k == 0 ? 0.0 : zb.y * ml.y));
+    a[pad(k)] = make_double2(va.x - vb.y, va.y + vb.x);
+    if (k != 0 && k != H) a[pad(L - k)] = make_double2(va.x + vb.y, vb.x - va.y);
+  };
+  if (act) {
+    const double *Ma = M + (size_t)(2 * p) * L, *Mb = Ma + L;
+#pragma unroll 4
+    for (int q = 0; q < 8; q++) {
+      const int k = j + q * T, l = k == 0 ? 0 : L - k;
+      turn(k, tw[k * st4], make_double2(Ma[k], Mb[k]), make_double2(Ma[l], Mb[l]));
+    }
+    if (j == 0) {
+      const double2 m = make_double2(Ma[H], Mb[H]);
+      turn(H, tw[H * st4], m, m);
     }
   }
-  for (int q = threadIdx.x; q < np; q += blockDim.x) W[q * SL + pad(n)] = make_double2(0, 0);
   __syncthreads();
-  fft_inplace<L, true, false, true>(W + sq * SL, sq < np, js, tb);          // outputs m < n = L/2
-  double2* Y = W;
-#pragma unroll 4
-  for (int idx = threadIdx.x; idx < np * n; idx += blockDim.x) {
-    const int m = idx / np, q = idx - m * np;
-    *reinterpret_cast<double2*>(D + (size_t)m * Nx + c0 + 2 * q) = Y[q * SL + pad(m)];
+  constexpr int NSL = last_ns<L, 16>();
+  fft_passes_below<L, 1, NSL, true, false, 16>(a, act, j, tb);
+  fft_last_pass_global<L, L / NSL, NSL, false, 16>(a, act, j, tb,
+                                                   [&](int i, double2 v) { D[spec_at(L, rowOf(i), p)] = v; });
+}
+
+// the multiplier of FFTW_dirichlet::_solve (FFTW_dirichlet.h:49-61), its
+// denominator in float where the reference's is
+__global__ void k_dct_multiplier(double* __restrict__ M, int Nx, int Ny, const float* __restrict__ cosX,
+                                 const float* __restrict__ cosY, double tol) {
+  const double MX = Nx, MY = Ny;
+  const double waveFactX = M_PI / MX, waveFactY = M_PI / MY, norm_factor = 0.25 / (MX * MY);
+  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < (size_t)Nx * Ny;
+       idx += (size_t)gridDim.x * blockDim.x) {
+    const int i = (int)(idx / Ny), jj = (int)(idx % Ny);
+    const double rkx = (i + 0.5) * waveFactX, rky = (jj + 0.5) * waveFactY;
+    const float denomF = 1 - cosX[i] / 2 - cosY[jj] / 2;                         // float, as written
+    const double denomFD = denomF;
+    const double denomSP = rkx * rkx + rky * rky;
+    M[idx] = idx == 0 ? 0.0 : -norm_factor / ((1 - tol) * denomFD + tol * denomSP);   // in_out[0] = 0
   }
 }
 
-// rows: DCT-III along x from D into p; L = Nx
-template <int L>
-__global__ void __launch_bounds__(Len<L>::NT, Len<L>::MINB)
-k_dct_rows_inv(const double* __restrict__ D, int Nx, int nrows, double* __restrict__ out, int rb,
-               const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen)
+// rows: DCT-III along x from D into p, n = 2L values
+template <int L, int E>
+__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+k_dct_rows_inv(const double* __restrict__ D, int nrows, double* __restrict__ out, const double2* __restrict__ tab,
+               const double2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_INV);
-  constexpr int SL = Len<L>::SL;
+  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B, NT = Row64<L, E>::NT, n = 2 * L, H = L / 2;
+  constexpr int KPT = (H + NT - 1) / NT;
   extern __shared__ double2 sm[];
   double2* A = sm;
-  const Tab tb = stage_tables<L, 16>(sm + rb * SL, tab);
+  const Tab tb = stage_tables<L, E>(sm + RB * SL, tab);
   cp_async_commit();
-  const int row0 = blockIdx.x * rb;
-  const int nb = min(rb, nrows - row0);
-  const int st2 = twLen / (2 * L), st4 = twLen / (4 * L);
-  // four iterations' global loads in flight before the first store
-#pragma unroll 4
-  for (int idx = threadIdx.x; idx < nb * L; idx += blockDim.x) {
-    const int r = idx / L, k = idx - r * L;
-    const double* Yr = D + (size_t)(row0 + r) * Nx;
-    // X_k = exp(i pi k/2n) Y_k, X_n = 0; then the c2r combination of k_rows_c2r
-    const double2 wk = conjg(tw[k * st4]);
-    double2 Xk = make_double2(wk.x * Yr[k], wk.y * Yr[k]);
-    double2 XL = make_double2(0, 0);
-    if (k > 0) { const double2 wl = conjg(tw[(L - k) * st4]); XL = make_double2(wl.x * Yr[L - k], wl.y * Yr[L - k]); }
-    if (k == 0) { Xk.y = 0; XL.y = 0; }
-    const double2 Xc = conjg(XL);
-    const double2 s = cadd(Xk, Xc), d = csub(Xk, Xc);
-    const double2 t = cmul(conjg(tw[k * st2]), d);
-    A[r * SL + pad(k)] = make_double2(s.x - t.y, s.y + t.x);
+  const int row0 = blockIdx.x * RB;
+  const int nb = min(RB, nrows - row0);
+  const int st2 = twLen / (2 * L), st8 = twLen / (8 * L);
+  auto get = [&](int r, int k) { return D[dct_at(nrows, row0 + r, k)]; };
+  // X_k = conj(w^k) (Y_k - i Y_(n-k)), then the merge of k_rows_c2r
+#pragma unroll
+  for (int q = 0; q < KPT; q++) {
+    const int k = threadIdx.x + q * NT;
+    if (k >= H) break;
+    const double2 w = conjg(tw[k * st2]), wk = conjg(tw[k * st8]), wl = conjg(tw[(L - k) * st8]);
+#pragma unroll
+    for (int r = 0; r < RB; r++) {
+      if (r >= nb) break;
+      const double2 Xk = cmul(wk, make_double2(get(r, k), k == 0 ? 0.0 : -get(r, n - k)));
+      const double2 Xc = conjg(cmul(wl, make_double2(get(r, L - k), -get(r, L + k))));
+      const double2 s = cadd(Xk, Xc), t = cmul(w, csub(Xk, Xc));
+      double2* a = A + r * SL;
+      a[pad(k)] = make_double2(s.x - t.y, s.y + t.x);
+      if (k > 0) a[pad(L - k)] = make_double2(s.x + t.y, t.x - s.y);
+    }
+  }
+  if (threadIdx.x < nb) {
+    const double2 x = cmul(conjg(tw[H * st8]), make_double2(get(threadIdx.x, H), -get(threadIdx.x, n - H)));
+    A[threadIdx.x * SL + pad(H)] = make_double2(2 * x.x, -2 * x.y);
   }
   cp_async_wait<0>();
   __syncthreads();
-  const int sq = threadIdx.x / (L / 16), js = threadIdx.x % (L / 16);
-  fft_inplace<L, true, false, true>(A + sq * SL, sq < nb, js, tb);          // outputs m < L/2
-  double2* z = A;
-  for (int idx = threadIdx.x; idx < nb * (L / 2); idx += blockDim.x) {
-    const int r = idx / (L / 2), m = idx - r * (L / 2);
-    *reinterpret_cast<double2*>(out + (size_t)(row0 + r) * Nx + 2 * m) = z[r * SL + pad(m)];
+  const int sq = threadIdx.x / (L / E), j = threadIdx.x % (L / E);
+  fft_inplace<L, true, false, false, E>(A + sq * SL, sq < nb, j, tb);
+  for (int idx = threadIdx.x; idx < nb * H; idx += NT) {
+    const int r = idx / H, m = idx % H;
+    const double2 z = A[r * SL + pad(m)], y = A[r * SL + pad(L - 1 - m)];
+    double2* o = reinterpret_cast<double2*>(out + (size_t)(row0 + r) * n + 4 * m);
+    o[0] = make_double2(z.x, y.y);
+    o[1] = make_double2(z.y, y.x);
   }
 }
 
@@ -865,10 +907,8 @@ inline bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 bool g_smemOk = true;
 void set_smem(const void* f) { if (allow_max_dynamic_smem(f) != cudaSuccess) g_smemOk = false; }
 
-// B padded sequences, the staged twiddles, and extraReals doubles
-template <int L> inline size_t smem_for(size_t extraReals = 0) {
-  return sizeof(double2) * ((size_t)Len<L>::B * Len<L>::SL + tab_staged<L, 16>()) + sizeof(double) * extraReals;
-}
+// the cosine solver's column lengths: Ny >= 32
+#define CUP2D_DCT_LENGTHS(X) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048)
 
 void set_all_smem() {
 #define X(L) set_smem((const void*)k_rows_r2c<L, false, 8, false>); set_smem((const void*)k_rows_r2c<L, true, 8, false>); \
@@ -877,9 +917,12 @@ void set_all_smem() {
              set_smem((const void*)k_rows_c2r<L, false, 8>); set_smem((const void*)k_rows_c2r<L, true, 8>); \
              set_smem((const void*)k_rows_c2r<L, false, 16>); set_smem((const void*)k_rows_c2r<L, true, 16>); \
              set_smem((const void*)k_cols<L, false, true>); set_smem((const void*)k_cols<L, true, true>); \
-             set_smem((const void*)k_cols<L, false, false>); set_smem((const void*)k_dct_rows_fwd<L>); \
-             set_smem((const void*)k_dct_cols<L>); set_smem((const void*)k_dct_rows_inv<L>);
+             set_smem((const void*)k_cols<L, false, false>); set_smem((const void*)k_dct_rows_fwd<L, dct_e<L>()>); \
+             set_smem((const void*)k_dct_rows_inv<L, 16>);
   CUP2D_FFT_LENGTHS(X)
+#undef X
+#define X(L) set_smem((const void*)k_dct_cols<L>);
+  CUP2D_DCT_LENGTHS(X)
 #undef X
   if (!poisson32_setup()) g_smemOk = false;
 }
@@ -989,34 +1032,34 @@ double2* make_tables(int L, int E, const std::vector<long double>& c, const std:
   return d;
 }
 
-bool dct_rows_fwd(int L, cudaStream_t st, const double* in, int Nx, int nrows, double* D,
-                  const double2* tab, const double2* tw, int twLen, FadeArgs fa) {
-  switch (L) {
-#define X(LL) case LL: launch_k(k_dct_rows_fwd<LL>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL>::NT, \
-                  smem_for<LL>((size_t)Len<LL>::B * LL), st, in, Nx, nrows, D, Len<LL>::B, tab, tw, twLen, fa); return true;
+bool dct_rows_fwd(const Poisson& P, cudaStream_t st, const double* in, int ny, const FadeArgs& fa) {
+  switch (P.Lrow) {
+#define X(LL) case LL: { constexpr int E = dct_e<LL>(); \
+    launch_k(k_dct_rows_fwd<LL, E>, (ny + Row64<LL, E>::B - 1) / Row64<LL, E>::B, Row64<LL, E>::NT, \
+             smem_row64<LL, E>(), st, in, ny, reinterpret_cast<double*>(P.spec), P.tRow[E == 16], P.tw, P.twLen, fa); \
+    return true; }
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }
   return false;
 }
 
-bool dct_cols(int L, cudaStream_t st, double* D, int Nx, int Ny, const float* cx, const float* cy, double tol,
-              const double2* tab, const double2* tw, int twLen) {
-  const int pairs = Nx / 2;
-  switch (L) {
-#define X(LL) case LL: launch_k(k_dct_cols<LL>, (pairs + Len<LL>::B - 1) / Len<LL>::B, Len<LL>::NT, smem_for<LL>(), st,  \
-                  D, Nx, Ny, Len<LL>::B, cx, cy, tol, tab, tw, twLen); return true;
-    CUP2D_FFT_LENGTHS(X)
+bool dct_cols(const Poisson& P, cudaStream_t st, int nx) {
+  const int pairs = nx / 2;
+  switch (P.Lcol) {
+#define X(LL) case LL: launch_k(k_dct_cols<LL>, (pairs + Col64<LL>::CB - 1) / Col64<LL>::CB, Col64<LL>::NT, \
+                  Col64<LL>::SMEM, st, P.spec, pairs, P.ghat, P.tCol, P.tw, P.twLen); return true;
+    CUP2D_DCT_LENGTHS(X)
 #undef X
   }
   return false;
 }
 
-bool dct_rows_inv(int L, cudaStream_t st, const double* D, int Nx, int nrows, double* out,
-                  const double2* tab, const double2* tw, int twLen) {
-  switch (L) {
-#define X(LL) case LL: launch_k(k_dct_rows_inv<LL>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL>::NT, smem_for<LL>(), st,  \
-                  D, Nx, nrows, out, Len<LL>::B, tab, tw, twLen); return true;
+bool dct_rows_inv(const Poisson& P, cudaStream_t st, int ny, double* out) {
+  switch (P.Lrow) {
+#define X(LL) case LL: launch_k(k_dct_rows_inv<LL, 16>, (ny + Row64<LL, 16>::B - 1) / Row64<LL, 16>::B, \
+                  Row64<LL, 16>::NT, smem_row64<LL, 16>(), st, reinterpret_cast<const double*>(P.spec), ny, out, \
+                  P.tRow[1], P.tw, P.twLen); return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }
@@ -1069,8 +1112,8 @@ Poisson* poisson_create(Ctx& c) {
     P->Lrow = Nx / 2;      // real length Nx
     P->Lcol = Ny;
   } else {
-    P->Lrow = Nx;          // DCT of length Nx via a real FFT of length 2Nx
-    P->Lcol = 2 * Ny;      // DCT of length Ny via a complex FFT of length 2Ny
+    P->Lrow = Nx / 2;      // DCT of length Nx via a real FFT of length Nx
+    P->Lcol = Ny;          // DCT of length Ny via a complex FFT of length Ny
   }
   // the built-in choice, measured on B200 (with the fade, as a step runs
   // them): forward rows with 8 and with 16 values per thread take 10.9 and 12.3
@@ -1083,7 +1126,7 @@ Poisson* poisson_create(Ctx& c) {
   if (!is_pow2(P->Lrow) || !is_pow2(P->Lcol) || P->Lrow < 16 || P->Lcol < 16 ||
       P->Lrow > 4096 || P->Lcol > 4096) { delete P; return nullptr; }   // shared-memory limit
   P->nkx = P->Lrow + 1;
-  P->twLen = 4 * (P->Lrow > P->Lcol ? P->Lrow : P->Lcol);
+  P->twLen = 4 * std::max(P->type == CUP2D_POISSON_COSINE ? Nx : P->Lrow, P->Lcol);
   std::vector<double2> tw(P->twLen);
   std::vector<long double> twc(P->twLen), tws(P->twLen);
   for (int k = 0; k < P->twLen; k++) {
@@ -1097,8 +1140,11 @@ Poisson* poisson_create(Ctx& c) {
   if (!(P->tRow[0] = make_tables(P->Lrow, 8, twc, tws, c.stream)) ||
       !(P->tRow[1] = make_tables(P->Lrow, 16, twc, tws, c.stream)) ||
       !(P->tCol = make_tables(P->Lcol, 16, twc, tws, c.stream))) { poisson_destroy(P); return nullptr; }
-  const size_t specRows = (size_t)P->Lcol;
-  if (cudaMalloc(&P->spec, sizeof(double2) * specRows * ((P->nkx + SPEC_K - 1) & ~(SPEC_K - 1))) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+  const size_t specRows = (size_t)P->Lcol, ncols = P->type == CUP2D_POISSON_COSINE ? Nx / 2 : P->nkx;
+  if (cudaMalloc(&P->spec, sizeof(double2) * specRows * ((ncols + SPEC_K - 1) / SPEC_K * SPEC_K)) != cudaSuccess) {
+    poisson_destroy(P);
+    return nullptr;
+  }
   set_all_smem();
   if (!g_smemOk) { poisson_destroy(P); return nullptr; }
   if (P->type == CUP2D_POISSON_COSINE) {
@@ -1110,6 +1156,9 @@ Poisson* poisson_create(Ctx& c) {
         cudaMalloc(&P->cosY, sizeof(float) * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
     h2d_sync(P->cosX, cx.data(), sizeof(float) * Nx, c.stream);
     h2d_sync(P->cosY, cy.data(), sizeof(float) * Ny, c.stream);
+    if (cudaMalloc(&P->ghat, sizeof(double) * Nx * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+    k_dct_multiplier<<<4 * c.sms, 256, 0, c.stream>>>(P->ghat, Nx, Ny, P->cosX, P->cosY, P->tol);
+    CUP2D_LAUNCHED(c);
   }
   if (P->type != CUP2D_POISSON_COSINE &&
       cudaMalloc(&P->ghat, sizeof(double) * (P->Lcol / 2 + 1) * P->nkx) != cudaSuccess) { poisson_destroy(P); return nullptr; }
@@ -1170,7 +1219,7 @@ void poisson_rows_fwd(Ctx& c) {
     CUP2D_LAUNCHED(c);
   }
   if (P->type == CUP2D_POISSON_COSINE) {
-    dct_rows_fwd(P->Lrow, c.stream, c.rhs, Nx, Ny, reinterpret_cast<double*>(P->spec), P->tRow[1], P->tw, P->twLen, fa);
+    dct_rows_fwd(*P, c.stream, c.rhs, Ny, fa);
     CUP2D_LAUNCHED(c);
     return;
   }
@@ -1187,7 +1236,7 @@ void poisson_cols(Ctx& c) {
   Poisson* P = c.poisson;
   const int Nx = c.g.nx, Ny = c.g.ny;
   if (P->type == CUP2D_POISSON_COSINE) {
-    dct_cols(P->Lcol, c.stream, reinterpret_cast<double*>(P->spec), Nx, Ny, P->cosX, P->cosY, P->tol, P->tCol, P->tw, P->twLen);
+    dct_cols(*P, c.stream, Nx);
   } else if (P->type == CUP2D_POISSON_FREESPACE) {
     if (P->fp32)
       cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), P->nkx, P->nkx, Ny, Ny, P->ghat32, 0,
@@ -1209,7 +1258,7 @@ void poisson_rows_inv(Ctx& c) {
   Poisson* P = c.poisson;
   const int Nx = c.g.nx, Ny = c.g.ny;
   if (P->type == CUP2D_POISSON_COSINE) {
-    dct_rows_inv(P->Lrow, c.stream, reinterpret_cast<const double*>(P->spec), Nx, Ny, c.pres, P->tRow[1], P->tw, P->twLen);
+    dct_rows_inv(*P, c.stream, Ny, c.pres);
     CUP2D_LAUNCHED(c);
     return;
   }
