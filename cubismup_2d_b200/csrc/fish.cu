@@ -10,8 +10,7 @@
 //   (FishLibrary.cpp:86-159).  None of this depends on the flow or on the
 //   body's position, only on t, so the pipeline computes the midline of step
 //   n+1 on a side branch while step n runs (double buffer by step parity).
-//   The Frenet recurrence is serial in s; it runs on one thread with its
-//   inputs and outputs in shared memory.
+//   The Frenet recurrence runs as block scans over the arclength points.
 // k_fish_frame (one CTA per fish): changeToCoMFrameAngular with the current
 //   theta_internal (FishLibrary.cpp:161-176) and the AreaSegment boxes in the
 //   computational frame (Fish.cpp:118-150, FishLibrary.cpp:295-342).
@@ -48,6 +47,134 @@ __device__ __forceinline__ void cubic_interp(double x0, double x1, double x, dou
   const double d = y0;
   y = a * xrel * xrel * xrel + b * xrel * xrel + c * xrel + d;
   dy = 3 * a * xrel * xrel + 2 * b * xrel + c;
+}
+
+// Exclusive block scan (512 threads at most, one value of K doubles each,
+// thread order) with an associative op(double*, const double*): a becomes
+// a o b; e is its neutral element.  Shuffles within the warps, then every warp
+// scans the warps' totals for itself (one barrier; a second before sm, 16 K
+// doubles, is written again).
+template <int K, class Op>
+__device__ __forceinline__ void block_scan_excl(double (&x)[K], const double (&e)[K], double* sm, Op op) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  auto warp_incl = [&](double (&v)[K]) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      double y[K];
+#pragma unroll
+      for (int q = 0; q < K; q++) y[q] = __shfl_up_sync(0xffffffffu, v[q], o);
+      if (lane >= o) {
+        op(y, v);
+#pragma unroll
+        for (int q = 0; q < K; q++) v[q] = y[q];
+      }
+    }
+  };
+  warp_incl(x);
+  if (lane == 31)
+#pragma unroll
+    for (int q = 0; q < K; q++) sm[wid * K + q] = x[q];
+  __syncthreads();
+  double t[K];
+#pragma unroll
+  for (int q = 0; q < K; q++) t[q] = lane < nw ? sm[lane * K + q] : e[q];
+  warp_incl(t);
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    t[q] = __shfl_sync(0xffffffffu, t[q], (wid + 31) & 31);           // the warps before this one
+    if (wid == 0) t[q] = e[q];
+    x[q] = __shfl_up_sync(0xffffffffu, x[q], 1);
+    if (lane == 0) x[q] = e[q];
+  }
+  op(t, x);
+#pragma unroll
+  for (int q = 0; q < K; q++) x[q] = t[q];
+  __syncthreads();
+}
+template <int K> struct AddOp {
+  __device__ void operator()(double* a, const double* b) const {
+#pragma unroll
+    for (int q = 0; q < K; q++) a[q] += b[q];
+  }
+};
+// (unit complex number, modulus): their products
+struct TurnOp {
+  __device__ void operator()(double* a, const double* b) const {
+    const double x = a[0] * b[0] - a[1] * b[1];
+    a[1] = a[0] * b[1] + a[1] * b[0];
+    a[0] = x;
+    a[2] *= b[2];
+  }
+};
+
+// IF2D_Frenet2D::solve (FishUtilities.h:15-79) as scans.  Its step from point
+// i - 1 to i, with a = ds curv and b = ds curv_dt of point i - 1, is
+//   ksi_i = normalised(ksi + a nor), nor_i = normalised(nor - a ksi),
+//   vKsi_i = vKsi + a vNor + b nor, vNor_i = vNor - a vKsi - b ksi,
+//   r_i = r + ds ksi, v_i = v + ds vKsi,
+// from ksi = (1, 0), nor = (0, 1), the rest 0.  As complex numbers nor = i ksi
+// and vNor = i vKsi throughout, so with q = 1 + i a, ksi_i is the product of
+// the q / |q|, and vKsi_i = q_i vKsi_(i-1) + i b_i ksi_(i-1) is ksi_i M_i W_i
+// with M_i the product of the |q| and W_i the sum of i b_j ksi_(j-1)
+// conj(ksi_j) / M_j; r and v are sums.  Three scans (the turns; r and W; v)
+// instead of a chain of Nm dependent steps of some 450 cycles each: 337
+// points had taken 80 us on one thread, off the step's critical path only
+// while the step took longer than the midline.  Each thread takes a run of
+// consecutive steps.
+__device__ __forceinline__ void frenet_scan(int Nm, const double* rS, const double* curv, const double* curv_dt,
+                                            double* rX, double* rY, double* vX, double* vY, double* norX,
+                                            double* norY, double* vNorX, double* vNorY, double* sm) {
+  const int n = Nm - 1, per = (n + blockDim.x - 1) / blockDim.x;
+  const int i0 = 1 + min(n, (int)threadIdx.x * per), i1 = 1 + min(n, ((int)threadIdx.x + 1) * per);
+  auto turn = [&](int i, double (&q)[3]) {             // of step i: q / |q| and |q|
+    const double a = (rS[i] - rS[i - 1]) * curv[i - 1], m = sqrt(1 + a * a);
+    q[0] = 1 / m; q[1] = a / m; q[2] = m;
+  };
+  // ksi and M before this thread's steps
+  double K[3] = {1, 0, 1};
+  for (int i = i0; i < i1; i++) { double q[3]; turn(i, q); TurnOp()(K, q); }
+  const double one[3] = {1, 0, 1};
+  block_scan_excl<3>(K, one, sm, TurnOp());
+  // the thread's sums of r and W; ksi_i goes to nor, M_i W_i's parts to vNor
+  double Q[4] = {0, 0, 0, 0};
+  {
+    double k[3] = {K[0], K[1], K[2]};
+    for (int i = i0; i < i1; i++) {
+      const double ds = rS[i] - rS[i - 1], b = ds * curv_dt[i - 1], x = k[0], y = k[1];
+      double q[3];
+      turn(i, q);
+      TurnOp()(k, q);
+      Q[0] += ds * x; Q[1] += ds * y;
+      // i b ksi_(i-1) conj(ksi_i) / M_i
+      Q[2] += b * (x * k[1] - y * k[0]) / k[2];
+      Q[3] += b * (x * k[0] + y * k[1]) / k[2];
+      rX[i] = Q[0]; rY[i] = Q[1]; vNorX[i] = Q[2]; vNorY[i] = Q[3];
+      norX[i] = k[0]; norY[i] = k[1]; vX[i] = k[2];
+    }
+  }
+  const double zero4[4] = {0, 0, 0, 0}, zero2[2] = {0, 0};
+  block_scan_excl<4>(Q, zero4, sm, AddOp<4>());
+  // r, vKsi = ksi M W, and the thread's sum of v
+  double V[2] = {0, 0};
+  {
+    double wx = K[2] * (K[0] * Q[2] - K[1] * Q[3]), wy = K[2] * (K[0] * Q[3] + K[1] * Q[2]);   // vKsi_(i-1)
+    for (int i = i0; i < i1; i++) {
+      const double ds = rS[i] - rS[i - 1], kx = norX[i], ky = norY[i], M = vX[i];
+      const double Wx = Q[2] + vNorX[i], Wy = Q[3] + vNorY[i];
+      V[0] += ds * wx; V[1] += ds * wy;
+      wx = M * (kx * Wx - ky * Wy); wy = M * (kx * Wy + ky * Wx);
+      rX[i] += Q[0]; rY[i] += Q[1];
+      norX[i] = -ky; norY[i] = kx;
+      vNorX[i] = -wy; vNorY[i] = wx;
+      vX[i] = V[0]; vY[i] = V[1];
+    }
+  }
+  block_scan_excl<2>(V, zero2, sm, AddOp<2>());
+  for (int i = i0; i < i1; i++) { vX[i] += V[0]; vY[i] += V[1]; }
+  if (threadIdx.x == 0) {
+    rX[0] = rY[0] = vX[0] = vY[0] = vNorX[0] = vNorY[0] = norX[0] = 0.0;
+    norY[0] = 1.0;
+  }
 }
 
 // mode 0: midline at sc->time into buffer (step & 1);
@@ -139,58 +266,7 @@ k_fish_midline(Scalars* sc, const DevShape* sh, int k, FishArrays F, int mode)
     }
     __syncthreads();
   CUP2D_TRACE_MARK(TRACE_ITEMS - 3, 2);
-    if (tid == 0) {                                     // IF2D_Frenet2D::solve
-      const double* curv = rK; const double* curv_dt = vK;
-      rX[0] = 0.0; rY[0] = 0.0;
-      double nX = 0.0, nY = 1.0;                        // norX[i-1], norY[i-1]
-      double ksiX = 1.0, ksiY = 0.0;
-      vX[0] = 0.0; vY[0] = 0.0;
-      double vnX = 0.0, vnY = 0.0;                      // vNorX[i-1], vNorY[i-1]
-      double vKsiX = 0.0, vKsiY = 0.0;
-      double rx = 0.0, ry = 0.0, vx = 0.0, vy = 0.0;
-      norX[0] = nX; norY[0] = nY; vNorX[0] = vnX; vNorY[0] = vnY;
-      double sPrev = rS[0];
-      // the next point's inputs are read one iteration ahead, off the
-      // recurrence's chain
-      double cN = curv[0], cdN = curv_dt[0], sN = rS[1];
-#pragma unroll 2
-      for (int i = 1; i < Nm; i++) {
-        const double c = cN, cd = cdN, sNow = sN;
-        if (i + 1 < Nm) { cN = curv[i]; cdN = curv_dt[i]; sN = rS[i + 1]; }
-        const double dksiX = c * nX;
-        const double dksiY = c * nY;
-        const double dnuX = -c * ksiX;
-        const double dnuY = -c * ksiY;
-        const double dvKsiX = cd * nX + c * vnX;
-        const double dvKsiY = cd * nY + c * vnY;
-        const double dvNuX = -cd * ksiX - c * vKsiX;
-        const double dvNuY = -cd * ksiY - c * vKsiY;
-        const double ds = sNow - sPrev;
-        rx = rx + ds * ksiX;
-        ry = ry + ds * ksiY;
-        nX = nX + ds * dnuX;
-        nY = nY + ds * dnuY;
-        ksiX += ds * dksiX;
-        ksiY += ds * dksiY;
-        vx = vx + ds * vKsiX;
-        vy = vy + ds * vKsiY;
-        vnX = vnX + ds * dvNuX;
-        vnY = vnY + ds * dvNuY;
-        vKsiX += ds * dvKsiX;
-        vKsiY += ds * dvKsiY;
-        const double d1 = ksiX * ksiX + ksiY * ksiY;
-        const double d2 = nX * nX + nY * nY;
-        // 1/sqrt(d) as the reference rounds it: the correctly rounded square
-        // root, then the correctly rounded reciprocal (both factors first, so
-        // the two sequences overlap)
-        const double nf1 = __drcp_rn(__dsqrt_rn(d1)), nf2 = __drcp_rn(__dsqrt_rn(d2));
-        if (d1 > EPSd) { ksiX *= nf1; ksiY *= nf1; }
-        if (d2 > EPSd) { nX *= nf2; nY *= nf2; }
-        rX[i] = rx; rY[i] = ry; vX[i] = vx; vY[i] = vy;
-        norX[i] = nX; norY[i] = nY; vNorX[i] = vnX; vNorY[i] = vnY;
-        sPrev = sNow;
-      }
-    }
+    frenet_scan(Nm, rS, rK, vK, rX, rY, vX, vY, norX, norY, vNorX, vNorY, red);
     __syncthreads();
   CUP2D_TRACE_MARK(TRACE_ITEMS - 3, 3);
   } else {
@@ -221,9 +297,16 @@ k_fish_midline(Scalars* sc, const DevShape* sh, int k, FishArrays F, int mode)
       vNorX[i - 1] = -dVy / ds; vNorY[i - 1] = dVx / ds;
     }
     __syncthreads();
+    {                                                   // running sums of the increments
+      const int n = Nm - 1, per = (n + nt - 1) / nt, i0 = 1 + min(n, tid * per), i1 = 1 + min(n, (tid + 1) * per);
+      double q[2] = {0, 0};
+      const double zero2[2] = {0, 0};
+      for (int i = i0; i < i1; i++) { q[0] += rK[i]; q[1] += vK[i]; rX[i] = q[0]; vX[i] = q[1]; }
+      block_scan_excl<2>(q, zero2, red, AddOp<2>());
+      for (int i = i0; i < i1; i++) { rX[i] += q[0]; vX[i] += q[1]; }
+    }
     if (tid == 0) {
       rX[0] = 0.0; vX[0] = 0.0;
-      for (int i = 1; i < Nm; i++) { rX[i] = rK[i] + rX[i - 1]; vX[i] = vK[i] + vX[i - 1]; }
       norX[Nm - 1] = norX[Nm - 2]; norY[Nm - 1] = norY[Nm - 2];
       vNorX[Nm - 1] = vNorX[Nm - 2]; vNorY[Nm - 1] = vNorY[Nm - 2];
     }
