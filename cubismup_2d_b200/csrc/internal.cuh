@@ -366,6 +366,48 @@ __device__ __forceinline__ void warp_sum_rows(const double* p, int n, int stride
   for (int k = 0; k < K; k++) out[k] = __shfl_sync(0xffffffffu, r, k * STRIDE);
 }
 
+// The sum of K (<= 32) values per thread over a CTA of 1024 threads, to
+// out[0..K) (global memory): a warp with no contribution (any false in all
+// its lanes, their values +0) skips its shuffles, then warp q adds the warps'
+// partial sums of value q.  The same trees as block_sum, so the same bits;
+// K warps side by side instead of one warp for all values, and no barrier
+// after the sums.  smem: 32 K doubles, free again after the caller's next
+// barrier.
+template <int K>
+__device__ __forceinline__ void tile_sum(double (&v)[K], bool any, double* smem, double* out) {
+  constexpr int KP = Pow2Up<K>::v, STRIDE = 32 / KP;
+  const int t = lin_tid(), lane = t & 31, wid = t >> 5;
+  double r = 0.0;
+  if (__any_sync(0xffffffffu, any)) {
+    double x[KP];
+#pragma unroll
+    for (int k = 0; k < KP; k++) x[k] = k < K ? v[k] : 0.0;
+    r = warp_reduce_scatter<KP>(x, lane);
+  }
+  if (lane % STRIDE == 0 && lane / STRIDE < K) smem[wid * K + lane / STRIDE] = r;
+  __syncthreads();
+  if (wid < K) {
+    const double s = warp_sum(smem[lane * K + wid]);
+    if (lane == 0) out[wid] = s;
+  }
+}
+// warp_sum_rows for a CTA of at least K warps, warp q adding value q: out[0..K)
+// (shared memory) holds the totals after the closing barrier
+template <int K>
+__device__ __forceinline__ void tile_sum_rows(const double* p, int n, double* out) {
+  const int t = lin_tid(), lane = t & 31, wid = t >> 5;
+  if (wid < K) {
+    double x = 0.0;
+    for (int i = lane; i < n; i += 32) x += __ldcg(&p[(size_t)K * i + wid]);
+    x = warp_sum(x);
+    if (lane == 0) out[wid] = x;
+  }
+  __syncthreads();
+}
+// the first tile of this CTA, read beside the tile count it is valid under
+__device__ __forceinline__ int first_tile(const ObstTiles& t) {
+  return (int)blockIdx.x < t.capacity ? t.tiles[blockIdx.x] : 0;
+}
 __device__ __forceinline__ double block_max(double v, double* smem) {
   const int t = lin_tid(), lane = t & 31, wid = t >> 5;
   const int nw = (lin_nthreads() + 31) >> 5;

@@ -143,16 +143,17 @@ k_chi_moments(GridDesc g, DevShape* sh, AllTiles T, const double* __restrict__ s
   const int k = blockIdx.y;
   DevShape& S = sh[k];
   const ObstTiles& t = T.t[k];
-  const int nt = S.ntiles;
+  const int nt = S.ntiles, b0 = first_tile(t);
   double* mp = partials + (size_t)k * partStride;
   const double C0 = S.s.com[0], C1 = S.s.com[1];
-  for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
+  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
   double I[7] = {0, 0, 0, 0, 0, 0, 0};
+  bool any = false;
   {
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = threadIdx.x, iy = threadIdx.y;
     const size_t o = (size_t)s * BS2 + iy * BS + ix;
-    const double sdf = t.dist[o];
+    const double sdf = t.dist[o], ux = t.udx[o], uy = t.udy[o];
     tile[iy][ix] = sdf;
     __syncthreads();
     const double h = g.h, i2h = 0.5 / h, fac = 0.5 * h;
@@ -183,7 +184,7 @@ k_chi_moments(GridDesc g, DevShape* sh, AllTiles T, const double* __restrict__ s
     if (X > 0) {
       const double p0 = cell_x(g, bx, ix) - C0, p1 = cell_y(g, by, iy) - C1;
       const double w = X * S.rhoTile * (h * h);
-      const double ux = t.udx[o], uy = t.udy[o];
+      any = true;
       I[0] = w * p0;
       I[1] = w * p1;
       I[2] = w;
@@ -207,15 +208,13 @@ k_chi_moments(GridDesc g, DevShape* sh, AllTiles T, const double* __restrict__ s
     }
     t.sD[o] = D; t.sdx[o] = sdx; t.sdy[o] = sdy;
   }
-  block_sum<7>(I, red);
-  if (lin_tid() == 0) for (int q = 0; q < 7; q++) mp[7 * s + q] = I[q];
+  tile_sum<7>(I, any, red, mp + 7 * s);
+  __syncthreads();
   }
   if (!last_block_done(counters + k, gridDim.x)) return;
-  const int tid = lin_tid();
-  if (tid >= 32) return;                               // one warp finishes
-  double I[7];
-  warp_sum_rows<7>(mp, nt, 7, I);
-  if (tid != 0 || nt == 0) return;
+  tile_sum_rows<7>(mp, nt, red);
+  if (lin_tid() != 0 || nt == 0) return;
+  const double* I = red;
   const double M = I[2];
   double d0 = 0, d1 = 0;
   if (M > EPSd) {                                      // PutObjectsOnGrid.cpp:118-122
@@ -265,10 +264,12 @@ k_rhs_obst(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restric
   CUP2D_TRACE_SCOPE(TR_RHSOBST);
   __shared__ double red[32 * 3];
   DevShape& S = sh[k];
-  for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
+  const int nt = S.ntiles, b0 = first_tile(t);
+  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
   double acc[3] = {0, 0, 0};   // sumRHS, posRHS, negRHS
+  bool any = false;
   {
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = threadIdx.x, iy = threadIdx.y;
     const int gx = bx * BS + ix, gy = by * BS + iy;
     auto CHI = [&](int x, int y) -> double {
@@ -276,13 +277,14 @@ k_rhs_obst(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restric
       y = y < 0 ? 0 : (y >= g.ny ? g.ny - 1 : y);
       return chig[(size_t)y * g.nx + x];
     };
-    const double chi = t.chi[(size_t)s * BS2 + iy * BS + ix];
-    if (!(CHI(gx, gy) > chi)) {
-      const double gradXx = CHI(gx + 1, gy) - CHI(gx - 1, gy);
-      const double gradXy = CHI(gx, gy + 1) - CHI(gx, gy - 1);
-      const size_t c = (size_t)gy * g.nx + gx;
-      const double tmp0 = rhs[c];
+    // every value the cell may need is loaded before the first test
+    const size_t c = (size_t)gy * g.nx + gx;
+    const double chi = t.chi[(size_t)s * BS2 + iy * BS + ix], tmp0 = rhs[c], own = CHI(gx, gy);
+    const double gradXx = CHI(gx + 1, gy) - CHI(gx - 1, gy);
+    const double gradXy = CHI(gx, gy + 1) - CHI(gx, gy - 1);
+    if (!(own > chi)) {
       const double srcBulk = -chi * tmp0;
+      any = true;
       acc[0] = srcBulk;
       const double tmp = tmp0 + srcBulk;
       rhs[c] = tmp;
@@ -291,14 +293,13 @@ k_rhs_obst(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restric
       if (isPerim && tmp < 0) acc[2] = -tmp;
     }
   }
-  block_sum<3>(acc, red);
-  if (lin_tid() == 0) for (int q = 0; q < 3; q++) partials[3 * s + q] = acc[q];
+  tile_sum<3>(acc, any, red, partials + 3 * s);
+  __syncthreads();
   }
   if (!last_block_done(counter, gridDim.x)) return;
-  if (lin_tid() >= 32) return;                           // one warp finishes
-  double tot[3];
-  warp_sum_rows<3>(partials, S.ntiles, 3, tot);
-  if (lin_tid() == 0) {                                  // PressureSingle.cpp:185-186
+  tile_sum_rows<3>(partials, nt, red);
+  if (lin_tid() == 0) {
+    const double* tot = red;                                  // PressureSingle.cpp:185-186
     const double corrDenom = tot[0] > 0 ? tot[1] : tot[2];
     S.rhsCorr = tot[0] / fmax(corrDenom, EPSd);
   }
@@ -316,22 +317,22 @@ k_rhs_corr(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __r
   __shared__ double red[32 * 3];
   const DevShape& S = sh[k];
   const double corr = S.rhsCorr;
+  const int nt = S.ntiles, b0 = first_tile(t);
   auto CHI = [&](int x, int y) -> double {
     x = x < 0 ? 0 : (x >= g.nx ? g.nx - 1 : x);
     y = y < 0 ? 0 : (y >= g.ny ? g.ny - 1 : y);
     return chig[(size_t)y * g.nx + x];
   };
-  for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = threadIdx.x, iy = threadIdx.y;
     const int gx = bx * BS + ix, gy = by * BS + iy;
-    const double chi = t.chi[(size_t)s * BS2 + iy * BS + ix];
-    if (!(CHI(gx, gy) > chi)) {
-      const double gradXx = CHI(gx + 1, gy) - CHI(gx - 1, gy);
-      const double gradXy = CHI(gx, gy + 1) - CHI(gx, gy - 1);
+    const size_t c = (size_t)gy * g.nx + gx;
+    const double chi = t.chi[(size_t)s * BS2 + iy * BS + ix], tmp = rhs[c], own = CHI(gx, gy);
+    const double gradXx = CHI(gx + 1, gy) - CHI(gx - 1, gy);
+    const double gradXy = CHI(gx, gy + 1) - CHI(gx, gy - 1);
+    if (!(own > chi)) {
       const bool isPerim = gradXx * gradXx + gradXy * gradXy > 0;
-      const size_t c = (size_t)gy * g.nx + gx;
-      const double tmp = rhs[c];
       if (isPerim && tmp > 0 && corr > 0) rhs[c] = tmp - corr * tmp;
       else if (isPerim && tmp < 0 && corr < 0) rhs[c] = tmp + corr * tmp;
     }
@@ -341,11 +342,8 @@ k_rhs_corr(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __r
       if (iy < 8)
         for (int r = 0; r < 4; r++)
           fade_accumulate(g, bx, by, ix, iy + 8 * r, rhs[(size_t)(by * BS + iy + 8 * r) * g.nx + gx], f);
-      block_sum<3>(f, red);
-      if (lin_tid() == 0) {
-        const int q = fadeSlot[b];
-        for (int k2 = 0; k2 < 3; k2++) fadePartials[3 * q + k2] = f[k2];
-      }
+      tile_sum<3>(f, iy < 8, red, fadePartials + 3 * fadeSlot[b]);
+      __syncthreads();
     }
   }
 }
@@ -374,27 +372,30 @@ k_momenta(GridDesc g, const Scalars* sc, DevShape* sh, AllTiles T, const double*
   const int k = blockIdx.y, tid = lin_tid();
   DevShape& S = sh[k];
   const ObstTiles& t = T.t[k];
-  const int nt = S.ntiles;
+  const int nt = S.ntiles, b0 = first_tile(t);
   double* mp = parts + (size_t)k * partStride + 10 * (size_t)t.capacity;
   for (int s = blockIdx.x; s < nt; s += gridDim.x) {
     const double Cx = S.s.com[0], Cy = S.s.com[1];
     const double hsq = g.h * g.h, rho = S.rhoTile;
     double A[7] = {0, 0, 0, 0, 0, 0, 0};   // PM, PJ, PX, PY, UM, VM, AM
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = tid % BS, iy = tid / BS;
     const size_t o = (size_t)s * BS2 + tid;
+    // every value the cell may need is loaded before the test of chi
+    const int gx = bx * BS + ix, gy = by * BS + iy, nx = g.nx, ny = g.ny;
+    const size_t c = (size_t)gy * nx + gx;
     const double chi = t.chi[o];
-    if (chi > 0) {
-      const int gx = bx * BS + ix, gy = by * BS + iy, nx = g.nx, ny = g.ny;
-      const size_t c = (size_t)gy * nx + gx;
-      double uc, vc;
-      if (VARRHO) {
-        uc = ui[c]; vc = vi[c];
-      } else {
+    double uc = ui[c], vc = vi[c], dpx = 0, dpy = 0;
+    if (!VARRHO) {
+      const double pW = p[gx > 0 ? c - 1 : c], pE = p[gx < nx - 1 ? c + 1 : c];
+      const double pS = p[gy > 0 ? c - nx : c], pN = p[gy < ny - 1 ? c + nx : c];
+      dpx = pE - pW; dpy = pN - pS;
+    }
+    const bool any = chi > 0;
+    if (any) {
+      if (!VARRHO) {
         const double pFac = -0.5 * sc->dt / g.h;
-        const double pW = p[gx > 0 ? c - 1 : c], pE = p[gx < nx - 1 ? c + 1 : c];
-        const double pS = p[gy > 0 ? c - nx : c], pN = p[gy < ny - 1 ? c + nx : c];
-        uc = ui[c] + pFac * (pE - pW); vc = vi[c] + pFac * (pN - pS);
+        uc = uc + pFac * dpx; vc = vc + pFac * dpy;
       }
       const double p0 = cell_x(g, bx, ix) - Cx, p1 = cell_y(g, by, iy) - Cy;
       double ud0 = uc, ud1 = vc;
@@ -417,14 +418,13 @@ k_momenta(GridDesc g, const Scalars* sc, DevShape* sh, AllTiles T, const double*
       A[5] = F * ud1;
       A[6] = F * (p0 * ud1 - p1 * ud0);
     }
-    block_sum<7>(A, red);
-    if (tid == 0) for (int q = 0; q < 7; q++) mp[7 * s + q] = A[q];
+    tile_sum<7>(A, any, red, mp + 7 * s);
+    __syncthreads();
   }
   if (!last_block_done(counters + k, gridDim.x)) return;
-  if (tid >= 32) return;                                // one warp finishes
-  double A[7];
-  warp_sum_rows<7>(mp, nt, 7, A);
+  tile_sum_rows<7>(mp, nt, red);
   if (tid != 0) return;
+  const double* A = red;
   S.s.fluidAngMom = A[6]; S.s.fluidMomX = A[4]; S.s.fluidMomY = A[5];
   S.s.penalDX = ITER ? 0.0 : A[2]; S.s.penalDY = ITER ? 0.0 : A[3];
   S.s.penalM = A[0]; S.s.penalJ = A[1];
@@ -579,13 +579,14 @@ k_penalize(GridDesc g, const Scalars* sc, const DevShape* sh, int k, ObstTiles t
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_PENALIZE);
   const DevShape& S = sh[k];
-  for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+  const int nt = S.ntiles, b0 = first_tile(t);
+  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = threadIdx.x, iy = threadIdx.y;
     const size_t o = (size_t)s * BS2 + iy * BS + ix;
     const size_t c = (size_t)(by * BS + iy) * g.nx + bx * BS + ix;
-    const double X = t.chi[o];
-    if (chig[c] > X) continue;
+    const double X = t.chi[o], Xg = chig[c], uc = u[c], vc = v[c];
+    if (Xg > X) continue;
     if (X <= 0) continue;
     const double p0 = cell_x(g, bx, ix) - S.s.com[0], p1 = cell_y(g, by, iy) - S.s.com[1];
     // PressureSingle.cpp:93-97: 1 / (1 + lambda dt X) without EXPL_INTEGRATE_MOM
@@ -594,8 +595,8 @@ k_penalize(GridDesc g, const Scalars* sc, const DevShape* sh, int k, ObstTiles t
     udef_at(t, o, S, p0, p1, ux, uy);
     const double US = S.s.u - S.s.omega * p1 + ux;
     const double VS = S.s.v + S.s.omega * p0 + uy;
-    u[c] = alpha * u[c] + (1 - alpha) * US;
-    v[c] = alpha * v[c] + (1 - alpha) * VS;
+    u[c] = alpha * uc + (1 - alpha) * US;
+    v[c] = alpha * vc + (1 - alpha) * VS;
   }
 }
 
@@ -615,26 +616,33 @@ k_forces(GridDesc g, Scalars* sc, int maxNext, DevShape* sh, AllTiles T, const d
   DevShape& S = sh[k];
   const ObstTiles& t = T.t[k];
   double* part = partials + (size_t)k * partStride;
+  const int nt = S.ntiles, b0 = first_tile(t);
+  __shared__ double redm[32];
   // maxNext (graph steps): the next step's findMaxU over this shape's tiles,
   // penalized by now (the blocks outside every tile are k_pcorr<true>'s)
   const double UINF = sc->uinfx, VINF = sc->uinfy;
-  double mx = 0.0;
-  int bad = 0;
-  for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
+  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
   double F[NFORCE];
+  bool any;
 #pragma unroll
   for (int q = 0; q < NFORCE; q++) F[q] = 0;
   {
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = threadIdx.x, iy = threadIdx.y;
     const size_t o = (size_t)s * BS2 + iy * BS + ix;
+    const double sD = t.sD[o];
     if (maxNext) {
       const size_t c = (size_t)(by * BS + iy) * g.nx + bx * BS + ix;
       const double a = u[c], w = v[c];
-      mx = fmax(mx, cell_speed(a, w, UINF, VINF));
-      bad |= !isfinite(a) || !isfinite(w);
+      const double mx = warp_max(cell_speed(a, w, UINF, VINF));
+      const bool bad = __any_sync(0xffffffffu, !isfinite(a) || !isfinite(w));
+      if (ix == 0) {
+        redm[iy] = mx;                                  // a warp is a row of the tile
+        if (bad) atomicOr(&sc->status, ST_NAN);
+      }
     }
-    if (t.sD[o] > 0) {
+    any = sD > 0;
+    if (any) {
       const int gx = bx * BS + ix, gy = by * BS + iy;
       auto I = [&](int x, int y) -> size_t {
         x = x < 0 ? 0 : (x >= g.nx ? g.nx - 1 : x);
@@ -678,23 +686,17 @@ k_forces(GridDesc g, Scalars* sc, int maxNext, DevShape* sh, AllTiles T, const d
       F[16] = fmin(0.0, powDef);                            // defPowerBnd
     }
   }
-  block_sum<NFORCE>(F, red);
-  if (lin_tid() == 0) for (int q = 0; q < NFORCE; q++) part[NFORCE * s + q] = F[q];
+  tile_sum<NFORCE>(F, any, red, part + NFORCE * s);
+  if (maxNext && threadIdx.y == 31) {                  // a warp that adds no force sums
+    const double mx = warp_max(redm[threadIdx.x]);
+    if (threadIdx.x == 0) atomic_max_nonneg(&sc->maxNext, mx);
   }
-  if (maxNext) {                                       // uniform over the launch
-    __shared__ double redm[32];
-    mx = block_max(mx, redm);
-    const int anyBad = __syncthreads_or(bad);
-    if (lin_tid() == 0) {
-      atomic_max_nonneg(&sc->maxNext, mx);
-      if (anyBad) atomicOr(&sc->status, ST_NAN);
-    }
+  __syncthreads();
   }
   if (!last_block_done(counters + k, gridDim.x)) return;
-  if (lin_tid() >= 32) return;                          // one warp finishes
-  double tot[NFORCE];
-  warp_sum_rows<NFORCE>(part, S.ntiles, NFORCE, tot);
+  tile_sum_rows<NFORCE>(part, nt, red);
   if (lin_tid() != 0) return;
+  const double* tot = red;
   cup2d_shape_state& st = S.s;
   st.perimeter = tot[0]; st.forcex = tot[1]; st.forcey = tot[2];
   st.forcex_P = tot[3]; st.forcey_P = tot[4]; st.forcex_V = tot[5]; st.forcey_V = tot[6];
