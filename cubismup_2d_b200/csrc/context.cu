@@ -173,7 +173,8 @@ struct StreamScope {
 // momentum integrals run side by side (the integrals evaluate the corrected
 // velocity of their own cells), then collisions and penalization.  The
 // integrals, the longer of the two, stay on the main stream.
-void launch_pressure_tail(Ctx& c, bool maxNext) {
+// joinMid: also waits for the midlines on side (where the tail joins anyway).
+void launch_pressure_tail(Ctx& c, bool maxNext, bool joinMid = false) {
   const double* ui = c.u();
   const double* vi = c.v();
   if (c.nshapes == 0) {
@@ -189,6 +190,7 @@ void launch_pressure_tail(Ctx& c, bool maxNext) {
   cudaEventRecord(c.evMom, c.side2);
   launch_momenta(c, ui, vi);
   cudaStreamWaitEvent(c.stream, c.evMom, 0);
+  if (joinMid) cudaStreamWaitEvent(c.stream, c.evJoin, 0);
   launch_collide_penalize(c);
 }
 
@@ -257,10 +259,10 @@ void enqueue_step(Ctx& c) {
   cudaStreamWaitEvent(c.stream, c.evObjDone, 0);
   launch_rhs_obstacles(c);
   poisson_solve(c);
-  launch_pressure_tail(c, true);
-  launch_forces(c, c.forcesOut, true);
-  if (anyAhead) cudaStreamWaitEvent(c.stream, c.evJoin, 0);
-  launch_end_step_dt(c);                    // t += dt, and the next step's dt
+  // (the next step's midlines read the time that the step end moves: joined in
+  // the tail, long after they are done)
+  launch_pressure_tail(c, true, anyAhead);
+  launch_forces(c, c.forcesOut, true, nullptr, 0, true);   // and t += dt, the next step's dt
 }
 
 // PressureIterator_unif::operator() (PressureIterator_unif.cpp:214-270): the

@@ -181,7 +181,7 @@ inline size_t fish_pool_len(int nm) { return 36 * (size_t)nm + 16; }
 
 // counter slots used by the kernels (each last-CTA reduction owns one)
 enum CounterSlot : int {
-  CNT_MAXU = 0, CNT_ADV = 1,
+  CNT_MAXU = 0, CNT_ADV = 1, CNT_STEP = 2,
   CNT_CHI = 8,          // + shape
   CNT_RHSOBST = 24,     // + shape
   CNT_FORCES = 40,      // + shape

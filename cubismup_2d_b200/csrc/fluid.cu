@@ -41,15 +41,7 @@ __global__ void k_end_step_dt(GridDesc g, Scalars* sc, const DevShape* sh, int n
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_ENDSTEP);
-  const double m = sc->maxNext;
-  sc->time += sc->dt;
-  sc->step += 1;
-  const double dtn = dt_from_max_u(g, sc, sh, nsh, m);
-  sc->dtNext = dtn;
-  sc->maxUNext = m;
-  sc->dtNextValid = 1;
-  if (dtOut) *dtOut = dtn;                    // to mapped host memory
-  signal_host(seqOut, seqVal);
+  end_step(g, sc, sh, nsh, dtOut, seqOut, seqVal);
 }
 
 // End of an operator-by-operator step: findMaxU on the final velocity (its

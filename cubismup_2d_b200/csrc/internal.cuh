@@ -439,7 +439,14 @@ __device__ __forceinline__ bool last_block_done(unsigned* counter, unsigned nblo
   return amLast;
 }
 
-// atomic max on doubles through the ordered-integer mapping of IEEE-754
+// last_block_done for single threads: true in the last of n callers
+__device__ __forceinline__ bool last_thread_done(unsigned* counter, unsigned n) {
+  unsigned t;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(t) : "l"(counter) : "memory");
+  if (t != n - 1) return false;
+  *counter = 0;
+  return true;
+}
 // Max of non-negative doubles (speeds: +0 and up, +inf, never NaN): their
 // bit patterns order as the values do, so one native 64-bit unsigned atomic
 // max (no compare-and-swap retries) suffices where many CTAs finishing at
@@ -447,16 +454,16 @@ __device__ __forceinline__ bool last_block_done(unsigned* counter, unsigned nblo
 __device__ __forceinline__ void atomic_max_nonneg(double* addr, double val) {
   atomicMax(reinterpret_cast<unsigned long long*>(addr), static_cast<unsigned long long>(__double_as_longlong(val)));
 }
+// Max of doubles of any sign without a compare-and-swap loop (two dependent
+// L2 round trips in each cell of the rasters): bit patterns of positive
+// doubles order as signed integers, above every negative one; those of
+// negative doubles order downwards as unsigned integers, above every
+// positive one.
 __device__ __forceinline__ void atomic_max_double(double* addr, double val) {
-  unsigned long long* a = reinterpret_cast<unsigned long long*>(addr);
-  unsigned long long old = *a, assumed;
-  do {
-    assumed = old;
-    if (__longlong_as_double(assumed) >= val) return;
-    old = atomicCAS(a, assumed, __double_as_longlong(val));
-  } while (old != assumed);
+  const long long b = __double_as_longlong(val);
+  if (b >= 0) atomicMax(reinterpret_cast<long long*>(addr), b);
+  else atomicMin(reinterpret_cast<unsigned long long*>(addr), static_cast<unsigned long long>(b));
 }
-
 // Per-tile udef after Shape::removeMoments (Shape.cpp:197-204), evaluated
 // where it is read: udef - (I.u - I.a p1), udef - (I.v + I.a p0), p = x - CoM.
 __device__ __forceinline__ void udef_at(const ObstTiles& t, size_t o, const DevShape& S,

@@ -88,8 +88,10 @@ void launch_collide_penalize(Ctx& c);                // PressureSingle.cpp:69-10
 // maxNext: with the next step's findMaxU over the shapes' tiles
 // out (mapped host memory, or null): each shape's final state; then
 // seqOut[k] = seqVal behind a system-scope fence
+// endStep (graph steps, with maxNext): the last CTA also ends the step, as
+// launch_end_step_dt does
 void launch_forces(Ctx& c, cup2d_shape_state* out, bool maxNext, unsigned long long* seqOut = nullptr,
-                   unsigned long long seqVal = 0);
+                   unsigned long long seqVal = 0, bool endStep = false);
 
 // poisson.cu
 struct Poisson;

@@ -110,6 +110,21 @@ __device__ __forceinline__ bool max_u_dt_cta(const GridDesc& g, Scalars* sc, con
   return true;
 }
 
+// Simulation.cpp:289-290 and the next step's calcMaxTimestep from sc->maxNext;
+// one thread.  dtOut (mapped host memory): the next dt, then seqOut = seqVal.
+__device__ __forceinline__ void end_step(const GridDesc& g, Scalars* sc, const DevShape* sh, int nsh, double* dtOut,
+                                         unsigned long long* seqOut, unsigned long long seqVal) {
+  const double m = __ldcg(&sc->maxNext);      // (other CTAs' atomics may be part of it)
+  sc->time += sc->dt;
+  sc->step += 1;
+  const double dtn = dt_from_max_u(g, sc, sh, nsh, m);
+  sc->dtNext = dtn;
+  sc->maxUNext = m;
+  sc->dtNextValid = 1;
+  if (dtOut) *dtOut = dtn;                    // to mapped host memory
+  signal_host(seqOut, seqVal);
+}
+
 // The PID controllers of StefanFish::create (StefanFish.cpp:264-364), run
 // after every body has moved and before the midline of this step is formed:
 // exponential averages of the lateral offset, the angle and the angular
