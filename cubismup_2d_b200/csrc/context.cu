@@ -265,6 +265,24 @@ void enqueue_step(Ctx& c) {
   launch_forces(c, c.forcesOut, true, nullptr, 0, true);   // and t += dt, the next step's dt
 }
 
+// Waits for a kernel's signal in mapped host memory: the word reaches want
+// (the kernel wrote its data first, behind a system-scope fence).  Spins on
+// the word for up to 20 ms -- waking on it costs less than on the event --
+// then waits on the event recorded after that kernel, which also reports
+// an error of the stream (a kernel that never signals ends up there).
+static cudaError_t wait_mapped(const unsigned long long* word, unsigned long long want, cudaEvent_t ev) {
+  const volatile unsigned long long* w = word;
+  const auto t0 = std::chrono::steady_clock::now();
+  for (unsigned it = 0;; it++) {
+    if (*w >= want) {
+      std::atomic_thread_fence(std::memory_order_acquire);
+      return cudaSuccess;
+    }
+    if ((it & 255) == 255 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) break;
+  }
+  return cudaEventSynchronize(ev);
+}
+
 // PressureIterator_unif::operator() (PressureIterator_unif.cpp:214-270): the
 // velocity after advDiff kept as TMPV, then per iteration the fluid velocity
 // UF = TMPV - (dt/2h) grad P (P of the previous iteration, or step), the
@@ -287,13 +305,16 @@ int pressure_iterative(cup2d_ctx* ctx) {
   for (iter = 0; iter < 1000; iter++) {
     launch_pcorr_from(c, c.itmp[0], c.itmp[1], c.ifluid[0], c.ifluid[1]);
     launch_momenta_iter(c, c.itmp[0], c.itmp[1]);    // UF's values, formed in place
-    launch_penalize_iter(c, c.itmp[0], c.itmp[1], c.ifluid[0], c.ifluid[1]);
+    const unsigned long long seq = ++c.mapSeq;
+    launch_penalize_iter(c, c.itmp[0], c.itmp[1], c.ifluid[0], c.ifluid[1], seq);
     launch_rhs_iter(c);
     poisson_solve(c);
-    CK(cudaMemcpyAsync(&c.pin->it.relDF, &c.dsc->it.relDF, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaStreamSynchronize(c.stream));
+    // the penalization wrote the change to mapped host memory: the next
+    // iteration (or the end) is enqueued while the solve runs
+    CK(cudaEventRecord(c.evIter, c.stream));
+    CK(wait_mapped(&c.map->seqIter, seq, c.evIter));
     if (int rc = check_launch(ctx)) return rc;
-    relDF = c.pin->it.relDF;
+    relDF = *const_cast<const volatile double*>(&c.map->relDF);
     if (relDF < st.target || iter > 100 || iter > 2 * st.oldNsteps) {
       launch_pcorr(c);                          // finalizePressure
       break;
@@ -345,12 +366,13 @@ int pressure_varrho(cup2d_ctx* ctx) {
     c.pres = c.rhs;                               // solve(tmp, tmp)
     poisson_solve(c);
     c.pres = P;
-    launch_vr_pcorr(c, false);
-    CK(cudaMemcpyAsync(&c.pin->it, &c.dsc->it, sizeof(IterState), cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaStreamSynchronize(c.stream));
+    const unsigned long long seq = ++c.mapSeq;
+    launch_vr_pcorr(c, false, seq);
+    CK(cudaEventRecord(c.evIter, c.stream));
+    CK(wait_mapped(&c.map->seqIter, seq, c.evIter));
     if (int rc = check_launch(ctx)) return rc;
-    relDF = c.pin->it.relDF;
-    relDP = c.pin->it.relDP;
+    relDF = *const_cast<const volatile double*>(&c.map->relDF);
+    relDP = *const_cast<const volatile double*>(&c.map->relDP);
     const bool converged = std::max(relDF, relDP) < st.target || iter > 2 * st.oldNsteps || iter > 100;
     if (converged) launch_vr_pcorr(c, true);     // finalizePressure
     std::swap(c.pres, c.rhs);                     // pres = tmp
@@ -510,6 +532,7 @@ int cup2d_create(const cup2d_config* cfg, cup2d_ctx** out) {
               cudaEventCreateWithFlags(&c.evObjDone, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&c.evPres, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&c.evMom, cudaEventDisableTiming) != cudaSuccess ||
+              cudaEventCreateWithFlags(&c.evIter, cudaEventDisableTiming) != cudaSuccess ||
               cudaEventCreateWithFlags(&c.evPlaced, cudaEventDisableTiming) != cudaSuccess))
     rc = fail(ctx, CUP2D_ECUDA, "stream/event creation failed");
   if (!rc && fish_setup_kernels() != cudaSuccess)
@@ -560,6 +583,7 @@ int cup2d_destroy(cup2d_ctx* ctx) {
   if (c.evJoin) cudaEventDestroy(c.evJoin);
   if (c.evPres) cudaEventDestroy(c.evPres);
   if (c.evMom) cudaEventDestroy(c.evMom);
+  if (c.evIter) cudaEventDestroy(c.evIter);
   if (c.evPlaced) cudaEventDestroy(c.evPlaced);
   for (auto& t : c.tiles) {
     cudaFree(t.tiles); cudaFree(t.slot); cudaFree(t.chi); cudaFree(t.dist); cudaFree(t.udx);
@@ -796,24 +820,6 @@ int cup2d_iteration_stats(cup2d_ctx* ctx, int* iterations, double* rel_df) {
   if (iterations) *iterations = c.pin->it.last;
   if (rel_df) *rel_df = c.pin->it.relDF;
   return CUP2D_OK;
-}
-
-// Waits for a kernel's signal in mapped host memory: the word reaches want
-// (the kernel wrote its data first, behind a system-scope fence).  Spins on
-// the word for up to 20 ms -- waking on it costs less than on the event --
-// then waits on the event recorded after that kernel, which also reports
-// an error of the stream (a kernel that never signals ends up there).
-static cudaError_t wait_mapped(const unsigned long long* word, unsigned long long want, cudaEvent_t ev) {
-  const volatile unsigned long long* w = word;
-  const auto t0 = std::chrono::steady_clock::now();
-  for (unsigned it = 0;; it++) {
-    if (*w >= want) {
-      std::atomic_thread_fence(std::memory_order_acquire);
-      return cudaSuccess;
-    }
-    if ((it & 255) == 255 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) break;
-  }
-  return cudaEventSynchronize(ev);
 }
 
 int cup2d_calc_dt(cup2d_ctx* ctx, double* dt_out) {

@@ -69,7 +69,7 @@ struct Ctx {
   cudaStream_t side2 = nullptr; // branch for the obstacle chain, beside advDiff
   cudaEvent_t evFork = nullptr, evJoin = nullptr, evObj = nullptr, evObjDone = nullptr;
   cudaEvent_t evStart = nullptr;   // the start of a graph step (fork of its first side launches)
-  cudaEvent_t evPres = nullptr, evMom = nullptr;
+  cudaEvent_t evPres = nullptr, evMom = nullptr, evIter = nullptr;
   cudaEvent_t evPlaced = nullptr;   // recorded after the obstacle tiles are placed
   bool recordPlaced = false;
   bool graphStep = false;           // enqueue_step is recording a graph step
@@ -123,6 +123,8 @@ struct Ctx {
     double dtNext;
     cup2d_shape_state shapes[MAX_SHAPES];
     unsigned long long seqDt, seqShape[MAX_SHAPES];
+    double relDF, relDP;            // an iterated pressure call's convergence, then seqIter
+    unsigned long long seqIter;
   };
   HostMapped* map = nullptr;      // host address
   HostMapped* mapDev = nullptr;   // its device address
@@ -181,7 +183,7 @@ inline size_t fish_pool_len(int nm) { return 36 * (size_t)nm + 16; }
 
 // counter slots used by the kernels (each last-CTA reduction owns one)
 enum CounterSlot : int {
-  CNT_MAXU = 0, CNT_ADV = 1, CNT_STEP = 2,
+  CNT_MAXU = 0, CNT_ADV = 1, CNT_STEP = 2, CNT_RELDF = 3,
   CNT_CHI = 8,          // + shape
   CNT_RHSOBST = 24,     // + shape
   CNT_FORCES = 40,      // + shape
@@ -202,12 +204,43 @@ inline AllTiles all_tiles(const Ctx& c) {
 }
 // CTAs of each shape's per-tile kernel (a kernel argument)
 struct PenalCtas { int n[MAX_SHAPES]; };
+// The relative momentum change of an iterated pressure call: the shapes'
+// per-CTA sums (four each, shape k's at parts + k stride), formed into
+// sc->it.relDF by the last CTA of the last shape's penalization
+struct Residual { Scalars* sc; int nsh; PenalCtas nc; double* parts; int stride; unsigned* counter; };
 // doubles of one shape's tile-reduction region
 inline size_t shape_region(const Ctx& c) { return (size_t)c.maxCapacity * 24; }
 // CTAs per shape of the per-tile kernels: one wave at most; each CTA loops
 // over tiles s = blockIdx.x, blockIdx.x + gridDim.x, ... < ntiles
 inline int tile_ctas(const Ctx& c, int capacity) { return capacity < c.sms ? capacity : c.sms; }
 inline double* shape_partials(const Ctx& c) { return c.partials + (size_t)3 * c.g.nblocks + 4096; }
+inline Residual residual(const Ctx& c) {
+  Residual R{c.dsc, c.nshapes, {}, shape_partials(c), (int)shape_region(c), c.counters + CNT_RELDF};
+  for (int k = 0; k < c.nshapes; k++) R.nc.n[k] = tile_ctas(c, c.tiles[k].capacity);
+  return R;
+}
+#ifdef __CUDACC__
+// sqrt((DMX + DMY) / (eps + MX + MY)) of all shapes' penalized cells
+// (PressureIterator_unif.cpp:185-186) from the per-CTA sums in a fixed order;
+// called by every CTA of the last shape's kernel (1024 threads) after its
+// sums.  relOut (mapped host memory, or null): the value, then seqOut = seqVal.
+__device__ __forceinline__ void relative_change(const Residual& R, double* red, double* relOut,
+                                                unsigned long long* seqOut, unsigned long long seqVal) {
+  if (!last_block_done(R.counter, gridDim.x)) return;
+  double a[4] = {0, 0, 0, 0};
+  for (int k = 0; k < R.nsh; k++) {
+    const double* pk = R.parts + (size_t)k * R.stride;
+    for (int i = lin_tid(); i < R.nc.n[k]; i += 1024)
+      for (int q = 0; q < 4; q++) a[q] += __ldcg(&pk[4 * i + q]);
+  }
+  block_sum<4>(a, red);
+  if (lin_tid() == 0) {
+    const double rel = sqrt((a[2] + a[3]) / (2.220446049250313e-16 + a[0] + a[1]));
+    R.sc->it.relDF = rel;
+    if (relOut) { *relOut = rel; signal_host(seqOut, seqVal); }
+  }
+}
+#endif
 
 #define CUP2D_LAUNCHED(c) ((c).launches++)
 

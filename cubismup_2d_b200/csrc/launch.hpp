@@ -76,13 +76,13 @@ void launch_advdiff_grav(Ctx& c);                    // advDiffGrav.cpp:14-137
 void launch_vr_init(Ctx& c);                         // pressureCorrectionInit :81-122
 void launch_vr_penalize(Ctx& c);                     // penalize :224-287 -> sc->it.relDF
 void launch_vr_rhs(Ctx& c);                          // updatePressureRHS :289-335
-void launch_vr_pcorr(Ctx& c, bool final_);           // pressureCorrection / finalizePressure
+// pressureCorrection / finalizePressure; not final_: relDF and relDP also to
+// mapped host memory, then its seqIter = seqVal
+void launch_vr_pcorr(Ctx& c, bool final_, unsigned long long seqVal = 0);
+// :137-187, residual -> sc->it.relDF and mapped host memory, then its seqIter = seqVal
 void launch_penalize_iter(Ctx& c, const double* tu, const double* tv,
-                          const double* fu, const double* fv);          // :137-187, residual -> sc->it.relDF
+                          const double* fu, const double* fv, unsigned long long seqVal);
 void launch_set_iter_state(Ctx& c, const IterState& st);                // :247-252 state after a call
-struct PenalCtas;
-// relDF = sqrt((DMX + DMY) / (eps + MX + MY)) from each shape's per-CTA sums
-void launch_reldf(Ctx& c, const PenalCtas& nc);
 void launch_collide_penalize(Ctx& c);                // PressureSingle.cpp:69-108, 243-344
 // ComputeForces.cpp:16-111; out (mapped host memory, or null): each shape's final state
 // maxNext: with the next step's findMaxU over the shapes' tiles

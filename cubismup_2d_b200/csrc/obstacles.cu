@@ -452,15 +452,18 @@ k_momenta(GridDesc g, const Scalars* sc, DevShape* sh, AllTiles T, const double*
 __global__ void __launch_bounds__(1024)
 k_penalize_iter(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
                 double* u, double* v, const double* __restrict__ tu, const double* __restrict__ tv,
-                const double* __restrict__ fu, const double* __restrict__ fv, double* part)
+                const double* __restrict__ fu, const double* __restrict__ fv, Residual R,
+                double* relOut, unsigned long long* seqOut, unsigned long long seqVal)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_PENALIZE);
   __shared__ double red[32 * 4];
   const DevShape& S = sh[k];
   double a[4] = {0, 0, 0, 0};                 // MX, MY, DMX, DMY
-  for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+  bool any = false;
+  const int nt = S.ntiles, b0 = first_tile(t);
+  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = threadIdx.x, iy = threadIdx.y;
     const size_t o = (size_t)s * BS2 + iy * BS + ix;
     const size_t c = (size_t)(by * BS + iy) * g.nx + bx * BS + ix;
@@ -478,27 +481,11 @@ k_penalize_iter(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double
     u[c] = un;
     v[c] = vn;
     a[0] += un * un; a[1] += vn * vn; a[2] += DPX * DPX; a[3] += DPY * DPY;
+    any = true;
   }
-  block_sum<4>(a, red);
-  if (lin_tid() == 0) for (int q = 0; q < 4; q++) part[4 * blockIdx.x + q] = a[q];
-}
-
-// The relative momentum change sqrt((DMX + DMY) / (eps + MX + MY)) of all
-// shapes' penalized cells (PressureIterator_unif.cpp:185-186), from the
-// per-CTA sums in a fixed order.
-__global__ void __launch_bounds__(256)
-k_reldf(Scalars* sc, int nsh, PenalCtas nc, const double* __restrict__ parts, int partStride)
-{
-  pdl_begin();
-  __shared__ double red[32 * 4];
-  double a[4] = {0, 0, 0, 0};
-  for (int k = 0; k < nsh; k++) {
-    const double* pk = parts + (size_t)k * partStride;
-    for (int i = threadIdx.x; i < nc.n[k]; i += blockDim.x)
-      for (int q = 0; q < 4; q++) a[q] += pk[4 * i + q];
-  }
-  block_sum<4>(a, red);
-  if (threadIdx.x == 0) sc->it.relDF = sqrt((a[2] + a[3]) / (DBL_EPSILON + a[0] + a[1]));
+  tile_sum<4>(a, any, red, R.parts + (size_t)k * R.stride + 4 * blockIdx.x);
+  __syncthreads();
+  if (k == R.nsh - 1) relative_change(R, red, relOut, seqOut, seqVal);
 }
 
 __global__ void k_set_iter_state(Scalars* sc, IterState st) { pdl_begin(); sc->it = st; }
@@ -851,22 +838,15 @@ void launch_momenta_iter(Ctx& c, const double* ui, const double* vi) {
 
 // the per-CTA sums of shape k sit at the start of its partial region (free
 // while the iterated operator runs: the placement's sums are consumed)
-void launch_penalize_iter(Ctx& c, const double* tu, const double* tv, const double* fu, const double* fv) {
-  PenalCtas nc{};
+void launch_penalize_iter(Ctx& c, const double* tu, const double* tv, const double* fu, const double* fv,
+                          unsigned long long seqVal) {
+  const Residual R = residual(c);
   for (int k = 0; k < c.nshapes; k++) {
-    nc.n[k] = tile_ctas(c, c.tiles[k].capacity);
-    launch_k(k_penalize_iter, nc.n[k], dim3(32, 32), 0, c.stream, c.g, (const DevShape*)c.dshapes, k,
-             c.tiles[k], (const double*)c.chi, c.u(), c.v(), tu, tv, fu, fv,
-             shape_partials(c) + (size_t)k * shape_region(c));
+    launch_k(k_penalize_iter, R.nc.n[k], dim3(32, 32), 0, c.stream, c.g, (const DevShape*)c.dshapes, k,
+             c.tiles[k], (const double*)c.chi, c.u(), c.v(), tu, tv, fu, fv, R, &c.mapDev->relDF,
+             &c.mapDev->seqIter, seqVal);
     CUP2D_LAUNCHED(c);
   }
-  launch_reldf(c, nc);
-}
-
-void launch_reldf(Ctx& c, const PenalCtas& nc) {
-  launch_k(k_reldf, 1, 256, 0, c.stream, c.dsc, c.nshapes, nc, (const double*)shape_partials(c),
-           (int)shape_region(c));
-  CUP2D_LAUNCHED(c);
 }
 
 void launch_set_iter_state(Ctx& c, const IterState& st) {

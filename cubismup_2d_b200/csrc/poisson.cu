@@ -27,6 +27,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 #include "poisson.cuh"
 
@@ -64,19 +65,6 @@ struct Poisson {
 
 namespace {
 
-// Per transform length L: padded stride SL of one sequence (one spare
-// element per 16, plus 4 so that consecutive sequences start in different
-// halves of the shared-memory banks), the staged quarter twiddle table
-// (w^j, j < L/4), the sequences per CTA B and the threads per CTA NT
-// (L/E per sequence: every thread owns E = 16 or 8 elements of a pass).
-template <int L, int E = 16> struct Len {
-  static constexpr int SL = L + L / 16 + 4;
-  static constexpr int B = 2048 / L < 1 ? 1 : (2048 / L > 8 ? 8 : 2048 / L);
-  static constexpr int NT0 = B * L / E;
-  static constexpr int NT = NT0 < 64 ? 64 : (NT0 > 512 ? 512 : NT0);
-  static constexpr int REGS = E == 16 ? 128 : 64;   // register budget per thread
-  static constexpr int MINB = 65536 / (NT * REGS) < 1 ? 1 : 65536 / (NT * REGS);
-};
 // ---- FP64: twiddles and DFT in one, on fused multiply-adds -----------------
 // A pass of radix R over sub-transforms of size NS, y_q = sum_m x_m W^(m k)
 // W_R^(m q) with W = exp(-2 pi i / (R NS)), as log2 R levels of two-point
@@ -388,10 +376,25 @@ __host__ __device__ __forceinline__ size_t spec_at(int rows, int r, int k) {
   return (((size_t)(k >> SPEC_LOG) * rows + r) << SPEC_LOG) | (k & (SPEC_K - 1));
 }
 
-// rows per CTA B, threads NT (L/E per row), padded stride SL of a row
-template <int L, int E> struct Row64 {
-  static constexpr int B = Len<L, E>::B, NT = Len<L, E>::NT, MINB = Len<L, E>::MINB, SL = Len<L, E>::SL;
+// Row passes: B rows per CTA, NT threads (L/E per row, E values each), stride SL
+// of a row (one spare element per 16, and 4 so that consecutive rows start in
+// different halves of the banks)
+template <int L> constexpr int rows_full() { return 2048 / L < 1 ? 1 : (2048 / L > 8 ? 8 : 2048 / L); }
+template <int L, int E, int ROWS> struct Row64 {
+  static constexpr int B = ROWS, SL = L + L / 16 + 4;
+  static constexpr int NT0 = B * L / E, NT = NT0 < 32 ? 32 : (NT0 > 512 ? 512 : NT0);
+  static constexpr int REGS = E == 16 ? 128 : 64;   // register budget per thread
+  static constexpr int MINB0 = 65536 / (NT * REGS), MINB = MINB0 < 1 ? 1 : (MINB0 > 16 ? 16 : MINB0);
 };
+// Grids whose rows fill less than half of the SMs with rows_full rows a CTA
+// take two a CTA (short rows only: from 1024 points on a CTA has at most two).
+// B200, forward and inverse rows with full and with two rows a CTA: 10.9, 11.9
+// and 9.4, 7.5 us at 256 x 128; 11.3, 10.7 and 11.1, 9.1 at 512 x 256; at
+// 1024 x 1024 periodic (256 full CTAs) 15.5, 11.5 and 17.5, 14.6.
+constexpr int ROWS_SMALL = 2, ROWS_SMALL_BELOW = 74;
+template <int L> inline bool rows_small(int nrows) {
+  return rows_full<L>() > ROWS_SMALL && nrows < ROWS_SMALL_BELOW * rows_full<L>();
+}
 // columns per CTA: consecutive lanes take the columns of one pair (CB > 1),
 // and the stride SL puts the columns of eight lanes in different banks
 template <int L> struct Col64 {
@@ -403,8 +406,8 @@ template <int L> struct Col64 {
   static constexpr int GR = L / 2 + 2;                  // multiplier values staged per column
   static constexpr size_t SMEM = sizeof(double2) * ((size_t)CB * SL + tab_staged<L, 16>()) + sizeof(double) * CB * GR;
 };
-template <int L, int E> constexpr size_t smem_row64() {
-  return sizeof(double2) * ((size_t)Row64<L, E>::B * Row64<L, E>::SL + tab_staged<L, E>());
+template <int L, int E, int B> constexpr size_t smem_row64() {
+  return sizeof(double2) * ((size_t)B * Row64<L, E, B>::SL + tab_staged<L, E>());
 }
 
 // Twice the real FFT of length 2L from the complex FFT Z of length L of its
@@ -412,11 +415,11 @@ template <int L, int E> constexpr size_t smem_row64() {
 // Fe = Z_k + conj(Z_(L-k)), Fo = -i (Z_k - conj(Z_(L-k))), W = exp(-i pi/L), k in
 // [0, L/2); 2 X[L/2] = 2 conj(Z_(L/2)).  (The column pass's multiplier carries
 // the 1/2.)  A thread's twiddles are read first, all in flight at once.
-template <int L, int E>
+template <int L, int E, int B>
 __device__ __forceinline__ void r2c_split(const double2* A, int nb, int row0, double2* __restrict__ out, int rows,
                                           const double2* __restrict__ tw, int twLen)
 {
-  constexpr int SL = Row64<L, E>::SL, NT = Row64<L, E>::NT, H = L / 2, KPT = (H + NT - 1) / NT;
+  constexpr int SL = Row64<L, E, B>::SL, NT = Row64<L, E, B>::NT, H = L / 2, KPT = (H + NT - 1) / NT;
   const int twStep = twLen / (2 * L);
   double2 w[KPT];
 #pragma unroll
@@ -446,15 +449,15 @@ __device__ __forceinline__ void r2c_split(const double2* A, int nb, int row0, do
 // on the MY x MX padded grid (FFTW_freespace.cpp:108-119), formed on the fly;
 // else rows of `in`, faded as they are read (cub2rhs, PoissonSolver.cpp:
 // 61-141) and the band cells written back.
-template <int L, bool HIN, int E, bool GREEN>
-__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+template <int L, bool HIN, int E, bool GREEN, int RB>
+__global__ void __launch_bounds__(Row64<L, E, RB>::NT, Row64<L, E, RB>::MINB)
 k_rows_r2c(const double* in, int inStride, int nrows, int ncolsIn, double2* __restrict__ out, int outRows,
            const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen, FadeArgs fa, double h,
            int MX, int MY)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_R2C);
-  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B;
+  constexpr int SL = Row64<L, E, RB>::SL;
   extern __shared__ double2 sm[];
   double2* A = sm;
   const int row0 = blockIdx.x * RB;
@@ -524,7 +527,7 @@ k_rows_r2c(const double* in, int inStride, int nrows, int ncolsIn, double2* __re
   }
   __syncthreads();
   fft_passes<L, E, false, false, false, E>(a, act, j, tb);
-  r2c_split<L, E>(A, nb, row0, out, outRows, tw, twLen);
+  r2c_split<L, E, RB>(A, nb, row0, out, outRows, tw, twLen);
 }
 
 // Column pass (at 4096 points: 172 us for 4097 columns, 280 before the
@@ -609,14 +612,14 @@ __global__ void k_periodic_multiplier(double* __restrict__ g, int nkx, int MX, i
 // values.  The pairs X[k], X[L - k] are read straight into registers and
 // merged: z[k] = s + i t, z[L - k] = conj(s) + i conj(t) with s = X_k +
 // conj(X_(L-k)), t = W^-k (X_k - conj(X_(L-k))), k < L/2; z[L/2] = 2 conj(X_(L/2)).
-template <int L, bool HOUT, int E>
-__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+template <int L, bool HOUT, int E, int RB>
+__global__ void __launch_bounds__(Row64<L, E, RB>::NT, Row64<L, E, RB>::MINB)
 k_rows_c2r(const double2* __restrict__ in, int inRows, int nrows, double* __restrict__ out,
            int outStride, int ncolsOut, const double2* __restrict__ tab, const double2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_C2R);
-  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B, NT = Row64<L, E>::NT, H = L / 2;
+  constexpr int SL = Row64<L, E, RB>::SL, NT = Row64<L, E, RB>::NT, H = L / 2;
   constexpr int KPT = (H + NT - 1) / NT;
   extern __shared__ double2 sm[];
   double2* A = sm;
@@ -694,14 +697,14 @@ __device__ __forceinline__ size_t dct_at(int rows, int r, int c) { return 2 * sp
 template <int L> constexpr int dct_e() { return L >= 1024 ? 16 : 8; }
 
 // rows: fade on load, DCT-II along x of n = 2L values into D
-template <int L, int E>
-__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+template <int L, int E, int RB>
+__global__ void __launch_bounds__(Row64<L, E, RB>::NT, Row64<L, E, RB>::MINB)
 k_dct_rows_fwd(const double* in, int nrows, double* __restrict__ D, const double2* __restrict__ tab,
                const double2* __restrict__ tw, int twLen, FadeArgs fa)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_FWD);
-  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B, NT = Row64<L, E>::NT, n = 2 * L, H = L / 2;
+  constexpr int SL = Row64<L, E, RB>::SL, NT = Row64<L, E, RB>::NT, n = 2 * L, H = L / 2;
   constexpr int PER = (RB * H + NT - 1) / NT;
   extern __shared__ double2 sm[];
   double2* A = sm;
@@ -851,14 +854,14 @@ __global__ void k_dct_multiplier(double* __restrict__ M, int Nx, int Ny, const f
 }
 
 // rows: DCT-III along x from D into p, n = 2L values
-template <int L, int E>
-__global__ void __launch_bounds__(Row64<L, E>::NT, Row64<L, E>::MINB)
+template <int L, int E, int RB>
+__global__ void __launch_bounds__(Row64<L, E, RB>::NT, Row64<L, E, RB>::MINB)
 k_dct_rows_inv(const double* __restrict__ D, int nrows, double* __restrict__ out, const double2* __restrict__ tab,
                const double2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_INV);
-  constexpr int SL = Row64<L, E>::SL, RB = Row64<L, E>::B, NT = Row64<L, E>::NT, n = 2 * L, H = L / 2;
+  constexpr int SL = Row64<L, E, RB>::SL, NT = Row64<L, E, RB>::NT, n = 2 * L, H = L / 2;
   constexpr int KPT = (H + NT - 1) / NT;
   extern __shared__ double2 sm[];
   double2* A = sm;
@@ -910,15 +913,27 @@ void set_smem(const void* f) { if (allow_max_dynamic_smem(f) != cudaSuccess) g_s
 // the cosine solver's column lengths: Ny >= 32
 #define CUP2D_DCT_LENGTHS(X) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048)
 
+// both row counts of a length, once where they are the same
+template <int L, class F> void for_rows(F f) {
+  f(std::integral_constant<int, rows_full<L>()>());
+  if constexpr (rows_full<L>() > ROWS_SMALL) f(std::integral_constant<int, ROWS_SMALL>());
+}
+template <int L> void set_smem_rows() {
+  for_rows<L>([](auto b) {
+    constexpr int B = decltype(b)::value;
+    set_smem((const void*)k_rows_r2c<L, false, 8, false, B>); set_smem((const void*)k_rows_r2c<L, true, 8, false, B>);
+    set_smem((const void*)k_rows_r2c<L, false, 16, false, B>); set_smem((const void*)k_rows_r2c<L, true, 16, false, B>);
+    set_smem((const void*)k_rows_c2r<L, false, 8, B>); set_smem((const void*)k_rows_c2r<L, true, 8, B>);
+    set_smem((const void*)k_rows_c2r<L, false, 16, B>); set_smem((const void*)k_rows_c2r<L, true, 16, B>);
+    set_smem((const void*)k_dct_rows_fwd<L, dct_e<L>(), B>); set_smem((const void*)k_dct_rows_inv<L, 16, B>);
+  });
+  set_smem((const void*)k_rows_r2c<L, false, 8, true, rows_full<L>()>);
+}
+
 void set_all_smem() {
-#define X(L) set_smem((const void*)k_rows_r2c<L, false, 8, false>); set_smem((const void*)k_rows_r2c<L, true, 8, false>); \
-             set_smem((const void*)k_rows_r2c<L, false, 16, false>); set_smem((const void*)k_rows_r2c<L, true, 16, false>); \
-             set_smem((const void*)k_rows_r2c<L, false, 8, true>); \
-             set_smem((const void*)k_rows_c2r<L, false, 8>); set_smem((const void*)k_rows_c2r<L, true, 8>); \
-             set_smem((const void*)k_rows_c2r<L, false, 16>); set_smem((const void*)k_rows_c2r<L, true, 16>); \
+#define X(L) set_smem_rows<L>(); \
              set_smem((const void*)k_cols<L, false, true>); set_smem((const void*)k_cols<L, true, true>); \
-             set_smem((const void*)k_cols<L, false, false>); set_smem((const void*)k_dct_rows_fwd<L, dct_e<L>()>); \
-             set_smem((const void*)k_dct_rows_inv<L, 16>);
+             set_smem((const void*)k_cols<L, false, false>);
   CUP2D_FFT_LENGTHS(X)
 #undef X
 #define X(L) set_smem((const void*)k_dct_cols<L>);
@@ -927,12 +942,21 @@ void set_all_smem() {
   if (!poisson32_setup()) g_smemOk = false;
 }
 
+// Launches a row pass, f(rows per CTA), with the row count of the grid's rows
+template <int L, class F> void with_rows(int nrows, F f) {
+  if constexpr (rows_full<L>() > ROWS_SMALL)
+    if (rows_small<L>(nrows)) { f(std::integral_constant<int, ROWS_SMALL>()); return; }
+  f(std::integral_constant<int, rows_full<L>()>());
+}
+
 template <int LL, int ER>
 void rows_r2c_e(const Poisson& P, cudaStream_t st, const double* in, int nx, int ny, const FadeArgs& fa, bool halfIn) {
-  const int grid = (ny + Row64<LL, ER>::B - 1) / Row64<LL, ER>::B;
-  const auto k = halfIn ? k_rows_r2c<LL, true, ER, false> : k_rows_r2c<LL, false, ER, false>;
-  launch_k(k, grid, Row64<LL, ER>::NT, smem_row64<LL, ER>(), st, in, nx, ny, nx, P.spec, ny, P.tRow[ER == 16], P.tw,
-           P.twLen, fa, 0.0, 0, 0);
+  with_rows<LL>(ny, [&](auto b) {
+    constexpr int B = decltype(b)::value;
+    const auto k = halfIn ? k_rows_r2c<LL, true, ER, false, B> : k_rows_r2c<LL, false, ER, false, B>;
+    launch_k(k, (ny + B - 1) / B, Row64<LL, ER, B>::NT, smem_row64<LL, ER, B>(), st, in, nx, ny, nx, P.spec, ny,
+             P.tRow[ER == 16], P.tw, P.twLen, fa, 0.0, 0, 0);
+  });
 }
 
 // e: elements per thread (8 or 16)
@@ -953,9 +977,9 @@ bool rows_r2c(const Poisson& P, cudaStream_t st, const double* in, int nx, int n
 bool rows_green(const Poisson& P, cudaStream_t st, double h) {
   FadeArgs fa{};
   switch (P.Lrow) {
-#define X(LL) case LL: launch_k(k_rows_r2c<LL, false, 8, true>, (P.MY + Row64<LL, 8>::B - 1) / Row64<LL, 8>::B, \
-        Row64<LL, 8>::NT, smem_row64<LL, 8>(), st, nullptr, 0, P.MY, P.MX, P.spec, P.MY, P.tRow[0], P.tw, P.twLen, \
-        fa, h, P.MX, P.MY); return true;
+#define X(LL) case LL: { constexpr int B = rows_full<LL>(); \
+    launch_k(k_rows_r2c<LL, false, 8, true, B>, (P.MY + B - 1) / B, Row64<LL, 8, B>::NT, smem_row64<LL, 8, B>(), st, \
+             nullptr, 0, P.MY, P.MX, P.spec, P.MY, P.tRow[0], P.tw, P.twLen, fa, h, P.MX, P.MY); return true; }
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }
@@ -989,10 +1013,12 @@ bool cols_green(const Poisson& P, cudaStream_t st, double norm) {
 
 template <int LL, int EC>
 void rows_c2r_e(const Poisson& P, cudaStream_t st, double* out, int nx, int ny, bool halfOut) {
-  const int grid = (ny + Row64<LL, EC>::B - 1) / Row64<LL, EC>::B;
-  const auto k = halfOut ? k_rows_c2r<LL, true, EC> : k_rows_c2r<LL, false, EC>;
-  launch_k(k, grid, Row64<LL, EC>::NT, smem_row64<LL, EC>(), st, P.spec, ny, ny, out, nx, nx, P.tRow[EC == 16], P.tw,
-           P.twLen);
+  with_rows<LL>(ny, [&](auto b) {
+    constexpr int B = decltype(b)::value;
+    const auto k = halfOut ? k_rows_c2r<LL, true, EC, B> : k_rows_c2r<LL, false, EC, B>;
+    launch_k(k, (ny + B - 1) / B, Row64<LL, EC, B>::NT, smem_row64<LL, EC, B>(), st, P.spec, ny, ny, out, nx, nx,
+             P.tRow[EC == 16], P.tw, P.twLen);
+  });
 }
 
 // e: elements per thread (8 or 16)
@@ -1034,10 +1060,11 @@ double2* make_tables(int L, int E, const std::vector<long double>& c, const std:
 
 bool dct_rows_fwd(const Poisson& P, cudaStream_t st, const double* in, int ny, const FadeArgs& fa) {
   switch (P.Lrow) {
-#define X(LL) case LL: { constexpr int E = dct_e<LL>(); \
-    launch_k(k_dct_rows_fwd<LL, E>, (ny + Row64<LL, E>::B - 1) / Row64<LL, E>::B, Row64<LL, E>::NT, \
-             smem_row64<LL, E>(), st, in, ny, reinterpret_cast<double*>(P.spec), P.tRow[E == 16], P.tw, P.twLen, fa); \
-    return true; }
+#define X(LL) case LL: with_rows<LL>(ny, [&](auto b) { \
+    constexpr int E = dct_e<LL>(), B = decltype(b)::value; \
+    launch_k(k_dct_rows_fwd<LL, E, B>, (ny + B - 1) / B, Row64<LL, E, B>::NT, smem_row64<LL, E, B>(), st, in, ny, \
+             reinterpret_cast<double*>(P.spec), P.tRow[E == 16], P.tw, P.twLen, fa); }); \
+    return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }
@@ -1057,9 +1084,11 @@ bool dct_cols(const Poisson& P, cudaStream_t st, int nx) {
 
 bool dct_rows_inv(const Poisson& P, cudaStream_t st, int ny, double* out) {
   switch (P.Lrow) {
-#define X(LL) case LL: launch_k(k_dct_rows_inv<LL, 16>, (ny + Row64<LL, 16>::B - 1) / Row64<LL, 16>::B, \
-                  Row64<LL, 16>::NT, smem_row64<LL, 16>(), st, reinterpret_cast<const double*>(P.spec), ny, out, \
-                  P.tRow[1], P.tw, P.twLen); return true;
+#define X(LL) case LL: with_rows<LL>(ny, [&](auto b) { \
+    constexpr int B = decltype(b)::value; \
+    launch_k(k_dct_rows_inv<LL, 16, B>, (ny + B - 1) / B, Row64<LL, 16, B>::NT, smem_row64<LL, 16, B>(), st, \
+             reinterpret_cast<const double*>(P.spec), ny, out, P.tRow[1], P.tw, P.twLen); }); \
+    return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
   }

@@ -216,42 +216,53 @@ k_vr_init(GridDesc g, const Scalars* sc, const double* __restrict__ P, const dou
 __global__ void __launch_bounds__(1024)
 k_vr_penalize(GridDesc g, const Scalars* sc, const DevShape* sh, int k, ObstTiles t,
               const double* __restrict__ chig, const double* __restrict__ uf, const double* __restrict__ vf,
-              double* fu, double* fv, double* part)
+              double* fu, double* fv, Residual R)
 {
   pdl_begin();
   __shared__ double red[32 * 4];
   const DevShape& S = sh[k];
   const double lambda = 1 / sc->dt;
   double a[4] = {0, 0, 0, 0};                 // MX, MY, DMX, DMY
-  for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
-    const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
+  bool any = false;
+  const int nt = S.ntiles, b0 = first_tile(t);
+  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
+    const int b = s == (int)blockIdx.x ? b0 : t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
     const int ix = threadIdx.x, iy = threadIdx.y;
     const size_t o = (size_t)s * BS2 + iy * BS + ix;
     const size_t c = (size_t)(by * BS + iy) * g.nx + bx * BS + ix;
-    const double X = t.chi[o];
-    if (chig[c] > X) continue;
+    const double X = t.chi[o], Xg = chig[c], uc = uf[c], vc = vf[c], old0 = fu[c], old1 = fv[c];
+    if (Xg > X) continue;
     if (X <= 0) continue;
+    any = true;
     const double p0 = cell_x(g, bx, ix) - S.s.com[0], p1 = cell_y(g, by, iy) - S.s.com[1];
     double ux, uy;
     udef_at(t, o, S, p0, p1, ux, uy);
     const double US = S.s.u - S.s.omega * p1 + ux;
     const double VS = S.s.v + S.s.omega * p0 + uy;
     const double pFac = lambda * X;
-    const double old0 = fu[c], old1 = fv[c];
-    const double new0 = pFac * (US - uf[c]), new1 = pFac * (VS - vf[c]);
+    const double new0 = pFac * (US - uc), new1 = pFac * (VS - vc);
     fu[c] = new0; fv[c] = new1;
     a[0] += new0 * new0; a[2] += (new0 - old0) * (new0 - old0);
     a[1] += new1 * new1; a[3] += (new1 - old1) * (new1 - old1);
   }
-  block_sum<4>(a, red);
-  if (lin_tid() == 0) for (int q = 0; q < 4; q++) part[4 * blockIdx.x + q] = a[q];
+  tile_sum<4>(a, any, red, R.parts + (size_t)k * R.stride + 4 * blockIdx.x);
+  __syncthreads();
+  if (k == R.nsh - 1) relative_change(R, red, nullptr, nullptr, 0);
 }
+
+// Rows per thread of the two full-grid kernels of an iteration: CTAs of 32 x 8
+// threads with four rows each, or, where the grid's blocks leave SMs idle, 32
+// x 32 threads with one (256 x 128, 32 blocks: the right-hand side 11 -> 7 us, the
+// correction 12 -> 8 us, serialised).  The sums keep the order of the
+// four-row form: thread (tx, ty < 8) adds rows ty, ty + 8, ty + 16, ty + 24.
+constexpr int VR_ROWS_BELOW = 296;
 
 // updatePressureRHS (PressureIterator_approx.cpp:289-335):
 // RHS = (1 - rho0 invRho) lap(P) - rho0 (dP/dx dinvRho/dx + dP/dy dinvRho/dy)
 //       + rho0 h/dt (vRHS + dt div F),
 // with the fade sums of the strip blocks for the Poisson solve.
-__global__ void __launch_bounds__(256)
+template <int RPT>
+__global__ void __launch_bounds__(1024 / RPT)
 k_vr_rhs(GridDesc g, const Scalars* sc, double rho0, const double* __restrict__ P,
          const double* __restrict__ ir, const double* __restrict__ fu, const double* __restrict__ fv,
          const double* __restrict__ prhs, double* __restrict__ rhs,
@@ -261,9 +272,10 @@ k_vr_rhs(GridDesc g, const Scalars* sc, double rho0, const double* __restrict__ 
   const double dt = sc->dt, facDiv = rho0 * g.h / dt;
   const int bx = blockIdx.x, by = blockIdx.y, gx = bx * BS + threadIdx.x;
   const bool touch = fade_touch(g, bx, by);
+  __shared__ double tile[RPT == 1 ? BS : 1][BS];
   double s[3] = {0, 0, 0};
 #pragma unroll
-  for (int r = 0; r < 4; r++) {
+  for (int r = 0; r < RPT; r++) {
     const int iy = threadIdx.y + 8 * r, gy = by * BS + iy;
     const size_t c = (size_t)gy * g.nx + gx;
     const double lap = (fdx_at(g, P, gx, gy, 1) - fdx_at(g, P, gx, gy, -1) +
@@ -275,10 +287,21 @@ k_vr_rhs(GridDesc g, const Scalars* sc, double rho0, const double* __restrict__ 
     const double divF = fdx(g, fu, gx, gy) + fdy(g, fv, gx, gy);
     const double b = hatPfac + facDiv * (prhs[c] + dt * divF);
     rhs[c] = b;
-    if (touch) fade_accumulate(g, bx, by, threadIdx.x, iy, b, s);
+    if (RPT == 1) tile[iy][threadIdx.x] = b;
+    else if (touch) fade_accumulate(g, bx, by, threadIdx.x, iy, b, s);
   }
   if (touch) {
     __shared__ double red[96];
+    if (RPT == 1) {
+      __syncthreads();
+      if (threadIdx.y < 8)
+        for (int r = 0; r < 4; r++) {
+          const int iy = threadIdx.y + 8 * r;
+          fade_accumulate(g, bx, by, threadIdx.x, iy, tile[iy][threadIdx.x], s);
+        }
+      tile_sum<3>(s, threadIdx.y < 8, red, fadePartials + 3 * fadeSlot[bx + g.bpdx * by]);
+      return;
+    }
     block_sum<3>(s, red);
     if (lin_tid() == 0) {
       const int q = fadeSlot[bx + g.bpdx * by];
@@ -292,21 +315,23 @@ k_vr_rhs(GridDesc g, const Scalars* sc, double rho0, const double* __restrict__ 
 // the sums of (Pcur - P)^2 and Pcur^2; the last CTA forms
 // relDP = sqrt(DP / max(EPS, NP)).  FINAL: finalizePressure (:337-376),
 // V += dt F + pFac (...) instead.
-template <bool FINAL>
-__global__ void __launch_bounds__(256)
+template <bool FINAL, int RPT>
+__global__ void __launch_bounds__(1024 / RPT)
 k_vr_pcorr(GridDesc g, Scalars* sc, double iRho0, const double* __restrict__ Pcur,
            const double* __restrict__ P, const double* __restrict__ ir, double* u, double* v,
            double* __restrict__ uf, double* __restrict__ vf, const double* __restrict__ fu,
-           const double* __restrict__ fv, double* partials, unsigned* counter)
+           const double* __restrict__ fv, double* partials, unsigned* counter, double* relOut,
+           unsigned long long* seqOut, unsigned long long seqVal)
 {
   pdl_begin();
   __shared__ double red[64];
+  __shared__ double2 tile[RPT == 1 && !FINAL ? BS : 1][BS];
   const double dt = sc->dt, pFac = -dt / g.h;
   const int gx = blockIdx.x * BS + threadIdx.x;
   double s[2] = {0, 0};
 #pragma unroll
-  for (int r = 0; r < 4; r++) {
-    const int gy = blockIdx.y * BS + threadIdx.y + 8 * r;
+  for (int r = 0; r < RPT; r++) {
+    const int iy = threadIdx.y + 8 * r, gy = blockIdx.y * BS + iy;
     const size_t c = (size_t)gy * g.nx + gx;
     const double dUdiv = fdx(g, P, gx, gy) * (ir[c] - iRho0);
     const double dVdiv = fdy(g, P, gx, gy) * (ir[c] - iRho0);
@@ -319,22 +344,37 @@ k_vr_pcorr(GridDesc g, Scalars* sc, double iRho0, const double* __restrict__ Pcu
       uf[c] = u[c] + pFac * (dUpre + dUdiv);
       vf[c] = v[c] + pFac * (dVpre + dVdiv);
       const double dp = Pcur[c] - P[c];
-      s[0] += dp * dp;
-      s[1] += Pcur[c] * Pcur[c];
+      if (RPT == 1) tile[iy][threadIdx.x] = make_double2(dp * dp, Pcur[c] * Pcur[c]);
+      else { s[0] += dp * dp; s[1] += Pcur[c] * Pcur[c]; }
     }
   }
   if (FINAL) return;
+  if (RPT == 1) {
+    __syncthreads();
+    if (threadIdx.y < 8)
+      for (int r = 0; r < 4; r++) {
+        const double2 q = tile[threadIdx.y + 8 * r][threadIdx.x];
+        s[0] += q.x; s[1] += q.y;
+      }
+  }
   block_sum<2>(s, red);
   const unsigned nb = gridDim.x * gridDim.y, bid = blockIdx.x + gridDim.x * blockIdx.y;
   if (lin_tid() == 0) { partials[2 * bid] = s[0]; partials[2 * bid + 1] = s[1]; }
   if (!last_block_done(counter, nb)) return;
   double t[2] = {0, 0};
-  for (unsigned i = lin_tid(); i < nb; i += 256) {
-    t[0] += __ldcg(&partials[2 * i]);
-    t[1] += __ldcg(&partials[2 * i + 1]);
-  }
+  if (lin_tid() < 256)
+    for (unsigned i = lin_tid(); i < nb; i += 256) {
+      t[0] += __ldcg(&partials[2 * i]);
+      t[1] += __ldcg(&partials[2 * i + 1]);
+    }
   block_sum<2>(t, red);
-  if (lin_tid() == 0) sc->it.relDP = sqrt(t[0] / fmax(EPSd, t[1]));
+  if (lin_tid() == 0) {
+    const double rel = sqrt(t[0] / fmax(EPSd, t[1]));
+    sc->it.relDP = rel;
+    relOut[0] = sc->it.relDF;                   // to mapped host memory, for the convergence test
+    relOut[1] = rel;
+    signal_host(seqOut, seqVal);
+  }
 }
 
 inline int fill_grid(const Ctx& c) {
@@ -377,35 +417,31 @@ void launch_vr_init(Ctx& c) {
 }
 
 void launch_vr_penalize(Ctx& c) {
-  PenalCtas nc{};
+  const Residual R = residual(c);
   for (int k = 0; k < c.nshapes; k++) {
-    nc.n[k] = tile_ctas(c, c.tiles[k].capacity);
-    launch_k(k_vr_penalize, nc.n[k], dim3(32, 32), 0, c.stream, c.g, (const Scalars*)c.dsc,
+    launch_k(k_vr_penalize, R.nc.n[k], dim3(32, 32), 0, c.stream, c.g, (const Scalars*)c.dsc,
              (const DevShape*)c.dshapes, k, c.tiles[k], (const double*)c.chi, (const double*)c.ifluid[0],
-             (const double*)c.ifluid[1], c.itmp[0], c.itmp[1], shape_partials(c) + (size_t)k * shape_region(c));
+             (const double*)c.ifluid[1], c.itmp[0], c.itmp[1], R);
     CUP2D_LAUNCHED(c);
   }
-  launch_reldf(c, nc);
 }
 
 void launch_vr_rhs(Ctx& c) {
-  launch_k(k_vr_rhs, dim3(c.g.bpdx, c.g.bpdy), dim3(32, 8), 0, c.stream, c.g, (const Scalars*)c.dsc, c.rho0,
-           (const double*)c.pres, (const double*)c.invRho, (const double*)c.itmp[0], (const double*)c.itmp[1],
-           (const double*)c.prhs, c.rhs, (const int*)c.fadeSlot, fade_partials(c));
+  const bool one = c.g.nblocks < VR_ROWS_BELOW;
+  launch_k(one ? k_vr_rhs<1> : k_vr_rhs<4>, dim3(c.g.bpdx, c.g.bpdy), dim3(32, one ? 32 : 8), 0, c.stream, c.g,
+           (const Scalars*)c.dsc, c.rho0, (const double*)c.pres, (const double*)c.invRho, (const double*)c.itmp[0],
+           (const double*)c.itmp[1], (const double*)c.prhs, c.rhs, (const int*)c.fadeSlot, fade_partials(c));
   CUP2D_LAUNCHED(c);
 }
 
-void launch_vr_pcorr(Ctx& c, bool final_) {
-  const dim3 grid(c.g.bpdx, c.g.bpdy), block(32, 8);
-  const double iRho0 = 1 / c.rho0;
-  if (final_)
-    launch_k(k_vr_pcorr<true>, grid, block, 0, c.stream, c.g, c.dsc, iRho0, (const double*)c.rhs,
-             (const double*)c.pres, (const double*)c.invRho, c.u(), c.v(), c.ifluid[0], c.ifluid[1],
-             (const double*)c.itmp[0], (const double*)c.itmp[1], c.partials, c.counters + CNT_ADV);
-  else
-    launch_k(k_vr_pcorr<false>, grid, block, 0, c.stream, c.g, c.dsc, iRho0, (const double*)c.rhs,
-             (const double*)c.pres, (const double*)c.invRho, c.u(), c.v(), c.ifluid[0], c.ifluid[1],
-             (const double*)c.itmp[0], (const double*)c.itmp[1], c.partials, c.counters + CNT_ADV);
+void launch_vr_pcorr(Ctx& c, bool final_, unsigned long long seqVal) {
+  const bool one = c.g.nblocks < VR_ROWS_BELOW;
+  const auto k = final_ ? (one ? k_vr_pcorr<true, 1> : k_vr_pcorr<true, 4>)
+                        : (one ? k_vr_pcorr<false, 1> : k_vr_pcorr<false, 4>);
+  launch_k(k, dim3(c.g.bpdx, c.g.bpdy), dim3(32, one ? 32 : 8), 0, c.stream, c.g, c.dsc, 1 / c.rho0,
+           (const double*)c.rhs, (const double*)c.pres, (const double*)c.invRho, c.u(), c.v(), c.ifluid[0],
+           c.ifluid[1], (const double*)c.itmp[0], (const double*)c.itmp[1], c.partials, c.counters + CNT_ADV,
+           &c.mapDev->relDF, &c.mapDev->seqIter, seqVal);
   CUP2D_LAUNCHED(c);
 }
 

@@ -20,7 +20,7 @@ def context(bpdx, bpdy, solver, tune):
 
 
 @pytest.mark.parametrize("bpdx,bpdy,solver", [
-    (1, 1, "freespace"), (2, 1, "freespace"), (3, 2, "freespace"), (4, 5, "freespace"), (8, 16, "freespace"),
+    (1, 1, "freespace"), (2, 1, "freespace"), (3, 2, "freespace"), (4, 5, "freespace"), (8, 16, "freespace"), (8, 20, "freespace"), (16, 10, "freespace"),
     (17, 9, "freespace"), (33, 31, "freespace"), (64, 33, "freespace"), (65, 40, "freespace"), (128, 64, "freespace"),
     (1, 1, "periodic"), (2, 4, "periodic"), (8, 2, "periodic"), (16, 64, "periodic"), (128, 16, "periodic"),
     (1, 1, "cosine"), (2, 8, "cosine"), (8, 2, "cosine"), (32, 4, "cosine"), (16, 32, "cosine"),
