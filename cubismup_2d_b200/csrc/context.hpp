@@ -190,8 +190,8 @@ enum CounterSlot : int {
   CNT_MOMENTS = 56,     // + shape
   CNT_MOMENTA = 72,     // + shape
 };
-// partials: [0, 3 nblocks) the grid reductions (findMaxU, advDiff's outflow,
-// the fade sums: three per strip block), then 4096 spare, then the
+// partials: [0, 3 nblocks) the grid reductions (findMaxU,
+// the fade sums: three per strip block), then 4096 (advDiff's outflow), then the
 // per-shape tile reductions
 inline double* fade_partials(const Ctx& c) { return c.partials; }
 
@@ -213,6 +213,9 @@ inline size_t shape_region(const Ctx& c) { return (size_t)c.maxCapacity * 24; }
 // CTAs per shape of the per-tile kernels: one wave at most; each CTA loops
 // over tiles s = blockIdx.x, blockIdx.x + gridDim.x, ... < ntiles
 inline int tile_ctas(const Ctx& c, int capacity) { return capacity < c.sms ? capacity : c.sms; }
+// advDiff's outflow partials, at most one per SM (the spare region: the
+// update that reads them writes the fade sums)
+inline double* outflow_partials(const Ctx& c) { return c.partials + (size_t)3 * c.g.nblocks; }
 inline double* shape_partials(const Ctx& c) { return c.partials + (size_t)3 * c.g.nblocks + 4096; }
 inline Residual residual(const Ctx& c) {
   Residual R{c.dsc, c.nshapes, {}, shape_partials(c), (int)shape_region(c), c.counters + CNT_RELDF};

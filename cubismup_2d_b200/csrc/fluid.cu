@@ -139,10 +139,12 @@ __device__ __forceinline__ void adv_cell(const GridDesc& g, const AdvCoef& k, co
 // values depend on the old velocity only, so they are formed here, before
 // the update, with the update's own arithmetic (adv_cell).  Item k walks
 // the west column (-u), the east column (+u), the south row (-v) and the
-// north row (+v); the CTA sums, then the last CTA sums those in block order.
+// north row (+v); one partial sum per CTA.  The update's CTAs on the edge add
+// the partials themselves while their tiles load: a last CTA here would add
+// a ticket and a second reduction to the chain before the update.
 __global__ void __launch_bounds__(256)
 k_outflow_flux(GridDesc g, const Scalars* sc, const double* __restrict__ u, const double* __restrict__ v,
-               double* partials, unsigned* counter, Scalars* scw)
+               double* parts, Scalars* scw)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_ADVDIFF);
@@ -170,13 +172,7 @@ k_outflow_flux(GridDesc g, const Scalars* sc, const double* __restrict__ u, cons
   }
   double s1[1] = {IF};
   block_sum<1>(s1, red);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s1[0];
-  if (!last_block_done(counter, gridDim.x)) return;
-  double t1[1] = {0.0};
-  for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) t1[0] += __ldcg(&partials[i]);
-  block_sum<1>(t1, red);
-  if (threadIdx.x == 0)                                   // advDiff.cpp:105
-    scw->outflowCorr = t1[0] / (2 * (BS * g.bpdy - 0) + 2 * (BS * g.bpdx - 0));
+  if (threadIdx.x == 0) parts[blockIdx.x] = s1[0];
 }
 
 // adv_cell on the staged tile: U, V hold the block's cells and a two-cell
@@ -296,8 +292,10 @@ __global__ void __launch_bounds__(256, 4)
 k_advdiff(const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmV,
           GridDesc g, Scalars* sc, unsigned txBytes,
           double* __restrict__ un, double* __restrict__ vn,
-          double* __restrict__ rhs, const int* __restrict__ fadeSlot, double* __restrict__ fadePartials)
+          double* __restrict__ rhs, const int* __restrict__ fadeSlot, double* __restrict__ fadePartials,
+          const double* __restrict__ parts, int nparts)
 {
+  __shared__ double sCorr;
   __shared__ __align__(128) double tU[ADV_HT * ADV_HT];
   __shared__ __align__(128) double tV[ADV_HT * ADV_HT];
   __shared__ __align__(8) unsigned long long bar;
@@ -321,10 +319,12 @@ k_advdiff(const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUten
   kc.fadeW = sc->advCoef[2]; kc.fadeS = sc->advCoef[3];
   kc.fadeE = sc->advCoef[4]; kc.fadeN = sc->advCoef[5];
   kc.U0 = sc->uinfx; kc.U1 = sc->uinfy;
-  const double corr = sc->outflowCorr;
   const double facDiv = sc->facDiv;
-  const int nx = g.nx, ny = g.ny;
-  const int gx = bx * BS + tx;
+  if (ty == 1 && (bx == 0 || by == 0 || bx == g.bpdx - 1 || by == g.bpdy - 1)) {
+    double t[1];
+    warp_sum_rows<1>(parts, nparts, 1, t);
+    if (tx == 0) sCorr = t[0] / (2 * (BS * g.bpdy - 0) + 2 * (BS * g.bpdx - 0));   // advDiff.cpp:105
+  }
   // one thread waits for the tiles (the others at the CTA barrier, where
   // they take no issue slots); its acquire of the barrier's phase and the
   // CTA barrier make the tiles visible to every thread
@@ -341,9 +341,9 @@ k_advdiff(const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUten
   }
   // blocks away from the domain edge: no ghost, outflow or one-sided tests
   if (bx > 0 && by > 0 && bx < g.bpdx - 1 && by < g.bpdy - 1)
-    advdiff_tile_body<false>(g, kc, tU, tV, su, sv, corr, facDiv, un, vn, rhs, fadeSlot, fadePartials);
+    advdiff_tile_body<false>(g, kc, tU, tV, su, sv, 0.0, facDiv, un, vn, rhs, fadeSlot, fadePartials);
   else
-    advdiff_tile_body<true>(g, kc, tU, tV, su, sv, corr, facDiv, un, vn, rhs, fadeSlot, fadePartials);
+    advdiff_tile_body<true>(g, kc, tU, tV, su, sv, sCorr, facDiv, un, vn, rhs, fadeSlot, fadePartials);
 }
 
 // PressureSingle.cpp:112-128: tmp = (h / 2dt) * div_2h(u); zero-gradient ghosts
@@ -594,19 +594,21 @@ void launch_end_step_dt(Ctx& c, double* dtOut, unsigned long long* seqOut, unsig
   CUP2D_LAUNCHED(c);
 }
 
+namespace {
+int outflow_ctas(const Ctx& c) { return std::min((2 * (c.g.nx + c.g.ny) + 255) / 256, c.sms); }
+} // namespace
+
 void launch_outflow_flux(Ctx& c) {
-  const int items = 2 * (c.g.nx + c.g.ny);
-  int grid = (items + 255) / 256;
-  if (grid > c.sms) grid = c.sms;
-  launch_k(k_outflow_flux, grid, 256, 0, c.stream, c.g, (const Scalars*)c.dsc, (const double*)c.u(),
-           (const double*)c.v(), c.partials, c.counters + CNT_ADV, c.dsc);
+  launch_k(k_outflow_flux, outflow_ctas(c), 256, 0, c.stream, c.g, (const Scalars*)c.dsc, (const double*)c.u(),
+           (const double*)c.v(), outflow_partials(c), c.dsc);
   CUP2D_LAUNCHED(c);
 }
 
 void launch_advdiff_rhs_div(Ctx& c) {
   dim3 grid(c.g.bpdx, c.g.bpdy), block(32, 8);
   launch_k(k_advdiff, grid, block, 0, c.stream, c.tmVel[c.cur][0], c.tmVel[c.cur][1], c.g, c.dsc, c.advTx,
-           c.uo(), c.vo(), c.rhs, (const int*)c.fadeSlot, fade_partials(c));
+           c.uo(), c.vo(), c.rhs, (const int*)c.fadeSlot, fade_partials(c),
+           (const double*)outflow_partials(c), outflow_ctas(c));
   CUP2D_LAUNCHED(c);
   c.cur = 1 - c.cur;
 }
