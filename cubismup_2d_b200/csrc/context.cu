@@ -558,6 +558,8 @@ int cup2d_destroy(cup2d_ctx* ctx) {
   Ctx& c = ctx->c;
   for (cup2d_ctx* sh : c.gaitShadows) cup2d_destroy(sh);
   c.gaitShadows.clear();
+  for (const Ctx::Chunk& k : c.adjChunks) cudaFree(k.p);
+  c.adjChunks.clear();
   if (c.stream) cudaStreamSynchronize(c.stream);
   invalidate_graph(c);
   for (int b = 0; b < 2; b++) for (int d = 0; d < 2; d++) cudaFree(c.vel[b][d]);

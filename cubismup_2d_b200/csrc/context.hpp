@@ -151,6 +151,12 @@ struct Ctx {
   std::vector<int> shapeKinds;
   std::vector<struct cup2d_ctx*> gaitShadows;
 
+  // device scratch of cup2d_adjoint_run, kept between calls up to ADJ_KEEP
+  // bytes (freed with the context)
+  struct Chunk { char* p; size_t bytes, used; };
+  std::vector<Chunk> adjChunks;
+  static constexpr size_t ADJ_KEEP = (size_t)1 << 30;
+
   cudaGraphExec_t graph = nullptr;
   void* flushBuf = nullptr;      // cup2d_time_kernel's L2 flush (256 MB, allocated on demand)
   unsigned long long* hashAcc = nullptr;   // checkpoint checksum accumulator (on demand)
