@@ -500,6 +500,7 @@ k_collide(GridDesc g, const Scalars* sc, DevShape* sh, int nsh, AllTiles T)
   CUP2D_TRACE_SCOPE(TR_COLLIDE);
   __shared__ double red[32 * 10];
   __shared__ double coll[MAX_SHAPES][10];
+  __shared__ int shared[1024];                // shape j's slot of the tiles of shape i, a chunk at a time
   const int tid = threadIdx.x;
   for (int i = 0; i < nsh; i++) {
     double a[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -509,10 +510,17 @@ k_collide(GridDesc g, const Scalars* sc, DevShape* sh, int nsh, AllTiles T)
       const double iUl = Si.s.u, iVl = Si.s.v, iW = Si.s.omega;
       const double jUl = Sj.s.u, jVl = Sj.s.v, jW = Sj.s.omega;
       const double iCx = Si.s.com[0], iCy = Si.s.com[1], jCx = Sj.s.com[0], jCy = Sj.s.com[1];
-      for (int s = 0; s < Si.ntiles; s++) {
-        const int b = T.t[i].tiles[s];
-        const int sj = T.t[j].slot[b];
+      const int nt = Si.ntiles;
+      for (int s0 = 0; s0 < nt; s0 += 1024) {
+      // one look-up per thread (a loop over the tiles had waited for two
+      // dependent loads each, mostly to find that no tile is shared)
+      const int mine = s0 + tid < nt ? T.t[j].slot[T.t[i].tiles[s0 + tid]] : -1;
+      shared[tid] = mine;
+      if (!__syncthreads_or(mine >= 0)) continue;
+      for (int s = s0; s < min(nt, s0 + 1024); s++) {
+        const int sj = shared[s - s0];
         if (sj < 0) continue;
+        const int b = T.t[i].tiles[s];
         const int bx = b % g.bpdx, by = b / g.bpdx, ix = tid % BS, iy = tid / BS;
         const double iChi = T.t[i].chi[(size_t)s * BS2 + tid], jChi = T.t[j].chi[(size_t)sj * BS2 + tid];
         if (iChi <= 0 || jChi <= 0) continue;
@@ -528,6 +536,8 @@ k_collide(GridDesc g, const Scalars* sc, DevShape* sh, int nsh, AllTiles T)
         a[5] += jChi; a[6] += jChi * p0; a[7] += jChi * p1;
         a[8] += jChi * (jUl + jUr + ju0);
         a[9] += jChi * (jVl + jVr + ju1);
+      }
+      __syncthreads();
       }
     }
     block_sum<10>(a, red);
