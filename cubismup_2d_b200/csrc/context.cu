@@ -245,7 +245,7 @@ void enqueue_step(Ctx& c) {
   // that any kernel beside it slows (measured: even the 12-CTA outflow flux),
   // while the rasters after it leave most SMs free; with disks only, from
   // the step's start (advDiff reads no obstacle data)
-  c.recordPlaced = anyFish;
+  c.recordPlaced = anyFish && c.g.nblocks < ADV_FIRST_BLOCKS;
   if (!c.recordPlaced) cudaEventRecord(c.evPlaced, c.stream);
   launch_objects_rest(c);
   c.recordPlaced = false;
@@ -888,8 +888,8 @@ int cup2d_put_objects(cup2d_ctx* ctx, double dt) {
   if (anyFishShape) CK(cudaEventRecord(c.evFork, c.stream));
   launch_objects_begin(c, false);
   if (c.nshapes > 0) {
-    c.recordPlaced = anyFishShape;
-    if (!anyFishShape) CK(cudaEventRecord(c.evPlaced, c.stream));
+    c.recordPlaced = anyFishShape && c.g.nblocks < ADV_FIRST_BLOCKS;
+    if (!c.recordPlaced) CK(cudaEventRecord(c.evPlaced, c.stream));
     launch_objects_rest(c);
     c.recordPlaced = false;
   }

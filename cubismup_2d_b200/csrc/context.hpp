@@ -216,6 +216,11 @@ struct PenalCtas { int n[MAX_SHAPES]; };
 struct Residual { Scalars* sc; int nsh; PenalCtas nc; double* parts; int stride; unsigned* counter; };
 // doubles of one shape's tile-reduction region
 inline size_t shape_region(const Ctx& c) { return (size_t)c.maxCapacity * 24; }
+// advDiff reads no obstacle data.  Beside a fish's placement it slows the
+// one-CTA frame kernel, so it starts once the tiles are placed; on grids
+// where it takes longer than the whole obstacle chain it starts with the
+// step instead (4096 x 2048: 8 + 70 us against 46; 2048 x 1024: 8 + 22 against 38).
+constexpr int ADV_FIRST_BLOCKS = 4096;
 // CTAs per shape of the per-tile kernels: one wave at most; each CTA loops
 // over tiles s = blockIdx.x, blockIdx.x + gridDim.x, ... < ntiles
 inline int tile_ctas(const Ctx& c, int capacity) { return capacity < c.sms ? capacity : c.sms; }
