@@ -956,7 +956,7 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
   double* lx = obv + 1;                      // the body-velocity adjoint (see above)
   double* lxPrev = obv + 4;
   double* lb = obv + 8;
-  const int tctas = tile_ctas(c, cap);
+  const int tctas = tile_ctas(c, c.maxExpect);
   for (int s = nseg - 1; s >= 0; s--) {
     const int i0 = s * every, i1 = std::min(nsteps, i0 + every);
     ALOAD(s);

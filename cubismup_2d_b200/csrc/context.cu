@@ -669,6 +669,10 @@ int cup2d_add_shape(cup2d_ctx* ctx, int kind, const cup2d_shape_params* p, int* 
   S.rhoTile = kind == CUP2D_SHAPE_DISK ? f.rhoS : 1.0;
   ObstTiles t{};
   t.capacity = cap;
+  // a disk's rectangle of blocks; a fish's length and amplitude at any angle
+  const int along = (int)std::ceil((kind == CUP2D_SHAPE_DISK ? 2 * f.radius : f.length) / (BS * h)) + 2;
+  t.expect = std::min(cap, kind == CUP2D_SHAPE_DISK ? along * along : 4 * along);
+  c.maxExpect = std::max(c.maxExpect, t.expect);
   int rc = dalloc(ctx, &t.tiles, cap);
   if (!rc) rc = dalloc(ctx, &t.slot, c.g.nblocks);
   double** arrs[] = {&t.chi, &t.dist, &t.udx, &t.udy, &t.sD, &t.sdx, &t.sdy};

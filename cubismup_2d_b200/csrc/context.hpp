@@ -51,6 +51,7 @@ struct Ctx {
   std::vector<FishArrays> fish;
   int nshapes = 0;
   int maxCapacity = 0;
+  int maxExpect = 0;
 
   // reduction scratch: per-CTA partial sums and "last CTA" tickets
   double* partials = nullptr;
@@ -219,18 +220,23 @@ inline size_t shape_region(const Ctx& c) { return (size_t)c.maxCapacity * 24; }
 // advDiff reads no obstacle data.  Beside a fish's placement it slows the
 // one-CTA frame kernel, so it starts once the tiles are placed; on grids
 // where it takes longer than the whole obstacle chain it starts with the
-// step instead (4096 x 2048: 8 + 70 us against 46; 2048 x 1024: 8 + 22 against 38).
-constexpr int ADV_FIRST_BLOCKS = 4096;
-// CTAs per shape of the per-tile kernels: one wave at most; each CTA loops
-// over tiles s = blockIdx.x, blockIdx.x + gridDim.x, ... < ntiles
-inline int tile_ctas(const Ctx& c, int capacity) { return capacity < c.sms ? capacity : c.sms; }
+// step instead (us a step, after the placement and from the start: 4096 x 2048
+// 537 and 517, 2048 x 2048 302 and 290, 2048 x 1024 175 and 172, 1024 x 1024 120
+// and 120).
+constexpr int ADV_FIRST_BLOCKS = 2048;
+// CTAs per shape of the per-tile kernels: as many as the body usually touches
+// tiles, one wave at most; each CTA loops over tiles s = blockIdx.x, blockIdx.x
+// + gridDim.x, ... < ntiles.  A swimmer's capacity (its bounding square, 324
+// tiles at 205 cells) had launched 148 CTAs of 1024 threads for some 30 tiles:
+// they delay whatever runs beside them, the other members of an ensemble most.
+inline int tile_ctas(const Ctx& c, int expect) { return expect < c.sms ? expect : c.sms; }
 // advDiff's outflow partials, at most one per SM (the spare region: the
 // update that reads them writes the fade sums)
 inline double* outflow_partials(const Ctx& c) { return c.partials + (size_t)3 * c.g.nblocks; }
 inline double* shape_partials(const Ctx& c) { return c.partials + (size_t)3 * c.g.nblocks + 4096; }
 inline Residual residual(const Ctx& c) {
   Residual R{c.dsc, c.nshapes, {}, shape_partials(c), (int)shape_region(c), c.counters + CNT_RELDF};
-  for (int k = 0; k < c.nshapes; k++) R.nc.n[k] = tile_ctas(c, c.tiles[k].capacity);
+  for (int k = 0; k < c.nshapes; k++) R.nc.n[k] = tile_ctas(c, c.tiles[k].expect);
   return R;
 }
 #ifdef __CUDACC__

@@ -151,6 +151,7 @@ struct ObstTiles {
   double* sdx;                    // dchidx = -D * gradUX (ObstacleBlock.h:98)
   double* sdy;
   int capacity;
+  int expect;                     // tiles the body usually touches (sizes the launches)
 };
 
 // One fish midline (the arrays of FishLibrary.h:49-60); the two step

@@ -734,7 +734,7 @@ void launch_objects_begin(Ctx& c, bool midlineReady) {
   if (c.nshapes == 0) return;
   // the last step's tiles reset and the body motion first: the midline
   // reads neither (a graph step runs them side by side)
-  launch_k(k_obj_begin, tile_ctas(c, c.maxCapacity), 256, 0, c.stream, 
+  launch_k(k_obj_begin, tile_ctas(c, c.maxExpect), 256, 0, c.stream, 
       c.g, c.dsc, c.dshapes, c.nshapes, all_tiles(c), c.chi, c.sdf);
   CUP2D_LAUNCHED(c);
   // fish midlines at the current time (Fish.cpp:79-95) unless the previous
@@ -773,7 +773,6 @@ void launch_step_begin(Ctx& c) {
 void launch_objects_rest(Ctx& c) {
   if (c.nshapes == 0) return;
   const AllTiles T = all_tiles(c);
-  const int cap = c.maxCapacity;
   bool anyDisk = false, anyFish = false;
   for (int k = 0; k < c.nshapes; k++) {
     if (c.hshapes[k].cfg.kind == CUP2D_SHAPE_DISK) anyDisk = true; else anyFish = true;
@@ -783,7 +782,7 @@ void launch_objects_rest(Ctx& c) {
     if (c.hshapes[k].cfg.kind != CUP2D_SHAPE_DISK) launch_fish_place(c, k);
   if (c.recordPlaced) cudaEventRecord(c.evPlaced, c.stream);
   if (anyDisk) {
-    launch_k(k_raster_disk, dim3(tile_ctas(c, cap), c.nshapes), dim3(32, 32), 0, c.stream, c.g, c.dsc, c.dshapes, T,
+    launch_k(k_raster_disk, dim3(tile_ctas(c, c.maxExpect), c.nshapes), dim3(32, 32), 0, c.stream, c.g, c.dsc, c.dshapes, T,
              c.sdf);
     CUP2D_LAUNCHED(c);
   }
@@ -791,7 +790,7 @@ void launch_objects_rest(Ctx& c) {
     for (int k = 0; k < c.nshapes; k++)
       if (c.hshapes[k].cfg.kind != CUP2D_SHAPE_DISK) launch_fish_raster(c, k);
   const int stride = (int)shape_region(c);
-  launch_k(k_chi_moments, dim3(tile_ctas(c, cap), c.nshapes), dim3(32, 32), 0, c.stream, c.g, c.dshapes, T,
+  launch_k(k_chi_moments, dim3(tile_ctas(c, c.maxExpect), c.nshapes), dim3(32, 32), 0, c.stream, c.g, c.dshapes, T,
            (const double*)c.sdf, c.chi, shape_partials(c), stride, c.counters + CNT_MOMENTS);
   CUP2D_LAUNCHED(c);
 }
@@ -803,7 +802,7 @@ void launch_objects(Ctx& c, bool midlineReady) {
 
 void launch_obj_vel_on_grid(Ctx& c) {
   for (int k = 0; k < c.nshapes; k++) {
-    launch_k(k_udef_grid, tile_ctas(c, c.tiles[k].capacity), dim3(32, 32), 0, c.stream, c.g, c.dshapes, k, c.tiles[k],
+    launch_k(k_udef_grid, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, c.g, c.dshapes, k, c.tiles[k],
                                                                    c.chi, c.udefx, c.udefy);
     CUP2D_LAUNCHED(c);
   }
@@ -811,13 +810,13 @@ void launch_obj_vel_on_grid(Ctx& c) {
 
 void launch_rhs_obstacles(Ctx& c) {
   for (int k = 0; k < c.nshapes; k++) {
-    launch_k(k_rhs_obst, tile_ctas(c, c.tiles[k].capacity), dim3(32, 32), 0, c.stream, 
+    launch_k(k_rhs_obst, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, 
         c.g, c.dshapes, k, c.tiles[k], c.chi, c.rhs, shape_partials(c) + (size_t)k * shape_region(c),
         c.counters + CNT_RHSOBST + k);
     CUP2D_LAUNCHED(c);
   }
   for (int k = 0; k < c.nshapes; k++) {
-    launch_k(k_rhs_corr, tile_ctas(c, c.tiles[k].capacity), dim3(32, 32), 0, c.stream, c.g, c.dshapes, k, c.tiles[k],
+    launch_k(k_rhs_corr, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, c.g, c.dshapes, k, c.tiles[k],
              (const double*)c.chi, c.rhs, (const int*)c.fadeSlot, fade_partials(c));
     CUP2D_LAUNCHED(c);
   }
@@ -825,7 +824,7 @@ void launch_rhs_obstacles(Ctx& c) {
 
 void launch_momenta(Ctx& c, const double* ui, const double* vi) {
   if (c.nshapes == 0) return;
-  launch_k(k_momenta<false>, dim3(tile_ctas(c, c.maxCapacity), c.nshapes), 1024, 0, c.stream, 
+  launch_k(k_momenta<false>, dim3(tile_ctas(c, c.maxExpect), c.nshapes), 1024, 0, c.stream, 
       c.g, c.dsc, c.dshapes, all_tiles(c), c.pres, ui, vi, shape_partials(c), (int)shape_region(c),
       c.counters + CNT_MOMENTA);
   CUP2D_LAUNCHED(c);
@@ -833,14 +832,14 @@ void launch_momenta(Ctx& c, const double* ui, const double* vi) {
 
 void launch_momenta_varrho(Ctx& c, const double* ui, const double* vi) {
   if (c.nshapes == 0) return;
-  launch_k(k_momenta<false, true>, dim3(tile_ctas(c, c.maxCapacity), c.nshapes), 1024, 0, c.stream,
+  launch_k(k_momenta<false, true>, dim3(tile_ctas(c, c.maxExpect), c.nshapes), 1024, 0, c.stream,
       c.g, c.dsc, c.dshapes, all_tiles(c), (const double*)nullptr, ui, vi, shape_partials(c), (int)shape_region(c),
       c.counters + CNT_MOMENTA);
   CUP2D_LAUNCHED(c);
 }
 void launch_momenta_iter(Ctx& c, const double* ui, const double* vi) {
   if (c.nshapes == 0) return;
-  launch_k(k_momenta<true>, dim3(tile_ctas(c, c.maxCapacity), c.nshapes), 1024, 0, c.stream, 
+  launch_k(k_momenta<true>, dim3(tile_ctas(c, c.maxExpect), c.nshapes), 1024, 0, c.stream, 
       c.g, c.dsc, c.dshapes, all_tiles(c), c.pres, ui, vi, shape_partials(c), (int)shape_region(c),
       c.counters + CNT_MOMENTA);
   CUP2D_LAUNCHED(c);
@@ -872,7 +871,7 @@ void launch_collide_penalize(Ctx& c) {
     CUP2D_LAUNCHED(c);
   }
   for (int k = 0; k < c.nshapes; k++) {
-    launch_k(k_penalize, tile_ctas(c, c.tiles[k].capacity), dim3(32, 32), 0, c.stream, c.g,
+    launch_k(k_penalize, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, c.g,
              (const Scalars*)c.dsc, (const DevShape*)c.dshapes, k, c.tiles[k], (const double*)c.chi, c.u(), c.v());
     CUP2D_LAUNCHED(c);
   }
@@ -882,7 +881,7 @@ void launch_forces(Ctx& c, cup2d_shape_state* out, bool maxNext, unsigned long l
                    unsigned long long seqVal, bool endStep) {
   if (c.nshapes == 0) return;
   const AllTiles T = all_tiles(c);
-  launch_k(k_forces, dim3(tile_ctas(c, c.maxCapacity), c.nshapes), dim3(32, 32), 0, c.stream,
+  launch_k(k_forces, dim3(tile_ctas(c, c.maxExpect), c.nshapes), dim3(32, 32), 0, c.stream,
       c.g, c.dsc, maxNext ? 1 : 0, c.dshapes, T, (const double*)c.u(), (const double*)c.v(),
       (const double*)c.pres, shape_partials(c), (int)shape_region(c), c.counters + CNT_FORCES, out,
       seqOut, seqVal, endStep ? c.counters + CNT_STEP : (unsigned*)nullptr);

@@ -388,7 +388,7 @@ void launch_invrho(Ctx& c) {
   launch_k(k_invrho_fill, fill_grid(c), 256, 0, c.stream, c.ncells(), c.invRho);
   CUP2D_LAUNCHED(c);
   for (int k = 0; k < c.nshapes; k++) {
-    launch_k(k_invrho_blend, tile_ctas(c, c.tiles[k].capacity), dim3(32, 32), 0, c.stream, c.g,
+    launch_k(k_invrho_blend, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, c.g,
              (const DevShape*)c.dshapes, k, all_tiles(c), c.invRho);
     CUP2D_LAUNCHED(c);
   }
