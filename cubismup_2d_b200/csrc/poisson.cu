@@ -41,7 +41,7 @@ struct Poisson {
   int Lrow = 0;          // complex FFT length of the row passes (M/2)
   int Lcol = 0;          // complex FFT length of the column pass
   int nkx = 0;           // spectrum columns (Lrow + 1)
-  double2* spec = nullptr;   // the half spectrum: FP64 in column pairs (spec_at), FP32 [Lcol rows][nkx]
+  double2* spec = nullptr;   // the half spectrum: in groups of columns (spec_at; FP32: spec32_at)
   // FP64: the column pass's multiplier [nkx][Lcol/2 + 1], the free-space
   // kernel or the periodic -1/|k|^2, halved (r2c_split writes twice the
   // spectrum); cosine: its multiplier [Nx][Ny]; a column's values are consecutive
@@ -52,7 +52,7 @@ struct Poisson {
   double2* tCol = nullptr;                 // and of the column transforms
   bool fp32 = false;         // CUP2D_PREC_FP32: float2 spectrum in spec, FP32 passes
   float2* tw32 = nullptr;    // tw rounded to FP32
-  float* ghat32 = nullptr;   // the free-space kernel rounded to FP32, [Lcol/2 + 1][nkx]
+  float* ghat32 = nullptr;   // the free-space kernel rounded to FP32, [nkx][Lcol/2 + 1]
   int rb = 1, cb = 1;        // rows / columns per CTA
   int MX = 0, MY = 0;        // free space: the padded grid (powers of two >= 2Nx, 2Ny)
   // elements per thread of the forward and inverse row passes (FP64 free
@@ -1217,9 +1217,7 @@ Poisson* poisson_create(Ctx& c) {
       if (cudaStreamSynchronize(c.stream) != cudaSuccess ||
           cudaMemcpy(g64.data(), P->ghat, sizeof(double) * ng, cudaMemcpyDeviceToHost) != cudaSuccess ||
           cudaMalloc(&P->ghat32, sizeof(float) * ng) != cudaSuccess) { poisson_destroy(P); return nullptr; }
-      const size_t gn = (size_t)P->Lcol / 2 + 1;
-      for (size_t k = 0; k < (size_t)P->nkx; k++)
-        for (size_t r = 0; r < gn; r++) g32[r * P->nkx + k] = (float)(2 * g64[k * gn + r]);
+      for (size_t i = 0; i < ng; i++) g32[i] = (float)(2 * g64[i]);
       h2d_sync(P->ghat32, g32.data(), sizeof(float) * ng, c.stream);
     }
   }
@@ -1254,7 +1252,7 @@ void poisson_rows_fwd(Ctx& c) {
   }
   // free space: the row's zero padding is the upper half of the length-Lrow sequence
   if (P->fp32)
-    rows_r2c32(P->Lrow, c.stream, c.rhs, Nx, Ny, Nx, reinterpret_cast<float2*>(P->spec), P->nkx, P->tw32,
+    rows_r2c32(P->Lrow, c.stream, c.rhs, Nx, Ny, Nx, reinterpret_cast<float2*>(P->spec), Ny, P->tw32,
                P->twLen, fa, P->type == CUP2D_POISSON_FREESPACE);
   else
     rows_r2c(*P, c.stream, c.rhs, Nx, Ny, fa, P->type == CUP2D_POISSON_FREESPACE, P->eR2C);
@@ -1268,14 +1266,14 @@ void poisson_cols(Ctx& c) {
     dct_cols(*P, c.stream, Nx);
   } else if (P->type == CUP2D_POISSON_FREESPACE) {
     if (P->fp32)
-      cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), P->nkx, P->nkx, Ny, Ny, P->ghat32, 0,
+      cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), Ny, P->nkx, Ny, Ny, P->ghat32, 0,
              P->tw32, P->twLen, 0.0, 0, 0);
     else
       cols(*P, c.stream, Ny, true);
   } else {
     const double norm = 1.0 / ((double)Nx * (double)Ny);
     if (P->fp32)
-      cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), P->nkx, P->nkx, Ny, Ny, nullptr, 2,
+      cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), Ny, P->nkx, Ny, Ny, nullptr, 2,
              P->tw32, P->twLen, norm, Nx, Ny);
     else
       cols(*P, c.stream, Ny, false);
@@ -1292,7 +1290,7 @@ void poisson_rows_inv(Ctx& c) {
     return;
   }
   if (P->fp32)
-    rows_c2r32(P->Lrow, c.stream, reinterpret_cast<const float2*>(P->spec), P->nkx, Ny, c.pres, Nx, Nx,
+    rows_c2r32(P->Lrow, c.stream, reinterpret_cast<const float2*>(P->spec), Ny, Ny, c.pres, Nx, Nx,
                P->tw32, P->twLen, P->type == CUP2D_POISSON_FREESPACE);
   else
     rows_c2r(*P, c.stream, c.pres, Nx, Ny, P->type == CUP2D_POISSON_FREESPACE, P->eC2R);        // free space keeps the first half

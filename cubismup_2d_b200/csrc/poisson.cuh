@@ -116,10 +116,10 @@ __device__ __forceinline__ double fade_cell(double row, double col, double b, do
 // poisson32.cu: the FP32 passes of the free-space and periodic solves
 bool poisson32_setup();                              // shared-memory limits of its kernels
 bool rows_r2c32(int L, cudaStream_t st, const double* in, int inStride, int nrows, int ncolsIn, float2* out,
-                int outStride, const float2* tw, int twLen, FadeArgs fa, bool halfIn);
-bool cols32(int L, cudaStream_t st, float2* data, int stride, int ncols, int nrowsIn, int nrowsOut,
+                int outRows, const float2* tw, int twLen, FadeArgs fa, bool halfIn);
+bool cols32(int L, cudaStream_t st, float2* data, int rows, int ncols, int nrowsIn, int nrowsOut,
             const float* ghat, int mode, const float2* tw, int twLen, double norm, int MXp, int MYp);
-bool rows_c2r32(int L, cudaStream_t st, const float2* in, int inStride, int nrows, double* out, int outStride,
+bool rows_c2r32(int L, cudaStream_t st, const float2* in, int inRows, int nrows, double* out, int outStride,
                 int ncolsOut, const float2* tw, int twLen, bool halfOut);
 
 } // namespace cup2d

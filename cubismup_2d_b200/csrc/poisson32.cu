@@ -10,6 +10,16 @@
 namespace cup2d {
 namespace {
 
+// The half spectrum lies in groups of eight columns, 64 bytes a row, as the
+// FP64 one does in groups of four (spec_at in poisson.cu): a column pass then
+// touches 16 lines for 32 rows instead of 32, and the kernel G^ lies by columns.
+// Column pass on B200: 180 -> 145 us at 4096 x 2048, 70 -> 45 at 2048 x 1024, 17.2 -> 14.3
+// at 1024 x 512 (row passes unchanged).
+constexpr int SPEC32_LOG = 3;
+__device__ __forceinline__ size_t spec32_at(int rows, int r, int k) {
+  return (((size_t)(k >> SPEC32_LOG) * rows + r) << SPEC32_LOG) | (k & ((1 << SPEC32_LOG) - 1));
+}
+
 // Per transform length L: padded stride SL of one sequence (one spare
 // element per 16, plus 4 so that consecutive sequences start in different
 // halves of the shared-memory banks), the staged quarter twiddle table
@@ -320,7 +330,7 @@ __device__ __forceinline__ void fft_convolve(C* A, int nseq, const C* tws, Mul m
 // inside the loop, every iteration waited for its own).
 template <int L, int ER, class C>
 __device__ __forceinline__ void r2c_split(const C* A, int nb, int row0, C* __restrict__ out,
-                                          int outStride, const C* __restrict__ tw, int twLen)
+                                          int outRows, const C* __restrict__ tw, int twLen)
 {
   using R = typename CT<C>::R;
   constexpr int SL = Len<L, ER>::SL, NT = Len<L, ER>::NT, KPT = (L + 1 + NT - 1) / NT;
@@ -344,7 +354,7 @@ __device__ __forceinline__ void r2c_split(const C* A, int nb, int row0, C* __res
         const C Fe = mk<C>(R(0.5) * (Zk.x + Zc.x), R(0.5) * (Zk.y + Zc.y));
         const C d = csub(Zk, Zc);
         const C Fo = mk<C>(R(0.5) * d.y, R(-0.5) * d.x);  // (Zk - Zc) / (2i)
-        out[(size_t)(row0 + r) * outStride + k] = cadd(Fe, cmul(w[q], Fo));
+        out[spec32_at(outRows, row0 + r, k)] = cadd(Fe, cmul(w[q], Fo));
       }
     }
   }
@@ -353,7 +363,7 @@ __device__ __forceinline__ void r2c_split(const C* A, int nb, int row0, C* __res
 template <int L, bool HIN>
 __global__ void __launch_bounds__(Len<L, E_ROWS32>::NT, Len<L, E_ROWS32>::MINB)
 k_rows_r2c32(const double* __restrict__ in, int inStride, int nrows, int ncolsIn,
-             float2* __restrict__ out, int outStride, const float2* __restrict__ tw, int twLen, FadeArgs fa)
+             float2* __restrict__ out, int outRows, const float2* __restrict__ tw, int twLen, FadeArgs fa)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_R2C);
@@ -404,14 +414,14 @@ k_rows_r2c32(const double* __restrict__ in, int inStride, int nrows, int ncolsIn
   }
   __syncthreads();
   fft_inplace<L, false, HIN, false, E_ROWS32>(A, nb, tws);
-  r2c_split<L, E_ROWS32>(A, nb, row0, out, outStride, tw, twLen);
+  r2c_split<L, E_ROWS32>(A, nb, row0, out, outRows, tw, twLen);
 }
 
 // mode 0: forward, x G^, inverse, keep nrowsOut rows; mode 2: the periodic
 // multiplier -1/|k|^2 / (MX MY) (formed in FP64, applied in FP32)
 template <int L, bool FS>
 __global__ void __launch_bounds__(Len<L, E_COLS32>::NT, Len<L, E_COLS32>::MINB)
-k_cols32(float2* __restrict__ data, int stride, int ncols, int nrowsIn, int nrowsOut,
+k_cols32(float2* __restrict__ data, int rows, int ncols, int nrowsIn, int nrowsOut,
          const float* __restrict__ ghat, int mode, const float2* __restrict__ tw, int twLen,
          double norm, int MXp, int MYp)
 {
@@ -426,12 +436,12 @@ k_cols32(float2* __restrict__ data, int stride, int ncols, int nrowsIn, int nrow
   const int nb = min(CB, ncols - c0);
   for (int idx = threadIdx.x; idx < CB * nrowsIn; idx += NT) {
     const int r = idx / CB, j = idx & (CB - 1);
-    if (j < nb) cp_async8(A + j * SL + pad(r), data + (size_t)r * stride + c0 + j);
+    if (j < nb) cp_async8(A + j * SL + pad(r), data + spec32_at(rows, r, c0 + j));
   }
   if (mode == 0)
     for (int idx = threadIdx.x; idx < CB * GR; idx += NT) {
-      const int r = idx / CB, j = idx & (CB - 1);
-      if (j < nb) cp_async4(Gs + r * CB + j, ghat + (size_t)r * stride + c0 + j);
+      const int j = idx / GR, r = idx - j * GR;
+      if (j < nb) cp_async4(Gs + r * CB + j, ghat + (size_t)(c0 + j) * GR + r);
     }
   cp_async_commit();
   // rows beyond the input are zero; the free-space solve never reads its
@@ -463,7 +473,7 @@ k_cols32(float2* __restrict__ data, int stride, int ncols, int nrowsIn, int nrow
   }
   for (int idx = threadIdx.x; idx < CB * nrowsOut; idx += NT) {
     const int r = idx / CB, j = idx & (CB - 1);
-    if (j < nb) data[(size_t)r * stride + c0 + j] = A[j * SL + pad(r)];
+    if (j < nb) data[spec32_at(rows, r, c0 + j)] = A[j * SL + pad(r)];
   }
 }
 
@@ -471,7 +481,7 @@ k_cols32(float2* __restrict__ data, int stride, int ncols, int nrowsIn, int nrow
 // ncolsOut values in FP64
 template <int L, bool HOUT>
 __global__ void __launch_bounds__(Len<L, E_C2R32>::NT, Len<L, E_C2R32>::MINB)
-k_rows_c2r32(const float2* __restrict__ in, int inStride, int nrows, double* __restrict__ out, int outStride,
+k_rows_c2r32(const float2* __restrict__ in, int inRows, int nrows, double* __restrict__ out, int outStride,
              int ncolsOut, const float2* __restrict__ tw, int twLen)
 {
   pdl_begin();
@@ -485,7 +495,7 @@ k_rows_c2r32(const float2* __restrict__ in, int inStride, int nrows, double* __r
   const int twStep = twLen / (2 * L);
   for (int idx = threadIdx.x; idx < RB * (L + 1); idx += NT) {
     const int r = idx / (L + 1), k = idx - r * (L + 1);
-    if (r < nb) cp_async8(A + r * SL + pad(k), in + (size_t)(row0 + r) * inStride + k);
+    if (r < nb) cp_async8(A + r * SL + pad(k), in + spec32_at(inRows, row0 + r, k));
   }
   cp_async_commit();
   load_twiddles<L, E_C2R32>(tws, tw, twLen);
@@ -558,13 +568,13 @@ bool poisson32_setup() {
 }
 
 bool rows_r2c32(int L, cudaStream_t st, const double* in, int inStride, int nrows, int ncolsIn,
-                float2* out, int outStride, const float2* tw, int twLen, FadeArgs fa, bool halfIn) {
+                float2* out, int outRows, const float2* tw, int twLen, FadeArgs fa, bool halfIn) {
   switch (L) {
 #define X(LL) case LL: \
     if (halfIn) launch_k(k_rows_r2c32<LL, true>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_ROWS32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outStride, tw, twLen, fa); \
+        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outRows, tw, twLen, fa); \
     else launch_k(k_rows_r2c32<LL, false>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_ROWS32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outStride, tw, twLen, fa); \
+        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outRows, tw, twLen, fa); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -572,15 +582,15 @@ bool rows_r2c32(int L, cudaStream_t st, const double* in, int inStride, int nrow
   return false;
 }
 
-bool cols32(int L, cudaStream_t st, float2* data, int stride, int ncols, int nrowsIn, int nrowsOut,
+bool cols32(int L, cudaStream_t st, float2* data, int rows, int ncols, int nrowsIn, int nrowsOut,
             const float* ghat, int mode, const float2* tw, int twLen, double norm, int MXp, int MYp) {
   switch (L) {
 #define X(LL) case LL: \
     if (mode == 0) launch_k(k_cols32<LL, true>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS32>::NT, \
-        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, stride, ncols, nrowsIn, nrowsOut, \
+        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, rows, ncols, nrowsIn, nrowsOut, \
         ghat, mode, tw, twLen, norm, MXp, MYp); \
     else launch_k(k_cols32<LL, false>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS32>::NT, \
-        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, stride, ncols, nrowsIn, nrowsOut, \
+        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, rows, ncols, nrowsIn, nrowsOut, \
         ghat, mode, tw, twLen, norm, MXp, MYp); \
     return true;
     CUP2D_FFT_LENGTHS(X)
@@ -589,14 +599,14 @@ bool cols32(int L, cudaStream_t st, float2* data, int stride, int ncols, int nro
   return false;
 }
 
-bool rows_c2r32(int L, cudaStream_t st, const float2* in, int inStride, int nrows, double* out, int outStride,
+bool rows_c2r32(int L, cudaStream_t st, const float2* in, int inRows, int nrows, double* out, int outStride,
                 int ncolsOut, const float2* tw, int twLen, bool halfOut) {
   switch (L) {
 #define X(LL) case LL: \
     if (halfOut) launch_k(k_rows_c2r32<LL, true>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_C2R32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, out, outStride, ncolsOut, tw, twLen); \
+        smem_for32<LL>(), st, in, inRows, nrows, out, outStride, ncolsOut, tw, twLen); \
     else launch_k(k_rows_c2r32<LL, false>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_C2R32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, out, outStride, ncolsOut, tw, twLen); \
+        smem_for32<LL>(), st, in, inRows, nrows, out, outStride, ncolsOut, tw, twLen); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
