@@ -20,9 +20,9 @@
 //   here each CTA walks the points of the block's segments in the
 //   reference's loop order (segment, s index, side or width offset), keeps
 //   those whose support reaches its 16x16 cells, and every cell applies them
-//   in that order, so its "keep the
-//   nearest" updates (ties included) and its hat-kernel sums see exactly the
-//   reference's sequence.
+//   so that its "keep the nearest" updates (ties included) end with the point
+//   of the reference's sequence; its hat-kernel sums take every other point
+//   in each of two threads.
 #include <cmath>
 #include "context.hpp"
 #include "fish.cuh"
@@ -623,9 +623,9 @@ struct IntPt { double ud[2], w[2][2]; int iap[2]; };
 
 constexpr int SUB = 16;                     // cells per sub-tile edge
 constexpr int NSUB = (BS / SUB) * (BS / SUB);
-constexpr int RT = SUB * SUB;               // threads per CTA (one per cell)
+constexpr int RT = 2 * SUB * SUB;           // threads per CTA: two per cell, a warp per row
 constexpr int NWARP = RT / 32;
-constexpr int CH = 4;                       // candidate points per thread and chunk
+constexpr int CH = 2;                       // candidate points per thread and chunk
 constexpr int CAP = RT * CH;                // points per chunk
 constexpr int MAX_SEG_PER_TILE = 256;
 constexpr int WU = 4;                       // list entries a cell evaluates at a time
@@ -671,38 +671,34 @@ __device__ __forceinline__ int find_range(const int* start, int n, int q) {
   return lo;
 }
 
-// Half-row lists: warp w owns the sub-tile rows 2w (lanes 0-15) and 2w+1
-// (lanes 16-31), each split into two halves of 8 columns, i.e. four lists
-// (list 2*row + half).  The warp walks the chunk's kept points in order, 32
-// at a time, and appends (ballot + popc, so order is kept) those whose
-// support covers the list's row and reaches its half.  Every cell then
-// visits only its half-row's points, in the reference's order, and skips
-// those whose columns miss it.
+// Half-row lists: warp w owns the sub-tile row w, split into two halves of 8
+// columns, i.e. two lists (list 2*row + half).  The warp walks the chunk's
+// kept points in order, 32 at a time, and appends (ballot + popc, so order is
+// kept) those whose support covers the list's row and reaches its half.
+// Every cell then visits only its half-row's points and skips those whose
+// columns miss it; its two threads take every other entry.
 constexpr int NLIST = 2 * SUB;
 
 __device__ __forceinline__ void rows_build(unsigned short* rowIdx, int* rowN, const uchar4* supp, int nc) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int n[4] = {0, 0, 0, 0};
+  int n[2] = {0, 0};
   for (int p0 = 0; p0 < nc; p0 += 32) {
     const int p = p0 + lane;
-    bool in[4] = {false, false, false, false};
+    bool in[2] = {false, false};
     if (p < nc) {
       const uchar4 sp = supp[p];          // x lo, x hi, y lo, y hi relative to the sub-tile
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int r = 2 * w + (q >> 1), h0 = 8 * (q & 1);
-        in[q] = sp.z <= r && r < sp.w && sp.x < h0 + 8 && h0 < sp.y;
-      }
+      for (int q = 0; q < 2; q++) in[q] = sp.z <= w && w < sp.w && sp.x < 8 * q + 8 && 8 * q < sp.y;
     }
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < 2; q++) {
       const unsigned m = __ballot_sync(0xffffffffu, in[q]);
-      if (in[q]) rowIdx[(4 * w + q) * CAP + n[q] + __popc(m & lt)] = (unsigned short)p;
+      if (in[q]) rowIdx[(2 * w + q) * CAP + n[q] + __popc(m & lt)] = (unsigned short)p;
       n[q] += __popc(m);
     }
   }
-  if (lane < 4) rowN[4 * w + lane] = lane == 0 ? n[0] : lane == 1 ? n[1] : lane == 2 ? n[2] : n[3];
+  if (lane < 2) rowN[2 * w + lane] = lane == 0 ? n[0] : n[1];
   __syncwarp();
 }
 
@@ -743,6 +739,10 @@ inline size_t raster_smem(int Nm) {
   return sizeof(double) * RSTAGE * (size_t)Nm + pts + sizeof(uchar4) * CAP + sizeof(unsigned short) * NLIST * CAP;
 }
 
+// Bound by latency: a swimmer of 205 cells has some 32 sub-tiles of up to 1200
+// candidate points.  Two threads per cell halve the candidates per thread, the
+// rows per warp and the list entries per thread: 22 -> 15 us in the graph at
+// 1024 x 512 (one thread per cell before).
 __global__ void __launch_bounds__(RT)
 k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, double* sdfg)
 {
@@ -786,7 +786,8 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
   CUP2D_TRACE_MARK(wi, 0);
   const int b = t.tiles[s], bx = b % g.bpdx, by = b / g.bpdx;
   const int sx0 = (sub % (BS / SUB)) * SUB, sy0 = (sub / (BS / SUB)) * SUB;
-  const int ix = sx0 + tid % SUB, iy = sy0 + tid / SUB;
+  const int cell = tid >> 1, part = tid & 1;            // the cell's threads are neighbouring lanes
+  const int ix = sx0 + cell % SUB, iy = sy0 + cell / SUB;
   const int row = iy - sy0, col = ix - sx0;
   const double org0 = cell_x(g, bx, 0), org1 = cell_y(g, by, 0);
 
@@ -822,12 +823,19 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
     }
   }
   const int nsl = nSegList < MAX_SEG_PER_TILE ? nSegList : MAX_SEG_PER_TILE;
-  if (tid == 0) {
-    surfStart[0] = 0; intStart[0] = 0;
-    for (int i = 0; i < nsl; i++) {
-      surfStart[i + 1] = surfStart[i] + segSurfCnt[i];
-      intStart[i + 1] = intStart[i] + segIntCnt[i];
+  if (tid < 32) {                                       // running sums of the counts
+    int cs = 0, ci = 0;
+    for (int i0 = 0; i0 < nsl; i0 += 32) {
+      const int i = i0 + tid;
+      int a = i < nsl ? segSurfCnt[i] : 0, c = i < nsl ? segIntCnt[i] : 0;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, c, o);
+        if (tid >= o) { a += x; c += y; }
+      }
+      if (i < nsl) { surfStart[i + 1] = cs + a; intStart[i + 1] = ci + c; }
+      cs += __shfl_sync(0xffffffffu, a, 31); ci += __shfl_sync(0xffffffffu, c, 31);
     }
+    if (tid == 0) { surfStart[0] = 0; intStart[0] = 0; }
   }
   __syncthreads();
   const int totSurf = surfStart[nsl], totInt = intStart[nsl];
@@ -839,7 +847,9 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
   // distM) is below |dist|, and then |dist| becomes dist1 (sign2d is +-1):
   // the cell ends with the first point, in the reference's order, attaining
   // the strict running minimum, so the sign, weight and velocity are
-  // evaluated once, for that point.
+  // evaluated once, for that point.  The cell's two threads each find theirs
+  // among every other entry; the lower distance, or the earlier entry of two
+  // equal ones, is the point that one pass would have kept.
   double dist = -1, chi = 0, ud0 = 0, ud1 = 0;
   double best = 1.0;                                    // |dist| of the initial -1
   for (int c0 = 0; c0 < totSurf; c0 += CAP) {
@@ -897,16 +907,16 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
     const int li = 2 * row + (col >> 3);                // this cell's half-row list
     const int n = rowN[li];
     const unsigned short* l = rowIdx + li * CAP;
-    int winner = -1;
+    int winner = -1, winE = 0x7fffffff;
     // WU list entries at a time: their loads and distances are independent,
     // the running minimum then takes them in list order
-    for (int e0 = 0; e0 < n; e0 += WU) {
+    for (int e0 = part; e0 < n; e0 += 2 * WU) {
       double d1[WU];
       int qs[WU];
       bool ok[WU];
 #pragma unroll
       for (int u = 0; u < WU; u++) {
-        const int e = e0 + u;
+        const int e = e0 + 2 * u;
         qs[u] = l[e < n ? e : e0];
         const uchar4 sp = supp[qs[u]];
         ok[u] = e < n && col >= sp.x && col < sp.y;
@@ -918,7 +928,12 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
       }
 #pragma unroll
       for (int u = 0; u < WU; u++)
-        if (ok[u] && best > d1[u]) { best = d1[u]; winner = qs[u]; }
+        if (ok[u] && best > d1[u]) { best = d1[u]; winner = qs[u]; winE = e0 + 2 * u; }
+    }
+    {
+      const double bo = __shfl_xor_sync(0xffffffffu, best, 1);
+      const int wo = __shfl_xor_sync(0xffffffffu, winner, 1), eo = __shfl_xor_sync(0xffffffffu, winE, 1);
+      if (wo >= 0 && (bo < best || (bo == best && eo < winE))) { best = bo; winner = wo; }
     }
     if (winner >= 0) {
       // evaluate the winner of this chunk now (its point data is in shared
@@ -967,7 +982,10 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
   }
 
   CUP2D_TRACE_MARK(wi, 2);
-  // constructInternl (FishLibrary.cpp:575-638)
+  // constructInternl (FishLibrary.cpp:575-638); each of the cell's threads sums
+  // every other entry, the first on top of the surface's values
+  if (part) { ud0 = 0; ud1 = 0; chi = 0; }
+  bool inside = false;
   for (int c0 = 0; c0 < totInt; c0 += CAP) {
     int2 sw[CH];                                      // (ss, iw) of the candidate
     double2 xw[CH];
@@ -1019,12 +1037,12 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
     const int li = 2 * row + (col >> 3);                // this cell's half-row list
     const int n = rowN[li];
     const unsigned short* l = rowIdx + li * CAP;
-    for (int e0 = 0; e0 < n; e0 += WU) {
+    for (int e0 = part; e0 < n; e0 += 2 * WU) {
       double w[WU], a0[WU], a1[WU];
       bool ok[WU];
 #pragma unroll
       for (int u = 0; u < WU; u++) {
-        const int e = e0 + u;
+        const int e = e0 + 2 * u;
         const int qi = l[e < n ? e : e0];
         const uchar4 sp = supp[qi];
         ok[u] = e < n && col >= sp.x && col < sp.y;
@@ -1040,20 +1058,29 @@ k_fish_raster(GridDesc g, const DevShape* sh, int k, ObstTiles t, FishArrays F, 
           ud0 += w[u] * a0[u];
           ud1 += w[u] * a1[u];
           chi += w[u];
-          if (fabs(dist + 1) < EPSd) dist = 1;
+          inside = true;
         }
     }
     __syncthreads();
   }
 
   CUP2D_TRACE_MARK(wi, 3);
+  ud0 += __shfl_xor_sync(0xffffffffu, ud0, 1);
+  ud1 += __shfl_xor_sync(0xffffffffu, ud1, 1);
+  chi += __shfl_xor_sync(0xffffffffu, chi, 1);
+  inside |= __shfl_xor_sync(0xffffffffu, (int)inside, 1) != 0;
+  if (inside && fabs(dist + 1) < EPSd) dist = 1;
   // signedDistanceSqrt (FishLibrary.cpp:419-436)
   const double normfac = chi > EPSd ? chi : 1;
   ud0 /= normfac; ud1 /= normfac;
   dist = dist >= 0 ? sqrt(dist) : -sqrt(-dist);
   const size_t o = (size_t)s * BS2 + iy * BS + ix;
-  t.dist[o] = dist; t.chi[o] = 0; t.udx[o] = ud0; t.udy[o] = ud1;
-  atomic_max_double(&sdfg[(size_t)(by * BS + iy) * g.nx + bx * BS + ix], dist);
+  if (part == 0) {
+    t.dist[o] = dist; t.chi[o] = 0;
+    atomic_max_double(&sdfg[(size_t)(by * BS + iy) * g.nx + bx * BS + ix], dist);
+  } else {
+    t.udx[o] = ud0; t.udy[o] = ud1;
+  }
   __syncthreads();                                      // shared state is reused by the next item
   CUP2D_TRACE_MARK(wi, 4);
 #ifdef CUP2D_TRACE
