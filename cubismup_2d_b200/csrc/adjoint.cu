@@ -36,6 +36,13 @@
 // schedule, or one given): it is not differentiated.  The gait gradient
 // contracts each step's sensitivity to the body's geometry with central
 // differences of the placement (see k_adj_geo_pen).
+//
+// A transposed step's kernels take 1-4 us each on the grids in use, so what
+// bounds it is the gaps between them: they are launched with programmatic
+// stream serialization like the forward's, their reductions are zeroed once
+// for all steps, and advDiff's boundary sum is formed by the kernel that
+// writes its input.  512x256, disk, 20 steps, mean drag: forward 2.3 -> 2.0
+// ms (no read-back a step, see k_adj_record), backward 3.5 -> 3.0 ms.
 #include <algorithm>
 #include <array>
 #include <cfloat>
@@ -87,6 +94,7 @@ __global__ void __launch_bounds__(256)
 k_adj_grad_T(GridDesc g, double pFac, const double* __restrict__ lu, const double* __restrict__ lv,
              double* __restrict__ lp)
 {
+  pdl_begin();
   const int gx = blockIdx.x * BS + threadIdx.x;
   for (int r = 0; r < 4; r++) {
     const Nb j = nb_of(g, gx, blockIdx.y * BS + threadIdx.y + 8 * r);
@@ -94,13 +102,19 @@ k_adj_grad_T(GridDesc g, double pFac, const double* __restrict__ lu, const doubl
   }
 }
 
-// (lu, lv) += facDiv D^T lr: the RHS divergence's transpose
+// (lu, lv) += facDiv D^T lr: the RHS divergence's transpose; the CTAs at the
+// domain's edge add up the result's Gamma = sum of sigma lambda over the
+// boundary cells (sigma: +1 on the W column / S row, -1 on the E column / N
+// row; u on the columns, v on the rows): the transpose of advDiff's rank-one
+// outflow correction
 __global__ void __launch_bounds__(256)
 k_adj_div_T(GridDesc g, double facDiv, const double* __restrict__ lr, double* __restrict__ lu,
-            double* __restrict__ lv)
+            double* __restrict__ lv, double* gamma)
 {
+  pdl_begin();
   const int gx = blockIdx.x * BS + threadIdx.x;
   const int nx = g.nx, ny = g.ny;
+  double a = 0;
   for (int r = 0; r < 4; r++) {
     const Nb j = nb_of(g, gx, blockIdx.y * BS + threadIdx.y + 8 * r);
     double ax = 0, ay = 0;
@@ -112,9 +126,17 @@ k_adj_div_T(GridDesc g, double facDiv, const double* __restrict__ lr, double* __
     if (j.y == ny - 1) ay += lr[j.c];
     if (j.y <= ny - 2) ay -= lr[j.c + nx];
     if (j.y == 0) ay -= lr[j.c];
-    lu[j.c] += facDiv * ax;
-    lv[j.c] += facDiv * ay;
+    const double U = lu[j.c] + facDiv * ax, V = lv[j.c] + facDiv * ay;
+    lu[j.c] = U;
+    lv[j.c] = V;
+    if (j.x == 0) a += U;
+    if (j.x == nx - 1) a -= U;
+    if (j.y == 0) a += V;
+    if (j.y == ny - 1) a -= V;
   }
+  if (blockIdx.x > 0 && blockIdx.x + 1 < gridDim.x && blockIdx.y > 0 && blockIdx.y + 1 < gridDim.y) return;
+  a = warp_sum(a);
+  if (threadIdx.x == 0 && a != 0) atomicAdd(gamma, a);
 }
 
 // Pen^T: lambda *= 1 - chi where the shape owns the cell (penalize's
@@ -125,6 +147,7 @@ __global__ void __launch_bounds__(1024)
 k_adj_pen(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
           double* lu, double* lv, double* gb)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   const double Cx = S.s.com[0], Cy = S.s.com[1];
   double a[3] = {0, 0, 0};
@@ -154,6 +177,7 @@ k_adj_pen(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __re
 // symmetric: lb = A^-1 lx, by the forward's own LU.
 __global__ void k_adj_solve(const DevShape* sh, int k, const double* lx, double* lb)
 {
+  pdl_begin();
   const cup2d_shape_state& s = sh[k].s;
   double A[3][3] = {{s.penalM, 0, -s.penalDY}, {0, s.penalM, s.penalDX}, {-s.penalDY, s.penalDX, s.penalJ}};
   const double b[3] = {lx[0], lx[1], lx[2]};
@@ -167,6 +191,7 @@ __global__ void __launch_bounds__(1024)
 k_adj_momenta(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ lb,
               double* lu, double* lv)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   const double Cx = S.s.com[0], Cy = S.s.com[1];
   const double l0 = lb[0], l1 = lb[1], l2 = lb[2];
@@ -186,6 +211,7 @@ k_adj_momenta(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* 
 // the objective's body-velocity weights of a step, added to lx
 __global__ void k_adj_add3(double* lx, double a, double b, double c)
 {
+  pdl_begin();
   lx[0] += a; lx[1] += b; lx[2] += c;
 }
 
@@ -200,6 +226,7 @@ __global__ void __launch_bounds__(1024)
 k_adj_force(GridDesc g, const DevShape* sh, int k, ObstTiles t, double wx, double wy, double wt, int part,
             double* lu, double* lv, double* lp)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   const double Cx = S.s.com[0], Cy = S.s.com[1];
   for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
@@ -227,13 +254,20 @@ k_adj_force(GridDesc g, const DevShape* sh, int k, ObstTiles t, double wx, doubl
 }
 
 // the objective's body terms of a step: acc += wx forcex + wy forcey + wt
-// |torque| + wb . (u, v, omega) of the state the step left; *tau = torque
-__global__ void k_adj_body_sum(const DevShape* sh, int k, double wx, double wy, double wt, double wb0,
-                               double wb1, double wb2, double* acc, double* tau)
+// |torque| + wb . (u, v, omega) of the state the step left (terms: there are
+// any); and what the backward step needs of it: the torque and the lab
+// velocity the placement set from the forced body.  Kept on the device until
+// the forward has ended: read back step by step they cost a wait for the
+// whole step, and the next one's launches were no longer hidden.
+struct StepRecord { double torque, uinfx, uinfy; };
+__global__ void k_adj_record(const DevShape* sh, int k, const Scalars* sc, bool terms, double wx, double wy,
+                             double wt, double wb0, double wb1, double wb2, double* acc, StepRecord* rec)
 {
+  pdl_begin();
   const cup2d_shape_state& s = sh[k].s;
-  *acc += wx * s.forcex + wy * s.forcey + wt * fabs(s.torque) + (wb0 * s.u + wb1 * s.v + wb2 * s.omega);
-  *tau = s.torque;
+  if (terms)
+    *acc += wx * s.forcex + wy * s.forcey + wt * fabs(s.torque) + (wb0 * s.u + wb1 * s.v + wb2 * s.omega);
+  *rec = {s.torque, sc->uinfx, sc->uinfy};
 }
 
 // ---- the obstacle RHS terms O (k_rhs_obst, k_rhs_corr) --------------------
@@ -263,6 +297,7 @@ __global__ void __launch_bounds__(1024)
 k_adj_obst_sums(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
                 const double* __restrict__ T, const double* __restrict__ lo, double* acc)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   double a[5] = {0, 0, 0, 0, 0};
   for (int s = blockIdx.x; s < S.ntiles; s += gridDim.x) {
@@ -286,6 +321,7 @@ __global__ void __launch_bounds__(1024)
 k_adj_obst_apply(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
                  const double* __restrict__ T, double* lo, const double* __restrict__ acc)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   const double s = acc[0], pos = acc[1], neg = acc[2], Lp = acc[3], Ln = acc[4];
   const double posF = fmax(pos, EPSd), negF = fmax(neg, EPSd);
@@ -330,6 +366,7 @@ k_adj_geo_pen(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* 
               const double* __restrict__ lu, const double* __restrict__ lv, double wFx, double wFy, double wt,
               double* gX, double* gU, double* gV, double* gSX, double* gSY, double* gCom)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   const double Cx = S.s.com[0], Cy = S.s.com[1];
   const double NUoH = g.nu / g.h;
@@ -371,6 +408,7 @@ k_adj_geo_obst(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double*
                const double* __restrict__ T, const double* __restrict__ lo, const double* __restrict__ acc,
                double* gX)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   const double s = acc[0], pos = acc[1], neg = acc[2], Lp = acc[3], Ln = acc[4];
   const double posF = fmax(pos, EPSd), negF = fmax(neg, EPSd);
@@ -402,6 +440,7 @@ k_adj_geo_dot(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* 
               const double* __restrict__ gSX, const double* __restrict__ gSY, const double* __restrict__ gCom,
               double* acc)
 {
+  pdl_begin();
   const DevShape& S = sh[k];
   const double Cx = S.s.com[0], Cy = S.s.com[1];
   double a = 0;
@@ -440,6 +479,7 @@ __device__ __forceinline__ double fade_w2(const GridDesc& g, int gx, int gy) {
 __global__ void __launch_bounds__(256)
 k_adj_fade_sums(GridDesc g, const double* __restrict__ f, const double* __restrict__ lb, double* acc)
 {
+  pdl_begin();
   const int bx = blockIdx.x, by = blockIdx.y;
   if (!fade_touch(g, bx, by)) return;
   const int gx = bx * BS + threadIdx.x;
@@ -463,6 +503,7 @@ k_adj_fade_sums(GridDesc g, const double* __restrict__ f, const double* __restri
 __global__ void __launch_bounds__(256)
 k_adj_fade_apply(GridDesc g, const double* __restrict__ f, double* lb, const double* __restrict__ acc)
 {
+  pdl_begin();
   // in place; outside the strip blocks w2 = 0 and lambda passes unchanged
   if (!fade_touch(g, blockIdx.x, blockIdx.y)) return;
   const double S = acc[0], Sp = acc[1], Sn = acc[2], Lp = acc[3], Ln = acc[4];
@@ -492,24 +533,6 @@ k_adj_fade_apply(GridDesc g, const double* __restrict__ f, double* lb, const dou
 // dW..dN: the inflow fades' derivatives with respect to (U0, U1)
 struct AdvC { double afac, dfac, fW, fS, fE, fN, U0, U1; double dW[2], dS[2], dE[2], dN[2]; int nb; };
 
-// Gamma = sum of sigma lambda over the boundary cells (sigma: +1 on the W
-// column / S row, -1 on the E column / N row; u on the columns, v on the
-// rows): the outflow correction's rank-one transpose
-__global__ void __launch_bounds__(256)
-k_adj_adv_gamma(GridDesc g, const double* __restrict__ lu, const double* __restrict__ lv, double* acc)
-{
-  const int nx = g.nx, ny = g.ny, n = 2 * (nx + ny);
-  double a = 0;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    if (q < ny) a += lu[(size_t)q * nx];
-    else if (q < 2 * ny) a -= lu[(size_t)(q - ny) * nx + nx - 1];
-    else if (q < 2 * ny + nx) a += lv[q - 2 * ny];
-    else a -= lv[(size_t)(ny - 1) * nx + (q - 2 * ny - nx)];
-  }
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if ((threadIdx.x & 31) == 0 && a != 0) atomicAdd(acc, a);
-}
-
 // lambda before the correction: lambda - sigma Gamma / Nb
 __device__ __forceinline__ double lpre_u(const GridDesc& g, const double* lu, size_t c, int x, double gn) {
   double v = lu[c];
@@ -531,6 +554,7 @@ k_adj_advdiff(GridDesc g, AdvC k, const double* __restrict__ u, const double* __
               const double* __restrict__ lu, const double* __restrict__ lv, const double* __restrict__ acc,
               double* __restrict__ ou, double* __restrict__ ov, double* gb)
 {
+  pdl_begin();
   const double gn = acc[0] / k.nb;
   const int nx = g.nx, ny = g.ny;
   const int gx = blockIdx.x * BS + threadIdx.x;
@@ -614,6 +638,7 @@ struct CopyList {
 };
 static_assert(sizeof(DevShape) % 4 == 0, "the shape snapshot is copied in 4-byte words");
 __global__ void __launch_bounds__(256) k_copy_many(CopyList L) {
+  pdl_begin();
   for (int q = 0; q < L.n; q++) {
     const unsigned* __restrict__ a = L.src[q];
     unsigned* __restrict__ b = L.dst[q];
@@ -628,6 +653,7 @@ __global__ void __launch_bounds__(256)
 k_adj_probe(GridDesc g, ProbeBox bx, const double* __restrict__ u, const double* __restrict__ v, double w,
             double* acc, double* lu, double* lv)
 {
+  pdl_begin();
   double a = 0;
   const int W = bx.x1 - bx.x0, H = bx.y1 - bx.y0;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < W * H; q += gridDim.x * blockDim.x) {
@@ -815,15 +841,18 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
   std::vector<void*> ck(nseg + 1);
   for (int s = 0; s <= nseg; s++)
     if (!(ck[s] = B.get<char>(ckBytes))) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint checkpoints");
-  double* acc = B.get<double>(8);          // [0..4] reductions of a transposed stage
+  // a step's reductions of its transposed stages, zeroed for all steps at
+  // once: the fade's five, the obstacle terms' five, advDiff's Gamma
+  constexpr int ACC = 16;
+  double* acc = B.get<double>(ACC * (size_t)nsteps);
   // [0] J; [1..3] the body-velocity gradient (forced: the held velocity's,
   // accumulated over the steps; free: the adjoint of the step's output
   // velocity); [4..6] a free body's adjoint of the previous output, formed
   // by advDiff's lab velocity; [8..10] the solve's transpose
   double* obv = B.get<double>(12);
-  double* tauRec = B.get<double>(nsteps);    // each step's torque (the |torque| term's sign)
-  if (!acc || !obv || !tauRec) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint scratch");
-  std::vector<double> dts(nsteps), U0s(nsteps), U1s(nsteps);
+  StepRecord* rec = B.get<StepRecord>(nsteps);
+  if (!acc || !obv || !rec) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint scratch");
+  std::vector<double> dts(nsteps);
   struct Ev {
     cudaEvent_t e[3] = {nullptr, nullptr, nullptr};
     ~Ev() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
@@ -857,13 +886,9 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
     else ARC(cup2d_calc_dt(ctx, &dt));
     dts[i] = dt;
     ARC(step(dt, nullptr, nullptr, nullptr, nullptr));
-    // the lab velocity of the step (set by the placement from the forced body)
-    double t_, dtd, ux, uy; int st;
-    ARC(cup2d_get_scalars(ctx, &t_, &dtd, &st, &ux, &uy));
-    U0s[i] = ux; U1s[i] = uy;
-    if (energy) k_adj_probe<<<probeGrid, 256, 0, c.stream>>>(g, bx, c.u(), c.v(), wE, obv, nullptr, nullptr);
-    if (force || bodyTerm)
-      k_adj_body_sum<<<1, 1, 0, c.stream>>>(c.dshapes, 0, wFx, wFy, wT, wB[0], wB[1], wB[2], obv, tauRec + i);
+    if (energy) launch_k(k_adj_probe, probeGrid, 256, 0, c.stream, g, bx, c.u(), c.v(), wE, obv, nullptr, nullptr);
+    launch_k(k_adj_record, 1, 1, 0, c.stream, c.dshapes, 0, c.dsc, force || bodyTerm, wFx, wFy, wT, wB[0], wB[1],
+             wB[2], obv, rec + i);
     ACK(cudaGetLastError());
   }
   ACK(cudaEventRecord(e1, c.stream));
@@ -877,11 +902,11 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
       return adj_fail(ctx, CUP2D_ENOTSUP, "the body is released (timeForced) within the run");
   }
   ACK(cudaMemcpyAsync(J, obv, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  std::vector<double> taus(nsteps, 0.0), wTs(nsteps, 0.0);
-  if (force || bodyTerm)
-    ACK(cudaMemcpyAsync(taus.data(), tauRec, sizeof(double) * nsteps, cudaMemcpyDeviceToHost, c.stream));
+  std::vector<StepRecord> recs(nsteps);
+  std::vector<double> wTs(nsteps);
+  ACK(cudaMemcpyAsync(recs.data(), rec, sizeof(StepRecord) * nsteps, cudaMemcpyDeviceToHost, c.stream));
   ACK(cudaStreamSynchronize(c.stream));
-  for (int i = 0; i < nsteps; i++) wTs[i] = taus[i] > 0 ? wT : (taus[i] < 0 ? -wT : 0.0);   // d|torque|
+  for (int i = 0; i < nsteps; i++) wTs[i] = recs[i].torque > 0 ? wT : (recs[i].torque < 0 ? -wT : 0.0);   // d|torque|
   if (dt_out) std::copy(dts.begin(), dts.end(), dt_out);
   float fms = 0;
   ACK(cudaEventElapsedTime(&fms, e0, e1));
@@ -952,6 +977,7 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
   ACK(cudaMemsetAsync(lu, 0, nb, c.stream));
   ACK(cudaMemsetAsync(lv, 0, nb, c.stream));
   ACK(cudaMemsetAsync(obv + 1, 0, sizeof(double) * 11, c.stream));
+  ACK(cudaMemsetAsync(acc, 0, sizeof(double) * ACC * nsteps, c.stream));
   ACK(cudaEventRecord(e2, c.stream));
   double* lx = obv + 1;                      // the body-velocity adjoint (see above)
   double* lxPrev = obv + 4;
@@ -986,7 +1012,7 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
         for (int q = 0; q < 6; q++) add(src[q], dst[q], sizeof(double) * tb);
         add(c.chi, chiSnap + o, nb);
       }
-      k_copy_many<<<2 * c.sms, 256, 0, c.stream>>>(L);
+      launch_k(k_copy_many, 2 * c.sms, 256, 0, c.stream, L);
       ACK(cudaGetLastError());
     }
     for (int i = i1 - 1; i >= i0; i--) {
@@ -995,29 +1021,32 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
       const DevShape* shI = keepObst ? shSnap + (i - i0) : c.dshapes;   // the step's obstacle state
       const ObstTiles tI = tilesAt(i - i0);
       const double* chiI = keepObst ? chiSnap + o : c.chi;
+      double* fadeAcc = acc + (size_t)ACC * i;
+      double* obstAcc = fadeAcc + 5;
+      double* gamma = fadeAcc + 10;
       // the objective's terms of u^(i+1), p^(i+1) and the body velocity
-      if (energy) k_adj_probe<<<probeGrid, 256, 0, c.stream>>>(g, bx, pu + o, pv + o, wE, nullptr, lu, lv);
+      if (energy) launch_k(k_adj_probe, probeGrid, 256, 0, c.stream, g, bx, pu + o, pv + o, wE, nullptr, lu, lv);
       if (force)
-        k_adj_force<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, wFx, wFy, wTs[i], 0, lu, lv, nullptr);
-      if (bodyTerm) k_adj_add3<<<1, 1, 0, c.stream>>>(lx, wB[0], wB[1], wB[2]);
+        launch_k(k_adj_force, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, wFx, wFy, wTs[i], 0, lu, lv, nullptr);
+      if (bodyTerm) launch_k(k_adj_add3, 1, 1, 0, c.stream, lx, wB[0], wB[1], wB[2]);
       if (gait) {
         const size_t og = (size_t)i * n;
-        k_adj_geo_pen<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, chiI, su1 + o, sv1 + o, sp + o,
+        launch_k(k_adj_geo_pen, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, chiI, su1 + o, sv1 + o, sp + o,
             -0.5 * dt / g.h, pu + o, pv + o, lu, lv, wFx, wFy, wTs[i], gG[0] + og, gG[1] + og, gG[2] + og,
             gG[3] + og, gG[4] + og, gCom + 2 * (size_t)i);
       }
       // penalization
-      k_adj_pen<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, chiI, lu, lv, lx);
+      launch_k(k_adj_pen, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, chiI, lu, lv, lx);
       if (freeBody) {
         // the body velocity of the step came from the momentum integrals of
         // the pressure-corrected velocity
-        k_adj_solve<<<1, 1, 0, c.stream>>>(shI, 0, lx, lb);
-        k_adj_momenta<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, lb, lu, lv);
+        launch_k(k_adj_solve, 1, 1, 0, c.stream, shI, 0, lx, lb);
+        launch_k(k_adj_momenta, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, lb, lu, lv);
       }
       // pressure correction: lambda_p, the force's pressure term, then the convolution
-      k_adj_grad_T<<<grid2, blk2, 0, c.stream>>>(g, -0.5 * dt / g.h, lu, lv, l1);
+      launch_k(k_adj_grad_T, grid2, blk2, 0, c.stream, g, -0.5 * dt / g.h, lu, lv, l1);
       if (force)
-        k_adj_force<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, wFx, wFy, wTs[i], 1, nullptr, nullptr, l1);
+        launch_k(k_adj_force, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, wFx, wFy, wTs[i], 1, nullptr, nullptr, l1);
       ACK(cudaGetLastError());
       {
         double* const R = c.rhs;
@@ -1028,26 +1057,22 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
       }
       // the fade, then the obstacle terms, both in place on l2 (over the
       // strip blocks and the shape's tiles)
-      ACK(cudaMemsetAsync(acc, 0, sizeof(double) * 8, c.stream));
-      k_adj_fade_sums<<<grid2, blk2, 0, c.stream>>>(g, sF + o, l2, acc);
-      k_adj_fade_apply<<<grid2, blk2, 0, c.stream>>>(g, sF + o, l2, acc);
-      ACK(cudaMemsetAsync(acc, 0, sizeof(double) * 8, c.stream));
-      k_adj_obst_sums<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, chiI, sT + o, l2, acc);
+      launch_k(k_adj_fade_sums, grid2, blk2, 0, c.stream, g, sF + o, l2, fadeAcc);
+      launch_k(k_adj_fade_apply, grid2, blk2, 0, c.stream, g, sF + o, l2, fadeAcc);
+      launch_k(k_adj_obst_sums, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, chiI, sT + o, l2, obstAcc);
       if (gait)
-        k_adj_geo_obst<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, chiI, sT + o, l2, acc,
+        launch_k(k_adj_geo_obst, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, chiI, sT + o, l2, obstAcc,
                                                             gG[0] + (size_t)i * n);
-      k_adj_obst_apply<<<tctas, dim3(32, 32), 0, c.stream>>>(g, shI, 0, tI, chiI, sT + o, l2, acc);
+      launch_k(k_adj_obst_apply, tctas, dim3(32, 32), 0, c.stream, g, shI, 0, tI, chiI, sT + o, l2, obstAcc);
       // the divergence, added to lambda of u1
-      k_adj_div_T<<<grid2, blk2, 0, c.stream>>>(g, 0.5 * g.h / dt, l2, lu, lv);
+      launch_k(k_adj_div_T, grid2, blk2, 0, c.stream, g, 0.5 * g.h / dt, l2, lu, lv, gamma);
       // advDiff about u^i
-      ACK(cudaMemsetAsync(acc, 0, sizeof(double) * 8, c.stream));
-      k_adj_adv_gamma<<<std::min(148, (2 * (g.nx + g.ny) + 255) / 256), 256, 0, c.stream>>>(g, lu, lv, acc);
       // (a free body: its previous velocity set the lab velocity of this
       // step; a forced one: its held velocity, accumulated)
       const double* un0 = i == i0 ? su : pu + o - n;     // u^n of the step
       const double* vn0 = i == i0 ? sv : pv + o - n;
-      k_adj_advdiff<<<grid2, blk2, 0, c.stream>>>(g, adv_coef_host(c, dt, U0s[i], U1s[i]), un0, vn0,
-                                                 lu, lv, acc, tu, tv, freeBody ? lxPrev : lx);
+      launch_k(k_adj_advdiff, grid2, blk2, 0, c.stream, g, adv_coef_host(c, dt, recs[i].uinfx, recs[i].uinfy), un0, vn0,
+                                                 lu, lv, gamma, tu, tv, freeBody ? lxPrev : lx);
       ACK(cudaGetLastError());
       std::swap(lu, tu);
       std::swap(lv, tv);
@@ -1089,7 +1114,7 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
         rc = cup2d_put_objects(x, dts[i]);
         if (rc) break;
         const size_t og = (size_t)i * n;
-        k_adj_geo_dot<<<tctas, dim3(32, 32), 0, cx.stream>>>(g, cx.dshapes, 0, cx.tiles[0], cx.chi, gG[0] + og,
+        launch_k(k_adj_geo_dot, tctas, dim3(32, 32), 0, cx.stream, g, cx.dshapes, 0, cx.tiles[0], cx.chi, gG[0] + og,
                                                             gG[1] + og, gG[2] + og, gG[3] + og, gG[4] + og,
                                                             gCom + 2 * (size_t)i, accx);
         if (cudaGetLastError() != cudaSuccess) return CUP2D_ECUDA;
