@@ -724,10 +724,20 @@ struct AdjBufs {
         k.used += want;
         return q;
       }
-    // a chunk of its own for a large buffer, 16 MB for small ones
-    const size_t bytes = std::max(want, (size_t)16 << 20);
+    // a chunk of its own for a large buffer, 16 MB for small ones; on a full
+    // device the buffer alone, with the chunks that this run does not use given
+    // back first
+    size_t bytes = std::max(want, (size_t)16 << 20);
     void* q = nullptr;
-    if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      auto unused = [](const Ctx::Chunk& k) { return k.used == 0; };
+      for (const Ctx::Chunk& k : c.adjChunks)
+        if (unused(k)) cudaFree(k.p);
+      c.adjChunks.erase(std::remove_if(c.adjChunks.begin(), c.adjChunks.end(), unused), c.adjChunks.end());
+      bytes = want;
+      if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
+    }
     c.adjChunks.push_back({static_cast<char*>(q), bytes, want});
     return static_cast<T*>(q);
   }
