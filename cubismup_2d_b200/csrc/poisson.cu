@@ -52,6 +52,8 @@ struct Poisson {
   double2* tCol = nullptr;                 // and of the column transforms
   bool fp32 = false;         // CUP2D_PREC_FP32: float2 spectrum in spec, FP32 passes
   float2* tw32 = nullptr;    // tw rounded to FP32
+  float2* tRow32 = nullptr;  // pass tables of the FP32 row and column transforms
+  float2* tCol32 = nullptr;
   float* ghat32 = nullptr;   // the free-space kernel rounded to FP32, [nkx][Lcol/2 + 1]
   int rb = 1, cb = 1;        // rows / columns per CTA
   int MX = 0, MY = 0;        // free space: the padded grid (powers of two >= 2Nx, 2Ny)
@@ -1210,6 +1212,8 @@ Poisson* poisson_create(Ctx& c) {
     for (int k = 0; k < P->twLen; k++) tw32[k] = make_float2((float)tw[k].x, (float)tw[k].y);
     if (cudaMalloc(&P->tw32, sizeof(float2) * P->twLen) != cudaSuccess) { poisson_destroy(P); return nullptr; }
     h2d_sync(P->tw32, tw32.data(), sizeof(float2) * P->twLen, c.stream);
+    if (!(P->tRow32 = make_tables32(P->Lrow, false, tw32, c.stream)) ||
+        !(P->tCol32 = make_tables32(P->Lcol, true, tw32, c.stream))) { poisson_destroy(P); return nullptr; }
     if (P->type == CUP2D_POISSON_FREESPACE) {
       const size_t ng = (size_t)(P->Lcol / 2 + 1) * P->nkx;
       std::vector<double> g64(ng);
@@ -1228,6 +1232,7 @@ void poisson_destroy(Poisson* P) {
   if (!P) return;
   cudaFree(P->spec); cudaFree(P->ghat); cudaFree(P->tw); cudaFree(P->cosX); cudaFree(P->cosY);
   cudaFree(P->tw32); cudaFree(P->ghat32);
+  cudaFree(P->tRow32); cudaFree(P->tCol32);
   cudaFree(P->tRow[0]); cudaFree(P->tRow[1]); cudaFree(P->tCol);
   delete P;
 }
@@ -1252,7 +1257,7 @@ void poisson_rows_fwd(Ctx& c) {
   }
   // free space: the row's zero padding is the upper half of the length-Lrow sequence
   if (P->fp32)
-    rows_r2c32(P->Lrow, c.stream, c.rhs, Nx, Ny, Nx, reinterpret_cast<float2*>(P->spec), Ny, P->tw32,
+    rows_r2c32(P->Lrow, c.stream, c.rhs, Nx, Ny, Nx, reinterpret_cast<float2*>(P->spec), Ny, P->tRow32, P->tw32,
                P->twLen, fa, P->type == CUP2D_POISSON_FREESPACE);
   else
     rows_r2c(*P, c.stream, c.rhs, Nx, Ny, fa, P->type == CUP2D_POISSON_FREESPACE, P->eR2C);
@@ -1267,14 +1272,14 @@ void poisson_cols(Ctx& c) {
   } else if (P->type == CUP2D_POISSON_FREESPACE) {
     if (P->fp32)
       cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), Ny, P->nkx, Ny, Ny, P->ghat32, 0,
-             P->tw32, P->twLen, 0.0, 0, 0);
+             P->tCol32, 0.0, 0, 0);
     else
       cols(*P, c.stream, Ny, true);
   } else {
     const double norm = 1.0 / ((double)Nx * (double)Ny);
     if (P->fp32)
       cols32(P->Lcol, c.stream, reinterpret_cast<float2*>(P->spec), Ny, P->nkx, Ny, Ny, nullptr, 2,
-             P->tw32, P->twLen, norm, Nx, Ny);
+             P->tCol32, norm, Nx, Ny);
     else
       cols(*P, c.stream, Ny, false);
   }
@@ -1291,7 +1296,7 @@ void poisson_rows_inv(Ctx& c) {
   }
   if (P->fp32)
     rows_c2r32(P->Lrow, c.stream, reinterpret_cast<const float2*>(P->spec), Ny, Ny, c.pres, Nx, Nx,
-               P->tw32, P->twLen, P->type == CUP2D_POISSON_FREESPACE);
+               P->tRow32, P->tw32, P->twLen, P->type == CUP2D_POISSON_FREESPACE);
   else
     rows_c2r(*P, c.stream, c.pres, Nx, Ny, P->type == CUP2D_POISSON_FREESPACE, P->eC2R);        // free space keeps the first half
   CUP2D_LAUNCHED(c);

@@ -47,10 +47,6 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
                :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n"
-               :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" :: "n"(N) : "memory");
 }
@@ -115,11 +111,13 @@ __device__ __forceinline__ double fade_cell(double row, double col, double b, do
 
 // poisson32.cu: the FP32 passes of the free-space and periodic solves
 bool poisson32_setup();                              // shared-memory limits of its kernels
+// device tables of the row (column) passes of length L, from tw rounded to FP32
+float2* make_tables32(int L, bool cols, const std::vector<float2>& tw, cudaStream_t st);
 bool rows_r2c32(int L, cudaStream_t st, const double* in, int inStride, int nrows, int ncolsIn, float2* out,
-                int outRows, const float2* tw, int twLen, FadeArgs fa, bool halfIn);
+                int outRows, const float2* tab, const float2* tw, int twLen, FadeArgs fa, bool halfIn);
 bool cols32(int L, cudaStream_t st, float2* data, int rows, int ncols, int nrowsIn, int nrowsOut,
-            const float* ghat, int mode, const float2* tw, int twLen, double norm, int MXp, int MYp);
+            const float* ghat, int mode, const float2* tab, double norm, int MXp, int MYp);
 bool rows_c2r32(int L, cudaStream_t st, const float2* in, int inRows, int nrows, double* out, int outStride,
-                int ncolsOut, const float2* tw, int twLen, bool halfOut);
+                int ncolsOut, const float2* tab, const float2* tw, int twLen, bool halfOut);
 
 } // namespace cup2d

@@ -5,6 +5,8 @@
 // The transforms keep their own radix passes: their twiddles are products of
 // table values in one fixed order, so FP32 results do not move with the FP64
 // passes.
+#include <algorithm>
+#include <vector>
 #include "poisson.cuh"
 
 namespace cup2d {
@@ -12,9 +14,12 @@ namespace {
 
 // The half spectrum lies in groups of eight columns, 64 bytes a row, as the
 // FP64 one does in groups of four (spec_at in poisson.cu): a column pass then
-// touches 16 lines for 32 rows instead of 32, and the kernel G^ lies by columns.
-// Column pass on B200: 180 -> 145 us at 4096 x 2048, 70 -> 45 at 2048 x 1024, 17.2 -> 14.3
-// at 1024 x 512 (row passes unchanged).
+// touches 16 lines for 32 rows instead of 32, and the kernel G^ lies by columns,
+// read where it is applied.  B200, forward rows, columns, inverse rows in us,
+// after (before) this, the tables laid out once, the first and last row passes
+// straight from and to global memory and Col32: 4096 x 2048 68, 112, 57 (81, 180,
+// 65); 2048 x 1024 25, 33, 19 (28, 70, 22); 1024 x 512 13.4, 14.0, 11.2 (14.4, 17.2,
+// 12.0).  The same arithmetic in the same order: the same bits.
 constexpr int SPEC32_LOG = 3;
 __device__ __forceinline__ size_t spec32_at(int rows, int r, int k) {
   return (((size_t)(k >> SPEC32_LOG) * rows + r) << SPEC32_LOG) | (k & ((1 << SPEC32_LOG) - 1));
@@ -22,8 +27,8 @@ __device__ __forceinline__ size_t spec32_at(int rows, int r, int k) {
 
 // Per transform length L: padded stride SL of one sequence (one spare
 // element per 16, plus 4 so that consecutive sequences start in different
-// halves of the shared-memory banks), the staged quarter twiddle table
-// (w^j, j < L/4), the sequences per CTA B and the threads per CTA NT
+// halves of the shared-memory banks), the room TW of the staged tables, the
+// rows per CTA B and the threads per CTA NT of the row passes
 // (L/E per sequence: every thread owns E = 16 or 8 elements of a pass).
 // ---- per-pass twiddle tables ---------------------------------------------
 // The passes of fft_inplace<L, ..., E> (fft_passes): sub-transform sizes
@@ -59,39 +64,44 @@ template <int L, int E = 16> struct Len {
   static constexpr int B = 2048 / L < 1 ? 1 : (2048 / L > 8 ? 8 : 2048 / L);
   static constexpr int NT0 = B * L / E;
   static constexpr int NT = NT0 < 64 ? 64 : (NT0 > 512 ? 512 : NT0);
-  static constexpr int REGS = E == 16 ? 128 : 64;   // register budget per thread
-  static constexpr int MINB = 65536 / (NT * REGS) < 1 ? 1 : 65536 / (NT * REGS);
+  static constexpr int MINB = 65536 / (NT * 64);    // 64 registers a thread
 };
 // elements per thread
 constexpr int E_ROWS32 = 8;
 constexpr int E_C2R32 = 8;
 constexpr int E_COLS32 = 16;
+// Columns per CTA of the column pass (of one group, so that a CTA reads runs
+// of 16 or 32 bytes) and a budget of 64 registers a thread, 32 warps an SM:
+// the pass waits for its exchanges, and more warps hide them.  4096 x 2048, in
+// us, with 1, 2 and 4 columns: 130 (80 registers), 115, 112; one column and 128
+// registers 137.  2048-point columns: 1, 2, 4 columns 40, 32, 35.
+template <int L> struct Col32 {
+  static constexpr int CB = L >= 4096 ? 4 : (L >= 1024 ? 2 : Len<L>::B);
+  static constexpr int NT0 = CB * L / E_COLS32, NT = NT0 < 64 ? 64 : NT0;
+  static constexpr int MINB = 65536 / (NT * 64);
+};
 
-constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n / 2); }
-
-// Stages the per-pass tables of fft_inplace<L, ..., E> from the global
-// table tw[j] = exp(-2 pi i j / twLen) (twLen a power of two, a multiple of
-// 4 L): the tables of the pass over sub-transforms of size NS and of every
-// later pass.  Entry t = p NS + k of a pass of radix R holds
-// W^(k 2^p) = tw[(k 2^p) twLen / (R NS)]; the passes' sizes are
-// compile-time powers of two, so every index is a shift.
-template <int L, int E, int NS, class C>
-__device__ __forceinline__ void load_twiddles_from(C* tws, const C* __restrict__ tw, int twShift) {
-  if constexpr (NS < L) {
-    constexpr int R = NS * E <= L ? E : L / NS;
-    if constexpr (NS > 1) {
-      constexpr int n = tw_npow(R) * NS, off = tw_off<L, E>(NS), sh = ilog2(R * NS);
-      for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int p = t / NS, k = t - p * NS;
-        tws[off + t] = tw[(size_t)(k << p) << (twShift - sh)];
-      }
-    }
-    load_twiddles_from<L, E, NS * R>(tws, tw, twShift);
-  }
-}
+// Stages the per-pass tables of fft_inplace<L, ..., E>, laid out once for all
+// CTAs (make_tables32).  Gathered by every CTA from the table of all
+// exp(-2 pi i j / twLen), a stride apart, the 14 KB of a 4096-point row had
+// taken as much L2 traffic as the row.
 template <int L, int E, class C>
-__device__ __forceinline__ void load_twiddles(C* tws, const C* __restrict__ tw, int twLen) {
-  load_twiddles_from<L, E, 1>(tws, tw, __ffs(twLen) - 1);
+__device__ __forceinline__ void load_twiddles(C* tws, const C* __restrict__ tab) {
+  for (int t = threadIdx.x; t < tw_size<L, E>(); t += blockDim.x) tws[t] = tab[t];
+}
+// the tables on the host, from tw[j] = exp(-2 pi i j / twLen) (twLen a
+// multiple of 2 L): entry p NS + k of a pass of radix R holds W^(k 2^p) =
+// tw[(k 2^p) twLen / (R NS)]
+template <int L, int E> void fill_tables32(const std::vector<float2>& tw, std::vector<float2>& out) {
+  out.assign(std::max(1, tw_size<L, E>()), make_float2(0, 0));
+  for (int ns = 1; ns < L;) {
+    const int r = ns * E <= L ? E : L / ns;
+    if (ns > 1)
+      for (int p = 0; p < tw_npow(r); p++)
+        for (int k = 0; k < ns; k++)
+          out[tw_off<L, E>(ns) + p * ns + k] = tw[(size_t)(k << p) * (tw.size() / (size_t)(r * ns))];
+    ns *= r;
+  }
 }
 
 // Scales xb[m], 0 < m < R, of the butterfly k of the pass over
@@ -363,86 +373,90 @@ __device__ __forceinline__ void r2c_split(const C* A, int nb, int row0, C* __res
 template <int L, bool HIN>
 __global__ void __launch_bounds__(Len<L, E_ROWS32>::NT, Len<L, E_ROWS32>::MINB)
 k_rows_r2c32(const double* __restrict__ in, int inStride, int nrows, int ncolsIn,
-             float2* __restrict__ out, int outRows, const float2* __restrict__ tw, int twLen, FadeArgs fa)
+             float2* __restrict__ out, int outRows, const float2* __restrict__ tab, const float2* __restrict__ tw,
+             int twLen, FadeArgs fa)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_R2C);
-  constexpr int SL = Len<L, E_ROWS32>::SL, RB = Len<L, E_ROWS32>::B, NT = Len<L, E_ROWS32>::NT;
-  constexpr int PER = (RB * L + NT - 1) / NT;          // value pairs per thread
+  constexpr int SL = Len<L, E_ROWS32>::SL, RB = Len<L, E_ROWS32>::B;
+  constexpr int E = E_ROWS32, Q = L / E, N = HIN ? E / 2 : E;
   extern __shared__ float2 sm32[];
   float2* A = sm32;
   float2* tws = sm32 + RB * SL;
   const int row0 = blockIdx.x * RB;
   const int nb = min(RB, nrows - row0);
-  double2 v[PER];                                      // this thread's pairs, all loads in flight
+  // this thread's inputs of the first pass, all loads in flight
+  const int sq = threadIdx.x / Q, j = threadIdx.x % Q, row = row0 + sq;
+  const bool act = sq < nb;
+  double2 v[N];
 #pragma unroll
-  for (int u = 0; u < PER; u++) {
-    const int idx = threadIdx.x + u * NT;
-    const int r = idx / L, n = idx & (L - 1), row = row0 + r;
-    v[u] = make_double2(0, 0);
-    if (idx < RB * L && r < nb) {
-      if (2 * n + 1 < ncolsIn) v[u] = *reinterpret_cast<const double2*>(in + (size_t)row * inStride + 2 * n);
-      else if (2 * n < ncolsIn) v[u].x = in[(size_t)row * inStride + 2 * n];
+  for (int m = 0; m < N; m++) {
+    const int n = j + m * Q;
+    v[m] = make_double2(0, 0);
+    if (act) {
+      if (2 * n + 1 < ncolsIn) v[m] = *reinterpret_cast<const double2*>(in + (size_t)row * inStride + 2 * n);
+      else if (2 * n < ncolsIn) v[m].x = in[(size_t)row * inStride + 2 * n];
     }
   }
   __shared__ double sCorr;
   if (fa.enabled) fade_corr_cta(fa, &sCorr);
-  load_twiddles<L, E_ROWS32>(tws, tw, twLen);
+  load_twiddles<L, E>(tws, tab);
   __syncthreads();
-  const double corr = fa.enabled ? sCorr : 0.0;
-  const int bandX = fa.enabled ? fa.bandX : 0;
-  const int bandY = fa.enabled ? fa.bandY : 0;
+  if (act) {
+    // fade band as in k_rows_r2c (cub2rhs, PoissonSolver.cpp:61-141; no band,
+    // and no cell looked at, with the fade off)
+    const bool rowBand = fa.enabled && (row < fa.bandY || row >= fa.g.ny - fa.bandY);
+    const int bandLo = !fa.enabled ? 0 : rowBand ? fa.g.nx : fa.bandX;
+    const int bandHi = fa.enabled ? fa.g.nx - fa.bandX : ncolsIn;
+    const double rowFade = fade_row(fa.g, row);
+    float2 x[E];
 #pragma unroll
-  for (int u = 0; u < PER; u++) {
-    const int idx = threadIdx.x + u * NT;
-    const int r = idx / L, n = idx & (L - 1), row = row0 + r;
-    if (idx >= RB * L || r >= nb) continue;
-    if (HIN && n >= L / 2) continue;                   // the zero upper half is never read
-    if (fa.enabled && 2 * n + 1 < ncolsIn) {
-      // fade band as in k_rows_r2c (cub2rhs, PoissonSolver.cpp:61-141)
-      const bool rowBand = row < bandY || row >= fa.g.ny - bandY;
-      double* x = &v[u].x;
-      for (int q = 0; q < 2; q++) {
-        const int col = 2 * n + q;
-        if (rowBand || col < bandX || col >= fa.g.nx - bandX) {
-          x[q] = fade_cell(fade_row(fa.g, row), fade_col(fa.g, col), x[q], corr);
-          fa.writeback[(size_t)row * inStride + col] = x[q];
+    for (int m = 0; m < E; m++) x[m] = make_float2(0, 0);    // HIN: the zero upper half
+#pragma unroll
+    for (int m = 0; m < N; m++) {
+      const int n = j + m * Q;
+      if ((2 * n < bandLo || 2 * n + 1 >= bandHi) && 2 * n + 1 < ncolsIn) {
+        double* y = &v[m].x;
+        for (int q = 0; q < 2; q++) {
+          const int col = 2 * n + q;
+          if (col < bandLo || col >= bandHi) {
+            y[q] = fade_cell(rowFade, fade_col(fa.g, col), y[q], sCorr);
+            fa.writeback[(size_t)row * inStride + col] = y[q];
+          }
         }
       }
+      x[m] = make_float2((float)v[m].x, (float)v[m].y);
     }
-    A[r * SL + pad(n)] = make_float2((float)v[u].x, (float)v[u].y);
+    dft<E, false>(x);
+    float2* a = A + sq * SL;
+    const int o = j * E, po = pad(o);
+#pragma unroll
+    for (int q = 0; q < E; q++) a[pad_out<1>(po, o, q)] = x[out_reg<E>(q)];
   }
   __syncthreads();
-  fft_inplace<L, false, HIN, false, E_ROWS32>(A, nb, tws);
+  fft_passes<L, E, false, false, false, E>(A, nb, tws);
   r2c_split<L, E_ROWS32>(A, nb, row0, out, outRows, tw, twLen);
 }
 
 // mode 0: forward, x G^, inverse, keep nrowsOut rows; mode 2: the periodic
 // multiplier -1/|k|^2 / (MX MY) (formed in FP64, applied in FP32)
 template <int L, bool FS>
-__global__ void __launch_bounds__(Len<L, E_COLS32>::NT, Len<L, E_COLS32>::MINB)
+__global__ void __launch_bounds__(Col32<L>::NT, Col32<L>::MINB)
 k_cols32(float2* __restrict__ data, int rows, int ncols, int nrowsIn, int nrowsOut,
-         const float* __restrict__ ghat, int mode, const float2* __restrict__ tw, int twLen,
-         double norm, int MXp, int MYp)
+         const float* __restrict__ ghat, int mode, const float2* __restrict__ tab, double norm, int MXp, int MYp)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_COLS);
-  constexpr int SL = Len<L, E_COLS32>::SL, CB = Len<L, E_COLS32>::B, NT = Len<L, E_COLS32>::NT, GR = L / 2 + 1;
+  constexpr int SL = Len<L>::SL, CB = Col32<L>::CB, NT = Col32<L>::NT, GR = L / 2 + 1;
   extern __shared__ float2 sm32[];
   float2* A = sm32;
   float2* tws = sm32 + CB * SL;
-  float* Gs = reinterpret_cast<float*>(tws + Len<L>::TW);   // [GR][CB] kernel rows
   const int c0 = blockIdx.x * CB;
   const int nb = min(CB, ncols - c0);
   for (int idx = threadIdx.x; idx < CB * nrowsIn; idx += NT) {
     const int r = idx / CB, j = idx & (CB - 1);
     if (j < nb) cp_async8(A + j * SL + pad(r), data + spec32_at(rows, r, c0 + j));
   }
-  if (mode == 0)
-    for (int idx = threadIdx.x; idx < CB * GR; idx += NT) {
-      const int j = idx / GR, r = idx - j * GR;
-      if (j < nb) cp_async4(Gs + r * CB + j, ghat + (size_t)(c0 + j) * GR + r);
-    }
   cp_async_commit();
   // rows beyond the input are zero; the free-space solve never reads its
   // upper half
@@ -450,13 +464,13 @@ k_cols32(float2* __restrict__ data, int rows, int ncols, int nrowsIn, int nrowsO
     const int r = nrowsIn + idx / CB, j = idx & (CB - 1);
     A[j * SL + pad(r)] = make_float2(0, 0);
   }
-  load_twiddles<L, E_COLS32>(tws, tw, twLen);
+  load_twiddles<L, E_COLS32>(tws, tab);
   cp_async_wait<0>();
   __syncthreads();
   if (mode == 0) {
     fft_convolve<L, FS, FS, E_COLS32>(A, nb, tws, [&](int j, int r, float2 z) {
       const int ky = r <= L / 2 ? r : L - r;
-      const float f = Gs[ky * CB + j];
+      const float f = __ldg(ghat + (size_t)(c0 + j) * GR + ky);
       return make_float2(z.x * f, z.y * f);
     });
   } else {
@@ -482,7 +496,7 @@ k_cols32(float2* __restrict__ data, int rows, int ncols, int nrowsIn, int nrowsO
 template <int L, bool HOUT>
 __global__ void __launch_bounds__(Len<L, E_C2R32>::NT, Len<L, E_C2R32>::MINB)
 k_rows_c2r32(const float2* __restrict__ in, int inRows, int nrows, double* __restrict__ out, int outStride,
-             int ncolsOut, const float2* __restrict__ tw, int twLen)
+             int ncolsOut, const float2* __restrict__ tab, const float2* __restrict__ tw, int twLen)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_C2R);
@@ -498,7 +512,7 @@ k_rows_c2r32(const float2* __restrict__ in, int inRows, int nrows, double* __res
     if (r < nb) cp_async8(A + r * SL + pad(k), in + spec32_at(inRows, row0 + r, k));
   }
   cp_async_commit();
-  load_twiddles<L, E_C2R32>(tws, tw, twLen);
+  load_twiddles<L, E_C2R32>(tws, tab);
   // the split's W^-k of the pairs (k, L - k) this thread forms, read while
   // the rows land (as in k_rows_c2r)
   constexpr int KPT = (H + NT - 1) / NT;
@@ -539,19 +553,37 @@ k_rows_c2r32(const float2* __restrict__ in, int inRows, int nrows, double* __res
     }
   }
   __syncthreads();
-  fft_inplace<L, true, false, HOUT, E_C2R32>(A, nb, tws);
-  const int half = (ncolsOut + 1) / 2;
-  for (int idx = threadIdx.x; idx < nb * half; idx += NT) {
-    const int r = idx / half, n = idx - r * half;
-    const float2 v = A[r * SL + pad(n)];
-    double* o = out + (size_t)(row0 + r) * outStride;
-    if (2 * n + 1 < ncolsOut) *reinterpret_cast<double2*>(o + 2 * n) = make_double2(v.x, v.y);
-    else o[2 * n] = v.x;
+  // the inverse FFT; its last pass writes the value pairs of the row
+  constexpr int E = E_C2R32, NS = last_ns<L, E>(), R = L / NS, T = L / E, NB = E / R, Q = L / R;
+  fft_passes_below<L, 1, NS, true, false, E>(A, nb, tws);
+  const int sq = threadIdx.x / T, j = threadIdx.x % T;
+  if (sq >= nb) return;
+  const float2* a = A + sq * SL;
+  double* o = out + (size_t)(row0 + sq) * outStride;
+  float2 x[E];
+  const int pj = pad(j);
+#pragma unroll
+  for (int u = 0; u < NB; u++)
+#pragma unroll
+    for (int m = 0; m < R; m++) x[u * R + m] = a[pad_at<T, Q>(pj, j, u, m)];
+#pragma unroll
+  for (int u = 0; u < NB; u++) {
+    float2* xb = x + u * R;
+    const int k = j + u * T;
+    if (k) apply_twiddles<L, E, R, NS, true>(xb, tws, k);
+    dft<R, true>(xb);
+#pragma unroll
+    for (int q = 0; q < (HOUT ? R / 2 : R); q++) {
+      const int n = k + q * NS;
+      const float2 v = xb[out_reg<R>(q)];
+      if (2 * n + 1 < ncolsOut) *reinterpret_cast<double2*>(o + 2 * n) = make_double2(v.x, v.y);
+      else if (2 * n < ncolsOut) o[2 * n] = v.x;
+    }
   }
 }
 
-template <int L> inline size_t smem_for32(size_t extraReals = 0) {
-  return sizeof(float2) * ((size_t)Len<L>::B * Len<L>::SL + Len<L>::TW) + sizeof(float) * extraReals;
+template <int L> inline size_t smem_for32(int nseq = Len<L>::B) {
+  return sizeof(float2) * ((size_t)nseq * Len<L>::SL + Len<L>::TW);
 }
 
 } // namespace
@@ -567,14 +599,28 @@ bool poisson32_setup() {
   return ok;
 }
 
+float2* make_tables32(int L, bool cols, const std::vector<float2>& tw, cudaStream_t st) {
+  static_assert(E_ROWS32 == E_C2R32, "one table serves both row passes");
+  std::vector<float2> t;
+  switch (L) {
+#define X(LL) case LL: if (cols) fill_tables32<LL, E_COLS32>(tw, t); else fill_tables32<LL, E_ROWS32>(tw, t); break;
+    CUP2D_FFT_LENGTHS(X)
+#undef X
+  }
+  float2* d = nullptr;
+  if (t.empty() || cudaMalloc(&d, sizeof(float2) * t.size()) != cudaSuccess) return nullptr;
+  h2d_sync(d, t.data(), sizeof(float2) * t.size(), st);
+  return d;
+}
+
 bool rows_r2c32(int L, cudaStream_t st, const double* in, int inStride, int nrows, int ncolsIn,
-                float2* out, int outRows, const float2* tw, int twLen, FadeArgs fa, bool halfIn) {
+                float2* out, int outRows, const float2* tab, const float2* tw, int twLen, FadeArgs fa, bool halfIn) {
   switch (L) {
 #define X(LL) case LL: \
     if (halfIn) launch_k(k_rows_r2c32<LL, true>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_ROWS32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outRows, tw, twLen, fa); \
+        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outRows, tab, tw, twLen, fa); \
     else launch_k(k_rows_r2c32<LL, false>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_ROWS32>::NT, \
-        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outRows, tw, twLen, fa); \
+        smem_for32<LL>(), st, in, inStride, nrows, ncolsIn, out, outRows, tab, tw, twLen, fa); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -583,15 +629,15 @@ bool rows_r2c32(int L, cudaStream_t st, const double* in, int inStride, int nrow
 }
 
 bool cols32(int L, cudaStream_t st, float2* data, int rows, int ncols, int nrowsIn, int nrowsOut,
-            const float* ghat, int mode, const float2* tw, int twLen, double norm, int MXp, int MYp) {
+            const float* ghat, int mode, const float2* tab, double norm, int MXp, int MYp) {
   switch (L) {
 #define X(LL) case LL: \
-    if (mode == 0) launch_k(k_cols32<LL, true>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS32>::NT, \
-        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, rows, ncols, nrowsIn, nrowsOut, \
-        ghat, mode, tw, twLen, norm, MXp, MYp); \
-    else launch_k(k_cols32<LL, false>, (ncols + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_COLS32>::NT, \
-        smem_for32<LL>((size_t)(LL / 2 + 1) * Len<LL>::B), st, data, rows, ncols, nrowsIn, nrowsOut, \
-        ghat, mode, tw, twLen, norm, MXp, MYp); \
+    if (mode == 0) launch_k(k_cols32<LL, true>, (ncols + Col32<LL>::CB - 1) / Col32<LL>::CB, Col32<LL>::NT, \
+        smem_for32<LL>(Col32<LL>::CB), st, data, rows, ncols, nrowsIn, nrowsOut, \
+        ghat, mode, tab, norm, MXp, MYp); \
+    else launch_k(k_cols32<LL, false>, (ncols + Col32<LL>::CB - 1) / Col32<LL>::CB, Col32<LL>::NT, \
+        smem_for32<LL>(Col32<LL>::CB), st, data, rows, ncols, nrowsIn, nrowsOut, \
+        ghat, mode, tab, norm, MXp, MYp); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -600,13 +646,13 @@ bool cols32(int L, cudaStream_t st, float2* data, int rows, int ncols, int nrows
 }
 
 bool rows_c2r32(int L, cudaStream_t st, const float2* in, int inRows, int nrows, double* out, int outStride,
-                int ncolsOut, const float2* tw, int twLen, bool halfOut) {
+                int ncolsOut, const float2* tab, const float2* tw, int twLen, bool halfOut) {
   switch (L) {
 #define X(LL) case LL: \
     if (halfOut) launch_k(k_rows_c2r32<LL, true>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_C2R32>::NT, \
-        smem_for32<LL>(), st, in, inRows, nrows, out, outStride, ncolsOut, tw, twLen); \
+        smem_for32<LL>(), st, in, inRows, nrows, out, outStride, ncolsOut, tab, tw, twLen); \
     else launch_k(k_rows_c2r32<LL, false>, (nrows + Len<LL>::B - 1) / Len<LL>::B, Len<LL, E_C2R32>::NT, \
-        smem_for32<LL>(), st, in, inRows, nrows, out, outStride, ncolsOut, tw, twLen); \
+        smem_for32<LL>(), st, in, inRows, nrows, out, outStride, ncolsOut, tab, tw, twLen); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
