@@ -192,7 +192,6 @@ inline size_t fish_pool_len(int nm) { return 36 * (size_t)nm + 16; }
 enum CounterSlot : int {
   CNT_MAXU = 0, CNT_ADV = 1, CNT_STEP = 2, CNT_RELDF = 3,
   CNT_CHI = 8,          // + shape
-  CNT_RHSOBST = 24,     // + shape
   CNT_FORCES = 40,      // + shape
   CNT_MOMENTS = 56,     // + shape
   CNT_MOMENTA = 72,     // + shape

@@ -268,16 +268,16 @@ k_udef_grid(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* ch
 }
 
 // ---------------------------------------------------------------------------
-// PressureSingle::updatePressureRHS, per-shape source (PressureSingle.cpp:136-168)
+// PressureSingle::updatePressureRHS, per-shape source (PressureSingle.cpp:136-168);
+// k_rhs_corr adds up the tiles' sums
 __global__ void __launch_bounds__(1024)
-k_rhs_obst(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
-           double* rhs, double* partials, unsigned* counter)
+k_rhs_obst(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
+           double* rhs, double* partials)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_RHSOBST);
   __shared__ double red[32 * 3];
-  DevShape& S = sh[k];
-  const int nt = S.ntiles, b0 = first_tile(t);
+  const int nt = sh[k].ntiles, b0 = first_tile(t);
   for (int s = blockIdx.x; s < nt; s += gridDim.x) {
   double acc[3] = {0, 0, 0};   // sumRHS, posRHS, negRHS
   bool any = false;
@@ -309,28 +309,24 @@ k_rhs_obst(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restric
   tile_sum<3>(acc, any, red, partials + 3 * s);
   __syncthreads();
   }
-  if (!last_block_done(counter, gridDim.x)) return;
-  tile_sum_rows<3>(partials, nt, red);
-  if (lin_tid() == 0) {
-    const double* tot = red;                                  // PressureSingle.cpp:185-186
-    const double corrDenom = tot[0] > 0 ? tot[1] : tot[2];
-    S.rhsCorr = tot[0] / fmax(corrDenom, EPSd);
-  }
 }
 
 // PressureSingle.cpp:173-212: perimeter correction of the same-sign RHS.
 // A tile that reaches the fade strip then rewrites its block's fade sums
-// (PoissonSolver.cpp:61-100) from the final RHS.
+// (PoissonSolver.cpp:61-100) from the final RHS.  Every CTA adds up the tiles'
+// sums for itself while its first tile's values are on their way: tens of values
+// from the L2, against the ticket and the last CTA's turn that k_rhs_obst would
+// end with (the two kernels 3.7 + 1.7 us with it, 2.2 + 2.4 without; swimmer
+// 1834 -> 1816 us a pass of 20 steps, ensemble 4158 -> 4115 of 10).
 __global__ void __launch_bounds__(1024)
-k_rhs_corr(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
-           double* rhs, const int* __restrict__ fadeSlot, double* fadePartials)
+k_rhs_corr(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
+           double* rhs, const double* partials, const int* __restrict__ fadeSlot, double* fadePartials)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_RHSCORR);
   __shared__ double red[32 * 3];
-  const DevShape& S = sh[k];
-  const double corr = S.rhsCorr;
-  const int nt = S.ntiles, b0 = first_tile(t);
+  double corr = 0;
+  const int nt = sh[k].ntiles, b0 = first_tile(t);
   auto CHI = [&](int x, int y) -> double {
     x = x < 0 ? 0 : (x >= g.nx ? g.nx - 1 : x);
     y = y < 0 ? 0 : (y >= g.ny ? g.ny - 1 : y);
@@ -344,6 +340,13 @@ k_rhs_corr(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __r
     const double chi = t.chi[(size_t)s * BS2 + iy * BS + ix], tmp = rhs[c], own = CHI(gx, gy);
     const double gradXx = CHI(gx + 1, gy) - CHI(gx - 1, gy);
     const double gradXy = CHI(gx, gy + 1) - CHI(gx, gy - 1);
+    if (s == (int)blockIdx.x) {
+      tile_sum_rows<3>(partials, nt, red);
+      const double corrDenom = red[0] > 0 ? red[1] : red[2];  // PressureSingle.cpp:185-186
+      corr = red[0] / fmax(corrDenom, EPSd);
+      if (s == 0 && lin_tid() == 0) sh[k].rhsCorr = corr;
+      __syncthreads();                                        // red is free again
+    }
     if (!(own > chi)) {
       const bool isPerim = gradXx * gradXx + gradXy * gradXy > 0;
       if (isPerim && tmp > 0 && corr > 0) rhs[c] = tmp - corr * tmp;
@@ -811,13 +814,14 @@ void launch_obj_vel_on_grid(Ctx& c) {
 void launch_rhs_obstacles(Ctx& c) {
   for (int k = 0; k < c.nshapes; k++) {
     launch_k(k_rhs_obst, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, 
-        c.g, c.dshapes, k, c.tiles[k], c.chi, c.rhs, shape_partials(c) + (size_t)k * shape_region(c),
-        c.counters + CNT_RHSOBST + k);
+        c.g, (const DevShape*)c.dshapes, k, c.tiles[k], (const double*)c.chi, c.rhs,
+        shape_partials(c) + (size_t)k * shape_region(c));
     CUP2D_LAUNCHED(c);
   }
   for (int k = 0; k < c.nshapes; k++) {
     launch_k(k_rhs_corr, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, c.g, c.dshapes, k, c.tiles[k],
-             (const double*)c.chi, c.rhs, (const int*)c.fadeSlot, fade_partials(c));
+             (const double*)c.chi, c.rhs, (const double*)(shape_partials(c) + (size_t)k * shape_region(c)),
+             (const int*)c.fadeSlot, fade_partials(c));
     CUP2D_LAUNCHED(c);
   }
 }
