@@ -141,12 +141,36 @@ k_raster_disk(GridDesc g, Scalars* sc, DevShape* sh, AllTiles T, double* sdf)
 //   A = sum w (p_x v - p_y u)       (p = x - C, u = udef).
 // J/M is the CoM correction d of putChiOnGrid; the moments about the
 // corrected CoM C + d that removeMoments integrates follow exactly in
-// algebra: M, U, V unchanged, Q - 2 d.J + M |d|^2, A - d_x V + d_y U.  The
-// last CTA of the shape adds the tile sums (fixed order) and finalises M,
-// J, the rigid udef part (removed where udef is read, udef_at) and d_gm.
+// algebra: M, U, V unchanged, Q - 2 d.J + M |d|^2, A - d_x V + d_y U.  One
+// CTA of the shape adds the tile sums (fixed order) and finalises M, J, the
+// rigid udef part (removed where udef is read, udef_at) and d_gm
+// (finish_moments): the last one of k_chi_moments or, in a graph step, where
+// nothing reads them before the momenta, one of k_rhs_obst beside the others
+// (k_chi_moments 6.0 -> 3.2 us; 512 x 256 with the cosine solver 1358 -> 1325 us
+// a pass of 20 steps, swimmer 1864 -> 1825).
+__device__ __forceinline__ void finish_moments(DevShape& S, const double* mp, double* red) {
+  const int nt = S.ntiles;
+  tile_sum_rows<7>(mp, nt, red);
+  if (lin_tid() != 0 || nt == 0) return;
+  const double* I = red;
+  const double M = I[2], C0 = S.s.com[0], C1 = S.s.com[1];
+  double d0 = 0, d1 = 0;
+  if (M > EPSd) {                                      // PutObjectsOnGrid.cpp:118-122
+    d0 = I[0] / M; d1 = I[1] / M;
+    S.s.com[0] = C0 + d0; S.s.com[1] = C1 + d1;
+  }
+  const double Q = I[3] - 2 * (d0 * I[0] + d1 * I[1]) + M * (d0 * d0 + d1 * d1);
+  const double A = I[6] - d0 * I[5] + d1 * I[4];
+  S.Iu = I[4] / M; S.Iv = I[5] / M; S.Ia = A / Q;
+  S.s.M = M; S.s.J = Q;
+  const double dCx = S.s.center[0] - S.s.com[0], dCy = S.s.center[1] - S.s.com[1];
+  const double co = S.cosO, si = S.sinO;         // cos/sin(orientation)
+  S.s.d_gm[0] = dCx * co + dCy * si;
+  S.s.d_gm[1] = -dCx * si + dCy * co;
+}
 __global__ void __launch_bounds__(1024)
 k_chi_moments(GridDesc g, DevShape* sh, AllTiles T, const double* __restrict__ sdfg,
-              double* chig, double* partials, int partStride, unsigned* counters)
+              double* chig, double* partials, int partStride, unsigned* counters, bool finish)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_CHI);
@@ -224,24 +248,7 @@ k_chi_moments(GridDesc g, DevShape* sh, AllTiles T, const double* __restrict__ s
   tile_sum<7>(I, any, red, mp + 7 * s);
   __syncthreads();
   }
-  if (!last_block_done(counters + k, gridDim.x)) return;
-  tile_sum_rows<7>(mp, nt, red);
-  if (lin_tid() != 0 || nt == 0) return;
-  const double* I = red;
-  const double M = I[2];
-  double d0 = 0, d1 = 0;
-  if (M > EPSd) {                                      // PutObjectsOnGrid.cpp:118-122
-    d0 = I[0] / M; d1 = I[1] / M;
-    S.s.com[0] = C0 + d0; S.s.com[1] = C1 + d1;
-  }
-  const double Q = I[3] - 2 * (d0 * I[0] + d1 * I[1]) + M * (d0 * d0 + d1 * d1);
-  const double A = I[6] - d0 * I[5] + d1 * I[4];
-  S.Iu = I[4] / M; S.Iv = I[5] / M; S.Ia = A / Q;
-  S.s.M = M; S.s.J = Q;
-  const double dCx = S.s.center[0] - S.s.com[0], dCy = S.s.center[1] - S.s.com[1];
-  const double co = S.cosO, si = S.sinO;         // cos/sin(orientation)
-  S.s.d_gm[0] = dCx * co + dCy * si;
-  S.s.d_gm[1] = -dCx * si + dCy * co;
+  if (finish && last_block_done(counters + k, gridDim.x)) finish_moments(S, mp, red);
 }
 
 // PutObjectsOnGrid::putObjectVelOnGrid (PutObjectsOnGrid.cpp:149-184), used at
@@ -269,16 +276,22 @@ k_udef_grid(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* ch
 
 // ---------------------------------------------------------------------------
 // PressureSingle::updatePressureRHS, per-shape source (PressureSingle.cpp:136-168);
-// k_rhs_corr adds up the tiles' sums
+// k_rhs_corr adds up the tiles' sums.  moments: the shape's sums of
+// k_chi_moments, finished by an additional, last CTA; or null.
 __global__ void __launch_bounds__(1024)
-k_rhs_obst(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
-           double* rhs, double* partials)
+k_rhs_obst(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
+           double* rhs, double* partials, const double* moments)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_RHSOBST);
   __shared__ double red[32 * 3];
+  const int ctas = gridDim.x - (moments ? 1 : 0);
+  if ((int)blockIdx.x == ctas) {
+    finish_moments(sh[k], moments, red);
+    return;
+  }
   const int nt = sh[k].ntiles, b0 = first_tile(t);
-  for (int s = blockIdx.x; s < nt; s += gridDim.x) {
+  for (int s = blockIdx.x; s < nt; s += ctas) {
   double acc[3] = {0, 0, 0};   // sumRHS, posRHS, negRHS
   bool any = false;
   {
@@ -794,7 +807,7 @@ void launch_objects_rest(Ctx& c) {
       if (c.hshapes[k].cfg.kind != CUP2D_SHAPE_DISK) launch_fish_raster(c, k);
   const int stride = (int)shape_region(c);
   launch_k(k_chi_moments, dim3(tile_ctas(c, c.maxExpect), c.nshapes), dim3(32, 32), 0, c.stream, c.g, c.dshapes, T,
-           (const double*)c.sdf, c.chi, shape_partials(c), stride, c.counters + CNT_MOMENTS);
+           (const double*)c.sdf, c.chi, shape_partials(c), stride, c.counters + CNT_MOMENTS, !c.graphStep);
   CUP2D_LAUNCHED(c);
 }
 
@@ -811,16 +824,23 @@ void launch_obj_vel_on_grid(Ctx& c) {
   }
 }
 
+// three values per tile, behind the seven of k_chi_moments, which a graph
+// step's k_rhs_obst still reads
+static double* rhs_partials(const Ctx& c, int k) {
+  return shape_partials(c) + (size_t)k * shape_region(c) + (size_t)7 * c.maxCapacity;
+}
+
 void launch_rhs_obstacles(Ctx& c) {
   for (int k = 0; k < c.nshapes; k++) {
-    launch_k(k_rhs_obst, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, 
-        c.g, (const DevShape*)c.dshapes, k, c.tiles[k], (const double*)c.chi, c.rhs,
-        shape_partials(c) + (size_t)k * shape_region(c));
+    double* const p = shape_partials(c) + (size_t)k * shape_region(c);
+    launch_k(k_rhs_obst, tile_ctas(c, c.tiles[k].expect) + (c.graphStep ? 1 : 0), dim3(32, 32), 0, c.stream,
+        c.g, c.dshapes, k, c.tiles[k], (const double*)c.chi, c.rhs, rhs_partials(c, k),
+        c.graphStep ? (const double*)p : nullptr);
     CUP2D_LAUNCHED(c);
   }
   for (int k = 0; k < c.nshapes; k++) {
     launch_k(k_rhs_corr, tile_ctas(c, c.tiles[k].expect), dim3(32, 32), 0, c.stream, c.g, c.dshapes, k, c.tiles[k],
-             (const double*)c.chi, c.rhs, (const double*)(shape_partials(c) + (size_t)k * shape_region(c)),
+             (const double*)c.chi, c.rhs, (const double*)rhs_partials(c, k),
              (const int*)c.fadeSlot, fade_partials(c));
     CUP2D_LAUNCHED(c);
   }
