@@ -250,6 +250,11 @@ class stdout_to_stderr:
         return False
 
 
+def reference_available():
+    from oracle import refsim
+    return refsim.available()
+
+
 def run_reference(args, world, rank, pg):
     """The reference's own operators (oracle/_ref) on the host cores.  For
     the ensemble: its first four members one after another, the steps split
@@ -886,6 +891,13 @@ def main():
         out = adjoint_measurement(local, rank, pg, nsteps=args.adjoint_only, every=args.adjoint_only)
         if rank == 0:
             print(json.dumps(out))
+        if pg is not None:
+            pg.barrier()
+            pg.destroy_process_group()
+        return
+    if args.impl == "reference" and not reference_available():
+        if rank == 0:
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's sources and its build are not present"}))
         if pg is not None:
             pg.barrier()
             pg.destroy_process_group()
