@@ -660,7 +660,9 @@ k_forces(GridDesc g, Scalars* sc, int maxNext, DevShape* sh, AllTiles T, const d
     if (maxNext) {
       const size_t c = (size_t)(by * BS + iy) * g.nx + bx * BS + ix;
       const double a = u[c], w = v[c];
-      const double mx = warp_max(cell_speed(a, w, UINF, VINF));
+      // (a cell whose components are both NaN counts as zero: the maximum
+      // below must be a number, and the status flag reports the cell)
+      const double mx = warp_max(fmax(0.0, cell_speed(a, w, UINF, VINF)));
       const bool bad = __any_sync(0xffffffffu, !isfinite(a) || !isfinite(w));
       if (ix == 0) {
         redm[iy] = mx;                                  // a warp is a row of the tile
