@@ -698,48 +698,43 @@ int adj_fail(cup2d_ctx* ctx, int code, const std::string& msg) {
     }                                                                           \
   } while (0)
 
-// Device scratch of an adjoint run, cut from the context's chunks.  A call
-// needs some 25 buffers; allocating and freeing each had taken 8 of the 14 ms
-// of a 20-step run at 512 x 256.  The chunks stay with the context for its
-// next run while they are at most ADJ_KEEP bytes, else they are freed on exit
-// as the buffers were.  Every use of a buffer is over when a run returns: the
-// device is waited for (a run that ends in an error may have left work).
-struct AdjBufs {
+// Device scratch of an adjoint run: its some 25 buffers laid out one after
+// another in the context's scratch (allocated and freed one by one they had
+// taken 7 to 8 ms of a 20-step run at 512 x 256).  Every use of it is over when
+// the run returns: the streams that may hold its work are waited for (a run
+// that ends in an error may have left some).
+struct AdjScratch {
   Ctx& c;
-  explicit AdjBufs(Ctx& ctx) : c(ctx) { for (Ctx::Chunk& k : c.adjChunks) k.used = 0; }
-  AdjBufs(const AdjBufs&) = delete;
-  ~AdjBufs() {
-    cudaDeviceSynchronize();
-    size_t total = 0;
-    for (const Ctx::Chunk& k : c.adjChunks) total += k.bytes;
-    if (total <= Ctx::ADJ_KEEP) return;
-    for (const Ctx::Chunk& k : c.adjChunks) cudaFree(k.p);
-    c.adjChunks.clear();
+  explicit AdjScratch(Ctx& ctx) : c(ctx) {}
+  AdjScratch(const AdjScratch&) = delete;
+  ~AdjScratch() {
+    if (!taken) return;
+    wait(c);
+    for (cup2d_ctx* x : c.gaitShadows) wait(x->c);
+    scratch_give(c);
   }
-  template <typename T> T* get(size_t n) {
-    const size_t want = (sizeof(T) * (n ? n : 1) + 255) / 256 * 256;
-    for (Ctx::Chunk& k : c.adjChunks)
-      if (k.bytes - k.used >= want) {
-        T* q = reinterpret_cast<T*>(k.p + k.used);
-        k.used += want;
-        return q;
-      }
-    // a chunk of its own for a large buffer, 16 MB for small ones; on a full
-    // device the buffer alone, with the chunks that this run does not use given
-    // back first
-    size_t bytes = std::max(want, (size_t)16 << 20);
-    void* q = nullptr;
-    if (cudaMalloc(&q, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      auto unused = [](const Ctx::Chunk& k) { return k.used == 0; };
-      for (const Ctx::Chunk& k : c.adjChunks)
-        if (unused(k)) cudaFree(k.p);
-      c.adjChunks.erase(std::remove_if(c.adjChunks.begin(), c.adjChunks.end(), unused), c.adjChunks.end());
-      bytes = want;
-      if (cudaMalloc(&q, bytes) != cudaSuccess) return nullptr;
-    }
-    c.adjChunks.push_back({static_cast<char*>(q), bytes, want});
-    return static_cast<T*>(q);
+  // n elements, their address to be in p once take() has returned true; p
+  // itself must stay where it is until then
+  template <class T> void add(T*& p, size_t n) {
+    p = nullptr;
+    parts.push_back({reinterpret_cast<void**>(&p), total});
+    total += (sizeof(T) * (n ? n : 1) + 255) / 256 * 256;
+  }
+  bool take() {
+    char* const base = scratch_take(c, total);
+    if (!base) return false;
+    taken = true;
+    for (const Part& q : parts) *q.p = base + q.at;
+    return true;
+  }
+
+private:
+  struct Part { void** p; size_t at; };
+  std::vector<Part> parts;
+  size_t total = 0;
+  bool taken = false;
+  static void wait(Ctx& x) {
+    for (cudaStream_t st : {x.stream, x.side, x.side2}) cudaStreamSynchronize(st);
   }
 };
 
@@ -844,24 +839,64 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
   const dim3 grid2(g.bpdx, g.bpdy), blk2(32, 8);
   const int probeGrid = energy ? std::min(1024, ((bx.x1 - bx.x0) * (bx.y1 - bx.y0) + 255) / 256) : 1;
 
-  AdjBufs B(c);
+  AdjScratch B(c);
   size_t ckBytes = 0;
   ARC(cup2d_checkpoint_size(ctx, &ckBytes));
   const int nseg = (nsteps + every - 1) / every;
-  std::vector<void*> ck(nseg + 1);
-  for (int s = 0; s <= nseg; s++)
-    if (!(ck[s] = B.get<char>(ckBytes))) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint checkpoints");
+  const size_t segN = (size_t)std::min(every, nsteps);   // steps of a segment
+  const bool backward = grad_u || grad_v || grad_body || gait;
+  std::vector<char*> ck(nseg + 1);
+  for (char*& q : ck) B.add(q, ckBytes);
   // a step's reductions of its transposed stages, zeroed for all steps at
   // once: the fade's five, the obstacle terms' five, advDiff's Gamma
   constexpr int ACC = 16;
-  double* acc = B.get<double>(ACC * (size_t)nsteps);
+  double *acc, *obv;
+  StepRecord* rec;
+  B.add(acc, ACC * (size_t)nsteps);
   // [0] J; [1..3] the body-velocity gradient (forced: the held velocity's,
   // accumulated over the steps; free: the adjoint of the step's output
   // velocity); [4..6] a free body's adjoint of the previous output, formed
   // by advDiff's lab velocity; [8..10] the solve's transpose
-  double* obv = B.get<double>(12);
-  StepRecord* rec = B.get<StepRecord>(nsteps);
-  if (!acc || !obv || !rec) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint scratch");
+  B.add(obv, 12);
+  B.add(rec, nsteps);
+  // backward: the velocity at the segment's start and after each of its steps
+  // (u^n of step j > 0 is u^(n+1) of step j - 1), the RHS before the obstacle
+  // terms and before the fade
+  double *su = nullptr, *sv = nullptr, *sT = nullptr, *sF = nullptr, *pu = nullptr, *pv = nullptr;
+  double *lu = nullptr, *lv = nullptr, *l1 = nullptr, *l2 = nullptr, *tu = nullptr, *tv = nullptr;
+  if (backward) {
+    for (double** q : {&su, &sv, &lu, &lv, &l1, &l2, &tu, &tv}) B.add(*q, n);
+    for (double** q : {&sT, &sF, &pu, &pv}) B.add(*q, n * segN);
+  }
+  // the gait: advDiff's velocity and the pressure of each step, and the
+  // geometry sensitivities of every step of the run
+  double *su1 = nullptr, *sv1 = nullptr, *sp = nullptr, *gCom = nullptr, *accs = nullptr;
+  double* gG[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // gX, gU, gV, gSX, gSY
+  constexpr int nrep = 2 * CUP2D_GAIT_PARAMS;
+  if (gait) {
+    for (double** q : {&su1, &sv1, &sp}) B.add(*q, n * segN);
+    for (double*& q : gG) B.add(q, n * (size_t)nsteps);
+    B.add(gCom, 2 * (size_t)nsteps);                     // d/d(centre of mass)
+    B.add(accs, nrep);
+  }
+  // a swimmer: each recomputed step's obstacle state (the shape's tile
+  // count and centre of mass, its tiles, the grid's chi); a disk's does not
+  // change from step to step, and the live one serves
+  const ObstTiles live = c.tiles[0];
+  const int cap = live.capacity;
+  const size_t tb = (size_t)cap * BS2;
+  const bool keepObst = sf.kind != CUP2D_SHAPE_DISK;
+  DevShape* shSnap = nullptr;
+  int* tlSnap = nullptr;
+  double* tSnap[6] = {};                                 // chi, udx, udy, sD, sdx, sdy
+  double* chiSnap = nullptr;
+  if (backward && keepObst) {
+    B.add(shSnap, segN);
+    B.add(tlSnap, (size_t)cap * segN);
+    for (double*& q : tSnap) B.add(q, tb * segN);
+    B.add(chiSnap, n * segN);
+  }
+  if (!B.take()) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint scratch");
   std::vector<double> dts(nsteps);
   struct Ev {
     cudaEvent_t e[3] = {nullptr, nullptr, nullptr};
@@ -921,60 +956,16 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
   float fms = 0;
   ACK(cudaEventElapsedTime(&fms, e0, e1));
   if (ms) { ms[0] = fms; ms[1] = 0; if (gait) ms[2] = 0; }
-  if (!grad_u && !grad_v && !grad_body && !gait) {
+  if (!backward) {
     ALOAD(nseg);
     return CUP2D_OK;
   }
 
   // backward
-  const size_t segN = (size_t)std::min(every, nsteps);   // steps of a segment
-  // the velocity at the segment's start and after each of its steps (u^n of
-  // step j > 0 is u^(n+1) of step j - 1)
-  double* su = B.get<double>(n);
-  double* sv = B.get<double>(n);
-  double* sT = B.get<double>(n * segN);      // RHS before the obstacle terms
-  double* sF = B.get<double>(n * segN);      // RHS before the fade
-  double* pu = B.get<double>(n * segN);
-  double* pv = B.get<double>(n * segN);
-  // the gait: advDiff's velocity and the pressure of each step, and the
-  // geometry sensitivities of every step of the run
-  double* su1 = gait ? B.get<double>(n * segN) : nullptr;
-  double* sv1 = gait ? B.get<double>(n * segN) : nullptr;
-  double* sp = gait ? B.get<double>(n * segN) : nullptr;
-  double* gG[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // gX, gU, gV, gSX, gSY
-  double* gCom = gait ? B.get<double>(2 * (size_t)nsteps) : nullptr;  // d/d(centre of mass)
   if (gait) {
-    if (!gCom) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint gait planes");
     ACK(cudaMemsetAsync(gCom, 0, sizeof(double) * 2 * nsteps, c.stream));
-    for (double*& q : gG) {
-      if (!(q = B.get<double>(n * (size_t)nsteps))) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint gait planes");
-      ACK(cudaMemsetAsync(q, 0, nb * nsteps, c.stream));
-    }
-    if (!su1 || !sv1 || !sp) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint segment buffers");
+    for (double* q : gG) ACK(cudaMemsetAsync(q, 0, nb * nsteps, c.stream));
   }
-  double* lu = B.get<double>(n);
-  double* lv = B.get<double>(n);
-  double* l1 = B.get<double>(n);
-  double* l2 = B.get<double>(n);
-  double* tu = B.get<double>(n);
-  double* tv = B.get<double>(n);
-  if (!su || !sv || !sT || !sF || !pu || !pv || !lu || !lv || !l1 || !l2 || !tu || !tv)
-    return adj_fail(ctx, CUP2D_ENOMEM, "adjoint segment buffers");
-  // a swimmer: each recomputed step's obstacle state (the shape's tile
-  // count and centre of mass, its tiles, the grid's chi); a disk's does not
-  // change from step to step, and the live one serves
-  const ObstTiles live = c.tiles[0];
-  const int cap = live.capacity;
-  const size_t tb = (size_t)cap * BS2;
-  const bool keepObst = sf.kind != CUP2D_SHAPE_DISK;
-  const size_t segK = keepObst ? segN : 0;
-  DevShape* shSnap = B.get<DevShape>(segK);
-  int* tlSnap = B.get<int>((size_t)cap * segK);
-  double* tSnap[6];
-  for (int q = 0; q < 6; q++) tSnap[q] = B.get<double>(tb * segK);   // chi, udx, udy, sD, sdx, sdy
-  double* chiSnap = B.get<double>(n * segK);
-  if (!shSnap || !tlSnap || !chiSnap) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint obstacle snapshots");
-  for (double* q : tSnap) if (!q) return adj_fail(ctx, CUP2D_ENOMEM, "adjoint obstacle snapshots");
   auto tilesAt = [&](int j) {
     if (!keepObst) return live;
     ObstTiles t = live;
@@ -1135,7 +1126,6 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
           cudaStreamSynchronize(cx.stream) != cudaSuccess) return CUP2D_ECUDA;
       return CUP2D_OK;
     };
-    const int nrep = 2 * np;
     std::vector<double> Cpm(nrep, 0.0);
     std::vector<std::array<double, CUP2D_GAIT_PARAMS>> ths(nrep);
     for (int j = 0; j < nrep; j++) {
@@ -1145,8 +1135,7 @@ int cup2d_adjoint_run(cup2d_ctx* ctx, int nsteps, int every, const cup2d_adjoint
     // side by side on contexts of this configuration, one host thread each
     // (the replays are latency-bound: the midline and the frame are
     // one-CTA kernels), else one after another on this context
-    double* accs = B.get<double>(nrep);
-    const bool side = accs && gait_shadows(ctx, nrep);   // (made on first use, not timed)
+    const bool side = gait_shadows(ctx, nrep);   // (made on first use, not timed)
     // host clock: the replays run on other contexts' streams
     const auto t0 = std::chrono::steady_clock::now();
     if (side) {

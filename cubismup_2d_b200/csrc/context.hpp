@@ -152,11 +152,10 @@ struct Ctx {
   std::vector<int> shapeKinds;
   std::vector<struct cup2d_ctx*> gaitShadows;
 
-  // device scratch of cup2d_adjoint_run, kept between calls up to ADJ_KEEP
-  // bytes (freed with the context)
-  struct Chunk { char* p; size_t bytes, used; };
-  std::vector<Chunk> adjChunks;
-  static constexpr size_t ADJ_KEEP = (size_t)1 << 30;
+  // device scratch of cup2d_adjoint_run; between runs it may stay for the next
+  // one (scratch_give)
+  char* scratch = nullptr;
+  size_t scratchBytes = 0;
 
   cudaGraphExec_t graph = nullptr;
   void* flushBuf = nullptr;      // cup2d_time_kernel's L2 flush (256 MB, allocated on demand)
@@ -187,6 +186,19 @@ inline bool midline_ahead(const Ctx& c, int k) {
 // two midline buffers, the frame midline, the integrals, then the skins of
 // the two midline buffers
 inline size_t fish_pool_len(int nm) { return 36 * (size_t)nm + 16; }
+
+// Device memory; where there is none left, the idle scratch of this process's
+// contexts is given back and the allocation tried again.  A failure leaves no
+// error pending in the runtime.
+cudaError_t device_malloc(void** p, size_t bytes);
+template <class T> cudaError_t device_malloc(T** p, size_t bytes) {
+  return device_malloc(reinterpret_cast<void**>(p), bytes);
+}
+// A context's scratch of at least `bytes` (null: no memory), its end of use
+// (no work on it is in flight any more), and its release.
+char* scratch_take(Ctx& c, size_t bytes);
+void scratch_give(Ctx& c);
+void scratch_drop(Ctx& c);
 
 // counter slots used by the kernels (each last-CTA reduction owns one)
 enum CounterSlot : int {

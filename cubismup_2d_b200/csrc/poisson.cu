@@ -1055,7 +1055,7 @@ double2* make_tables(int L, int E, const std::vector<long double>& c, const std:
     ns *= R;
   }
   double2* d = nullptr;
-  if (cudaMalloc(&d, sizeof(double2) * std::max<size_t>(1, t.size())) != cudaSuccess) return nullptr;
+  if (device_malloc(&d, sizeof(double2) * std::max<size_t>(1, t.size())) != cudaSuccess) return nullptr;
   if (!t.empty()) h2d_sync(d, t.data(), sizeof(double2) * t.size(), st);
   return d;
 }
@@ -1166,13 +1166,13 @@ Poisson* poisson_create(Ctx& c) {
     tws[k] = sinl(a);
     tw[k] = make_double2((double)twc[k], (double)tws[k]);
   }
-  if (cudaMalloc(&P->tw, sizeof(double2) * P->twLen) != cudaSuccess) { delete P; return nullptr; }
+  if (device_malloc(&P->tw, sizeof(double2) * P->twLen) != cudaSuccess) { delete P; return nullptr; }
   h2d_sync(P->tw, tw.data(), sizeof(double2) * P->twLen, c.stream);
   if (!(P->tRow[0] = make_tables(P->Lrow, 8, twc, tws, c.stream)) ||
       !(P->tRow[1] = make_tables(P->Lrow, 16, twc, tws, c.stream)) ||
       !(P->tCol = make_tables(P->Lcol, 16, twc, tws, c.stream))) { poisson_destroy(P); return nullptr; }
   const size_t specRows = (size_t)P->Lcol, ncols = P->type == CUP2D_POISSON_COSINE ? Nx / 2 : P->nkx;
-  if (cudaMalloc(&P->spec, sizeof(double2) * specRows * ((ncols + SPEC_K - 1) / SPEC_K * SPEC_K)) != cudaSuccess) {
+  if (device_malloc(&P->spec, sizeof(double2) * specRows * ((ncols + SPEC_K - 1) / SPEC_K * SPEC_K)) != cudaSuccess) {
     poisson_destroy(P);
     return nullptr;
   }
@@ -1183,16 +1183,16 @@ Poisson* poisson_create(Ctx& c) {
     std::vector<float> cx(Nx), cy(Ny);
     for (int j = 0; j < Ny; j++) cy[j] = (float)std::cos(M_PI / Ny * 2.0 * j);
     for (int i = 0; i < Nx; i++) cx[i] = (float)std::cos(M_PI / Nx * 2.0 * i);
-    if (cudaMalloc(&P->cosX, sizeof(float) * Nx) != cudaSuccess ||
-        cudaMalloc(&P->cosY, sizeof(float) * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+    if (device_malloc(&P->cosX, sizeof(float) * Nx) != cudaSuccess ||
+        device_malloc(&P->cosY, sizeof(float) * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
     h2d_sync(P->cosX, cx.data(), sizeof(float) * Nx, c.stream);
     h2d_sync(P->cosY, cy.data(), sizeof(float) * Ny, c.stream);
-    if (cudaMalloc(&P->ghat, sizeof(double) * Nx * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+    if (device_malloc(&P->ghat, sizeof(double) * Nx * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
     k_dct_multiplier<<<4 * c.sms, 256, 0, c.stream>>>(P->ghat, Nx, Ny, P->cosX, P->cosY, P->tol);
     CUP2D_LAUNCHED(c);
   }
   if (P->type != CUP2D_POISSON_COSINE &&
-      cudaMalloc(&P->ghat, sizeof(double) * (P->Lcol / 2 + 1) * P->nkx) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+      device_malloc(&P->ghat, sizeof(double) * (P->Lcol / 2 + 1) * P->nkx) != cudaSuccess) { poisson_destroy(P); return nullptr; }
   if (P->type == CUP2D_POISSON_FREESPACE) {
     // G^ = Re FFT[G] / (MX MY) on the MY x MX padded grid, kept for ky <= MY/2;
     // a quarter of norm: twice the spectrum comes in here and in the solve
@@ -1210,7 +1210,7 @@ Poisson* poisson_create(Ctx& c) {
     P->fp32 = true;
     std::vector<float2> tw32(P->twLen);
     for (int k = 0; k < P->twLen; k++) tw32[k] = make_float2((float)tw[k].x, (float)tw[k].y);
-    if (cudaMalloc(&P->tw32, sizeof(float2) * P->twLen) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+    if (device_malloc(&P->tw32, sizeof(float2) * P->twLen) != cudaSuccess) { poisson_destroy(P); return nullptr; }
     h2d_sync(P->tw32, tw32.data(), sizeof(float2) * P->twLen, c.stream);
     if (!(P->tRow32 = make_tables32(P->Lrow, false, tw32, c.stream)) ||
         !(P->tCol32 = make_tables32(P->Lcol, true, tw32, c.stream))) { poisson_destroy(P); return nullptr; }
@@ -1220,7 +1220,7 @@ Poisson* poisson_create(Ctx& c) {
       std::vector<float> g32(ng);
       if (cudaStreamSynchronize(c.stream) != cudaSuccess ||
           cudaMemcpy(g64.data(), P->ghat, sizeof(double) * ng, cudaMemcpyDeviceToHost) != cudaSuccess ||
-          cudaMalloc(&P->ghat32, sizeof(float) * ng) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+          device_malloc(&P->ghat32, sizeof(float) * ng) != cudaSuccess) { poisson_destroy(P); return nullptr; }
       for (size_t i = 0; i < ng; i++) g32[i] = (float)(2 * g64[i]);
       h2d_sync(P->ghat32, g32.data(), sizeof(float) * ng, c.stream);
     }

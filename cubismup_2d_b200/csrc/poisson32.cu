@@ -608,7 +608,7 @@ float2* make_tables32(int L, bool cols, const std::vector<float2>& tw, cudaStrea
 #undef X
   }
   float2* d = nullptr;
-  if (t.empty() || cudaMalloc(&d, sizeof(float2) * t.size()) != cudaSuccess) return nullptr;
+  if (t.empty() || device_malloc(&d, sizeof(float2) * t.size()) != cudaSuccess) return nullptr;
   h2d_sync(d, t.data(), sizeof(float2) * t.size(), st);
   return d;
 }
