@@ -203,7 +203,6 @@ void scratch_drop(Ctx& c);
 // counter slots used by the kernels (each last-CTA reduction owns one)
 enum CounterSlot : int {
   CNT_MAXU = 0, CNT_ADV = 1, CNT_STEP = 2, CNT_RELDF = 3,
-  CNT_CHI = 8,          // + shape
   CNT_FORCES = 40,      // + shape
   CNT_MOMENTS = 56,     // + shape
   CNT_MOMENTA = 72,     // + shape

@@ -36,53 +36,10 @@ __device__ __forceinline__ bool segment_hits_block(const Segment& S, const doubl
   return true;
 }
 
+// a rectangle of blocks clipped to the grid
 __device__ __forceinline__ void clip_rect(const GridDesc& g, int& bx0, int& bx1, int& by0, int& by1) {
   bx0 = bx0 < 0 ? 0 : bx0; by0 = by0 < 0 ? 0 : by0;
   bx1 = bx1 > g.bpdx - 1 ? g.bpdx - 1 : bx1; by1 = by1 > g.bpdy - 1 ? g.bpdy - 1 : by1;
-}
-
-// Ordered tile selection: the blocks of the rectangle [bx0, bx1] x [by0, by1]
-// (clipped to the grid) for which touch(bx, by) holds, in increasing block
-// index (the order of obstacleBlocks[blockID]), become t.tiles[0..n) with
-// t.slot[b]; n goes to *ntilesOut, overflow of the capacity raises
-// ST_CAPACITY.  touch(q, bx, by) gets the candidate's row-major index q in
-// the clipped rectangle (clip_rect).  Called by a whole 1D CTA whose size
-// is a multiple of 32.
-template <class Touch>
-__device__ void select_tiles(const GridDesc& g, ObstTiles t, int bx0, int bx1, int by0, int by1,
-                             Touch touch, int* ntilesOut, int* status)
-{
-  __shared__ int wcnt[32];
-  __shared__ int base;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  clip_rect(g, bx0, bx1, by0, by1);
-  const int W = bx1 - bx0 + 1, H = by1 - by0 + 1, n = (W > 0 && H > 0) ? W * H : 0;
-  if (tid == 0) base = 0;
-  __syncthreads();
-  for (int q0 = 0; q0 < n; q0 += blockDim.x) {
-    const int q = q0 + tid;
-    int b = -1;
-    bool f = false;
-    if (q < n) {
-      const int by = by0 + q / W, bx = bx0 + q % W;
-      b = by * g.bpdx + bx;
-      f = touch(q, bx, by);
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, f);
-    if (lane == 0) wcnt[wid] = __popc(m);
-    __syncthreads();
-    int off = 0, tot = 0;
-    for (int w = 0; w < nw; w++) { if (w < wid) off += wcnt[w]; tot += wcnt[w]; }
-    const int pos = base + off + __popc(m & ((1u << lane) - 1u));
-    if (f) {
-      if (pos < t.capacity) { t.tiles[pos] = b; t.slot[b] = pos; }
-      else atomicOr(status, ST_CAPACITY);
-    }
-    __syncthreads();
-    if (tid == 0) base += tot;
-    __syncthreads();
-  }
-  if (tid == 0) *ntilesOut = base < t.capacity ? base : t.capacity;
 }
 
 // Block index range whose cells' AABB, widened by `safe`, can overlap
@@ -92,17 +49,6 @@ __device__ __forceinline__ void block_range(double lo, double hi, double h, doub
   const double bw = BS * h;
   b0 = (int)floor(fmax((lo - safe) / bw, -2.0)) - 1;
   b1 = (int)floor(fmin((hi + safe) / bw, 1e8)) + 1;
-}
-
-// Fish::create step 6 (Fish.cpp:158-173): does any segment intersect block?
-__device__ __forceinline__ bool fish_block_touching(const GridDesc& g, const Segment* seg, int nseg,
-                                                    int bx, int by)
-{
-  const double start[2] = {cell_x(g, bx, 0), cell_y(g, by, 0)};
-  const double end[2] = {cell_x(g, bx, BS - 1), cell_y(g, by, BS - 1)};
-  for (int s = 0; s < nseg; s++)
-    if (segment_hits_block(seg[s], start, end, 2 * g.h)) return true;
-  return false;
 }
 
 } // namespace cup2d

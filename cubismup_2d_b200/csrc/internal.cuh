@@ -52,7 +52,7 @@ struct IterState {
 struct Scalars {
   double time, dt, uinfx, uinfy, lambda;
   double maxU;
-  double outflowCorr;             // advDiff.cpp:105
+  double outflowCorr;             // advDiffGrav's outflow correction (variable density)
   double fadeCorr;                // PoissonSolver.cpp:86
   int step;
   int status;
@@ -122,7 +122,7 @@ struct DevShape {
   int ntiles;                     // obstacle tiles this step
   int ntilesPrev;
   double rhoTile;                 // ObstacleBlock::rho: rhoS (disk), 1 (fish)
-  double rhsCorr;                 // PressureSingle.cpp:183-186 corr of this shape
+  double reserved;                // zero; checkpoints hold this structure as it is
   double bbox[2][2];              // disk bounding box (ShapeLibrary.h:40-43)
   double cosO, sinO;              // cos/sin(orientation), set where the orientation moves
   int nseg;                       // fish AreaSegments this step
@@ -192,11 +192,11 @@ struct FishArrays {
 // (atomicMax into slot 2*id+1), so one step's overlapped schedule can be
 // read back.  Without the define the scope compiles to nothing.
 enum TraceId : int {
-  TR_MAXU, TR_SETDT, TR_ENDSTEP, TR_ADVDIFF, TR_RHSDIV, TR_PCORR, TR_FADE,
-  TR_OBJBEGIN, TR_DISK_PLACE, TR_RASTER_DISK, TR_CHI, TR_MOMENTS,
+  TR_MAXU, TR_SETDT, TR_ENDSTEP, TR_ADVDIFF, TR_RHSDIV, TR_PCORR,
+  TR_OBJBEGIN, TR_RASTER_DISK, TR_CHI,
   TR_UDEF, TR_RHSOBST, TR_RHSCORR, TR_MOMENTA, TR_COLLIDE, TR_PENALIZE, TR_FORCES,
   TR_MIDLINE, TR_FRAME, TR_RASTER, TR_R2C, TR_COLS, TR_C2R, TR_DCT_FWD, TR_DCT_COLS,
-  TR_DCT_INV, TR_SELECT, TR_MAXNEXT, TR_N
+  TR_DCT_INV, TR_SELECT, TR_N
 };
 // per-work-item phase stamps of the trace build: slot 2*TR_N + 8*item + phase
 constexpr int TRACE_ITEMS = 4096;

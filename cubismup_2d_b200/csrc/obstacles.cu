@@ -332,7 +332,7 @@ k_rhs_obst(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restric
 // end with (the two kernels 3.7 + 1.7 us with it, 2.2 + 2.4 without; swimmer
 // 1834 -> 1816 us a pass of 20 steps, ensemble 4158 -> 4115 of 10).
 __global__ void __launch_bounds__(1024)
-k_rhs_corr(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
+k_rhs_corr(GridDesc g, const DevShape* sh, int k, ObstTiles t, const double* __restrict__ chig,
            double* rhs, const double* partials, const int* __restrict__ fadeSlot, double* fadePartials)
 {
   pdl_begin();
@@ -357,7 +357,6 @@ k_rhs_corr(GridDesc g, DevShape* sh, int k, ObstTiles t, const double* __restric
       tile_sum_rows<3>(partials, nt, red);
       const double corrDenom = red[0] > 0 ? red[1] : red[2];  // PressureSingle.cpp:185-186
       corr = red[0] / fmax(corrDenom, EPSd);
-      if (s == 0 && lin_tid() == 0) sh[k].rhsCorr = corr;
       __syncthreads();                                        // red is free again
     }
     if (!(own > chi)) {

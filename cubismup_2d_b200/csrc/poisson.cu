@@ -55,7 +55,6 @@ struct Poisson {
   float2* tRow32 = nullptr;  // pass tables of the FP32 row and column transforms
   float2* tCol32 = nullptr;
   float* ghat32 = nullptr;   // the free-space kernel rounded to FP32, [nkx][Lcol/2 + 1]
-  int rb = 1, cb = 1;        // rows / columns per CTA
   int MX = 0, MY = 0;        // free space: the padded grid (powers of two >= 2Nx, 2Ny)
   // elements per thread of the forward and inverse row passes (FP64 free
   // space and periodic), and the times the autotuner measured (us; r2c with
@@ -279,25 +278,6 @@ __device__ __forceinline__ void fft_turn(double2* a, bool act, int j, Tab tab, M
     for (int q = 0; q < E; q++) a[pad_out<1>(pad(j * E), j * E, q)] = y[out_reg<E>(q)];
   }
   __syncthreads();
-}
-
-// Spectral convolution in place: fft_inplace<L, false, HIN>, X[r] = mul(r,
-// X[r]), fft_inplace<L, true, false, HOUT>, with the turn in registers.  With
-// L <= E (one pass each way) the three steps run one after the other.
-template <int L, bool HIN, bool HOUT, int E, class Mul>
-__device__ __forceinline__ void fft_convolve(double2* a, bool act, int j, Tab tab, Mul mul)
-{
-  if constexpr (L <= E) {
-    fft_inplace<L, false, HIN, false, E>(a, act, j, tab);
-    if (act)
-      for (int r = j; r < L; r += L / E) a[pad(r)] = mul(r, a[pad(r)]);
-    __syncthreads();
-    fft_inplace<L, true, false, HOUT, E>(a, act, j, tab);
-  } else {
-    fft_passes_below<L, 1, last_ns<L, E>(), false, HIN, E>(a, act, j, tab);
-    fft_turn<L, E>(a, act, j, tab, mul);
-    fft_passes<L, E, true, false, HOUT, E>(a, act, j, tab);
-  }
 }
 
 // The first pass of a forward FFT (NS = 1, radix E) with its inputs read

@@ -27,11 +27,11 @@ from . import abi, build
 from .synthetic import FORCED_CYLINDER_RE100, SWIMMER_1024x512, noise_field
 
 # the order of TraceId in csrc/internal.cuh
-KERNELS = ["step_begin/max_u", "set_dt", "end_step", "advdiff", "rhs_div", "pcorr", "fade_sums",
-           "obj_begin", "disk_place", "raster_disk", "chi", "moments", "udef_grid",
+KERNELS = ["step_begin/max_u", "set_dt", "end_step", "advdiff", "rhs_div", "pcorr",
+           "obj_begin", "raster_disk", "chi", "udef_grid",
            "rhs_obst", "rhs_corr", "momenta", "collide", "penalize", "forces", "fish_midline",
            "fish_frame", "fish_raster", "rows_r2c", "cols", "rows_c2r", "dct_rows_fwd", "dct_cols",
-           "dct_rows_inv", "fish_tile_search", "max_next"]
+           "dct_rows_inv", "fish_tile_search"]
 TRACE_ITEMS = 4096
 WORKLOADS = {"swimmer": SWIMMER_1024x512, "cylinder": FORCED_CYLINDER_RE100}
 
