@@ -71,14 +71,20 @@ constexpr int E_ROWS32 = 8;
 constexpr int E_C2R32 = 8;
 constexpr int E_COLS32 = 16;
 // Columns per CTA of the column pass (of one group, so that a CTA reads runs
-// of 16 or 32 bytes) and a budget of 64 registers a thread, 32 warps an SM:
-// the pass waits for its exchanges, and more warps hide them.  4096 x 2048, in
-// us, with 1, 2 and 4 columns: 130 (80 registers), 115, 112; one column and 128
-// registers 137.  2048-point columns: 1, 2, 4 columns 40, 32, 35.
+// of 16 or 32 bytes): 4096 x 2048, in us, with 1, 2 and 4 columns 130 (80
+// registers), 115, 112; 2048-point columns with 1, 2, 4 columns 40, 32, 35.
+// Registers a thread: from 2048 points on 64, so that 32 warps an SM hide the
+// exchanges that the pass waits for: 2048 x 2048 periodic 26.6 us (28.8 with 128),
+// 4096 x 2048 periodic 41.5 (43.5), free space 112 (112, and 137 with 128 and one
+// column).  Shorter passes do not fill the chip with warps either way, and the
+// 64 registers spill: 64 points (64 x 32) 8.3 us with 64 registers and 8.05 with
+// 128; 128 points 8.55, 8.55; 256 8.4, 8.4 and 12.8, 12.7; 512 10.4, 10.4 and 12.5,
+// 12.5; 1024 14.0, 14.0 and 14.2, 14.3.
 template <int L> struct Col32 {
   static constexpr int CB = L >= 4096 ? 4 : (L >= 1024 ? 2 : Len<L>::B);
   static constexpr int NT0 = CB * L / E_COLS32, NT = NT0 < 64 ? 64 : NT0;
-  static constexpr int MINB = 65536 / (NT * 64);
+  static constexpr int REGS = L >= 2048 ? 64 : 128;
+  static constexpr int MINB = 65536 / (NT * REGS);
 };
 
 // Stages the per-pass tables of fft_inplace<L, ..., E>, laid out once for all
