@@ -251,11 +251,14 @@ k_vr_penalize(GridDesc g, const Scalars* sc, const DevShape* sh, int k, ObstTile
 }
 
 // Rows per thread of the two full-grid kernels of an iteration: CTAs of 32 x 8
-// threads with four rows each, or, where the grid's blocks leave SMs idle, 32
-// x 32 threads with one (256 x 128, 32 blocks: the right-hand side 11 -> 7 us, the
-// correction 12 -> 8 us, serialised).  The sums keep the order of the
-// four-row form: thread (tx, ty < 8) adds rows ty, ty + 8, ty + 16, ty + 24.
-constexpr int VR_ROWS_BELOW = 296;
+// threads with four rows each, or, on grids of fewer blocks than two an SM, which
+// leave warps idle, 32 x 32 threads with one (256 x 128, 32 blocks: the right-hand
+// side 11 -> 7 us, the correction 12 -> 8 us, serialised).  A step of the falling
+// disk (59 to 102 iterations) with four rows and with one, in us: 32 blocks 3005,
+// 2786; 96 5101, 4683; 192 5466, 5356; 288 6215, 6107; 384 6441, 6636; 640 8594, 8955.
+// The sums keep the order of the four-row form: thread (tx, ty < 8) adds rows
+// ty, ty + 8, ty + 16, ty + 24.
+inline bool one_row_a_thread(const Ctx& c) { return c.g.nblocks < 2 * c.sms; }
 
 // updatePressureRHS (PressureIterator_approx.cpp:289-335):
 // RHS = (1 - rho0 invRho) lap(P) - rho0 (dP/dx dinvRho/dx + dP/dy dinvRho/dy)
@@ -427,7 +430,7 @@ void launch_vr_penalize(Ctx& c) {
 }
 
 void launch_vr_rhs(Ctx& c) {
-  const bool one = c.g.nblocks < VR_ROWS_BELOW;
+  const bool one = one_row_a_thread(c);
   launch_k(one ? k_vr_rhs<1> : k_vr_rhs<4>, dim3(c.g.bpdx, c.g.bpdy), dim3(32, one ? 32 : 8), 0, c.stream, c.g,
            (const Scalars*)c.dsc, c.rho0, (const double*)c.pres, (const double*)c.invRho, (const double*)c.itmp[0],
            (const double*)c.itmp[1], (const double*)c.prhs, c.rhs, (const int*)c.fadeSlot, fade_partials(c));
@@ -435,7 +438,7 @@ void launch_vr_rhs(Ctx& c) {
 }
 
 void launch_vr_pcorr(Ctx& c, bool final_, unsigned long long seqVal) {
-  const bool one = c.g.nblocks < VR_ROWS_BELOW;
+  const bool one = one_row_a_thread(c);
   const auto k = final_ ? (one ? k_vr_pcorr<true, 1> : k_vr_pcorr<true, 4>)
                         : (one ? k_vr_pcorr<false, 1> : k_vr_pcorr<false, 4>);
   launch_k(k, dim3(c.g.bpdx, c.g.bpdy), dim3(32, one ? 32 : 8), 0, c.stream, c.g, c.dsc, 1 / c.rho0,
