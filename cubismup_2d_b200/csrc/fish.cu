@@ -1141,9 +1141,10 @@ void launch_fish_place(Ctx& c, int k) {
 }
 
 void launch_fish_raster(Ctx& c, int k) {
-  // two resident CTAs per SM at most (registers); each loops over
-  // (tile, sub-tile) items
-  const int items = c.tiles[k].capacity * NSUB, grid = items < 2 * c.sms ? items : 2 * c.sms;
+  // one resident CTA per SM (512 threads of 128 registers); each loops over
+  // (tile, sub-tile) items.  Two per SM, as for 256 threads, had launched a second
+  // wave that mostly exited: ensemble of 16 4084 us, 4069 without.
+  const int items = c.tiles[k].capacity * NSUB, grid = items < c.sms ? items : c.sms;
   launch_k(k_fish_raster, grid, RT, raster_smem(c.fish[k].nm), c.stream, c.g, c.dshapes, k, c.tiles[k],
                                                                 c.fish[k], c.sdf);
   CUP2D_LAUNCHED(c);
