@@ -201,10 +201,14 @@ int cup2d_compute_forces(cup2d_ctx* ctx, double dt);   /* ComputeForces.cpp:16-1
 int cup2d_poisson_solve(cup2d_ctx* ctx, int src, int dst);
 /* With cup2d_config.iterative, cup2d_pressure_single runs the iterated
  * penalization and projection of PressureIterator_unif::operator()
- * (PressureIterator_unif.cpp:214-270): it waits for each iteration's
- * residual on the host, as the reference decides convergence there, and
- * cup2d_advance / the ensemble return CUP2D_ENOTSUP.  The iteration count
- * and the last relative momentum change of the latest call: */
+ * (PressureIterator_unif.cpp:214-270), or, with a body of rhoS != 1, the
+ * variable-density one (PressureIterator_approx.cpp:378-468): it waits for
+ * each iteration's residual on the host, as the reference decides
+ * convergence there, and cup2d_advance / the ensemble return
+ * CUP2D_ENOTSUP.  Each wait spins on a word that the iteration's kernels
+ * write to mapped host memory (one host thread busy for up to 20 ms), and
+ * only then blocks on the stream's event.  The iteration count and the last
+ * relative momentum change of the latest call: */
 int cup2d_iteration_stats(cup2d_ctx* ctx, int* iterations, double* rel_df);
 /* time += dt; step++ (Simulation.cpp:289-290). */
 int cup2d_end_step(cup2d_ctx* ctx);
