@@ -262,16 +262,18 @@ void launch_pressure_tail(Ctx& c, bool maxNext, bool joinMid = false) {
 // One pass of Simulation::simulate's loop body (Simulation.cpp:245-251) as a
 // graph with three branches:
 //   main : dt + reset of last step's tiles + body motion -> fish frames and
-//          tile search, rasters, Towers chi with the moments -> [join side2] -> RHS
-//          obstacle terms, Poisson -> momentum integrals [beside the
-//          pressure correction on side2] -> collisions, penalization, forces
-//          -> [join side, side2] -> t += dt and the next step's dt
+//          tile search, rasters, Towers chi -> [join side2] -> RHS obstacle
+//          terms (with the moments' totals), Poisson -> momentum integrals
+//          [beside the pressure correction on side2] -> [join side2, side] ->
+//          collisions, penalization, forces; the last thread of the forces
+//          ends the step: t += dt and the next step's dt
 //   side : the fish midlines of the next step (they depend on time only):
 //          from the graph's start when the step's dt was carried, else
 //          once step_begin has set it
-//   side2: once the tiles are placed, advDiff's outflow flux, then advDiff
-//          with the RHS divergence in place (advDiff reads no obstacle data);
-//          later the pressure correction (with the next step's findMaxU
+//   side2: advDiff's outflow flux, then advDiff with the RHS divergence in
+//          place (it reads no obstacle data): from the step's start with disks
+//          only or on grids of ADV_FIRST_BLOCKS, else once a fish's tiles are
+//          placed; later the pressure correction (with the next step's findMaxU
 //          over the blocks without obstacle tiles; the tiles' part follows
 //          the penalization on main)
 void enqueue_step(Ctx& c) {

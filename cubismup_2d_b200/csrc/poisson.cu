@@ -47,6 +47,7 @@ struct Poisson {
   // spectrum); cosine: its multiplier [Nx][Ny]; a column's values are consecutive
   double* ghat = nullptr;
   double2* tw = nullptr;     // exp(-2 pi i k / twLen)
+  double2* dct = nullptr;    // cosine: DctCoef's four tables of its rows
   int twLen = 0;
   double2* tRow[2] = {nullptr, nullptr};   // pass tables of the row transforms, 8 and 16 values per thread
   double2* tCol = nullptr;                 // and of the column transforms
@@ -75,7 +76,8 @@ namespace {
 // table holding (c, t) = (cos, tan) of an angle, w b = c (b.x - t b.y, b.y +
 // t b.x) and a butterfly is six multiply-adds (the "ratio" butterfly of
 // Linzer and Feig, 1993); c t is the sine to rounding at every angle, so no
-// branch on it is needed (c is never zero: cos(pi/2) rounds to 6e-17).  A
+// branch on it is needed (c is never zero: formed in long double, the cosine
+// of the rounded pi/2 is some -3e-20, its tangent 4e19).  A
 // radix-16 pass takes 192 FP64 instructions a thread instead of about 280
 // (15 scalings, 11 products for the powers of W that the table did not hold,
 // 9 internal twiddles and 144 additions).
@@ -516,7 +518,7 @@ k_rows_r2c(const double* in, int inStride, int nrows, int ncolsIn, double2* __re
 // multiply-add butterflies, the grouped spectrum, the multiplier stored by
 // columns, and the first and last passes straight from and to global memory).
 // Bound by the L1: 23 M shared-memory wavefronts (four exchanges of 64 KB a
-// column) and 10 M of global accesses, 73% of its cycles; FP64 pipe 36%,
+// column) and 10 M of global accesses, 68% of its cycles; FP64 pipe 36%,
 // DRAM 30%.  CONV: forward, times the real multiplier g (symmetric in ky),
 // inverse, keep nrowsOut rows; else (set-up of the free-space kernel) forward
 // alone, Re * norm of the first L/2 + 1 values to gOut.  Rows r >= nrowsIn of
@@ -668,12 +670,63 @@ k_rows_c2r(const double2* __restrict__ in, int inRows, int nrows, double* __rest
 // A real row of n = 2L values is a complex FFT of length L as in k_rows_r2c;
 // two real columns are one complex FFT of length Ny.  The spectrum lies as
 // the other solvers' (spec_at, entry (r, p) = columns 2p and 2p + 1).
+// The error of a solve (2-norm, long double, means of 8 to 200 solves, before
+// and now): of vorticity-like right-hand sides 3.0-4.1e-16 and 2.6-3.3e-16 on eight
+// grids, 4.1 and 4.4 (within their scatter) on 256 x 2048; of a step's 3.2-3.7e-16
+// and 3.1-3.6e-16, of its gradient 4 to 6% lower; of white noise 3.3-4.2e-16 and
+// 3.0-4.4e-16, lower on six grids of nine, the others within the scatter.
 // B200, forward rows, columns, inverse rows (events around a launch, about 7 us of
-// them launch): 512 x 256 14.1, 12.3, 12.4 us (21.5, 17.9, 12.3 before);
-// 4096 x 2048 69, 87, 80 us (211, 188, 88 before).
+// them launch): 512 x 256 12.5, 12.5, 12.1 us (21.5, 17.9, 12.3 before);
+// 4096 x 2048 66, 86, 63 us (211, 188, 88 before; 68, 86, 78 with separate tables).
 
 // one real value of the spectrum
 __device__ __forceinline__ size_t dct_at(int rows, int r, int c) { return 2 * spec_at(rows, r, c >> 1) + (c & 1); }
+
+// A row's split and its w^k in one: with W = exp(-i pi / L), w^(L-k) and the
+// real-FFT split of r2c_split, 2 w^k V_k = conj(a) Z_k + b conj(Z_(L-k)) and
+// 2 w^(L-k) V_(L-k) = c conj(Z_k) + conj(d) Z_(L-k) with
+//   a = (1 + i W^-k) w^-k, b = (1 + i W^k) w^k, c = (1 - i W^-k) w^(L-k), d = (1 - i W^k) w^(k-L);
+// the inverse's merge is the transpose: z_k = a X + c conj(Y), z_(L-k) = b conj(X) + d Y of
+// X = Y_k - i Y_(n-k) and Y = Y_(L-k) - i Y_(L+k).  As tables of a, b, c, d, k < L/2, each is
+// rounded once, and a row's loads are four runs instead of three gathers.  The
+// rounding of a table is the same in every step, so its error adds up: with
+// separate tables of W and w the flow past a disk at 512 x 256 was 2.3e-15 off (2-norm,
+// long double) after 20 steps, 1.5e-15 with the even extension.  Two choices keep
+// it down.  b takes a's rounding (v's even entries see Re(a + b), its odd ones Im(a +
+// b), and neighbouring cells hold one of each), and the tables hold DCT_SCALE times
+// a..d (the multiplier its inverse square), so that the low modes' components lie
+// below 1, not on both sides.  Over ten grids of 128 x 128 to 1024 x 512, six flows each,
+// geometric means in 1e-15: even extension 1.23, separate tables 1.17, a..d rounded
+// apart 1.10, with one choice or the other 0.95 and 1.04, with both 0.95 and none of
+// the ten above the even extension's (512 x 256: 1.4).
+constexpr double DCT_SCALE = 0.9375;
+struct DctCoef { double2 a, b, c, d; };
+template <int L> __device__ __forceinline__ DctCoef dct_coef(const double2* __restrict__ t, int k) {
+  constexpr int H = L / 2;
+  return {t[k], t[H + k], t[2 * H + k], t[3 * H + k]};
+}
+// the tables on the host: W^-k = exp(4 i u), w^-k = exp(i u), u = pi k / 4L
+std::vector<double2> dct_coef_tables(int L) {
+  const int H = L / 2;
+  const long double pi = 3.14159265358979323846264338327950288L, q = pi / 4;
+  std::vector<double2> t(4 * H);
+  auto polar = [](long double r, long double phi) { return make_double2((double)(r * cosl(phi)), (double)(r * sinl(phi))); };
+  for (int k = 0; k < H; k++) {
+    const long double u = pi * k / (4 * L), p = 2 * DCT_SCALE * cosl(q + 2 * u), m = 2 * DCT_SCALE * cosl(q - 2 * u);
+    const double2 a = t[k] = polar(p, q + 3 * u);
+    // b takes a's rounding: v's even entries see Re(a + b), its odd ones Im(a + b)
+    t[H + k] = make_double2((double)(p * cosl(q + 3 * u) + m * cosl(q - 3 * u) - a.x),
+                            (double)(p * sinl(q + 3 * u) + m * sinl(q - 3 * u) - a.y));
+    t[2 * H + k] = polar(m, 3 * u - 2 * q);
+    t[3 * H + k] = polar(p, -3 * u);
+  }
+  return t;
+}
+// a x + b y
+__device__ __forceinline__ double2 cmul2(double2 a, double2 x, double2 b, double2 y) {
+  return make_double2(fma(a.x, x.x, fma(-a.y, x.y, fma(b.x, y.x, -(b.y * y.y)))),
+                      fma(a.x, x.y, fma(a.y, x.x, fma(b.x, y.y, b.y * y.x))));
+}
 
 // values per thread of the cosine solver's row passes
 template <int L> constexpr int dct_e() { return L >= 1024 ? 16 : 8; }
@@ -682,7 +735,7 @@ template <int L> constexpr int dct_e() { return L >= 1024 ? 16 : 8; }
 template <int L, int E, int RB>
 __global__ void __launch_bounds__(Row64<L, E, RB>::NT, Row64<L, E, RB>::MINB)
 k_dct_rows_fwd(const double* in, int nrows, double* __restrict__ D, const double2* __restrict__ tab,
-               const double2* __restrict__ tw, int twLen, FadeArgs fa)
+               const double2* __restrict__ tw, int twLen, const double2* __restrict__ coef, FadeArgs fa)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_FWD);
@@ -736,27 +789,25 @@ k_dct_rows_fwd(const double* in, int nrows, double* __restrict__ D, const double
   __syncthreads();
   const int sq = threadIdx.x / (L / E), j = threadIdx.x % (L / E);
   fft_inplace<L, false, false, false, E>(A + sq * SL, sq < nb, j, tb);
-  // the real-FFT split (r2c_split), then C_k and C_(n-k) of k and of L - k
+  // C_k and C_(n-k) of k and of L - k
   constexpr int KPT = (H + NT - 1) / NT;
-  const int st2 = twLen / (2 * L), st8 = twLen / (8 * L);
   auto put = [&](int r, int k, double2 z) {            // z = 2 w^k V_k
     D[dct_at(nrows, row0 + r, k)] = z.x;
     if (k != 0 && k != L) D[dct_at(nrows, row0 + r, n - k)] = -z.y;
   };
   if (threadIdx.x < nb) {
     const double2 z = A[threadIdx.x * SL + pad(H)];
-    put(threadIdx.x, H, cmul(tw[H * st8], make_double2(2 * z.x, -2 * z.y)));
+    put(threadIdx.x, H, cmul(tw[H * (twLen / (8 * L))], make_double2(2 * DCT_SCALE * z.x, -2 * DCT_SCALE * z.y)));
   }
 #pragma unroll
   for (int q = 0; q < KPT; q++) {
     const int k = threadIdx.x + q * NT;
     if (k >= H) break;                                  // k grows with q
-    const double2 w = tw[k * st2], wk = tw[k * st8], wl = tw[(L - k) * st8];
+    const DctCoef c = dct_coef<L>(coef, k);
     for (int r = 0; r < nb; r++) {
-      const double2 Za = A[r * SL + pad(k)], Zb = conjg(A[r * SL + pad(k == 0 ? 0 : L - k)]);
-      const double2 Fe = cadd(Za, Zb), d = csub(Za, Zb), t = cmul(w, make_double2(d.y, -d.x));
-      put(r, k, cmul(wk, cadd(Fe, t)));
-      put(r, L - k, cmul(wl, conjg(csub(Fe, t))));
+      const double2 Zk = A[r * SL + pad(k)], Zl = A[r * SL + pad(k == 0 ? 0 : L - k)];
+      put(r, k, cmul2(conjg(c.a), Zk, c.b, conjg(Zl)));
+      put(r, L - k, cmul2(c.c, conjg(Zk), conjg(c.d), Zl));
     }
   }
 }
@@ -823,7 +874,8 @@ k_dct_cols(double2* D, int npairs, const double* __restrict__ M, const double2* 
 __global__ void k_dct_multiplier(double* __restrict__ M, int Nx, int Ny, const float* __restrict__ cosX,
                                  const float* __restrict__ cosY, double tol) {
   const double MX = Nx, MY = Ny;
-  const double waveFactX = M_PI / MX, waveFactY = M_PI / MY, norm_factor = 0.25 / (MX * MY);
+  const double waveFactX = M_PI / MX, waveFactY = M_PI / MY;
+  const double norm_factor = 0.25 / (DCT_SCALE * DCT_SCALE) / (MX * MY);
   for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < (size_t)Nx * Ny;
        idx += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(idx / Ny), jj = (int)(idx % Ny);
@@ -839,7 +891,7 @@ __global__ void k_dct_multiplier(double* __restrict__ M, int Nx, int Ny, const f
 template <int L, int E, int RB>
 __global__ void __launch_bounds__(Row64<L, E, RB>::NT, Row64<L, E, RB>::MINB)
 k_dct_rows_inv(const double* __restrict__ D, int nrows, double* __restrict__ out, const double2* __restrict__ tab,
-               const double2* __restrict__ tw, int twLen)
+               const double2* __restrict__ tw, int twLen, const double2* __restrict__ coef)
 {
   pdl_begin();
   CUP2D_TRACE_SCOPE(TR_DCT_INV);
@@ -851,28 +903,25 @@ k_dct_rows_inv(const double* __restrict__ D, int nrows, double* __restrict__ out
   cp_async_commit();
   const int row0 = blockIdx.x * RB;
   const int nb = min(RB, nrows - row0);
-  const int st2 = twLen / (2 * L), st8 = twLen / (8 * L);
   auto get = [&](int r, int k) { return D[dct_at(nrows, row0 + r, k)]; };
-  // X_k = conj(w^k) (Y_k - i Y_(n-k)), then the merge of k_rows_c2r
 #pragma unroll
   for (int q = 0; q < KPT; q++) {
     const int k = threadIdx.x + q * NT;
     if (k >= H) break;
-    const double2 w = conjg(tw[k * st2]), wk = conjg(tw[k * st8]), wl = conjg(tw[(L - k) * st8]);
+    const DctCoef c = dct_coef<L>(coef, k);
 #pragma unroll
     for (int r = 0; r < RB; r++) {
       if (r >= nb) break;
-      const double2 Xk = cmul(wk, make_double2(get(r, k), k == 0 ? 0.0 : -get(r, n - k)));
-      const double2 Xc = conjg(cmul(wl, make_double2(get(r, L - k), -get(r, L + k))));
-      const double2 s = cadd(Xk, Xc), t = cmul(w, csub(Xk, Xc));
+      const double2 X = make_double2(get(r, k), k == 0 ? 0.0 : -get(r, n - k));
+      const double2 Y = make_double2(get(r, L - k), -get(r, L + k));
       double2* a = A + r * SL;
-      a[pad(k)] = make_double2(s.x - t.y, s.y + t.x);
-      if (k > 0) a[pad(L - k)] = make_double2(s.x + t.y, t.x - s.y);
+      a[pad(k)] = cmul2(c.a, X, c.c, conjg(Y));
+      if (k > 0) a[pad(L - k)] = cmul2(c.b, conjg(X), c.d, Y);
     }
   }
   if (threadIdx.x < nb) {
-    const double2 x = cmul(conjg(tw[H * st8]), make_double2(get(threadIdx.x, H), -get(threadIdx.x, n - H)));
-    A[threadIdx.x * SL + pad(H)] = make_double2(2 * x.x, -2 * x.y);
+    const double2 x = cmul(conjg(tw[H * (twLen / (8 * L))]), make_double2(get(threadIdx.x, H), -get(threadIdx.x, n - H)));
+    A[threadIdx.x * SL + pad(H)] = make_double2(2 * DCT_SCALE * x.x, -2 * DCT_SCALE * x.y);
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -1045,7 +1094,7 @@ bool dct_rows_fwd(const Poisson& P, cudaStream_t st, const double* in, int ny, c
 #define X(LL) case LL: with_rows<LL>(ny, [&](auto b) { \
     constexpr int E = dct_e<LL>(), B = decltype(b)::value; \
     launch_k(k_dct_rows_fwd<LL, E, B>, (ny + B - 1) / B, Row64<LL, E, B>::NT, smem_row64<LL, E, B>(), st, in, ny, \
-             reinterpret_cast<double*>(P.spec), P.tRow[E == 16], P.tw, P.twLen, fa); }); \
+             reinterpret_cast<double*>(P.spec), P.tRow[E == 16], P.tw, P.twLen, P.dct, fa); }); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -1069,7 +1118,7 @@ bool dct_rows_inv(const Poisson& P, cudaStream_t st, int ny, double* out) {
 #define X(LL) case LL: with_rows<LL>(ny, [&](auto b) { \
     constexpr int B = decltype(b)::value; \
     launch_k(k_dct_rows_inv<LL, 16, B>, (ny + B - 1) / B, Row64<LL, 16, B>::NT, smem_row64<LL, 16, B>(), st, \
-             reinterpret_cast<const double*>(P.spec), ny, out, P.tRow[1], P.tw, P.twLen); }); \
+             reinterpret_cast<const double*>(P.spec), ny, out, P.tRow[1], P.tw, P.twLen, P.dct); }); \
     return true;
     CUP2D_FFT_LENGTHS(X)
 #undef X
@@ -1167,6 +1216,9 @@ Poisson* poisson_create(Ctx& c) {
         device_malloc(&P->cosY, sizeof(float) * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
     h2d_sync(P->cosX, cx.data(), sizeof(float) * Nx, c.stream);
     h2d_sync(P->cosY, cy.data(), sizeof(float) * Ny, c.stream);
+    const std::vector<double2> coef = dct_coef_tables(P->Lrow);
+    if (device_malloc(&P->dct, sizeof(double2) * coef.size()) != cudaSuccess) { poisson_destroy(P); return nullptr; }
+    h2d_sync(P->dct, coef.data(), sizeof(double2) * coef.size(), c.stream);
     if (device_malloc(&P->ghat, sizeof(double) * Nx * Ny) != cudaSuccess) { poisson_destroy(P); return nullptr; }
     k_dct_multiplier<<<4 * c.sms, 256, 0, c.stream>>>(P->ghat, Nx, Ny, P->cosX, P->cosY, P->tol);
     CUP2D_LAUNCHED(c);
@@ -1211,7 +1263,7 @@ Poisson* poisson_create(Ctx& c) {
 void poisson_destroy(Poisson* P) {
   if (!P) return;
   cudaFree(P->spec); cudaFree(P->ghat); cudaFree(P->tw); cudaFree(P->cosX); cudaFree(P->cosY);
-  cudaFree(P->tw32); cudaFree(P->ghat32);
+  cudaFree(P->tw32); cudaFree(P->ghat32); cudaFree(P->dct);
   cudaFree(P->tRow32); cudaFree(P->tCol32);
   cudaFree(P->tRow[0]); cudaFree(P->tRow[1]); cudaFree(P->tCol);
   delete P;
