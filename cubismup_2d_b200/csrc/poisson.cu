@@ -689,16 +689,17 @@ __device__ __forceinline__ size_t dct_at(int rows, int r, int c) { return 2 * sp
 // the inverse's merge is the transpose: z_k = a X + c conj(Y), z_(L-k) = b conj(X) + d Y of
 // X = Y_k - i Y_(n-k) and Y = Y_(L-k) - i Y_(L+k).  As tables of a, b, c, d, k < L/2, each is
 // rounded once, and a row's loads are four runs instead of three gathers.  The
-// rounding of a table is the same in every step, so its error adds up: with
-// separate tables of W and w the flow past a disk at 512 x 256 was 2.3e-15 off (2-norm,
-// long double) after 20 steps, 1.5e-15 with the even extension.  Two choices keep
-// it down.  b takes a's rounding (v's even entries see Re(a + b), its odd ones Im(a +
-// b), and neighbouring cells hold one of each), and the tables hold DCT_SCALE times
-// a..d (the multiplier its inverse square), so that the low modes' components lie
-// below 1, not on both sides.  Over ten grids of 128 x 128 to 1024 x 512, six flows each,
-// geometric means in 1e-15: even extension 1.23, separate tables 1.17, a..d rounded
-// apart 1.10, with one choice or the other 0.95 and 1.04, with both 0.95 and none of
-// the ten above the even extension's (512 x 256: 1.4).
+// rounding of a table is the same in every step, so its error adds up: most of a
+// flow's is its mean velocity, which follows the pressure's difference between the
+// edge columns x_0 and x_(n-1), that is the low modes' relative error there (both are
+// even entries of v: Re(a + b)).  Two choices keep it down: b takes a's rounding, and
+// the tables hold DCT_SCALE times a..d (the multiplier its inverse square), so that
+// the low modes' components lie below 1, not on both sides.  Flows past a disk, in
+// 1e-15 (2-norm, long double), with the even extension, with separate tables of W
+// and w, and now: 512 x 256, 20 steps, 32 flows 1.40, 2.25, 1.50; geometric mean of
+// ten grids of 128 x 128 to 1024 x 512, six flows each, 1.23, 1.17, 0.95 (a..d rounded
+// apart 1.10, with b's choice alone 0.95, with the scale alone 1.04); of five of
+// them, twelve flows each, 1.72, 1.89, 1.31 (1.71, 1.39, 1.41).
 constexpr double DCT_SCALE = 0.9375;
 struct DctCoef { double2 a, b, c, d; };
 template <int L> __device__ __forceinline__ DctCoef dct_coef(const double2* __restrict__ t, int k) {
