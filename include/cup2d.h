@@ -352,11 +352,13 @@ int cup2d_checkpoint_load(cup2d_ctx* ctx, const void* buf, size_t bytes);
  *    way (forced in all three, no PID: its chi and udef move with its gait
  *    alone, each step's kept by the recomputation); anything else
  *    CUP2D_ENOTSUP;
- *  - device scratch: (nsteps/every + 2) checkpoints and 4 min(every, nsteps)
- *    + 8 planes (for a gradient); up to 256 MB of it, over all contexts of
- *    the process, stay allocated for the next runs.  cup2d_destroy gives a
- *    context's back, and so does any allocation of this library that finds
- *    the device full;
+ *  - device scratch, allocated before the run: (nsteps/every + 2)
+ *    checkpoints; for a gradient, 4 min(every, nsteps) + 8 planes; a
+ *    swimmer's also min(every, nsteps) times its obstacle tiles; with
+ *    grad_gait 3 min(every, nsteps) + 5 nsteps more planes.  Up to 256 MB of
+ *    it, over all contexts of the process, stay allocated for the next
+ *    runs.  cup2d_destroy gives a context's back, and so does any allocation
+ *    of this library that finds the device full;
  *  - the context ends in the forward's final state (as after nsteps
  *    steps), its gait as it was; synchronises.  After an error its state is
  *    unspecified: load a checkpoint taken before the call. */
